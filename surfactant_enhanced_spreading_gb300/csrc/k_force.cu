@@ -22,7 +22,7 @@ void upload_tables_force(const Tables &t, cudaStream_t st) {
 }
 
 constexpr int NEAR_THREADS = 128;
-constexpr int SORT_CAP = 2048;
+constexpr int SORT_CAP = 2048, SORT_SHIFT = 29;   // site indices stay below 2^29
 
 __device__ inline void cell_xyz(const Rep &r, int c, int &ix, int &iy, int &iz) {
     int l = c - r.cell0;
@@ -60,15 +60,23 @@ __device__ inline int block_exscan(int v, int *total) {
     return res;
 }
 
+// groups of four that hold n sites in up to five padded runs
+__host__ __device__ inline int pair_groups(int n) { return n > 0 ? (n + 15) >> 2 : 0; }
+
+// first slot of every cell, and the first group of its pair layout
 __global__ void k_scan(Dev d, int ncell) {
     int per = (ncell + blockDim.x - 1) / blockDim.x;
     int b = threadIdx.x * per, e = min(ncell, b + per);
-    int s = 0;
-    for (int c = b; c < e; c++) s += d.ccount[c];
-    int total;
-    int acc = block_exscan(s, &total);
+    int s = 0, q = 0;
+    for (int c = b; c < e; c++) { const int n = d.ccount[c]; s += n; q += pair_groups(n); }
+    int total, qtotal;
+    int acc = block_exscan(s, &total), qacc = block_exscan(q, &qtotal);
     if (threadIdx.x == 0) d.cstart[ncell] = total;
-    for (int c = b; c < e; c++) { d.cstart[c] = acc; acc += d.ccount[c]; d.cfill[c] = 0; }
+    for (int c = b; c < e; c++) {
+        const int n = d.ccount[c];
+        d.cstart[c] = acc; acc += n; d.cfill[c] = 0;
+        d.crun[8 * (size_t)c] = qacc; qacc += pair_groups(n);
+    }
 }
 
 __global__ void k_scatter(Dev d, int nsite) {
@@ -108,51 +116,89 @@ __device__ int molecule_cells(const Dev &d, int c, int v) {
     return mask;
 }
 
-// order the sites of each cell by site index, so the slot order (and with it
-// every floating-point sum) is independent of the scatter's atomics
-// (order within a cell: sites with LJ first - every kind but water H - then
-// water H, each group by site index; cnh[c] counts the first group, so the
-// FP32 pair loop runs its LJ test on a prefix of every partner cell only)
-constexpr int SORT_HBIT = 1 << 30;   // site indices stay below 2^30
+// order the sites of each cell by class and site index, so the slot order (and
+// with it every floating-point sum) is independent of the scatter's atomics.
+// Classes: water O, other LJ sites, water H (cno and cnh count the first and
+// the first two), so the pair loops run over sites of one charge and test for
+// LJ on a prefix only; waters whose molecule lies in this cell alone come
+// before the others in theirs, so that a neighbour cell's same-molecule test
+// is needed in a run's second part only (a fifth of its sites).  The FP32
+// paths' pair layout holds the same order with every run padded to fours.
 __global__ void k_sort_cells(Dev d) {
-    __shared__ int buf[SORT_CAP];
-    __shared__ int nonh;
+    __shared__ unsigned buf[SORT_CAP];
+    __shared__ int xm[SORT_CAP];
+    __shared__ int cnt[5];
     int c = blockIdx.x;
     int s0 = d.cstart[c], n = d.cstart[c + 1] - s0;
-    if (threadIdx.x == 0) nonh = 0;
-    if (threadIdx.x == 0 && n > 0) atomicMax(&d.counters[3], (unsigned long long)n);
+    int *run = d.crun + 8 * (size_t)c;
+    if (n == 0) {
+        if (threadIdx.x < 5) run[1 + threadIdx.x] = 0;
+        if (threadIdx.x == 0) d.cnh[c] = d.cno[c] = 0;
+        return;
+    }
+    if (threadIdx.x < 5) cnt[threadIdx.x] = 0;
+    if (threadIdx.x == 0) atomicMax(&d.counters[3], (unsigned long long)n);
     __syncthreads();
+    float *xyz = (float *)(d.pair_xyz + 3 * (size_t)run[0]);
+    int *keys = (int *)(d.pair_key + run[0]);
+    auto place = [&](int slot, int v, int mask, int pair) {
+        const int key = d.smol[v] << 5 | (int)d.ptype[v];
+        d.srt_site[s0 + slot] = v;
+        d.sslot[v] = s0 + slot;
+        d.srt_meta[s0 + slot] = make_int2(d.smol[v], (int)d.ptype[v]);
+        d.srt_key[s0 + slot] = key;
+        d.srt_xmask[s0 + slot] = mask;
+        d.srt_pair[s0 + slot] = 4 * run[0] + pair;
+        keys[pair] = key;
+    };
+    auto pad = [&](int pair) {   // no molecule, kind 0, far away
+        float *o = xyz + 12 * (pair >> 2) + (pair & 3);
+        o[0] = o[4] = o[8] = 1e18f;
+        keys[pair] = -32;
+    };
     if (n > SORT_CAP) {
         // counted as an overflow; the cell keeps the scatter's order (its sums
-        // then depend on timing), with every per-slot field still written
+        // then depend on timing), with every per-slot field still written; the
+        // pair loops take every slot's own charge and kind
         if (threadIdx.x == 0) atomicAdd(&d.counters[1], 1ull);
-        for (int t = threadIdx.x; t < n; t += blockDim.x) {
-            const int v = d.srt_site[s0 + t];
-            d.sslot[v] = s0 + t;
-            d.srt_meta[s0 + t] = make_int2(d.smol[v], (int)d.ptype[v]);
-            d.srt_key[s0 + t] = d.smol[v] << 5 | (int)d.ptype[v];
-            d.srt_xmask[s0 + t] = molecule_cells(d, c, v);
+        for (int t = threadIdx.x; t < n; t += blockDim.x) place(t, d.srt_site[s0 + t], molecule_cells(d, c, d.srt_site[s0 + t]), t);
+        if (threadIdx.x < (-n & 3)) pad(n + threadIdx.x);
+        if (threadIdx.x == 0) {
+            d.cnh[c] = n; d.cno[c] = 0;
+            run[1] = run[2] = 0;
+            run[3] = run[4] = run[5] = (n + 3) >> 2;
         }
-        if (threadIdx.x == 0) d.cnh[c] = n;   // the pair loop then tests every slot for LJ
         return;
     }
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int v = d.srt_site[s0 + t];
-        const bool h = d.ptype[v] == 1;
-        buf[t] = v | (h ? SORT_HBIT : 0);
-        if (!h) atomicAdd(&nonh, 1);
+        const int v = d.srt_site[s0 + t], ty = d.ptype[v], mask = molecule_cells(d, c, v);
+        const int whole = mask == 1 << 13;   // bit of the cell itself
+        const int cls = ty == 0 ? 1 - whole : ty == 1 ? 4 - whole : 2;
+        buf[t] = (unsigned)cls << SORT_SHIFT | (unsigned)v;
+        xm[t] = mask;
+        atomicAdd(&cnt[cls], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) d.cnh[c] = nonh;
+    int first[6], quad[6];   // slots and groups before each class
+    first[0] = quad[0] = 0;
+#pragma unroll
+    for (int k = 0; k < 5; k++) { first[k + 1] = first[k] + cnt[k]; quad[k + 1] = quad[k] + ((cnt[k] + 3) >> 2); }
+    if (threadIdx.x == 0) { d.cnh[c] = first[3]; d.cno[c] = first[2]; }
+#pragma unroll
+    for (int k = 0; k < 5; k++) {
+        if (threadIdx.x == 0) run[1 + k] = quad[k + 1];
+        if (threadIdx.x < (-cnt[k] & 3)) pad(4 * quad[k] + cnt[k] + threadIdx.x);
+    }
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
-        const int k = buf[t], v = k & (SORT_HBIT - 1);
+        const unsigned k = buf[t];
         int rank = 0;
         for (int u = 0; u < n; u++) rank += buf[u] < k;
-        d.srt_site[s0 + rank] = v;
-        d.sslot[v] = s0 + rank;
-        d.srt_meta[s0 + rank] = make_int2(d.smol[v], (int)d.ptype[v]);
-        d.srt_key[s0 + rank] = d.smol[v] << 5 | (int)d.ptype[v];
-        d.srt_xmask[s0 + rank] = molecule_cells(d, c, v);
+        const int cls = k >> SORT_SHIFT;
+        int f = 0, q = 0;
+#pragma unroll
+        for (int a = 1; a < 5; a++)
+            if (cls == a) { f = first[a]; q = quad[a]; }
+        place(rank, (int)(k & ((1u << SORT_SHIFT) - 1)), xm[t], 4 * q + rank - f);
     }
 }
 
@@ -193,8 +239,12 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mixed) {
         const Rep r = rr;
         int ix, iy, iz;
         cell_xyz(r, c, ix, iy, iz);
-        d.srt_pos32[s] = make_float4((float)(x - cell_centre(d, r, 0, ix)), (float)(y - cell_centre(d, r, 1, iy)),
+        const float4 p = make_float4((float)(x - cell_centre(d, r, 0, ix)), (float)(y - cell_centre(d, r, 1, iy)),
                                      (float)(z - cell_centre(d, r, 2, iz)), (float)q);
+        d.srt_pos32[s] = p;
+        const int k = d.srt_pair[s];
+        float *o = (float *)d.pair_xyz + 12 * (size_t)(k >> 2) + (k & 3);
+        o[0] = -p.x; o[4] = -p.y; o[8] = -p.z;
     }
 }
 
@@ -309,8 +359,22 @@ __device__ inline double rsqrt_fp64(double r2) {
 // chunk of `tile` target sites).  A partner row is the (up to) 3 cells at
 // (dy, dz) from the target cell along x, contiguous in slot order; the 9 rows
 // (3 planes x 3 rows) of a cell cover its 27-cell shell.  tile is 64 (two
-// target sites per lane of a warp) or 32 (one); the autotuner picks it.
-// item.x = cell, item.y = (plane * 3 + row) << 8 | chunk.
+// target sites per lane of a warp), 32 (one) or 128 (64 twice); the autotuner
+// picks it.  near_split: one per partner cell instead of row.
+// Chunks do not mix LJ-carrying targets (the first nh of a cell) and water H:
+// the two take different loops, and a target's loop must not depend on the tile.
+// item.x = cell, item.y = part << 24 | chunk, part = plane * 3 + row, or
+// 3 (plane * 3 + row) + cell with near_split.
+
+__host__ __device__ inline int near_chunks(int nh, int ni, int tile) {
+    return (nh + tile - 1) / tile + (ni - nh + tile - 1) / tile;
+}
+// first and past-the-end target of a chunk
+__device__ inline void near_chunk(int nh, int ni, int tile, int ch, int &b, int &e) {
+    const int k = (nh + tile - 1) / tile;
+    b = ch < k ? ch * tile : nh + (ch - k) * tile;
+    e = min(b + tile, ch < k ? nh : ni);
+}
 
 // rows of the 27-cell shell inside the box (periodic preset: every row in y)
 __device__ inline int near_row_mask(const Rep &r, int iy, int iz) {
@@ -350,7 +414,9 @@ __global__ void k_near_items_count(Dev d, int ncell, int tile) {
         const Rep r = d.rep[d.crep[c]];
         int ix, iy, iz;
         cell_xyz(r, c, ix, iy, iz);
-        n = __popc(near_row_mask(r, iy, iz)) * ((ni + tile - 1) / tile);
+        int jx0, jx1;
+        row_x(r, ix, jx0, jx1);
+        n = __popc(near_row_mask(r, iy, iz)) * near_chunks(d.cnh[c], ni, tile) * (d.near_split ? jx1 - jx0 + 1 : 1);
     }
     d.near_icount[c] = n;
 }
@@ -373,29 +439,29 @@ __device__ inline void near_items_fill_cell(const Dev &d, int c, int ni, int til
     int ix, iy, iz;
     cell_xyz(r, c, ix, iy, iz);
     const int mask = near_row_mask(r, iy, iz);
-    const int nch = (ni + tile - 1) / tile;
+    const int nh = d.cnh[c], nch = near_chunks(nh, ni, tile);
     int jx0, jx1;
     row_x(r, ix, jx0, jx1);
     int k = d.near_icount[c];
+    const int step = d.near_split ? 1 : jx1 - jx0 + 1;   // cells of an item
     for (int pr = 0; pr < 9; pr++) {
         if (!(mask >> pr & 1)) continue;
-        int npart = 0;
-        if (r.per) {
-            for (int jx = jx0; jx <= jx1; jx++) {
+        for (int x0 = jx0; x0 <= jx1; x0 += step) {
+            int npart = 0;
+            for (int jx = x0; jx < x0 + step; jx++) {
                 const int cn = shell_cell(r, jx, iy + pr % 3 - 1, iz + pr / 3 - 1);
                 npart += d.cstart[cn + 1] - d.cstart[cn];
             }
-        } else {
-            const int c0 = cell_index(r, jx0, iy + pr % 3 - 1, iz + pr / 3 - 1);
-            npart = d.cstart[c0 + (jx1 - jx0) + 1] - d.cstart[c0];
-        }
-        for (int ch = 0; ch < nch; ch++) {
-            const int nt = min(tile, ni - ch * tile);
-            const int cls = 31 - __clz(nt * npart + 1);
-            d.near_items_tmp[k] = make_int2(c, pr << 24 | ch);
-            d.near_cls[k] = cls;
-            atomicAdd(&hist[cls], 1);
-            k++;
+            const int p = d.near_split ? 3 * pr + x0 - ix + 1 : pr;
+            for (int ch = 0; ch < nch; ch++) {
+                int tb, te;
+                near_chunk(nh, ni, tile, ch, tb, te);
+                const int cls = 31 - __clz((te - tb) * npart + 1);
+                d.near_items_tmp[k] = make_int2(c, p << 24 | ch);
+                d.near_cls[k] = cls;
+                atomicAdd(&hist[cls], 1);
+                k++;
+            }
         }
     }
 }
@@ -449,23 +515,19 @@ void launch_near_items(const Dev &d, int ncell, int nitems_max, int tile, cudaSt
     k_near_items_place<<<(nitems_max + 255) / 256, 256, 0, st>>>(d);
 }
 
-// One partner's force on the two target sites of a lane (src/evalw1w1n.f90:86-104
-// form): qq / r^3 without cutoff plus 48 eps sg6 r^-6 (sg6 r^-6 - 1/2) / r^2
-// within rc; zero for a partner of the same molecule (src/evalSS.f90:36).  The
-// LJ part runs only when some lane of the warp has a target within rc of the
-// partner (the partner is the same for the whole warp).
-// The pair's (48 eps sg6, sg6) from the kind-pair table (the
-// Lorentz-Berthelot rule of src/init_arrays.f90:476-502, formed in FP64;
-// FP32 copy for the FP32 path).
-struct Tgt32 {
-    float x, y, z, q;   // position relative to the target cell's centre, shifted into the partner cell's frame; q * xpi
-    int m;              // molecule
-    int trow;           // kind * NTYPE: the target's row of the kind-pair table
-};
-struct Tgt64 {
-    double x, y, z, q;
-    int m, trow;        // molecule, type * NTYPE
-};
+// One partner's force on a target site (src/evalw1w1n.f90:86-104 form):
+// qq / r^3 without cutoff plus 48 eps sg6 r^-6 (sg6 r^-6 - 1/2) / r^2 within
+// rc; zero for a partner of the same molecule (src/evalSS.f90:36).
+//
+// The cell sort orders a cell's sites as water O, other LJ sites, water H, so
+// a partner cell is up to three runs.  The two water runs have one charge
+// each: their Coulomb sums S = sum d / r^3 carry no charge per pair and are
+// scaled by q_target q_run xpi once per run.  LJ runs only on targets that
+// have it: a chunk of water H alone (two thirds of the target sites of water)
+// takes the water-O run as plain Coulomb too.
+//
+// Order of a target's sums, the same for every launch shape: the partners of
+// one cell in slot order, then the (up to) 3 cells of a row, then the 9 rows.
 
 // 1/sqrt(x) of the special-function unit (the approximation rsqrtf uses)
 // without the handling of denormal inputs: pair distances are never
@@ -476,447 +538,617 @@ __device__ __forceinline__ float rsqrt_ftz(float x) {
     return y;
 }
 
-// Per-target force sums of an FP32 work item.  COMP: compensated (Kahan)
-// summation, each term's rounding error carried in a second register and
-// folded back when the sum is read.
+// add v to the compensated sum s with carry c (the sum is s - c)
+__device__ __forceinline__ void kahan(float &s, float &c, float v) {
+    const float y = __fsub_rn(v, c);
+    const float t = __fadd_rn(s, y);
+    c = __fsub_rn(__fsub_rn(t, s), y);
+    s = t;
+}
+
+// ---- FP32: two partners at a time in Blackwell's paired arithmetic
+
+// Partners are read from the pair layout of the cell sort: groups of four as
+// negated coordinates x[4], y[4], z[4] (target + partner = difference, and a
+// pair of partners is one register pair of a 128-bit shared load; pairing two
+// targets instead needs every partner coordinate duplicated by moves), every
+// run padded to a multiple of four with partners at 1e18, whose terms are
+// exactly zero: r^-3 underflows.  A warp stages a whole partner cell (up to
+// NEAR_Q groups at a time) by 16-byte cp.async while it works on the one
+// before: staging run by run in blocks of 64 partners cost 250 issue slots a
+// block, 15 % of the kernel.
+constexpr int NEAR_Q = 56;
+struct Buf32 {
+    float4 xyz[NEAR_Q][3];
+    int4 key[NEAR_Q];
+};
+// row: the item's sums over the cells done, by component and target.
+template <bool COMP>
+struct Stage32 {
+    Buf32 b[2];
+    float row[3][64], rowe[COMP ? 3 : 1][COMP ? 64 : 1];
+};
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <int K>
+struct Tgt32 {
+    float x[K], y[K], z[K], q[K];   // position in the partner cell's frame; q * xpi
+    int m[K], trow[K];              // molecule, kind * NTYPE (row of the kind-pair table)
+};
+
+// Per-target sums of a run: the even and the odd partners' in the halves of
+// a pair.  COMP: compensated (Kahan) sums with the carries in e.
 template <int K, bool COMP>
 struct Acc32 {
-    float f[K][3];
-    __device__ __forceinline__ void zero() {
-#pragma unroll
-        for (int j = 0; j < K; j++) f[j][0] = f[j][1] = f[j][2] = 0.f;
-    }
-    __device__ __forceinline__ void add(int j, float dx, float dy, float dz, float ft) {
-        f[j][0] = __fmaf_rn(dx, ft, f[j][0]); f[j][1] = __fmaf_rn(dy, ft, f[j][1]); f[j][2] = __fmaf_rn(dz, ft, f[j][2]);
-    }
-    __device__ __forceinline__ float get(int j, int a) const { return f[j][a]; }
-};
-template <int K>
-struct Acc32<K, true> {
-    float f[K][3], e[K][3];
+    float2 f[K][3], e[COMP ? K : 1][3];
     __device__ __forceinline__ void zero() {
 #pragma unroll
         for (int j = 0; j < K; j++)
 #pragma unroll
-            for (int a = 0; a < 3; a++) f[j][a] = e[j][a] = 0.f;
+            for (int a = 0; a < 3; a++) {
+                f[j][a] = make_float2(0.f, 0.f);
+                if constexpr (COMP) e[j][a] = make_float2(0.f, 0.f);
+            }
     }
-    __device__ __forceinline__ void add1(float &s, float &c, float v) {
-        const float y = __fsub_rn(v, c);
-        const float t = __fadd_rn(s, y);
-        c = __fsub_rn(__fsub_rn(t, s), y);
-        s = t;
+    __device__ __forceinline__ void add1(int j, int a, float2 d, float2 ft) {
+        if constexpr (COMP) {
+            const float2 m1 = make_float2(-1.f, -1.f);
+            const float2 y = __ffma2_rn(d, ft, __fmul2_rn(m1, e[j][a]));
+            const float2 t = __fadd2_rn(f[j][a], y);
+            e[j][a] = __fadd2_rn(__ffma2_rn(m1, f[j][a], t), __fmul2_rn(m1, y));
+            f[j][a] = t;
+        } else {
+            f[j][a] = __ffma2_rn(d, ft, f[j][a]);
+        }
     }
-    __device__ __forceinline__ void add(int j, float dx, float dy, float dz, float ft) {
-        add1(f[j][0], e[j][0], __fmul_rn(dx, ft));
-        add1(f[j][1], e[j][1], __fmul_rn(dy, ft));
-        add1(f[j][2], e[j][2], __fmul_rn(dz, ft));
+    __device__ __forceinline__ void add(int j, float2 dx, float2 dy, float2 dz, float2 ft) {
+        add1(j, 0, dx, ft); add1(j, 1, dy, ft); add1(j, 2, dz, ft);
     }
-    __device__ __forceinline__ float get(int j, int a) const { return __fsub_rn(f[j][a], e[j][a]); }
 };
 
-// FP32 path, K target sites per lane: one partner against targets t[0..K),
-// Coulomb plus, for a partner with LJ, the LJ term of each target within rc
-// (run when some lane of the warp has one); pairk_coul32 for a water-H
-// partner (no LJ).  A partner of the target's own molecule (and the target
-// itself, at r = 0) is excluded by one select that zeroes the reciprocal
-// distance: its Coulomb and LJ terms are then exactly zero (EXCL: only
-// in partner cells that hold a site of some target's molecule).
-template <int K, bool EXCL, bool COMP>
-__device__ __forceinline__ void pairk_acc32(const Tgt32 (&t)[K], float4 pj, int key, const float2 *ljt, float rc2,
-                                            Acc32<K, COMP> &f) {
-    const int mj = key >> 5, tj = key & 31;
-    float dx[K], dy[K], dz[K], r2[K], ir2[K], ft[K];
+// A cell's force per target, compensated with COMP.
+template <int K, bool COMP>
+struct Sum32 {
+    float f[K][3], e[COMP ? K : 1][3];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-    for (int j = 0; j < K; j++) {
-        dx[j] = __fsub_rn(t[j].x, pj.x); dy[j] = __fsub_rn(t[j].y, pj.y); dz[j] = __fsub_rn(t[j].z, pj.z);
-        r2[j] = __fmaf_rn(dz[j], dz[j], __fmaf_rn(dy[j], dy[j], __fmul_rn(dx[j], dx[j])));
-        const float ira = EXCL && mj == t[j].m ? 0.f : rsqrt_ftz(r2[j]);
-        ir2[j] = __fmul_rn(ira, ira);
-        ft[j] = __fmul_rn(__fmul_rn(__fmul_rn(t[j].q, pj.w), ira), ir2[j]);
-    }
-    {   // (a water H in the prefix, only in an overflowing cell, has zero LJ table entries)
-        bool n[K], any = false;
+        for (int j = 0; j < K; j++)
 #pragma unroll
-        for (int j = 0; j < K; j++) { n[j] = r2[j] <= rc2; any = any || n[j]; }
-        if (__any_sync(0xffffffffu, any)) {
-#pragma unroll
-            for (int j = 0; j < K; j++) {
-                const float2 v = ljt[t[j].trow + tj];
-                const float r6 = __fmul_rn(__fmul_rn(ir2[j], ir2[j]), ir2[j]);   // zero for an excluded partner
-                const float w = __fmaf_rn(v.y, r6, -0.5f);
-                ft[j] = __fmaf_rn(__fmul_rn(__fmul_rn(n[j] ? v.x : 0.f, r6), w), ir2[j], ft[j]);
+            for (int a = 0; a < 3; a++) {
+                f[j][a] = 0.f;
+                if constexpr (COMP) e[j][a] = 0.f;
             }
-        }
     }
+    // += s * (both halves of a run's sums)
+    __device__ __forceinline__ void run(const Acc32<K, COMP> &r, const float (&s)[K]) {
 #pragma unroll
-    for (int j = 0; j < K; j++) f.add(j, dx[j], dy[j], dz[j], ft[j]);
-}
-// (t[j].q already holds q_target xpi q_H: every water H carries the same charge)
-template <int K, bool EXCL, bool COMP>
-__device__ __forceinline__ void pairk_coul32(const Tgt32 (&t)[K], float4 pj, int mj, Acc32<K, COMP> &f) {
+        for (int j = 0; j < K; j++)
 #pragma unroll
-    for (int j = 0; j < K; j++) {
-        const float dx = __fsub_rn(t[j].x, pj.x), dy = __fsub_rn(t[j].y, pj.y), dz = __fsub_rn(t[j].z, pj.z);
-        const float r2 = __fmaf_rn(dz, dz, __fmaf_rn(dy, dy, __fmul_rn(dx, dx)));
-        const float ira = EXCL && mj == t[j].m ? 0.f : rsqrt_ftz(r2);
-        const float ft = __fmul_rn(__fmul_rn(t[j].q, ira), __fmul_rn(ira, ira));
-        f.add(j, dx, dy, dz, ft);
+            for (int a = 0; a < 3; a++) {
+                if constexpr (COMP) {
+                    const float2 v = r.f[j][a], c = r.e[j][a];
+                    const float px = __fmul_rn(s[j], v.x), py = __fmul_rn(s[j], v.y);
+                    kahan(f[j][a], e[j][a], px);
+                    kahan(f[j][a], e[j][a], py);
+                    kahan(f[j][a], e[j][a], __fmaf_rn(s[j], v.x, -px));
+                    kahan(f[j][a], e[j][a], __fmaf_rn(s[j], v.y, -py));
+                    kahan(f[j][a], e[j][a], -__fmul_rn(s[j], __fadd_rn(c.x, c.y)));
+                } else {
+                    f[j][a] = __fmaf_rn(s[j], __fadd_rn(r.f[j][a].x, r.f[j][a].y), f[j][a]);
+                }
+            }
     }
-}
+    __device__ __forceinline__ float get(int j, int a) const {
+        if constexpr (COMP) return __fsub_rn(f[j][a], e[j][a]);
+        else return f[j][a];
+    }
+};
 
-// Two targets per lane in Blackwell's paired FP32 arithmetic (fma / add /
-// mul .rn.f32x2: one instruction for both targets; the reciprocal square
-// root stays one MUFU each).  The pair field is issue-bound, so half the
-// FP32 instructions of the two-target items is most of its gain.  The
-// scalar forms above spell out the same roundings in the same order
-// (explicit __fmaf_rn / __fmul_rn / __fsub_rn, so the compiler contracts
-// nothing of its own): a target's force does not depend on whether its item
-// took one, two or four targets per lane, i.e. on the launch shape.
-// Water-H partners, no exclusion test, plain sums:
-__device__ __forceinline__ void coul_h_x2(const Tgt32 (&u)[2], const float4 *wpos, int n, float (&f)[2][3]) {
-    const float2 tx = make_float2(u[0].x, u[1].x), ty = make_float2(u[0].y, u[1].y), tz = make_float2(u[0].z, u[1].z);
-    const float2 tq = make_float2(u[0].q, u[1].q);
-    float2 fx = make_float2(f[0][0], f[1][0]), fy = make_float2(f[0][1], f[1][1]), fz = make_float2(f[0][2], f[1][2]);
-#pragma unroll 2
-    for (int k = 0; k < n; k++) {
-        const float4 p = wpos[k];
-        const float2 dx = __fadd2_rn(tx, make_float2(-p.x, -p.x));
-        const float2 dy = __fadd2_rn(ty, make_float2(-p.y, -p.y));
-        const float2 dz = __fadd2_rn(tz, make_float2(-p.z, -p.z));
-        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const float2 ira = make_float2(rsqrt_ftz(r2.x), rsqrt_ftz(r2.y));
-        const float2 ft = __fmul2_rn(__fmul2_rn(tq, ira), __fmul2_rn(ira, ira));
-        fx = __ffma2_rn(dx, ft, fx); fy = __ffma2_rn(dy, ft, fy); fz = __ffma2_rn(dz, ft, fz);
-    }
-    f[0][0] = fx.x; f[1][0] = fx.y; f[0][1] = fy.x; f[1][1] = fy.y; f[0][2] = fz.x; f[1][2] = fz.y;
-}
-// the LJ-carrying prefix with both targets of a lane in f32x2 arithmetic
-// (same-molecule test per target; LJ only when some lane has a target within rc)
-__device__ __forceinline__ void lj_x2(const Tgt32 (&u)[2], const float4 *wpos, const int *wkey, int n, const float2 *ljt,
-                                      float rc2, float (&f)[2][3]) {
-    const float2 tx = make_float2(u[0].x, u[1].x), ty = make_float2(u[0].y, u[1].y), tz = make_float2(u[0].z, u[1].z);
-    const float2 tq = make_float2(u[0].q, u[1].q);
-    float2 fx = make_float2(f[0][0], f[1][0]), fy = make_float2(f[0][1], f[1][1]), fz = make_float2(f[0][2], f[1][2]);
-#pragma unroll 2
-    for (int k = 0; k < n; k++) {
-        const float4 p = wpos[k];
-        const int key = wkey[k], mj = key >> 5, tj = key & 31;
-        const float2 dx = __fadd2_rn(tx, make_float2(-p.x, -p.x));
-        const float2 dy = __fadd2_rn(ty, make_float2(-p.y, -p.y));
-        const float2 dz = __fadd2_rn(tz, make_float2(-p.z, -p.z));
-        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const float2 ira = make_float2(mj == u[0].m ? 0.f : rsqrt_ftz(r2.x), mj == u[1].m ? 0.f : rsqrt_ftz(r2.y));
-        const float2 ir2 = __fmul2_rn(ira, ira);
-        float2 ft = __fmul2_rn(__fmul2_rn(__fmul2_rn(tq, make_float2(p.w, p.w)), ira), ir2);
-        const bool n0 = r2.x <= rc2, n1 = r2.y <= rc2;
-        if (__any_sync(0xffffffffu, n0 || n1)) {
-            const float2 v0 = ljt[u[0].trow + tj], v1 = ljt[u[1].trow + tj];
-            const float2 r6 = __fmul2_rn(__fmul2_rn(ir2, ir2), ir2);
-            const float2 on = make_float2(n0 ? v0.x : 0.f, n1 ? v1.x : 0.f);
-            const float2 w = __ffma2_rn(make_float2(v0.y, v1.y), r6, make_float2(-0.5f, -0.5f));
-            ft = __ffma2_rn(__fmul2_rn(__fmul2_rn(on, r6), w), ir2, ft);
-        }
-        fx = __ffma2_rn(dx, ft, fx); fy = __ffma2_rn(dy, ft, fy); fz = __ffma2_rn(dz, ft, fz);
-    }
-    f[0][0] = fx.x; f[1][0] = fx.y; f[0][1] = fy.x; f[1][1] = fy.y; f[0][2] = fz.x; f[1][2] = fz.y;
-}
-// water-H partners with the same-molecule test, f32x2
-__device__ __forceinline__ void coul_h_x2_excl(const Tgt32 (&u)[2], const float4 *wpos, const int *wkey, int n,
-                                               float (&f)[2][3]) {
-    const float2 tx = make_float2(u[0].x, u[1].x), ty = make_float2(u[0].y, u[1].y), tz = make_float2(u[0].z, u[1].z);
-    const float2 tq = make_float2(u[0].q, u[1].q);
-    float2 fx = make_float2(f[0][0], f[1][0]), fy = make_float2(f[0][1], f[1][1]), fz = make_float2(f[0][2], f[1][2]);
+// The pairs of the staged groups k0..k1.  LJ: 0 Coulomb of a run with one
+// charge (unscaled), 1 water-O partners with LJ, 2 any partners (charge and LJ
+// parameters by kind).  EXCL: partners of the target's own molecule (and the
+// target itself, at r = 0) get a zero reciprocal distance, so all their terms
+// vanish.  LJ is evaluated when some lane has a pair within rc.
+template <int K, int LJ, bool EXCL, bool COMP>
+__device__ __forceinline__ void near_block32(const Tgt32<K> &t, const float (&qq)[K], const Buf32 &s, int k0, int k1,
+                                             const float2 *ljt, const float *qt, Acc32<K, COMP> &acc) {
+    const float rc2 = (float)(RC * RC);
 #pragma unroll 1
-    for (int k = 0; k < n; k++) {
-        const float4 p = wpos[k];
-        const int mj = wkey[k] >> 5;
-        const float2 dx = __fadd2_rn(tx, make_float2(-p.x, -p.x));
-        const float2 dy = __fadd2_rn(ty, make_float2(-p.y, -p.y));
-        const float2 dz = __fadd2_rn(tz, make_float2(-p.z, -p.z));
-        const float2 r2 = __ffma2_rn(dz, dz, __ffma2_rn(dy, dy, __fmul2_rn(dx, dx)));
-        const float2 ira = make_float2(mj == u[0].m ? 0.f : rsqrt_ftz(r2.x), mj == u[1].m ? 0.f : rsqrt_ftz(r2.y));
-        const float2 ft = __fmul2_rn(__fmul2_rn(tq, ira), __fmul2_rn(ira, ira));
-        fx = __ffma2_rn(dx, ft, fx); fy = __ffma2_rn(dy, ft, fy); fz = __ffma2_rn(dz, ft, fz);
-    }
-    f[0][0] = fx.x; f[1][0] = fx.y; f[0][1] = fy.x; f[1][1] = fy.y; f[0][2] = fz.x; f[1][2] = fz.y;
-}
-
-// One partner cell's sites (slots t0..t1, LJ-carrying ones before th) on
-// the targets u, in the partner cell's frame.  The LJ-carrying prefix always
-// tests for partners of a target's own molecule; the water-H suffix (about
-// two thirds of the pairs) does so only when EXCL says some target's molecule
-// has a site in this cell.  Only that loop comes in two versions, and the
-// testing one is not unrolled: a second LJ loop and more unrolling cost more
-// in instruction-cache stalls than they saved in instructions.  The warp
-// stages 32 partners at a time in its shared-memory slot (one coalesced
-// load per lane) and reads them back as broadcasts: shorter load latency
-// than a broadcast L1 load per partner.
-// Two-target items of the plain mixed path take the paired forms above.
-template <int K, bool EXCL, bool COMP>
-__device__ __forceinline__ void near_cell32(const float4 *__restrict__ pos32, const int *__restrict__ keys,
-                                            Tgt32 (&u)[K], int t0, int th, int t1, const float2 *ljt, float rc2,
-                                            Acc32<K, COMP> &f, float4 *wpos, int *wkey, int lane) {
-    for (int b0 = t0; b0 < th; b0 += 32) {
-        const int n = min(32, th - b0);
-        __syncwarp();
-        if (lane < n) { wpos[lane] = pos32[b0 + lane]; wkey[lane] = keys[b0 + lane]; }
-        __syncwarp();
-        if constexpr (K == 2 && !COMP) {
-            lj_x2(u, wpos, wkey, n, ljt, rc2, f.f);
-        } else {
-#pragma unroll 2
-            for (int k = 0; k < n; k++) pairk_acc32<K, true, COMP>(u, wpos[k], wkey[k], ljt, rc2, f);
-        }
-    }
-    if (th < t1) {
-        const float qh = pos32[th].w;
+    for (int k = k0; k < k1; k++) {
+        const float4 X = s.xyz[k][0], Y = s.xyz[k][1], Z = s.xyz[k][2];
+        const float2 px[2] = {make_float2(X.x, X.y), make_float2(X.z, X.w)};
+        const float2 py[2] = {make_float2(Y.x, Y.y), make_float2(Y.z, Y.w)};
+        const float2 pz[2] = {make_float2(Z.x, Z.y), make_float2(Z.z, Z.w)};
+        int4 M = make_int4(0, 0, 0, 0);
+        if constexpr (EXCL || LJ == 2) M = s.key[k];
+        const int key[4] = {M.x, M.y, M.z, M.w};
+        // the 2 K chains (two pairs of partners, K targets) step by step
+        constexpr int C = 2 * K;
+        float2 dx[C], dy[C], dz[C], r2[C], ir[C], i2[C], ft[C];
 #pragma unroll
-        for (int j = 0; j < K; j++) u[j].q *= qh;
-    }
-    if constexpr (EXCL) {
-        for (int b0 = th; b0 < t1; b0 += 32) {
-            const int n = min(32, t1 - b0);
-            __syncwarp();
-            if (lane < n) { wpos[lane] = pos32[b0 + lane]; wkey[lane] = keys[b0 + lane]; }
-            __syncwarp();
-            if constexpr (K == 2 && !COMP) {
-                coul_h_x2_excl(u, wpos, wkey, n, f.f);
-            } else {
-#pragma unroll 1
-                for (int k = 0; k < n; k++) pairk_coul32<K, true, COMP>(u, wpos[k], wkey[k] >> 5, f);
+        for (int c = 0; c < C; c++) {
+            const int h = c / K, j = c % K;
+            dx[c] = __fadd2_rn(make_float2(t.x[j], t.x[j]), px[h]);
+            dy[c] = __fadd2_rn(make_float2(t.y[j], t.y[j]), py[h]);
+            dz[c] = __fadd2_rn(make_float2(t.z[j], t.z[j]), pz[h]);
+        }
+#pragma unroll
+        for (int c = 0; c < C; c++) r2[c] = __fmul2_rn(dx[c], dx[c]);
+#pragma unroll
+        for (int c = 0; c < C; c++) r2[c] = __ffma2_rn(dy[c], dy[c], r2[c]);
+#pragma unroll
+        for (int c = 0; c < C; c++) r2[c] = __ffma2_rn(dz[c], dz[c], r2[c]);
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            const int h = c / K, j = c % K;
+            ir[c] = make_float2(rsqrt_ftz(r2[c].x), rsqrt_ftz(r2[c].y));
+            if constexpr (EXCL) {
+                if ((key[2 * h] >> 5) == t.m[j]) ir[c].x = 0.f;
+                if ((key[2 * h + 1] >> 5) == t.m[j]) ir[c].y = 0.f;
             }
         }
-    } else {
-        for (int b0 = th; b0 < t1; b0 += 32) {
-            const int n = min(32, t1 - b0);
-            __syncwarp();
-            if (lane < n) wpos[lane] = pos32[b0 + lane];
-            __syncwarp();
-            if constexpr (K == 2 && !COMP) {
-                coul_h_x2(u, wpos, n, f.f);
-            } else {
-#pragma unroll 2
-                for (int k = 0; k < n; k++) pairk_coul32<K, false, COMP>(u, wpos[k], 0, f);
+#pragma unroll
+        for (int c = 0; c < C; c++) i2[c] = __fmul2_rn(ir[c], ir[c]);
+#pragma unroll
+        for (int c = 0; c < C; c++) ft[c] = __fmul2_rn(ir[c], i2[c]);
+        if constexpr (LJ != 0) {
+            bool any = false;
+#pragma unroll
+            for (int c = 0; c < C; c++) any = any || r2[c].x <= rc2 || r2[c].y <= rc2;
+            any = __any_sync(0xffffffffu, any);
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const int h = c / K, j = c % K;
+                float2 q = make_float2(qq[j], qq[j]);
+                if constexpr (LJ == 2) q = __fmul2_rn(q, make_float2(qt[key[2 * h] & 31], qt[key[2 * h + 1] & 31]));
+                const float2 i3 = ft[c];
+                ft[c] = __fmul2_rn(q, i3);
+                if (any) {
+                    float2 v0, v1;
+                    if constexpr (LJ == 2) { v0 = ljt[t.trow[j] + (key[2 * h] & 31)]; v1 = ljt[t.trow[j] + (key[2 * h + 1] & 31)]; }
+                    else v0 = v1 = ljt[t.trow[j]];
+                    const float2 on = make_float2(r2[c].x <= rc2 ? v0.x : 0.f, r2[c].y <= rc2 ? v1.x : 0.f);
+                    const float2 i6 = __fmul2_rn(i3, i3);
+                    const float2 w = __ffma2_rn(make_float2(v0.y, v1.y), i6, make_float2(-0.5f, -0.5f));
+                    ft[c] = __ffma2_rn(__fmul2_rn(__fmul2_rn(on, i6), w), i2[c], ft[c]);
+                }
             }
         }
+#pragma unroll
+        for (int c = 0; c < C; c++) acc.add(c % K, dx[c], dy[c], dz[c], ft[c]);
     }
 }
 
-// One FP32 work item with K target sites per lane (lane + 32 j of the chunk):
-// the force of partner row pr on them, written to that row's partial.
+// One FP32 work item with K target sites per lane (lane + 32 j from `first`):
+// the force of the partner cells xo0..xo1 of row pr on them, written to
+// partial `part`.  qt: charges by kind.
 template <int K, bool PER, bool COMP>
-__device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, int nslot, int c, int pr, int first,
-                                            int ni, int lane, float4 *wpos, int *wkey) {
-    const float4 *__restrict__ pos32 = d.srt_pos32;
-    const int *__restrict__ keys = d.srt_key;
+__device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, const float *qt, float *part, int c, int pr,
+                                            int xo0, int xo1, int first, int ni, int lane, Stage32<COMP> &st) {
     const int dzc = pr / 3 - 1, dyc = pr % 3 - 1;
     const int s0 = d.cstart[c];
-    const Rep r = d.rep[d.crep[c]];
-    int ix, iy, iz;
-    cell_xyz(r, c, ix, iy, iz);
-    const int jy = iy + dyc, jz = iz + dzc;
-    int jx0, jx1;
-    if constexpr (PER) { jx0 = ix - 1; jx1 = ix + 1; }
-    else row_x(r, ix, jx0, jx1);
-    const int wy = PER ? wrap1(jy, r.nc[1]) : jy;
-    Tgt32 t[K];
-    bool act[K];
+    // lane l holds the pair layout of the row's cell at x offset l - 1: first
+    // group, and the ends of its runs (water O whose molecule lies in this
+    // cell alone, other water O, other LJ sites, water H likewise twice)
+    int base = 0, e0 = 0, e1 = 0, e2 = 0, e3 = 0, e4 = 0;
+    if (lane >= xo0 + 1 && lane <= xo1 + 1) {
+        const Rep &r = d.rep[d.crep[c]];
+        int ix, iy, iz;
+        cell_xyz(r, c, ix, iy, iz);
+        const int jx = ix + lane - 1, jy = iy + dyc;
+        const int *cr = d.crun + 8 * (size_t)cell_index(r, PER ? wrap1(jx, r.nc[0]) : jx, PER ? wrap1(jy, r.nc[1]) : jy, iz + dzc);
+        const int4 a = *(const int4 *)cr;
+        const int2 b = *(const int2 *)(cr + 4);
+        base = a.x; e0 = a.y; e1 = a.z; e2 = a.w; e3 = b.x; e4 = b.y;
+    }
+    Tgt32<K> t;
+    float tx[K];
+    unsigned xm = 0;
+    const int rowsh = 3 * (dyc + 1) + 9 * (dzc + 1);
+    const float rs = (float)RS, sy = (float)-dyc * rs, sz = (float)-dzc * rs;
 #pragma unroll
     for (int j = 0; j < K; j++) {
         const int i = first + lane + 32 * j;
-        act[j] = i < ni;
-        t[j] = {0.f, 0.f, 0.f, 0.f, -1, 0};
-        if (act[j]) {
-            const float4 p = pos32[s0 + i];
-            const int kk = keys[s0 + i];
-            t[j] = {p.x, p.y, p.z, p.w * (float)XPI, kk >> 5, (kk & 31) * NTYPE};
+        tx[j] = t.y[j] = t.z[j] = t.q[j] = 0.f;
+        t.m[j] = -2; t.trow[j] = NTYPE;   // no molecule; water H (no LJ)
+        if (i < ni) {
+            const float4 p = d.srt_pos32[s0 + i];
+            const int kk = d.srt_key[s0 + i];
+            tx[j] = p.x; t.y[j] = p.y + sy; t.z[j] = p.z + sz; t.q[j] = p.w * (float)XPI;
+            t.m[j] = kk >> 5; t.trow[j] = (kk & 31) * NTYPE;
+            // the row's partner cells holding a site of the target's molecule: bit jx - ix + 1
+            xm |= ((unsigned)d.srt_xmask[s0 + i] >> rowsh) & 7u;
         }
     }
-    // the row's partner cells holding a site of some target's molecule:
-    // bit jx - ix + 1 (from the targets' molecule-cell masks)
-    unsigned xm = 0;
-    const int rowsh = 3 * (dyc + 1) + 9 * (dzc + 1);
-#pragma unroll
-    for (int j = 0; j < K; j++)
-        if (act[j]) xm |= ((unsigned)d.srt_xmask[s0 + first + lane + 32 * j] >> rowsh) & 7u;
     const unsigned excl = __reduce_or_sync(0xffffffffu, xm);
-    const float rc2 = (float)(RC * RC);
-    const float sy = (float)(-dyc * RS), sz = (float)(-dzc * RS);
-    Acc32<K, COMP> f;
-    f.zero();
-    for (int jx = jx0; jx <= jx1; jx++) {
-        // positions are cell-relative: the shift is the unwrapped offset
-        const int cn = cell_index(r, PER ? wrap1(jx, r.nc[0]) : jx, wy, jz);
-        const int t0 = d.cstart[cn], t1 = d.cstart[cn + 1];
-        const float sx = (float)((ix - jx) * RS);
-        Tgt32 u[K];   // targets in the partner cell's frame
-#pragma unroll
-        for (int j = 0; j < K; j++) { u[j] = t[j]; u[j].x += sx; u[j].y += sy; u[j].z += sz; }
-        // partners with LJ first (the cell sort puts water H last)
-        const int th = t0 + d.cnh[cn];
-        // (items of one target per lane keep one loop body: less code)
-        if (K == 1 || ((excl >> (jx - ix + 1)) & 1u)) near_cell32<K, true, COMP>(pos32, keys, u, t0, th, t1, ljt, rc2, f, wpos, wkey, lane);
-        else near_cell32<K, false, COMP>(pos32, keys, u, t0, th, t1, ljt, rc2, f, wpos, wkey, lane);
-    }
-    float *part = (float *)d.near_part + (size_t)pr * 3 * nslot;   // FP32 row partials on the mixed path
+    const bool lj = first < d.cnh[c];   // the other chunks are water H alone
+    // a block: groups q0..q0 + NEAR_Q of the cell at offset xo
+    int xo = xo0, q0 = -NEAR_Q;
+    auto advance = [&]() -> bool {   // to the next block; false past the last
+        q0 += NEAR_Q;
+        while (q0 >= __shfl_sync(0xffffffffu, e4, xo + 1)) {
+            q0 = 0;
+            if (++xo > xo1) return false;
+        }
+        return true;
+    };
+    auto issue = [&](Buf32 &s) {
+        const int n = min(NEAR_Q, __shfl_sync(0xffffffffu, e4, xo + 1) - q0), g = __shfl_sync(0xffffffffu, base, xo + 1) + q0;
+        const float4 *src = d.pair_xyz + 3 * (size_t)g;
+        float4 *dst = &s.xyz[0][0];
+        for (int i = lane; i < 3 * n; i += 32) cp_async16(dst + i, src + i);
+        const int4 *ks = d.pair_key + g;
+        for (int i = lane; i < n; i += 32) cp_async16(s.key + i, ks + i);
+    };
 #pragma unroll
     for (int j = 0; j < K; j++)
-        if (act[j]) {
-            const size_t o = 3 * (size_t)(s0 + first + lane + 32 * j);
-            part[o] = f.get(j, 0); part[o + 1] = f.get(j, 1); part[o + 2] = f.get(j, 2);
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            st.row[a][lane + 32 * j] = 0.f;
+            if constexpr (COMP) st.rowe[a][lane + 32 * j] = 0.f;
         }
+    Acc32<K, COMP> acc;
+    Sum32<K, COMP> cell;
+    acc.zero();
+    cell.zero();
+    __syncwarp();   // the previous item's last block has been read
+    bool more = advance();
+    if (more) issue(st.b[0]);
+    for (int buf = 0; more; buf ^= 1) {
+        const int bx = xo, b0 = q0, l = xo + 1;
+        const int r0 = __shfl_sync(0xffffffffu, e0, l), r1 = __shfl_sync(0xffffffffu, e1, l), r2 = __shfl_sync(0xffffffffu, e2, l),
+                  r3 = __shfl_sync(0xffffffffu, e3, l), r4 = __shfl_sync(0xffffffffu, e4, l);
+        const int b1 = min(b0 + NEAR_Q, r4);
+        cp_async_wait();
+        __syncwarp();   // this block is staged, the previous one read by every lane
+        more = advance();
+        if (more) issue(st.b[buf ^ 1]);
+        const Buf32 &s = st.b[buf];
+        const float sx = (float)-bx * rs;
+#pragma unroll
+        for (int j = 0; j < K; j++) t.x[j] = tx[j] + sx;
+        const bool own = bx == 0 && pr == 4, ex = (excl >> l) & 1u;
+#pragma unroll 1
+        for (int g = 0; g < 3; g++) {   // water O, other LJ sites, water H
+            const int ga = g == 0 ? 0 : g == 1 ? r1 : r2, gb = g == 0 ? r1 : g == 1 ? r2 : r4;
+            const int ka = max(ga, b0), kb = min(gb, b1);
+            if (ka >= kb) continue;
+            float qq[K], sc[K];
+#pragma unroll
+            for (int j = 0; j < K; j++) {
+                qq[j] = g == 1 ? t.q[j] : __fmul_rn(t.q[j], qt[g >> 1]);
+                sc[j] = g == 1 || (g == 0 && lj) ? 1.f : qq[j];
+            }
+            if (g == 1) {
+                near_block32<K, 2, true, COMP>(t, qq, s, ka - b0, kb - b0, ljt, qt, acc);
+            } else if (g == 0 && lj) {
+                near_block32<K, 1, true, COMP>(t, qq, s, ka - b0, kb - b0, ljt, qt, acc);
+            } else {
+                // same-molecule partners: anywhere in the targets' own cell, else in the run's second part
+                const int m = min(max(own ? ga : ex ? (g == 0 ? r0 : r3) : gb, ka), kb);
+                near_block32<K, 0, false, COMP>(t, qq, s, ka - b0, m - b0, ljt, qt, acc);
+                near_block32<K, 0, true, COMP>(t, qq, s, m - b0, kb - b0, ljt, qt, acc);
+            }
+            if (gb <= b1) {   // the run ends here
+                cell.run(acc, sc);
+                acc.zero();
+            }
+        }
+        if (b1 == r4) {   // the cell ends
+#pragma unroll
+            for (int j = 0; j < K; j++)
+#pragma unroll
+                for (int a = 0; a < 3; a++) {
+                    float &rw = st.row[a][lane + 32 * j];
+                    if constexpr (COMP) {
+                        float r = rw, e = st.rowe[a][lane + 32 * j];
+                        kahan(r, e, cell.get(j, a));
+                        rw = r; st.rowe[a][lane + 32 * j] = e;
+                    } else {
+                        rw = __fadd_rn(rw, cell.get(j, a));
+                    }
+                }
+            cell.zero();
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const int i = first + lane + 32 * j;
+        if (i < ni) {
+            float *o = part + 3 * (size_t)(s0 + i);
+#pragma unroll
+            for (int a = 0; a < 3; a++) {
+                const float r = st.row[a][lane + 32 * j];
+                if constexpr (COMP) o[a] = __fsub_rn(r, st.rowe[a][lane + 32 * j]);
+                else o[a] = r;
+            }
+        }
+    }
 }
 
-__device__ __forceinline__ void pair2_acc64(const Tgt64 &a, const Tgt64 &b, bool two, double4 pj, int key,
-                                            const double2 *lj, double rc2, double (&fa)[3], double (&fb)[3]) {
-    const int mj = key >> 5, tj = key & 31;
-    const double dxa = a.x - pj.x, dya = a.y - pj.y, dza = a.z - pj.z;
-    const bool samea = mj == a.m;
-    const double r2a = samea ? 1.0 : dxa * dxa + dya * dya + dza * dza;
-    const double ira = rsqrt_fp64(r2a), ir2a = ira * ira;
-    double fta = (samea ? 0.0 : a.q * pj.w) * ira * ir2a;
-    double dxb = 0.0, dyb = 0.0, dzb = 0.0, r2b = 1.0, ir2b = 0.0, ftb = 0.0;
-    bool sameb = true;
-    if (two) {
-        dxb = b.x - pj.x; dyb = b.y - pj.y; dzb = b.z - pj.z;
-        sameb = mj == b.m;
-        r2b = sameb ? 1.0 : dxb * dxb + dyb * dyb + dzb * dzb;
-        const double irb = rsqrt_fp64(r2b);
-        ir2b = irb * irb;
-        ftb = (sameb ? 0.0 : b.q * pj.w) * irb * ir2b;
-    }
-    if (tj != 1) {
-        const bool na = r2a <= rc2 && !samea, nb = two && r2b <= rc2 && !sameb;
-        if (__any_sync(0xffffffffu, na || nb)) {   // a zero LJ term leaves the sum unchanged, so skipping it is exact
-            {
-                const double2 v = lj[a.trow + tj];
-                const double on = na ? v.x : 0.0;
-                const double r6 = ir2a * ir2a * ir2a;
-                fta += on * r6 * (v.y * r6 - 0.5) * ir2a;
+// ---- FP64
+
+// GB300 issues an FP64 warp instruction in 16 cycles of an SM (2 FMA per SM
+// per cycle) and everything else 32 times as fast, so the FP64 pair loop
+// counts FP64 instructions alone: 15 for a Coulomb pair.  r^-3 comes from the
+// special-function unit's y ~ r^-1 (relative error below 2^-21): y^2 is exact
+// (48 bits), e = 1 - r^2 y^2 has one rounding, and r^-3 = y^3 (1 - e)^(-3/2) =
+// y^3 (1 + e (3/2 + 15/8 e)) up to 35/16 e^3 < 2^-61.  The conversions of r^2
+// to FP32 and of y to FP64 are bit moves on the integer pipe (GB300 converts
+// at its FP64 rate), and the cutoff is compared on the bits too.
+struct Rinv64 { double y2, e, i3; };   // y^2, 1 - r^2 y^2, r^-3
+
+// r2 within 2^-100 .. 2^100 (the FP32 seed's range, with room for y^3)
+__device__ __forceinline__ bool rinv_plain(double r2) {
+    return (unsigned)(__double2hiint(r2) - ((1023 - 100) << 20)) < (200u << 20);
+}
+__device__ __forceinline__ Rinv64 rinv64(double r2) {
+    // FP32 bits of r2 (truncated): exponent bias 1023 -> 127, mantissa's top 23 bits
+    const unsigned f = __funnelshift_l((unsigned)__double2loint(r2), (unsigned)__double2hiint(r2), 3) + 0x40000000u;
+    const unsigned b = __float_as_uint(rsqrt_ftz(__uint_as_float(f)));
+    const double y = __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    Rinv64 o;
+    o.y2 = y * y;
+    o.e = fma(-r2, o.y2, 1.0);
+    const double y3 = o.y2 * y;
+    o.i3 = fma(y3, o.e * fma(o.e, 1.875, 1.5), y3);
+    return o;
+}
+// any r2 (coincident or blown-up sites: infinities and NaN as 1 / r gives them)
+__device__ __noinline__ Rinv64 rinv64_any(double r2) {
+    const double i = 1.0 / sqrt(r2);
+    return {i * i, 0.0, i * i * i};
+}
+
+constexpr int NEAR_STAGE64 = 32;
+struct Stage64 {
+    double x[NEAR_STAGE64], y[NEAR_STAGE64], z[NEAR_STAGE64], q[NEAR_STAGE64];
+    int key[NEAR_STAGE64];
+};
+template <int K>
+struct Tgt64 {
+    double x[K], y[K], z[K], q[K];
+    int m[K], trow[K];
+};
+
+// The pairs of one staged block (LJ and EXCL as in near_block32).
+template <int K, int LJ, bool EXCL>
+__device__ __forceinline__ void near_block64(const Tgt64<K> &t, const double (&qq)[K], const Stage64 &s, int n,
+                                             const double2 *ljt, double (&f)[K][3]) {
+    const long long rc2 = __double_as_longlong(RC * RC);   // positive doubles order as their bits
+#pragma unroll 2
+    for (int k = 0; k < n; k++) {
+        const double px = s.x[k], py = s.y[k], pz = s.z[k];
+        const int key = EXCL || LJ == 2 ? s.key[k] : 0;
+        double dx[K], dy[K], dz[K], r2[K];
+        bool out = false, same[K];
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+            dx[j] = t.x[j] - px; dy[j] = t.y[j] - py; dz[j] = t.z[j] - pz;
+            r2[j] = fma(dz[j], dz[j], fma(dy[j], dy[j], dx[j] * dx[j]));
+            same[j] = EXCL && (key >> 5) == t.m[j];
+            out = out || !(same[j] || rinv_plain(r2[j]));
+        }
+        Rinv64 v[K];
+#pragma unroll
+        for (int j = 0; j < K; j++) v[j] = rinv64(r2[j]);
+        if (__any_sync(0xffffffffu, out)) {
+#pragma unroll
+            for (int j = 0; j < K; j++)
+                if (!rinv_plain(r2[j])) v[j] = rinv64_any(r2[j]);
+        }
+        double ft[K];
+#pragma unroll
+        for (int j = 0; j < K; j++) ft[j] = same[j] ? 0.0 : v[j].i3;
+        if constexpr (LJ != 0) {
+            bool in[K], any = false;
+#pragma unroll
+            for (int j = 0; j < K; j++) {
+                in[j] = !same[j] && __double_as_longlong(r2[j]) <= rc2;
+                any = any || in[j];
             }
-            if (two) {
-                const double2 v = lj[b.trow + tj];
-                const double on = nb ? v.x : 0.0;
-                const double r6 = ir2b * ir2b * ir2b;
-                ftb += on * r6 * (v.y * r6 - 0.5) * ir2b;
+            any = __any_sync(0xffffffffu, any);
+#pragma unroll
+            for (int j = 0; j < K; j++) {
+                const double i3 = ft[j];
+                double c = qq[j];
+                if constexpr (LJ == 2) c *= s.q[k];
+                ft[j] = c * i3;
+                if (any) {   // a zero LJ term leaves the sum unchanged
+                    const double2 p = ljt[t.trow[j] + (LJ == 2 ? key & 31 : 0)];
+                    const double i6 = i3 * i3, i2 = fma(v[j].y2, fma(v[j].e, v[j].e, v[j].e), v[j].y2);
+                    ft[j] = fma(((in[j] ? p.x : 0.0) * i6) * fma(p.y, i6, -0.5), i2, ft[j]);
+                }
             }
         }
+#pragma unroll
+        for (int j = 0; j < K; j++) {
+            f[j][0] = fma(dx[j], ft[j], f[j][0]); f[j][1] = fma(dy[j], ft[j], f[j][1]); f[j][2] = fma(dz[j], ft[j], f[j][2]);
+        }
     }
-    fa[0] += dxa * fta; fa[1] += dya * fta; fa[2] += dza * fta;
-    if (two) { fb[0] += dxb * ftb; fb[1] += dyb * ftb; fb[2] += dzb * ftb; }
+}
+
+template <int K, int LJ, bool EXCL>
+__device__ __forceinline__ void near_run64(const Dev &d, const Tgt64<K> &t, int t0, int t1, const double2 *ljt,
+                                           double (&cell)[K][3], Stage64 &st, int lane) {
+    if (t0 >= t1) return;
+    double qq[K], f[K][3];
+    const double qr = d.srt_pos[t0].w;
+#pragma unroll
+    for (int j = 0; j < K; j++) { qq[j] = LJ == 2 ? t.q[j] : t.q[j] * qr; f[j][0] = f[j][1] = f[j][2] = 0.0; }
+    for (int b0 = t0; b0 < t1; b0 += NEAR_STAGE64) {
+        const int n = min(NEAR_STAGE64, t1 - b0);
+        __syncwarp();
+        if (lane < n) {
+            const double4 p = d.srt_pos[b0 + lane];
+            st.x[lane] = p.x; st.y[lane] = p.y; st.z[lane] = p.z;
+            if constexpr (LJ == 2) st.q[lane] = p.w;
+            if constexpr (EXCL || LJ == 2) st.key[lane] = d.srt_key[b0 + lane];
+        }
+        __syncwarp();
+        near_block64<K, LJ, EXCL>(t, qq, st, n, ljt, f);
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++)
+#pragma unroll
+        for (int a = 0; a < 3; a++) cell[j][a] = LJ == 0 ? fma(qq[j], f[j][a], cell[j][a]) : cell[j][a] + f[j][a];
+}
+
+template <int K, bool PER>
+__device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, double *part, int c, int pr, int xo0,
+                                            int xo1, int first, int ni, int lane, Stage64 &st) {
+    const int dzc = pr / 3 - 1, dyc = pr % 3 - 1;
+    const int s0 = d.cstart[c];
+    const Rep &r = d.rep[d.crep[c]];
+    int ix, iy, iz;
+    cell_xyz(r, c, ix, iy, iz);
+    const int jy = iy + dyc, jz = iz + dzc, wy = PER ? wrap1(jy, r.nc[1]) : jy;
+    Tgt64<K> t;
+    double tx[K];
+    unsigned xm = 0;
+    const int rowsh = 3 * (dyc + 1) + 9 * (dzc + 1);
+    // a partner cell across a periodic face holds positions one box length
+    // away, so the targets move by that length into its frame
+    const double sy = (double)(jy - wy) * RS;
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const int i = first + lane + 32 * j;
+        tx[j] = t.y[j] = t.z[j] = 1e9;   // no site: far from every partner
+        t.q[j] = 0.0; t.m[j] = -2; t.trow[j] = NTYPE;
+        if (i < ni) {
+            const double4 p = d.srt_pos[s0 + i];
+            const int kk = d.srt_key[s0 + i];
+            tx[j] = p.x; t.y[j] = p.y - sy; t.z[j] = p.z; t.q[j] = p.w * XPI;
+            t.m[j] = kk >> 5; t.trow[j] = (kk & 31) * NTYPE;
+            xm |= ((unsigned)d.srt_xmask[s0 + i] >> rowsh) & 7u;
+        }
+    }
+    const unsigned excl = __reduce_or_sync(0xffffffffu, xm);
+    const bool lj = first < d.cnh[c];
+    double row[K][3];
+#pragma unroll
+    for (int j = 0; j < K; j++) row[j][0] = row[j][1] = row[j][2] = 0.0;
+    for (int xo = xo0; xo <= xo1; xo++) {
+        const int wx = PER ? wrap1(ix + xo, r.nc[0]) : ix + xo;
+        const int cn = cell_index(r, wx, wy, jz);
+        const int t0 = d.cstart[cn], to = t0 + d.cno[cn], th = t0 + d.cnh[cn], t1 = d.cstart[cn + 1];
+        const double sx = (double)(ix + xo - wx) * RS;
+        double cell[K][3];
+#pragma unroll
+        for (int j = 0; j < K; j++) { t.x[j] = tx[j] - sx; cell[j][0] = cell[j][1] = cell[j][2] = 0.0; }
+        const bool ex = (excl >> (xo + 1)) & 1u;
+        if (lj) near_run64<K, 1, true>(d, t, t0, to, ljt, cell, st, lane);
+        else if (ex) near_run64<K, 0, true>(d, t, t0, to, ljt, cell, st, lane);
+        else near_run64<K, 0, false>(d, t, t0, to, ljt, cell, st, lane);
+        near_run64<K, 2, true>(d, t, to, th, ljt, cell, st, lane);
+        if (ex) near_run64<K, 0, true>(d, t, th, t1, ljt, cell, st, lane);
+        else near_run64<K, 0, false>(d, t, th, t1, ljt, cell, st, lane);
+#pragma unroll
+        for (int j = 0; j < K; j++)
+#pragma unroll
+            for (int a = 0; a < 3; a++) row[j][a] += cell[j][a];
+    }
+#pragma unroll
+    for (int j = 0; j < K; j++) {
+        const int i = first + lane + 32 * j;
+        if (i < ni) {
+            double *o = part + 3 * (size_t)(s0 + i);
+            o[0] = row[j][0]; o[1] = row[j][1]; o[2] = row[j][2];
+        }
+    }
 }
 
 // Near field as a persistent kernel: each warp takes items from a global
 // counter until none are left, and for its item sums the force of one
-// partner row on 64 target sites (2 per lane), reading the partners as
-// broadcasts (FP32: staged 32 at a time in the warp's shared-memory slot;
-// FP64: one broadcast L1 load per partner).  Each item
-// writes its own partial per slot (near_part[plane * 3 + row]); k_near_finish
-// adds the 9 partials in a fixed order.  Which warp takes which item does not
-// change any arithmetic, so results are bit-reproducible.
-// MIXED: FP32 positions relative to the cell centres, FP32 pair terms summed
-// in FP32 over one row (at most 3 cells).
+// partner row (or one of its cells, near_split) on up to `tile` target
+// sites, two per lane.  Each item writes its own partial per slot; the
+// finish kernel adds the cells of a row and the 9 rows in a fixed order.
+// Which warp takes which item does not change any arithmetic, so results are
+// bit-reproducible.
+// A warp's first item is fixed: warp w of CTA b takes item w * grid + b.  All
+// CTAs wait together for the predecessor kernel, and taken from the counter
+// the first items went to the 20 to 32 warps of the SMs nearest to it: with
+// fewer items than warps the other SMs had none (3,000 sites in FP64: 3.2 ms,
+// 0.61 with the fixed first items, 0.32 with an item per cell as well).
+//
+// FP32, what bounds it: the FMA pipe and the registers that feed it.  A pair
+// of partners takes 11 paired instructions and two reciprocal square roots; a
+// loop of nothing else runs 2.85 T pairs/s (three-operand paired FMAs issue
+// at 0.6 of the rate of two-operand ones), which is 0.42 ms for the 1.19 G
+// pairs of the 312,000-site configuration.  Lanes without a target (14 %) and
+// LJ (a ninth of the pairs, at three times the cost) make it 0.53; measured
+// 0.64, and 0.72 with two targets per pair register, LJ arithmetic on water-H
+// targets, and partners staged 32 at a time.
+// MODE 0: FP64; 1: FP32 positions relative to the cell centres, FP32 pair
+// terms; 2: FP32 with compensated (Kahan) sums (SESP_MIXED_COMP).
 // PER: the periodic preset's instantiation (rows wrap around x and y)
-// COMP: compensated (Kahan) FP32 sums per target (SESP_MIXED_COMP)
-// (the FP32 two-target instantiations are held to 8 CTAs per SM, 64
-// registers: the paired loops want 67 and the compensated ones 80, and
-// fewer CTAs per SM ran slower)
-template <bool MIXED, int KMAX, bool PER, bool COMP = false>
-__global__ void __launch_bounds__(NEAR_THREADS, (MIXED && KMAX == 2) ? 8 : 1) k_near(Dev d, int nslot, int tile) {
+// CTAs per SM: the FP32 loops want 110 to 146 registers, and one CTA more than
+// they leave room for spills into them (312,000 sites: 0.640 ms at 4 CTAs,
+// 0.736 at 5, 0.675 at 3; compensated, 41,600 sites: 0.164 ms at 3, 0.176 at
+// 4; FP64, 62,400 sites: 7.14 ms at 4, 7.25 at 5).
+constexpr int near_ctas(int mode) { return mode == 2 ? 3 : 4; }
+template <int MODE, bool PER>
+__global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, int nslot, int tile, int split) {
     griddep_wait();
-    __shared__ float2 s_lj32[MIXED ? NTYPE * NTYPE : 1];
-    __shared__ float4 s_stage[MIXED ? NEAR_THREADS / 32 : 1][32];
-    __shared__ int s_key[MIXED ? NEAR_THREADS / 32 : 1][32];
-    __shared__ double2 s_lj64[MIXED ? 1 : NTYPE * NTYPE];
-    if constexpr (MIXED) {
-        for (int t = threadIdx.x; t < NTYPE * NTYPE; t += blockDim.x) s_lj32[t] = d.ljt32[t];
-    } else {
-        for (int t = threadIdx.x; t < NTYPE * NTYPE; t += blockDim.x) s_lj64[t] = d.ljt[t];
+    constexpr int NW = NEAR_THREADS / 32;
+    typedef typename std::conditional<MODE != 0, float2, double2>::type LJ2;
+    typedef typename std::conditional<MODE != 0, float, double>::type R;
+    __shared__ LJ2 s_lj[NTYPE * NTYPE];
+    __shared__ __align__(16) typename std::conditional<MODE != 0, Stage32<MODE == 2>, Stage64>::type s_stage[NW];
+    for (int t = threadIdx.x; t < NTYPE * NTYPE; t += blockDim.x) {
+        if constexpr (MODE != 0) s_lj[t] = d.ljt32[t];
+        else s_lj[t] = d.ljt[t];
     }
+    __shared__ float s_q[MODE != 0 ? NTYPE : 1];
+    if constexpr (MODE != 0)
+        if (threadIdx.x < NTYPE) s_q[threadIdx.x] = (float)d.tq[threadIdx.x];
     __syncthreads();
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nitems = d.near_ctl[1];
-    const float4 *__restrict__ pos32 = d.srt_pos32;
-    const double4 *__restrict__ pos64 = d.srt_pos;
-    const int *__restrict__ keys = d.srt_key;
-    for (;;) {
-        int k = 0;
-        if (lane == 0) k = atomicAdd(&d.near_ctl[0], 1);
-        k = __shfl_sync(0xffffffffu, k, 0);
-        if (k >= nitems) break;
+    int k = w * gridDim.x + blockIdx.x;
+    while (k < nitems) {
         const int2 item = d.near_items[k];
-        const int c = item.x, pr = item.y >> 24, chunk = item.y & 0xFFFFFF;
-        const int dzc = pr / 3 - 1, dyc = pr % 3 - 1;
-        const int s0 = d.cstart[c], ni = d.cstart[c + 1] - s0;
-        const int i0 = chunk * tile + lane, i1 = tile == 64 ? i0 + 32 : ni;
-        const bool a0 = i0 < ni, a1 = i1 < ni;
-        const bool two = __any_sync(0xffffffffu, a1);
-        const Rep r = d.rep[d.crep[c]];
-        int ix, iy, iz;
-        cell_xyz(r, c, ix, iy, iz);
-        const int jy = iy + dyc, jz = iz + dzc;
-        int jx0, jx1;
-        row_x(r, ix, jx0, jx1);
-        double *part = d.near_part + (size_t)pr * 3 * nslot;
-        if constexpr (MIXED) {
-            // K = targets per lane: ceil(targets of the chunk / 32), at most KMAX
-            const int nt = min(tile, ni - chunk * tile), kk = (nt + 31) >> 5;
-            if (kk <= 1) near_item32<1, PER, COMP>(d, s_lj32, nslot, c, pr, chunk * tile, ni, lane, s_stage[threadIdx.x >> 5], s_key[threadIdx.x >> 5]);
-            else if (kk == 2 || KMAX == 2) near_item32<2, PER, COMP>(d, s_lj32, nslot, c, pr, chunk * tile, ni, lane, s_stage[threadIdx.x >> 5], s_key[threadIdx.x >> 5]);
-            else if (kk == 3) near_item32<(KMAX > 2 ? 3 : 2), PER, COMP>(d, s_lj32, nslot, c, pr, chunk * tile, ni, lane, s_stage[threadIdx.x >> 5], s_key[threadIdx.x >> 5]);
-            else near_item32<KMAX, PER, COMP>(d, s_lj32, nslot, c, pr, chunk * tile, ni, lane, s_stage[threadIdx.x >> 5], s_key[threadIdx.x >> 5]);
-        } else {
-            Tgt64 ta = {0.0, 0.0, 0.0, 0.0, -1, 0}, tb = ta;
-            if (a0) {
-                const double4 p = pos64[s0 + i0];
-                const int kk = keys[s0 + i0];
-                ta = {p.x, p.y, p.z, p.w * XPI, kk >> 5, (kk & 31) * NTYPE};
-            }
-            if (a1) {
-                const double4 p = pos64[s0 + i1];
-                const int kk = keys[s0 + i1];
-                tb = {p.x, p.y, p.z, p.w * XPI, kk >> 5, (kk & 31) * NTYPE};
-            }
-            const double rc2 = RC * RC;
-            double fa[3] = {0.0, 0.0, 0.0}, fb[3] = {0.0, 0.0, 0.0};
-            if constexpr (PER) {
-                // one cell at a time: a partner cell across a periodic face
-                // holds positions one box length away, so the targets move
-                // by that length into its frame
-                const int wy = wrap1(jy, r.nc[1]);
-                const double sy = (double)(jy - wy) * RS;
-                for (int jx = jx0; jx <= jx1; jx++) {
-                    const int wx = wrap1(jx, r.nc[0]);
-                    const double sx = (double)(jx - wx) * RS;
-                    Tgt64 ua = ta, ub = tb;
-                    ua.x -= sx; ua.y -= sy; ub.x -= sx; ub.y -= sy;
-                    const int cn = cell_index(r, wx, wy, jz);
-                    const int t0 = d.cstart[cn], t1 = d.cstart[cn + 1];
-#pragma unroll 2
-                    for (int sl = t0; sl < t1; sl++) pair2_acc64(ua, ub, two, pos64[sl], keys[sl], s_lj64, rc2, fa, fb);
-                }
+        int next = 0;   // the next item's number, asked for before this one's work
+        if (lane == 0) next = atomicAdd(&d.near_ctl[0], 1) + NW * gridDim.x;
+        const int c = item.x, p = item.y >> 24, chunk = item.y & 0xFFFFFF;
+        const int pr = split ? p / 3 : p;
+        const int ni = d.cstart[c + 1] - d.cstart[c];
+        int xo0 = -1, xo1 = 1;
+        if (split) {
+            xo0 = xo1 = p - 3 * pr - 1;
+        } else if constexpr (!PER) {
+            const Rep &r = d.rep[d.crep[c]];
+            const int ix = (c - r.cell0) % r.nc[0];
+            if (ix == 0) xo0 = 0;
+            if (ix == r.nc[0] - 1) xo1 = 0;
+        }
+        R *part = (R *)d.near_part + (size_t)p * 3 * nslot;
+        // 64 targets at a time, two per lane where there are more than 32
+        int first, end;
+        near_chunk(d.cnh[c], ni, tile, chunk, first, end);
+        for (; first < end; first += 64) {
+            const int e = min(first + 64, end);
+            if constexpr (MODE != 0) {
+                if (e - first > 32) near_item32<2, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
+                else near_item32<1, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
             } else {
-                const int ca = cell_index(r, jx0, jy, jz);
-                const int t0 = d.cstart[ca], t1 = d.cstart[ca + (jx1 - jx0) + 1];
-#pragma unroll 2
-                for (int sl = t0; sl < t1; sl++) pair2_acc64(ta, tb, two, pos64[sl], keys[sl], s_lj64, rc2, fa, fb);
-            }
-            if (a0) {
-                const size_t o = 3 * (size_t)(s0 + i0);
-                part[o] = fa[0]; part[o + 1] = fa[1]; part[o + 2] = fa[2];
-            }
-            if (a1) {
-                const size_t o = 3 * (size_t)(s0 + i1);
-                part[o] = fb[0]; part[o + 1] = fb[1]; part[o + 2] = fb[2];
+                if (e - first > 32) near_item64<2, PER>(d, s_lj, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
+                else near_item64<1, PER>(d, s_lj, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
             }
         }
+        k = __shfl_sync(0xffffffffu, next, 0);
     }
 }
 
 // Sum of the 9 row partials (fixed order) plus the local-expansion force of
-// src/evalLjk4.f90:31-282 for every slot; writes nf.
+// src/evalLjk4.f90:31-282 for every slot; writes nf.  split: the partials are
+// single cells', and a row is the sum of its cells first.
 template <bool MIXED, bool COMP = false>
-__global__ void k_near_finish(Dev d, int nslot, int ncell, int terms) {
+__global__ void k_near_finish(Dev d, int nslot, int ncell, int terms, int split) {
     griddep_wait();
     typedef typename std::conditional<MIXED, float, double>::type R;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -926,31 +1158,38 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms) {
     const Rep r = d.rep[d.crep[c]];
     int ix, iy, iz;
     cell_xyz(r, c, ix, iy, iz);
-    // the 9 row partials in row order: FP32 rows summed in FP32 on the mixed
-    // path (one conversion to FP64 per component), FP64 on the plain path
-    // (COMP: compensated FP32 sums of the rows, as in the pair field)
-    R fx = 0, fy = 0, fz = 0;
+    // FP32 partials summed in FP32 on the mixed path (one conversion to FP64
+    // per component), FP64 on the plain path (COMP: compensated FP32 sums, as
+    // in the pair field)
+    R fs[3] = {0, 0, 0}, es[3] = {0, 0, 0};
+    auto add = [](R &sum, R &car, R v) {
+        if constexpr (COMP) kahan(sum, car, v);
+        else sum += v;
+    };
     if (terms & SESP_T_NEAR) {
         const int mask = near_row_mask(r, iy, iz);
-        const R *part = (const R *)d.near_part;
-        R ex = 0, ey = 0, ez = 0;
+        const R *part = (const R *)d.near_part + 3 * (size_t)s;
+        const size_t stride = 3 * (size_t)nslot;
+        int x0, x1;
+        row_x(r, ix, x0, x1);
         for (int pr = 0; pr < 9; pr++) {
             if (!(mask >> pr & 1)) continue;
-            const R *p = part + (size_t)pr * 3 * nslot + 3 * (size_t)s;
-            if constexpr (COMP) {
-                R v[3] = {p[0], p[1], p[2]}, *sm[3] = {&fx, &fy, &fz}, *em[3] = {&ex, &ey, &ez};
-                for (int a = 0; a < 3; a++) {
-                    const float y = __fsub_rn(v[a], *em[a]);
-                    const float t = __fadd_rn(*sm[a], y);
-                    *em[a] = __fsub_rn(__fsub_rn(t, *sm[a]), y);
-                    *sm[a] = t;
+            R v[3];
+            if (split) {
+                R rs[3] = {0, 0, 0}, re[3] = {0, 0, 0};
+                for (int xo = x0 - ix; xo <= x1 - ix; xo++) {
+                    const R *p = part + (size_t)(3 * pr + xo + 1) * stride;
+                    for (int a = 0; a < 3; a++) add(rs[a], re[a], p[a]);
                 }
+                for (int a = 0; a < 3; a++) v[a] = rs[a] - re[a];
             } else {
-                fx += p[0]; fy += p[1]; fz += p[2];
+                const R *p = part + (size_t)pr * stride;
+                for (int a = 0; a < 3; a++) v[a] = p[a];
             }
+            for (int a = 0; a < 3; a++) add(fs[a], es[a], v[a]);
         }
-        if constexpr (COMP) { fx = __fsub_rn(fx, ex); fy = __fsub_rn(fy, ey); fz = __fsub_rn(fz, ez); }
     }
+    R fx = fs[0] - es[0], fy = fs[1] - es[1], fz = fs[2] - es[2];
     if (terms & SESP_T_FAR) {
         R x, y, z, q;
         // the cell's local expansion: the FP32 copy of L4 on the mixed path
@@ -972,44 +1211,36 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms) {
     d.nf[3 * (size_t)s] = (double)fx; d.nf[3 * (size_t)s + 1] = (double)fy; d.nf[3 * (size_t)s + 2] = (double)fz;
 }
 
-// mixed: 0 plain FP64, 1 FP32, 2 FP32 with compensated sums
-template <bool PER>
-int near_max_ctas_t(int mixed, int tile) {
+// mode: 0 plain FP64, 1 FP32, 2 FP32 with compensated sums
+int near_resident_ctas(int mode, int per) {
     int nb = 0;
-    if (mixed == 2 && tile > 64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_near<true, 4, PER, true>, NEAR_THREADS, 0);
-    else if (mixed == 2) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_near<true, 2, PER, true>, NEAR_THREADS, 0);
-    else if (mixed && tile > 64) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_near<true, 4, PER>, NEAR_THREADS, 0);
-    else if (mixed) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_near<true, 2, PER>, NEAR_THREADS, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_near<false, 2, PER>, NEAR_THREADS, 0);
+    auto q = [&](auto *k) { cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, NEAR_THREADS, 0); };
+    if (mode == 2) per ? q(k_near<2, true>) : q(k_near<2, false>);
+    else if (mode == 1) per ? q(k_near<1, true>) : q(k_near<1, false>);
+    else per ? q(k_near<0, true>) : q(k_near<0, false>);
     return nb > 0 ? nb : 1;
 }
-int near_max_ctas_per_sm(int mixed, int tile, int per) {
-    return per ? near_max_ctas_t<true>(mixed, tile) : near_max_ctas_t<false>(mixed, tile);
-}
+// Shapes up to this many CTAs per SM are accepted; CTAs past the resident
+// ones start as those finish.
+int near_max_ctas_per_sm(int mode, int per) { return max(near_resident_ctas(mode, per), mode ? 8 : 5); }
 
 // reset_counter: the work counter is cleared here (otherwise the step's
 // gather kernel has cleared it)
-template <bool PER>
-void launch_near_t(const Dev &d, int nslot, int mixed, const NearShape &shape, cudaStream_t st) {
-    const dim3 g(shape.grid), b(NEAR_THREADS);
-    if (mixed == 2 && shape.tile > 64) launch_pdl(k_near<true, 4, PER, true>, g, b, 0, st, d, nslot, shape.tile);
-    else if (mixed == 2) launch_pdl(k_near<true, 2, PER, true>, g, b, 0, st, d, nslot, shape.tile);
-    else if (mixed && shape.tile > 64) launch_pdl(k_near<true, 4, PER>, g, b, 0, st, d, nslot, shape.tile);
-    else if (mixed) launch_pdl(k_near<true, 2, PER>, g, b, 0, st, d, nslot, shape.tile);
-    else launch_pdl(k_near<false, 2, PER>, g, b, 0, st, d, nslot, shape.tile);
-}
-
-void launch_near(const Dev &d, int ncell, int nslot, int mixed, int terms, const NearShape &shape, cudaStream_t st,
+void launch_near(const Dev &d, int ncell, int nslot, int mode, int terms, const NearShape &shape, cudaStream_t st,
                  bool reset_counter, int per) {
+    const int split = d.near_split;
     if (terms & SESP_T_NEAR) {
         if (reset_counter) cudaMemsetAsync(d.near_ctl, 0, sizeof(int), st);
-        if (per) launch_near_t<true>(d, nslot, mixed, shape, st);
-        else launch_near_t<false>(d, nslot, mixed, shape, st);
+        const dim3 g(shape.grid), b(NEAR_THREADS);
+        auto go = [&](auto *k) { launch_pdl(k, g, b, 0, st, d, nslot, shape.tile, split); };
+        if (mode == 2) per ? go(k_near<2, true>) : go(k_near<2, false>);
+        else if (mode == 1) per ? go(k_near<1, true>) : go(k_near<1, false>);
+        else per ? go(k_near<0, true>) : go(k_near<0, false>);
     }
     const dim3 g((nslot + 127) / 128 > 0 ? (nslot + 127) / 128 : 1), b(128);
-    if (mixed == 2) launch_pdl(k_near_finish<true, true>, g, b, 0, st, d, nslot, ncell, terms);
-    else if (mixed) launch_pdl(k_near_finish<true>, g, b, 0, st, d, nslot, ncell, terms);
-    else launch_pdl(k_near_finish<false>, g, b, 0, st, d, nslot, ncell, terms);
+    if (mode == 2) launch_pdl(k_near_finish<true, true>, g, b, 0, st, d, nslot, ncell, terms, split);
+    else if (mode) launch_pdl(k_near_finish<true>, g, b, 0, st, d, nslot, ncell, terms, split);
+    else launch_pdl(k_near_finish<false>, g, b, 0, st, d, nslot, ncell, terms, split);
 }
 
 // ------------------------------------------------------------------ multipoles

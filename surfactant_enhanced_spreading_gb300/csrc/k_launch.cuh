@@ -50,17 +50,18 @@ void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st);
 void launch_gather(const Dev &d, int nslot, int ncell, int mixed, cudaStream_t st);
 // launch shape of the pair field (results do not depend on it)
 struct NearShape {
-    int tile;   // target sites per work item: 32, 64 or (FP32 path) 128, up to 4 per lane
+    int tile;   // target sites per work item: 32, 64 or (FP32 paths) 128
     int grid;   // CTAs of the persistent kernel
 };
 void launch_near_items(const Dev &d, int ncell, int nitems_max, int tile, cudaStream_t st);
-// per: the periodic preset's kernels
-int near_max_ctas_per_sm(int mixed, int tile, int per);
+// mode: 0 FP64, 1 FP32, 2 FP32 with compensated sums; per: the periodic preset's kernels
+int near_resident_ctas(int mode, int per);
+int near_max_ctas_per_sm(int mode, int per);
 // reset_counter: clear the pair field's work counter first; without it the
 // caller must have launched launch_gather (which clears it) on the same
 // stream since the last pair-field launch, or the launch finds every work
 // item taken and computes nothing
-void launch_near(const Dev &d, int ncell, int nslot, int mixed, int terms, const NearShape &shape, cudaStream_t st,
+void launch_near(const Dev &d, int ncell, int nslot, int mode, int terms, const NearShape &shape, cudaStream_t st,
                  bool reset_counter, int per);
 // d2: the largest L2 offset per axis (the H table's half-widths)
 void launch_fma_build(const Dev &d, int ncell, int n3, int n2, int mixed, int3 d2, cudaStream_t st);

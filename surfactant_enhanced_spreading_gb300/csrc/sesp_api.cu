@@ -462,8 +462,17 @@ int dalloc(sesp_ctx *c, T **p, size_t n) {
     return 0;
 }
 
-// work items of the pair field: at most 9 rows x ceil(sites / 32) chunks per cell
-size_t near_items_max(int nsite, int ncell) { return 9 * ((size_t)nsite / 32 + ncell) + 16; }
+// Systems up to this size run the pair field with one work item per partner
+// cell (27 partials per site) instead of per row of three (9): a small system
+// has too few rows to fill the GPU (us per call, rows against cells: 3,000
+// sites 30.9 / 26.6, FP64 614 / 317; 21,400 sites 69.2 / 63.6; 62,400 sites
+// 142.6 / 150.7).
+constexpr int NEAR_SPLIT_MAX = 40000;
+// work items of the pair field: 9 rows (or 27 cells) x the chunks of every
+// occupied cell (LJ-carrying sites and water H, each rounded up to 32s)
+size_t near_items_max(int nsite, int ncell) {
+    return (nsite <= NEAR_SPLIT_MAX ? 27 : 9) * ((size_t)nsite / 32 + 2 * (size_t)std::min(nsite, ncell)) + 16;
+}
 
 void free_state(sesp_ctx *c) {
     for (auto &g : c->g_step)
@@ -697,7 +706,7 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
         cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, dev);
         const int mixed = c->p.precision != SESP_PLAIN_FP64;
         c->near.tile = 64;   // 128 (mixed paths) only where the autotuner measures it faster
-        c->near.grid = c->n_sm * near_max_ctas_per_sm(near_mode(c), c->near.tile, c->chains);
+        c->near.grid = c->n_sm * near_resident_ctas(near_mode(c), c->chains);
         c->cshape.grid = c->n_sm;
     }
     c->sync_check = getenv("SESP_SYNC_CHECK") != nullptr;
@@ -818,10 +827,12 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
     memset(&d, 0, sizeof d);
     int N = nsite, M = nmol, C = ncell;
     d.nsite = N;
+    d.near_split = N <= NEAR_SPLIT_MAX;
     int e = 0;
     double **a12[12] = {&d.x, &d.y, &d.z, &d.vx, &d.vy, &d.vz, &d.ax, &d.ay, &d.az, &d.fx, &d.fy, &d.fz};
     for (auto q : a12) if ((e = dalloc(c, q, N))) return e;
     lap("replica checks");
+    const size_t pair_max = (size_t)N / 4 + 4 * (size_t)std::min(N, C) + 8;   // groups of the pair layout
     if ((e = dalloc(c, &d.ptype, N)) || (e = dalloc(c, &d.smol, N)) || (e = dalloc(c, &d.mrep, M)) ||
         (e = dalloc(c, &d.mfirst, M)) || (e = dalloc(c, &d.mkind, M)) || (e = dalloc(c, &d.mkey, M)) ||
         (e = dalloc(c, &d.mw1, M)) || (e = dalloc(c, &d.ke, 2 * M)) || (e = dalloc(c, &d.mfail, M)) ||
@@ -830,8 +841,9 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.ccount, C)) || (e = dalloc(c, &d.cfill, C)) || (e = dalloc(c, &d.sloc, N)) ||
         (e = dalloc(c, &d.sslot, N)) || (e = dalloc(c, &d.srt_site, N)) || (e = dalloc(c, &d.srt_pos, N)) ||
         (e = dalloc(c, &d.srt_pos32, N)) || (e = dalloc(c, &d.srt_meta, N)) || (e = dalloc(c, &d.srt_key, N)) ||
-        (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
-        (e = dalloc(c, &d.near_part, 27 * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
+        (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) ||
+        (e = dalloc(c, &d.pair_xyz, 3 * pair_max)) || (e = dalloc(c, &d.pair_key, pair_max)) || (e = dalloc(c, &d.crun, 8 * (size_t)C)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
+        (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
         (e = dalloc(c, &d.near_items_tmp, near_items_max(N, C))) || (e = dalloc(c, &d.near_cls, near_items_max(N, C))) ||
         (e = dalloc(c, &d.near_icount, C + 1)) || (e = dalloc(c, &d.near_ctl, 66)) ||
         (e = dalloc(c, &d.isub, (size_t)c->ssite * nsm)) || (e = dalloc(c, &d.O4, (size_t)LP * C)) ||
@@ -844,7 +856,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.wlist_a, nwm)) || (e = dalloc(c, &d.wlist_b, nwm)) || (e = dalloc(c, &d.wsw_a, M)) ||
         (e = dalloc(c, &d.wsw_b, M)) || (e = dalloc(c, &d.cctl, 8)) || (e = dalloc(c, &d.wsort_off, 256)) ||
         (e = dalloc(c, &d.eta_part, 64 * (size_t)R)) || (e = dalloc(c, &d.eta_ctl, R)) ||
-        (e = dalloc(c, &d.cnh, C)) || (e = dalloc(c, &d.tq, NTYPE)) || (e = dalloc(c, &d.tmass, NTYPE)) ||
+        (e = dalloc(c, &d.cnh, C)) || (e = dalloc(c, &d.cno, C)) || (e = dalloc(c, &d.tq, NTYPE)) || (e = dalloc(c, &d.tmass, NTYPE)) ||
         (e = dalloc(c, &d.tgr, NTYPE)) || (e = dalloc(c, &d.simg, N)) || (e = dalloc(c, &d.tbuf, (size_t)R * (1 + TEMP_SLICES))))
         return e;
     const int w2x = 2 * d2.x + 1, w2y = 2 * d2.y + 1, w2z = 2 * d2.z + 1;
@@ -1501,8 +1513,8 @@ int sesp_set_tuning(sesp_ctx *c, int tile, int ctas_per_sm) {
     const int mixed = c->p.precision != SESP_PLAIN_FP64;
     if (tile != 32 && tile != 64 && !(mixed && tile == 128))
         return fail(SESP_EINVAL, "tile must be 32 or 64 (or 128 on the mixed paths)");
-    if (ctas_per_sm < 1 || ctas_per_sm > near_max_ctas_per_sm(near_mode(c), tile, c->chains))
-        return fail(SESP_EINVAL, "ctas_per_sm must be 1..%d", near_max_ctas_per_sm(near_mode(c), tile, c->chains));
+    if (ctas_per_sm < 1 || ctas_per_sm > near_max_ctas_per_sm(near_mode(c), c->chains))
+        return fail(SESP_EINVAL, "ctas_per_sm must be 1..%d", near_max_ctas_per_sm(near_mode(c), c->chains));
     if (set_device(c)) return SESP_ECUDA;
     const bool retile = tile != c->near.tile;
     c->near = {tile, c->n_sm * ctas_per_sm};
@@ -1518,7 +1530,7 @@ int sesp_tuning(sesp_ctx *c, int out[3]) {
     if (!out) return fail(SESP_EINVAL, "null output");
     out[0] = c->near.tile;
     out[1] = c->n_sm ? c->near.grid / c->n_sm : 0;
-    out[2] = near_max_ctas_per_sm(near_mode(c), c->near.tile, c->chains);
+    out[2] = near_max_ctas_per_sm(near_mode(c), c->chains);
     return 0;
 }
 
@@ -1622,7 +1634,7 @@ int sesp_autotune(sesp_ctx *c, int out[3]) {
     NearShape pick = c->near;
     for (int tile : {128, 64, 32}) {
         if (tile == 128 && !mixed) continue;
-        const int mx = near_max_ctas_per_sm(near_mode(c), tile, c->chains);
+        const int mx = near_resident_ctas(near_mode(c), c->chains);
         const int cands[4] = {mx, (3 * mx) / 4, mx / 2, mx / 4};
         launch_near_items(c->d, c->ncell, (int)near_items_max(c->nsite, c->ncell), tile, c->st);
         for (int k = 0; k < 4; k++) {
@@ -1653,7 +1665,7 @@ int sesp_autotune(sesp_ctx *c, int out[3]) {
     CK(cudaStreamSynchronize(c->st));
     out[0] = pick.tile;
     out[1] = pick.grid / c->n_sm;
-    out[2] = near_max_ctas_per_sm(near_mode(c), pick.tile, c->chains);
+    out[2] = near_max_ctas_per_sm(near_mode(c), c->chains);
     return 0;
 }
 

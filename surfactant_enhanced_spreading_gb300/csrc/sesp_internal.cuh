@@ -158,21 +158,30 @@ struct Dev {
     int *cstart, *ccount, *cfill;
     int *sloc, *sslot;
     int *cnh;            // per cell: slots with LJ (every kind but water H), which the sort puts first
+    int *cno;            // per cell: water O among them, which come first of all
     int *srt_site;
     double4 *srt_pos;    // x, y, z, q in slot order (FP64)
     float4 *srt_pos32;   // x, y, z relative to the slot's own cell centre, q (mixed)
+    // pair layout (mixed): the slots of a cell in groups of four, negated
+    // cell-relative coordinates x[4], y[4], z[4] and keys, every run padded;
+    // crun: per cell its first group and the ends of its five runs in groups
+    // (stride 8); srt_pair: a slot's place, 4 group + k
+    float4 *pair_xyz;
+    int4 *pair_key;
+    int *crun, *srt_pair;
     int2 *srt_meta;      // molecule, type
     int *srt_key;        // molecule << 5 | type
     int *srt_xmask;      // per slot: bit dx + 3 dy + 9 dz (each offset + 1) set when the cell at that
                          // offset from the slot's own holds a site of the slot's molecule (itself
                          // included), so the pair loop tests same-molecule partners there only
     double *nf;          // near + far force by slot [3 * nslot]
-    double *near_part;   // per partner row partial near force [9][3 * nslot] (float on the mixed path)
+    double *near_part;   // partial near forces [9 rows, or 27 cells with near_split][3 * nslot] (float on the mixed path)
+    int near_split;      // pair-field items are single partner cells, not rows of three
     int2 *near_items;    // near-field work items (cell, row << 24 | chunk), most expensive first
     int2 *near_items_tmp;   // the same in cell order
     int *near_cls;       // cost class of each item in cell order
     int *near_icount;    // per cell: item count, then first item
-    int *near_ctl;       // [0] item counter of the running launch, [1] item count,
+    int *near_ctl;       // [0] items taken past each warp's first in the running launch, [1] item count,
                          // [2..33] items per cost class, [34..65] next slot per class
     // graphite columns of the bottom layer
     int *gcol_start;
