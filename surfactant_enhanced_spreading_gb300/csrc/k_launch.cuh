@@ -47,6 +47,8 @@ void init_constraint_kernels();   // shared-memory limits of the constraint laun
 // k_force.cu
 void upload_tables_force(const Tables &t, cudaStream_t st);
 void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st);
+// lists of the occupied boxes, and the packed multipoles cleared (with the cell lists, before launch_fma_build)
+void launch_far_lists(const Dev &d, int ncell, cudaStream_t st);
 void launch_gather(const Dev &d, int nslot, int ncell, int mixed, cudaStream_t st);
 // launch shape of the pair field (results do not depend on it)
 struct NearShape {

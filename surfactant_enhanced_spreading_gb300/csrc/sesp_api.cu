@@ -543,11 +543,14 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
     const int mixed = c->p.precision != SESP_PLAIN_FP64;
     if (rebuild) {
         tstart(c, 5);
-        cudaMemsetAsync(d.ccount, 0, sizeof(int) * c->ncell, c->st);
+        // sites per cell, then the far field's counts
+        cudaMemsetAsync(d.ccount, 0, sizeof(int) * (c->ncell + 16 * c->nrep + 3), c->st);
         launch_locate(d, c->nmol, c->smols, c->nsm * c->ssite, c->chains, c->nsite, c->st);
         family(c, "locate");
         launch_sort(d, c->nsite, c->ncell, c->st);
         family(c, "cell sort");
+        launch_far_lists(d, c->ncell, c->st);
+        family(c, "far-field lists");
         launch_near_items(d, c->ncell, (int)near_items_max(c->nsite, c->ncell), c->near.tile, c->st);
         family(c, "near-field items");
         launch_isub(d, c->nsm * c->ssite, c->smols, c->chains, c->st);
@@ -827,6 +830,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
     memset(&d, 0, sizeof d);
     int N = nsite, M = nmol, C = ncell;
     d.nsite = N;
+    d.nrep = R;
     d.near_split = N <= NEAR_SPLIT_MAX;
     int e = 0;
     double **a12[12] = {&d.x, &d.y, &d.z, &d.vx, &d.vy, &d.vz, &d.ax, &d.ay, &d.az, &d.fx, &d.fy, &d.fz};
@@ -838,7 +842,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.mw1, M)) || (e = dalloc(c, &d.ke, 2 * M)) || (e = dalloc(c, &d.mfail, M)) ||
         (e = dalloc(c, &d.rep, R)) || (e = dalloc(c, &d.eta, R)) || (e = dalloc(c, &d.crep, C)) ||
         (e = dalloc(c, &d.b3rep, n3)) || (e = dalloc(c, &d.b2rep, n2)) || (e = dalloc(c, &d.cstart, C + 1)) ||
-        (e = dalloc(c, &d.ccount, C)) || (e = dalloc(c, &d.cfill, C)) || (e = dalloc(c, &d.sloc, N)) ||
+        (e = dalloc(c, &d.ccount, C + 16 * (size_t)R + 3)) || (e = dalloc(c, &d.cfill, C)) || (e = dalloc(c, &d.sloc, N)) ||
         (e = dalloc(c, &d.sslot, N)) || (e = dalloc(c, &d.srt_site, N)) || (e = dalloc(c, &d.srt_pos, N)) ||
         (e = dalloc(c, &d.srt_pos32, N)) || (e = dalloc(c, &d.srt_meta, N)) || (e = dalloc(c, &d.srt_key, N)) ||
         (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) ||
@@ -862,11 +866,12 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
     const int w2x = 2 * d2.x + 1, w2y = 2 * d2.y + 1, w2z = 2 * d2.z + 1;
     const size_t nh2 = (size_t)w2x * w2y * w2z * NHARM;
     lap("allocation");
-    // real-form M2L at L4 and L3: work items of M2C_TILE targets of one parity
+    // real-form M2L at L4 and L3: work items (tiles of targets) of one parity
     // class, each split into M2C_GROUPS offset groups (a constant, so a
     // replica's sums do not depend on what else is batched with it)
     const int mixed = c->p.precision != SESP_PLAIN_FP64;
     const size_t rsz = mixed ? sizeof(float) : sizeof(double);
+    const int tile = mixed ? M2C_TILE : M2C_TILE64;
     std::vector<int4> m2c_items;
     for (int lev = 4; lev >= 3; lev--)
         for (int q = 0; q < R; q++) {
@@ -874,20 +879,22 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
             const int div = lev == 4 ? 2 : 4;
             const int ncls = (r.nc[0] / div) * (r.nc[1] / div) * (r.nc[2] / div);
             for (int cls = 0; cls < 8; cls++)
-                for (int t0 = 0; t0 < ncls; t0 += M2C_TILE)
-                    m2c_items.push_back(make_int4(lev << 28 | q, cls, t0, std::min(M2C_TILE, ncls - t0)));
+                for (int t0 = 0; t0 < ncls; t0 += tile)
+                    m2c_items.push_back(make_int4(lev << 28 | q, cls, t0, std::min(tile, ncls - t0)));
         }
     d.m2c_nitems = (int)m2c_items.size();
     d.m2c_groups = M2C_GROUPS;
     {
-        char *p4 = nullptr, *p3 = nullptr, *q4 = nullptr, *q3 = nullptr, *o4 = nullptr, *o3 = nullptr;
+        char *p4 = nullptr, *q4 = nullptr, *q3 = nullptr, *o4 = nullptr, *o3 = nullptr;
         if ((e = dalloc(c, &o4, (size_t)343 * LP * M2C_LD * rsz)) || (e = dalloc(c, &o3, (size_t)343 * LP * M2C_LD * rsz)) ||
-            (e = dalloc(c, &p4, npk4 * rsz)) || (e = dalloc(c, &p3, npk3 * rsz)) ||
+            (e = dalloc(c, &p4, (npk4 + npk3) * rsz)) ||
+            (e = dalloc(c, &d.fm_list, (size_t)C + n3)) || (e = dalloc(c, &d.occ4, C)) || (e = dalloc(c, &d.occ3, n3)) ||
+            (e = dalloc(c, &d.occ2, n2)) || (e = dalloc(c, &d.has3, n3)) || (e = dalloc(c, &d.has2, n2)) ||
             (e = dalloc(c, &q4, (size_t)d.m2c_groups * LP * C * rsz)) ||
             (e = dalloc(c, &q3, (size_t)d.m2c_groups * LP * n3 * rsz)) ||
             (e = dalloc(c, &d.m2c_items, m2c_items.size())) || (e = dalloc(c, &d.m2c_off, (size_t)8 * M2C_NOFF)))
             return e;
-        d.rop4 = o4; d.rop3 = o3; d.pk4 = p4; d.pk3 = p3; d.part4 = q4; d.part3 = q3;
+        d.rop4 = o4; d.rop3 = o3; d.pk4 = p4; d.pk3 = p4 + npk4 * rsz; d.pk_bytes = (npk4 + npk3) * rsz; d.fm_cnt = d.ccount + C; d.part4 = q4; d.part3 = q3;
     }
     CK(cudaMemcpyAsync(d.m2c_items, m2c_items.data(), m2c_items.size() * sizeof(int4), cudaMemcpyHostToDevice, c->st));
     {

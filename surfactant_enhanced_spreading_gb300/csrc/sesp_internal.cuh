@@ -73,8 +73,9 @@ constexpr double DTSQ2 = 0.00127362 * 0.00127362 / 2.0;
 
 constexpr int M2C_NOFF = 189; // M2L offsets of a cell (6^3 - 3^3 for its parity class)
 constexpr int M2C_LD = 28;    // padded output stride of a real M2L operator row
-constexpr int M2C_W = 2;      // warps of an M2L CTA, 64 targets each (2 per lane)
-constexpr int M2C_TILE = 64 * M2C_W;
+constexpr int M2C_W = 4;      // warps of an M2L CTA, 64 targets each (2 per lane)
+constexpr int M2C_FEW = 16;   // targets of a tile that are taken one per warp
+constexpr int M2C_TILE = 64 * M2C_W, M2C_TILE64 = M2C_FEW;   // targets of a tile, FP32 and FP64
 constexpr int M2C_GROUPS = 21; // offset groups of an M2L work item, 9 offsets each (partial sums added in group order)
 constexpr int GGRP = 8;       // carbon groups per graphite column
 constexpr int GBIN = 32;      // y bins per group
@@ -193,7 +194,8 @@ struct Dev {
     int *gsite, *gcount;   // sites the graphite acts on (rebuilt with the lists)
     // intramolecular correction lists (bit k: site k+1 of the molecule)
     uint32_t *isub;
-    // multipoles / local expansions (double2 = complex)
+    // multipoles / local expansions (complex; L4 FP64, the others FP64 or FP32
+    // by precision), of occupied boxes only
     double2 *O4, *L4, *O3, *L3, *O2, *L2;
     float2 *L4f;         // FP32 copy of L4 (mixed path)
     double *fside;       // graphite + intramolecular forces of the step, [3][nsite]; the site forces add and clear them
@@ -225,6 +227,11 @@ struct Dev {
     int4 *m2c_items;     // work items: (level << 28 | replica, class, first target, targets)
     int *m2c_off;        // per class its 189 offsets, (dx + 3) + 7 (dy + 3) + 49 (dz + 3)
     int m2c_nitems, m2c_groups;
+    // occupied boxes: class targets and their counts, boxes per level, flags (see k_far_lists)
+    int *fm_list, *fm_cnt, *occ4, *occ3, *occ2;
+    uint8_t *has3, *has2;
+    size_t pk_bytes;     // pk4 and pk3, which follows it
+    int nrep;
     // LJ pair table (eps, sg6), NTYPE^2
     double2 *ljt;
     float2 *ljt32;       // FP32 copy of ljt

@@ -117,13 +117,13 @@ def estimate_bytes(system: S.System) -> int:
     per_site = 12 * 8 + 1 + 4 * 4 + 32 + 16 + 8 + 4 + 3 * 8 + parts * 3 * 8 + 6 + 3 * 8 + 12 * 8 + 4 + 16 + parts * 20 / 32
     per_mol = 5 * 4 + 2 * 8 + 4 + 4 + 2 * 4 + 2   # incl. the constraint halves' water lists and sweep counts
     cz = 25 * 16
-    cells = ncell * (6 * 4 + 2 * cz + 4 + 32 + 25 * 8) + min(n, ncell) * (parts * 40 + 4 * 64) + n3 * (4 + 2 * cz) + n2 * (4 + 2 * cz)
+    cells = ncell * (8 * 4 + 2 * cz + 4 + 32 + 25 * 8) + min(n, ncell) * (parts * 40 + 4 * 64) + n3 * (13 + 2 * cz) + n2 * (9 + 2 * cz) + 80
     ops = (w2 ** 3 + 4 * 8) * 15 * 25 * 16 + w2 ** 3 * 45 * 24
     # real-form M2L at L4 and L3: operators, class-packed multipoles, partial
     # sums of 21 offset groups (FP64 sizes: an upper bound)
     pad4 = int(np.prod(nc // 2 + 4)) * 200
     pad3 = int(np.prod(nc // 4 + 4)) * 200
-    ops += 8 * (2 * 343 * 25 * 28 + pad4 + pad3 + 21 * 25 * (ncell + n3)) + 16 * 16 * (ncell // 1024 + 1) + 8 * 189 * 4
+    ops += 8 * (2 * 343 * 25 * 28 + pad4 + pad3 + 21 * 25 * (ncell + n3)) + 16 * 16 * (ncell // 128 + 1) + 8 * 189 * 4
     ncarb = system.carbons.reshape(-1, 3).shape[0]
     ncol = int(nc[0] * nc[1])
     # each carbon lies within reach of about 8 bottom-layer columns (12 with
