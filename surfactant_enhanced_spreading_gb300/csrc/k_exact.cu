@@ -154,43 +154,381 @@ __global__ void k_isub(Dev d, int nsurf_sites, const int *surf_mol_of) {
 
 // ---------------------------------------------------------------- integrator
 
-template <int NSITE>
-struct MolTopo;
+// The waters' halves of the plain path.  What bounds them is FP64 issue: a warp
+// instruction takes its scheduler's FP64 unit 64 cycles, whatever its active
+// lanes, so a water's sweeps take 64 cycles x its warp's instructions.  CTAs
+// are single warps, spread over all schedulers; the reciprocal masses, the
+// fixed bond vectors and divisions by constants leave the sweeps; and up to
+// MOVE_SPLIT_MAX waters, the number that fills every scheduler once, a water
+// takes three lanes, one per component (26 FP64 instructions a corrected SHAKE
+// bond, 46 with a lane per water; more waters than that are bound by the sum
+// over all of them, which a lane per water keeps smaller).  1,000 waters at
+// tolerance 1e-8: SHAKE 204 -> 109 us, RATTLE 218 -> 187 us; 20,000 waters
+// (a lane each) 381 -> 252 and 417 -> 346 us.
+constexpr int WATERS_SPLIT = 10;                       // waters of a warp with three lanes each
+constexpr int MOVE_SPLIT_MAX = WATERS_SPLIT * 4 * 152;
+constexpr int MOVE_BLOCK = 32;
 
-template <>
-struct MolTopo<3> {
-    static constexpr int NB = 3;
-    __device__ static int bi(int b) { return b; }
-    __device__ static int bj(int b) { return b == 2 ? 0 : b + 1; }
-    __device__ static double dsq(int b) { return cT.dsqw[b]; }
-    __device__ static double mass(int i) { return cT.mass[i == 0 ? 0 : 1]; }
-};
-template <>
-struct MolTopo<NSURF> {
-    static constexpr int NB = NBOND;
-    __device__ static int bi(int b) { return cT.bi[b]; }
-    __device__ static int bj(int b) { return cT.bj[b]; }
-    __device__ static double dsq(int b) { return cT.dsqs[b]; }
-    __device__ static double mass(int i) { return cT.mass[2 + i]; }
+// a / b, correctly rounded, from y = 1 / b correctly rounded (P. Markstein,
+// IBM J. Res. Dev. 34, 111 (1990)): the first step brings the quotient within
+// an ulp, the second rounds it.  Infinities and NaN take the division.
+__device__ __forceinline__ double div_by(double a, double b, double y) {
+    double q = a * y;
+    q = fma(fma(-q, b, a), y, q);
+    q = fma(fma(-q, b, a), y, q);
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = a / b;
+    return q;
+}
+
+// a / DT: RN(1 / DT) lies within 0.14 x 2^-53 of 1 / DT, so a y is within an
+// ulp of the quotient and the second step alone rounds it
+__device__ __forceinline__ double div_dt(double a) {
+    constexpr double y = 1.0 / DT;
+    double q = a * y;
+    q = fma(fma(-q, DT, a), y, q);
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = a / DT;
+    return q;
+}
+
+// The plain path's surfactants: the Gauss-Seidel sweeps over 28 bonds of
+// src/move_surfactant_a.f90:36-134 and src/move_surfactant_b.f90:30-118, bit
+// for bit, as a wavefront.  Sweep k takes bond b in step 8 k + b, on the k-th
+// (mod 4) of four groups of three lanes, one lane per component.  Bonds that
+// share a site are at most 7 apart in the reference's order, so when sweep k
+// takes bond b, sweep k - 1 has done every bond that shares a site with it and
+// is at b + 8, which shares none: each site sees the sequential order's
+// updates.  Once a sweep has changed nothing, neither have the later ones
+// under way.  A sum over components is formed by every lane in the
+// reference's order from its neighbours' products.
+// Bound by FP64 issue and latency along one molecule's steps (a step of a
+// correcting bond is 32 FP64 warp instructions; a thread per molecule took 52,
+// in sequence over all sweeps, and spilled): 12 surfactants with 701 waters,
+// SHAKE 280 -> 75 us, RATTLE 571 -> 149 us.
+constexpr int SURF_MOLS = 2;   // molecules of a warp, 12 lanes each
+struct SurfShared {
+    double p[SURF_MOLS][NSURF][3], v[SURF_MOLS][NSURF][3], r[SURF_MOLS][NBOND][3], ke[SURF_MOLS][NSURF];
+    double m[NSURF], rm[NSURF], c0[NBOND], c1[NBOND], c2[NBOND];   // masses and their reciprocals; per-bond constants
+    int i[NBOND], j[NBOND];
 };
 
-// move_*_a for one molecule: Nose-Hoover scaled predictor, SHAKE
-// (src/move_w1_a.f90:36-134, src/move_surfactant_a.f90:36-134), and the
-// kinetic sums before and after (src/nh_water1.f90, src/nh_surfactant.f90)
-template <int NSITE>
-__global__ void k_move_a(Dev d, const int *mols, int nm, double tol, int maxit) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
+// sum of a group's three components (lanes first..first + 2) in the reference's order
+__device__ __forceinline__ double sum3(double v, int first) {
+    const double a = __shfl_sync(0xffffffffu, v, first), b = __shfl_sync(0xffffffffu, v, first + 1),
+                 c = __shfl_sync(0xffffffffu, v, first + 2);
+    return a + b + c;
+}
+
+// Runs the sweeps of the warp's molecules; act(b, on) takes bond b for the
+// lane's group (every lane calls it; `on`: the group has a bond in this step)
+// and says whether it corrected it.  True if the lane's molecule met the
+// tolerance within maxit + 1 sweeps.
+template <typename F>
+__device__ __forceinline__ bool surf_sweeps(int slot, unsigned mol, bool mine, int maxit, F act) {
+    bool ok = false, done = !mine || maxit < 0, dirty = false;
+    int sweep = slot;
+    for (int step = 0; __any_sync(0xffffffffu, !done); step++) {
+        int b = step - 8 * sweep;
+        if (b == NBOND) { sweep += 4; b -= 32; }   // this group's next sweep starts in 4 steps
+        const bool on = !done && b >= 0 && sweep <= maxit;
+        if (b == 0) dirty = false;
+        if (act(on ? b : 0, on)) dirty = true;
+        __syncwarp();
+        const bool ends = on && b == NBOND - 1;
+        const unsigned clean = __ballot_sync(0xffffffffu, ends && !dirty) & mol;
+        const unsigned out = __ballot_sync(0xffffffffu, ends && sweep == maxit) & mol;
+        if (!done && clean) ok = done = true;
+        else if (!done && out) done = true;
+    }
+    return ok;
+}
+
+// which molecule of the warp, sweep slot and component a lane has
+struct SurfLane {
+    int lane, mo, l, slot, a, first;
+    unsigned mol;
+    bool in;
+    __device__ SurfLane() {
+        lane = threadIdx.x & 31;
+        mo = lane >= 12 && lane < 24;
+        in = lane < 12 * SURF_MOLS;
+        l = in ? lane - 12 * mo : lane - 24;   // 0..11 (0..7 past the molecules)
+        slot = l / 3; a = l % 3;
+        first = min(lane - a, 29);
+        mol = in ? 0xfffu << (12 * mo) : 0u;
+    }
+};
+
+__device__ void surf_move_a(const Dev &d, const int *mols, int nm, double tol, int maxit, SurfShared &s, int block) {
+    const SurfLane L;
+    for (int k = L.lane; k < NSURF; k += 32) { s.m[k] = cT.mass[2 + k]; s.rm[k] = 1.0 / cT.mass[2 + k]; }
+    for (int b = L.lane; b < NBOND; b += 32) {
+        const int i = cT.bi[b], j = cT.bj[b];
+        s.i[b] = i; s.j[b] = j;
+        s.c0[b] = cT.dsqs[b];
+        s.c1[b] = cT.dsqs[b] * (2.0 * tol);
+        s.c2[b] = 2.0 * (1.0 / cT.mass[2 + i] + 1.0 / cT.mass[2 + j]);
+    }
+    const int t = block * SURF_MOLS + L.mo;
+    const bool mine = L.in && t < nm;
+    const int m = mine ? mols[t] : 0, g0 = mine ? d.mfirst[m] : 0;
+    const double escale = mine ? 1.0 - d.eta[d.mrep[m]] * DT / 2.0 : 1.0;
+    double *const xs[3] = {d.x, d.y, d.z}, *const vs[3] = {d.vx, d.vy, d.vz}, *const as[3] = {d.ax, d.ay, d.az};
+    auto each = [&](auto f) {   // every (site, component) of the molecule over its 12 lanes
+        if (mine)
+            for (int k = L.l; k < 3 * NSURF; k += 12) f(k / 3, k % 3);
+        __syncwarp();
+    };
+    auto kinetic = [&]() {   // sum of m v^2 in site order
+        if (mine)
+            for (int k = L.l; k < NSURF; k += 12) {
+                const double vx = s.v[L.mo][k][0], vy = s.v[L.mo][k][1], vz = s.v[L.mo][k][2];
+                s.ke[L.mo][k] = s.m[k] * (vx * vx + vy * vy + vz * vz);
+            }
+        __syncwarp();
+        double sum = 0.0;
+        if (mine && L.l == 0)
+            for (int k = 0; k < NSURF; k++) sum += s.ke[L.mo][k];
+        __syncwarp();
+        return sum;
+    };
+    each([&](int k, int a) { s.p[L.mo][k][a] = xs[a][g0 + k]; s.v[L.mo][k][a] = vs[a][g0 + k]; });
+    const double ke0 = kinetic();
+    if (mine)
+        for (int k = L.l; k < 3 * NBOND; k += 12) {
+            const int b = k / 3, a = k % 3;
+            s.r[L.mo][b][a] = s.p[L.mo][s.i[b]][a] - s.p[L.mo][s.j[b]][a];
+        }
+    __syncwarp();
+    each([&](int k, int a) {
+        const double v = s.v[L.mo][k][a], acc = as[a][g0 + k];
+        s.p[L.mo][k][a] = s.p[L.mo][k][a] + v * escale + acc;
+        s.v[L.mo][k][a] = v * escale + acc;
+    });
+    const bool ok = surf_sweeps(L.slot, L.mol, mine, maxit, [&](int b, bool on) {
+        const int i = s.i[b], j = s.j[b], a = L.a, mo = L.mo;
+        const double p = s.p[mo][i][a] - s.p[mo][j][a];
+        const double diffsq = s.c0[b] - sum3(p * p, L.first);
+        const bool cor = on && fabs(diffsq) > s.c1[b];
+        if (__any_sync(0xffffffffu, cor)) {
+            const double r = s.r[mo][b][a], rpab = sum3(r * p, L.first);
+            const double gab = diffsq / (s.c2[b] * rpab);
+            if (cor) {
+                const double dx = r * gab, di = s.rm[i] * dx, dj = s.rm[j] * dx;
+                s.p[mo][i][a] = s.p[mo][i][a] + di; s.p[mo][j][a] = s.p[mo][j][a] - dj;
+                s.v[mo][i][a] = s.v[mo][i][a] + di; s.v[mo][j][a] = s.v[mo][j][a] - dj;
+            }
+        }
+        return cor;
+    });
+    each([&](int k, int a) { xs[a][g0 + k] = s.p[L.mo][k][a]; vs[a][g0 + k] = s.v[L.mo][k][a]; });
+    const double ke1 = kinetic();
+    if (mine && L.l == 0) {
+        d.ke[2 * m] = ke0;
+        d.ke[2 * m + 1] = ke1;
+        if (!ok) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
+    }
+}
+
+__device__ void surf_move_b(const Dev &d, const int *mols, int nm, double tol, int maxit, SurfShared &s, int block) {
+    const SurfLane L;
+    for (int k = L.lane; k < NSURF; k += 32) { s.m[k] = cT.mass[2 + k]; s.rm[k] = 1.0 / cT.mass[2 + k]; }
+    for (int b = L.lane; b < NBOND; b += 32) {
+        const int i = cT.bi[b], j = cT.bj[b];
+        s.i[b] = i; s.j[b] = j;
+        s.c0[b] = (1.0 / cT.mass[2 + i] + 1.0 / cT.mass[2 + j]) * cT.dsqs[b];
+        s.c1[b] = 1.0 / s.c0[b];
+    }
+    const int t = block * SURF_MOLS + L.mo;
+    const bool mine = L.in && t < nm;
+    const int m = mine ? mols[t] : 0, g0 = mine ? d.mfirst[m] : 0;
+    const double escale = mine ? 2.0 / (2.0 + d.eta[d.mrep[m]] * DT) : 1.0;
+    double *const xs[3] = {d.x, d.y, d.z}, *const vs[3] = {d.vx, d.vy, d.vz}, *const as[3] = {d.ax, d.ay, d.az};
+    double *const fs[3] = {d.fx, d.fy, d.fz};
+    __syncwarp();   // the constants are in place
+    if (mine)
+        for (int k = L.l; k < 3 * NSURF; k += 12) {
+            const int n = k / 3, a = k % 3;
+            const double acc = div_by(fs[a][g0 + n] * DTSQ2, s.m[n], s.rm[n]);
+            as[a][g0 + n] = acc;
+            s.p[L.mo][n][a] = xs[a][g0 + n];
+            s.v[L.mo][n][a] = escale * (vs[a][g0 + n] + acc);
+        }
+    __syncwarp();
+    if (mine)
+        for (int k = L.l; k < 3 * NBOND; k += 12) {
+            const int b = k / 3, a = k % 3;
+            s.r[L.mo][b][a] = s.p[L.mo][s.i[b]][a] - s.p[L.mo][s.j[b]][a];
+        }
+    __syncwarp();
+    const bool ok = surf_sweeps(L.slot, L.mol, mine, maxit, [&](int b, bool on) {
+        const int i = s.i[b], j = s.j[b], a = L.a, mo = L.mo;
+        const double r = s.r[mo][b][a], v = s.v[mo][i][a] - s.v[mo][j][a];
+        const double rvab = div_dt(sum3(r * v, L.first));
+        const double gab = div_by(-rvab, s.c0[b], s.c1[b]);
+        const bool cor = on && fabs(gab) > tol;
+        if (cor) {
+            const double dx = r * gab;
+            s.v[mo][i][a] = s.v[mo][i][a] + s.rm[i] * dx * DT;
+            s.v[mo][j][a] = s.v[mo][j][a] - s.rm[j] * dx * DT;
+        }
+        return cor;
+    });
+    if (mine)
+        for (int k = L.l; k < 3 * NSURF; k += 12) vs[k % 3][g0 + k / 3] = s.v[L.mo][k / 3][k % 3];
+    if (mine && L.l == 0 && !ok) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
+}
+
+// A water over three lanes, one per component: the same operations in the
+// same order as the kernels below (every lane forms the sums over components).
+struct WaterLane {
+    int a, first;
+    bool mine;
+    int m, g0;
+    __device__ WaterLane(const Dev &d, const int *mols, int nm, int block) {
+        const int lane = threadIdx.x & 31, w = block * WATERS_SPLIT + lane / 3;
+        a = lane % 3;
+        first = min(lane - a, 29);
+        mine = lane < 3 * WATERS_SPLIT && w < nm;
+        m = mine ? mols[w] : 0;
+        g0 = mine ? d.mfirst[m] : 0;
+    }
+};
+__device__ void water_split_a(const Dev &d, const int *mols, int nm, double tol, int maxit, int block) {
+    const WaterLane L(d, mols, nm, block);
+    double *const x = L.a == 0 ? d.x : L.a == 1 ? d.y : d.z, *const vel = L.a == 0 ? d.vx : L.a == 1 ? d.vy : d.vz;
+    const double *const acc = L.a == 0 ? d.ax : L.a == 1 ? d.ay : d.az;
+    const double mass[3] = {cT.mass[0], cT.mass[1], cT.mass[1]};
+    const double rmO = 1.0 / mass[0], rmH = 1.0 / mass[1], rm[3] = {rmO, rmH, rmH};
+    const double escale = L.mine ? 1.0 - d.eta[d.mrep[L.m]] * DT / 2.0 : 1.0;
+    double p[3], v[3], r[3], lim[3], mm[3], ke0 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        const double vg = L.mine ? vel[L.g0 + i] : 0.0, ag = L.mine ? acc[L.g0 + i] : 0.0;
+        ke0 += mass[i] * sum3(vg * vg, L.first);
+        p[i] = L.mine ? x[L.g0 + i] : 0.0;
+        v[i] = vg * escale + ag;
+        r[i] = p[i];
+        p[i] = p[i] + vg * escale + ag;
+    }
+    const double x0 = r[0];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const int j = b == 2 ? 0 : b + 1;
+        r[b] = r[b] - (b == 2 ? x0 : r[j]);
+        lim[b] = cT.dsqw[b] * (2.0 * tol);
+        mm[b] = 2.0 * (rm[b] + rm[j]);
+    }
+    bool ldone = !L.mine;
+    for (int it = 0; it <= maxit && __any_sync(0xffffffffu, !ldone); it++) {
+        bool clean = true;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int j = b == 2 ? 0 : b + 1;
+            const double pab = p[b] - p[j];
+            const double diffsq = cT.dsqw[b] - sum3(pab * pab, L.first);
+            const bool cor = !ldone && fabs(diffsq) > lim[b];
+            if (__any_sync(0xffffffffu, cor)) {
+                const double rpab = sum3(r[b] * pab, L.first);
+                const double gab = diffsq / (mm[b] * rpab);
+                if (cor) {
+                    const double dx = r[b] * gab, di = rm[b] * dx, dj = rm[j] * dx;
+                    p[b] = p[b] + di; p[j] = p[j] - dj;
+                    v[b] = v[b] + di; v[j] = v[j] - dj;
+                    clean = false;
+                }
+            }
+        }
+        ldone = ldone || clean;
+    }
+    double ke1 = 0.0;
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        if (L.mine) { x[L.g0 + i] = p[i]; vel[L.g0 + i] = v[i]; }
+        ke1 += mass[i] * sum3(v[i] * v[i], L.first);
+    }
+    if (L.mine && L.a == 0) {
+        d.ke[2 * L.m] = ke0;
+        d.ke[2 * L.m + 1] = ke1;
+        if (!ldone) { d.mfail[L.m] += 1; atomicAdd(&d.counters[0], 1ull); }
+    }
+}
+__device__ void water_split_b(const Dev &d, const int *mols, int nm, double tol, int maxit, int block) {
+    const WaterLane L(d, mols, nm, block);
+    const double *const x = L.a == 0 ? d.x : L.a == 1 ? d.y : d.z, *const f = L.a == 0 ? d.fx : L.a == 1 ? d.fy : d.fz;
+    double *const vel = L.a == 0 ? d.vx : L.a == 1 ? d.vy : d.vz, *const acc = L.a == 0 ? d.ax : L.a == 1 ? d.ay : d.az;
+    const double mass[3] = {cT.mass[0], cT.mass[1], cT.mass[1]};
+    const double rmO = 1.0 / mass[0], rmH = 1.0 / mass[1], rm[3] = {rmO, rmH, rmH};
+    const double escale = L.mine ? 2.0 / (2.0 + d.eta[d.mrep[L.m]] * DT) : 1.0;
+    double xs[3], v[3], r[3], den[3], iden[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
+        xs[i] = L.mine ? x[L.g0 + i] : 0.0;
+        const double ag = div_by(L.mine ? f[L.g0 + i] * DTSQ2 : 0.0, mass[i], rm[i]);
+        if (L.mine) acc[L.g0 + i] = ag;
+        v[i] = escale * ((L.mine ? vel[L.g0 + i] : 0.0) + ag);
+    }
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const int j = b == 2 ? 0 : b + 1;
+        r[b] = xs[b] - xs[j];
+        den[b] = (rm[b] + rm[j]) * cT.dsqw[b];
+        iden[b] = 1.0 / den[b];
+    }
+    bool ldone = !L.mine;
+    for (int it = 0; it <= maxit && __any_sync(0xffffffffu, !ldone); it++) {
+        bool clean = true;
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int j = b == 2 ? 0 : b + 1;
+            const double rvab = div_dt(sum3(r[b] * (v[b] - v[j]), L.first));
+            const double gab = div_by(-rvab, den[b], iden[b]);
+            if (!ldone && fabs(gab) > tol) {
+                const double dx = r[b] * gab;
+                v[b] = v[b] + rm[b] * dx * DT;
+                v[j] = v[j] - rm[j] * dx * DT;
+                clean = false;
+            }
+        }
+        ldone = ldone || clean;
+    }
+    if (L.mine) {
+#pragma unroll
+        for (int i = 0; i < 3; i++) vel[L.g0 + i] = v[i];
+        if (L.a == 0 && !ldone) { d.mfail[L.m] += 1; atomicAdd(&d.counters[0], 1ull); }
+    }
+}
+
+// move_*_a of a water: Nose-Hoover scaled predictor, SHAKE
+// (src/move_w1_a.f90:36-134), and the kinetic sums before and after
+// (src/nh_water1.f90)
+// (the first CTAs take the surfactants, smols[0..ns))
+__global__ void __launch_bounds__(MOVE_BLOCK) k_move_a(Dev d, const int *mols, int nm, const int *smols, int ns, double tol,
+                                                      int maxit) {
+    __shared__ SurfShared surf;
+    const int sb = (ns + SURF_MOLS - 1) / SURF_MOLS;
+    if ((int)blockIdx.x < sb) {
+        surf_move_a(d, smols, ns, tol, maxit, surf, blockIdx.x);
+        return;
+    }
+    if (nm <= MOVE_SPLIT_MAX) {
+        water_split_a(d, mols, nm, tol, maxit, blockIdx.x - sb);
+        return;
+    }
+    int t = (blockIdx.x - sb) * blockDim.x + threadIdx.x;
     if (t >= nm) return;
     int m = mols[t];
     int rep = d.mrep[m];
     int g0 = d.mfirst[m];
     double escale = 1.0 - d.eta[rep] * DT / 2.0;
-    double rx[NSITE], ry[NSITE], rz[NSITE], px[NSITE], py[NSITE], pz[NSITE], vx[NSITE], vy[NSITE], vz[NSITE];
+    const double mass[3] = {cT.mass[0], cT.mass[1], cT.mass[1]};
+    const double rmO = 1.0 / mass[0], rmH = 1.0 / mass[1], rm[3] = {rmO, rmH, rmH};
+    double rx[3], ry[3], rz[3], px[3], py[3], pz[3], vx[3], vy[3], vz[3];
     double ke0 = 0.0;
-    for (int i = 0; i < NSITE; i++) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
         int g = g0 + i;
         double vxg = d.vx[g], vyg = d.vy[g], vzg = d.vz[g];
-        ke0 += MolTopo<NSITE>::mass(i) * (vxg * vxg + vyg * vyg + vzg * vzg);
+        ke0 += mass[i] * (vxg * vxg + vyg * vyg + vzg * vzg);
         rx[i] = d.x[g]; ry[i] = d.y[g]; rz[i] = d.z[g];
         px[i] = d.x[g] + vxg * escale + d.ax[g];
         py[i] = d.y[g] + vyg * escale + d.ay[g];
@@ -199,23 +537,30 @@ __global__ void k_move_a(Dev d, const int *mols, int nm, double tol, int maxit) 
         vy[i] = vyg * escale + d.ay[g];
         vz[i] = vzg * escale + d.az[g];
     }
-    const double tol2 = 2.0 * tol;
+    double rxab[3], ryab[3], rzab[3], rabsq[3], lim[3], mm[3];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const int i = b, j = b == 2 ? 0 : b + 1;
+        rxab[b] = rx[i] - rx[j]; ryab[b] = ry[i] - ry[j]; rzab[b] = rz[i] - rz[j];
+        rabsq[b] = cT.dsqw[b];
+        lim[b] = rabsq[b] * (2.0 * tol);
+        mm[b] = 2.0 * (rm[i] + rm[j]);
+    }
     int it = 0;
     bool ldone = false;
     while (!ldone && it <= maxit) {
         ldone = true;
-        for (int b = 0; b < MolTopo<NSITE>::NB; b++) {
-            int i = MolTopo<NSITE>::bi(b), j = MolTopo<NSITE>::bj(b);
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int i = b, j = b == 2 ? 0 : b + 1;
             double pxab = px[i] - px[j], pyab = py[i] - py[j], pzab = pz[i] - pz[j];
             double pabsq = pxab * pxab + pyab * pyab + pzab * pzab;
-            double rabsq = MolTopo<NSITE>::dsq(b);
-            double diffsq = rabsq - pabsq;
-            if (fabs(diffsq) > rabsq * tol2) {
-                double rxab = rx[i] - rx[j], ryab = ry[i] - ry[j], rzab = rz[i] - rz[j];
-                double rpab = rxab * pxab + ryab * pyab + rzab * pzab;
-                double rma = 1.0 / MolTopo<NSITE>::mass(i), rmb = 1.0 / MolTopo<NSITE>::mass(j);
-                double gab = diffsq / (2.0 * (rma + rmb) * rpab);
-                double dx = rxab * gab, dy = ryab * gab, dz = rzab * gab;
+            double diffsq = rabsq[b] - pabsq;
+            if (fabs(diffsq) > lim[b]) {
+                double rpab = rxab[b] * pxab + ryab[b] * pyab + rzab[b] * pzab;
+                double rma = rm[i], rmb = rm[j];
+                double gab = diffsq / (mm[b] * rpab);
+                double dx = rxab[b] * gab, dy = ryab[b] * gab, dz = rzab[b] * gab;
                 px[i] = px[i] + rma * dx; py[i] = py[i] + rma * dy; pz[i] = pz[i] + rma * dz;
                 px[j] = px[j] - rmb * dx; py[j] = py[j] - rmb * dy; pz[j] = pz[j] - rmb * dz;
                 vx[i] = vx[i] + rma * dx; vy[i] = vy[i] + rma * dy; vz[i] = vz[i] + rma * dz;
@@ -226,153 +571,15 @@ __global__ void k_move_a(Dev d, const int *mols, int nm, double tol, int maxit) 
         it++;
     }
     double ke1 = 0.0;
-    for (int i = 0; i < NSITE; i++) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
         int g = g0 + i;
         d.x[g] = px[i]; d.y[g] = py[i]; d.z[g] = pz[i];
         d.vx[g] = vx[i]; d.vy[g] = vy[i]; d.vz[g] = vz[i];
-        ke1 += MolTopo<NSITE>::mass(i) * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
+        ke1 += mass[i] * (vx[i] * vx[i] + vy[i] * vy[i] + vz[i] * vz[i]);
     }
     d.ke[2 * m] = ke0;
     d.ke[2 * m + 1] = ke1;
-    if (!ldone) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
-}
-
-// The surfactant halves with the bond graph of src/init_arrays.f90:229-264
-// unrolled at compile time, so the 29 iterated positions (SHAKE) or
-// velocities (RATTLE) live in registers; the fixed positions and the velocity
-// copies sit in shared memory.  Same Gauss-Seidel order and arithmetic as the
-// generic kernel above (and as src/move_surfactant_a.f90 / _b.f90).
-__device__ constexpr int SBI[NBOND] = {0, 1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17,
-                                        17, 19, 20, 20, 20, 17, 24, 25, 25, 25};
-__device__ constexpr int SBJ[NBOND] = {1, 2, 3, 4, 5, 6, 7, 8, 9, 10, 11, 12, 13, 14, 15, 16, 17, 18,
-                                        19, 20, 21, 22, 23, 24, 25, 26, 27, 28};
-constexpr int SURF_BLOCK = 32;
-
-__global__ void __launch_bounds__(SURF_BLOCK) k_move_a_surf(Dev d, const int *mols, int nm, double tol, int maxit) {
-    __shared__ double s_rm[NSURF], s_dsq[NBOND];
-    if (threadIdx.x < NSURF) s_rm[threadIdx.x] = 1.0 / cT.mass[2 + threadIdx.x];
-    if (threadIdx.x < NBOND) s_dsq[threadIdx.x] = cT.dsqs[threadIdx.x];
-    __syncthreads();
-    volatile double *vrm = s_rm, *vdsq = s_dsq;
-    __shared__ double sr[3][NSURF][SURF_BLOCK];
-    __shared__ double sv[3][NSURF][SURF_BLOCK];
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nm) return;
-    const int l = threadIdx.x;
-    int m = mols[t];
-    int g0 = d.mfirst[m];
-    double escale = 1.0 - d.eta[d.mrep[m]] * DT / 2.0;
-    double px[NSURF], py[NSURF], pz[NSURF];
-    double ke0 = 0.0;
-#pragma unroll
-    for (int i = 0; i < NSURF; i++) {
-        int g = g0 + i;
-        double vxg = d.vx[g], vyg = d.vy[g], vzg = d.vz[g];
-        ke0 += cT.mass[2 + i] * (vxg * vxg + vyg * vyg + vzg * vzg);
-        sr[0][i][l] = d.x[g]; sr[1][i][l] = d.y[g]; sr[2][i][l] = d.z[g];
-        px[i] = d.x[g] + vxg * escale + d.ax[g];
-        py[i] = d.y[g] + vyg * escale + d.ay[g];
-        pz[i] = d.z[g] + vzg * escale + d.az[g];
-        sv[0][i][l] = vxg * escale + d.ax[g];
-        sv[1][i][l] = vyg * escale + d.ay[g];
-        sv[2][i][l] = vzg * escale + d.az[g];
-    }
-    const double tol2 = 2.0 * tol;
-    volatile double(*vr)[NSURF][SURF_BLOCK] = sr;
-    volatile double(*vv)[NSURF][SURF_BLOCK] = sv;
-    int it = 0;
-    bool ldone = false;
-    while (!ldone && it <= maxit) {
-        ldone = true;
-#pragma unroll
-        for (int b = 0; b < NBOND; b++) {
-            const int i = SBI[b], j = SBJ[b];
-            double pxab = px[i] - px[j], pyab = py[i] - py[j], pzab = pz[i] - pz[j];
-            double pabsq = pxab * pxab + pyab * pyab + pzab * pzab;
-            double rabsq = vdsq[b];
-            double diffsq = rabsq - pabsq;
-            if (fabs(diffsq) > rabsq * tol2) {
-                double rxab = vr[0][i][l] - vr[0][j][l], ryab = vr[1][i][l] - vr[1][j][l], rzab = vr[2][i][l] - vr[2][j][l];
-                double rpab = rxab * pxab + ryab * pyab + rzab * pzab;
-                double rma = vrm[i], rmb = vrm[j];
-                double gab = diffsq / (2.0 * (rma + rmb) * rpab);
-                double dx = rxab * gab, dy = ryab * gab, dz = rzab * gab;
-                px[i] = px[i] + rma * dx; py[i] = py[i] + rma * dy; pz[i] = pz[i] + rma * dz;
-                px[j] = px[j] - rmb * dx; py[j] = py[j] - rmb * dy; pz[j] = pz[j] - rmb * dz;
-                vv[0][i][l] = vv[0][i][l] + rma * dx; vv[1][i][l] = vv[1][i][l] + rma * dy; vv[2][i][l] = vv[2][i][l] + rma * dz;
-                vv[0][j][l] = vv[0][j][l] - rmb * dx; vv[1][j][l] = vv[1][j][l] - rmb * dy; vv[2][j][l] = vv[2][j][l] - rmb * dz;
-                ldone = false;
-            }
-        }
-        it++;
-    }
-    double ke1 = 0.0;
-#pragma unroll
-    for (int i = 0; i < NSURF; i++) {
-        int g = g0 + i;
-        double vx = sv[0][i][l], vy = sv[1][i][l], vz = sv[2][i][l];
-        d.x[g] = px[i]; d.y[g] = py[i]; d.z[g] = pz[i];
-        d.vx[g] = vx; d.vy[g] = vy; d.vz[g] = vz;
-        ke1 += cT.mass[2 + i] * (vx * vx + vy * vy + vz * vz);
-    }
-    d.ke[2 * m] = ke0;
-    d.ke[2 * m + 1] = ke1;
-    if (!ldone) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
-}
-
-__global__ void __launch_bounds__(SURF_BLOCK) k_move_b_surf(Dev d, const int *mols, int nm, double tol, int maxit) {
-    __shared__ double s_rm[NSURF], s_dsq[NBOND];
-    if (threadIdx.x < NSURF) s_rm[threadIdx.x] = 1.0 / cT.mass[2 + threadIdx.x];
-    if (threadIdx.x < NBOND) s_dsq[threadIdx.x] = cT.dsqs[threadIdx.x];
-    __syncthreads();
-    volatile double *vrm = s_rm, *vdsq = s_dsq;
-    __shared__ double sr[3][NSURF][SURF_BLOCK];
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nm) return;
-    const int l = threadIdx.x;
-    int m = mols[t];
-    int g0 = d.mfirst[m];
-    double escale = 2.0 / (2.0 + d.eta[d.mrep[m]] * DT);
-    double vx[NSURF], vy[NSURF], vz[NSURF];
-#pragma unroll
-    for (int i = 0; i < NSURF; i++) {
-        int g = g0 + i;
-        double mi = cT.mass[2 + i];
-        sr[0][i][l] = d.x[g]; sr[1][i][l] = d.y[g]; sr[2][i][l] = d.z[g];
-        double axg = d.fx[g] * DTSQ2 / mi, ayg = d.fy[g] * DTSQ2 / mi, azg = d.fz[g] * DTSQ2 / mi;
-        d.ax[g] = axg; d.ay[g] = ayg; d.az[g] = azg;
-        vx[i] = escale * (d.vx[g] + axg);
-        vy[i] = escale * (d.vy[g] + ayg);
-        vz[i] = escale * (d.vz[g] + azg);
-    }
-    volatile double(*vr)[NSURF][SURF_BLOCK] = sr;
-    int it = 0;
-    bool ldone = false;
-    while (!ldone && it <= maxit) {
-        ldone = true;
-#pragma unroll
-        for (int b = 0; b < NBOND; b++) {
-            const int i = SBI[b], j = SBJ[b];
-            double vxab = vx[i] - vx[j], vyab = vy[i] - vy[j], vzab = vz[i] - vz[j];
-            double rxab = vr[0][i][l] - vr[0][j][l], ryab = vr[1][i][l] - vr[1][j][l], rzab = vr[2][i][l] - vr[2][j][l];
-            double rvab = rxab * vxab + ryab * vyab + rzab * vzab;
-            double rma = vrm[i], rmb = vrm[j];
-            rvab = rvab / DT;
-            double gab = -rvab / ((rma + rmb) * vdsq[b]);
-            if (fabs(gab) > tol) {
-                double dx = rxab * gab, dy = ryab * gab, dz = rzab * gab;
-                vx[i] = vx[i] + rma * dx * DT; vy[i] = vy[i] + rma * dy * DT; vz[i] = vz[i] + rma * dz * DT;
-                vx[j] = vx[j] - rmb * dx * DT; vy[j] = vy[j] - rmb * dy * DT; vz[j] = vz[j] - rmb * dz * DT;
-                ldone = false;
-            }
-        }
-        it++;
-    }
-#pragma unroll
-    for (int i = 0; i < NSURF; i++) {
-        int g = g0 + i;
-        d.vx[g] = vx[i]; d.vy[g] = vy[i]; d.vz[g] = vz[i];
-    }
     if (!ldone) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
 }
 
@@ -416,41 +623,63 @@ __global__ void __launch_bounds__(ETA_THREADS) k_eta(Dev d) {
     }
 }
 
-// move_*_b for one molecule: acceleration from force, friction, RATTLE
-// (src/move_w1_b.f90:30-119, src/move_surfactant_b.f90:30-118)
-template <int NSITE>
-__global__ void k_move_b(Dev d, const int *mols, int nm, double tol, int maxit) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
+// move_*_b of a water: acceleration from force, friction, RATTLE
+// (src/move_w1_b.f90:30-119)
+// (the first CTAs take the surfactants, smols[0..ns))
+__global__ void __launch_bounds__(MOVE_BLOCK) k_move_b(Dev d, const int *mols, int nm, const int *smols, int ns, double tol,
+                                                      int maxit) {
+    __shared__ SurfShared surf;
+    const int sb = (ns + SURF_MOLS - 1) / SURF_MOLS;
+    if ((int)blockIdx.x < sb) {
+        surf_move_b(d, smols, ns, tol, maxit, surf, blockIdx.x);
+        return;
+    }
+    if (nm <= MOVE_SPLIT_MAX) {
+        water_split_b(d, mols, nm, tol, maxit, blockIdx.x - sb);
+        return;
+    }
+    int t = (blockIdx.x - sb) * blockDim.x + threadIdx.x;
     if (t >= nm) return;
     int m = mols[t];
     int rep = d.mrep[m];
     int g0 = d.mfirst[m];
     double escale = 2.0 / (2.0 + d.eta[rep] * DT);
-    double rx[NSITE], ry[NSITE], rz[NSITE], vx[NSITE], vy[NSITE], vz[NSITE];
-    for (int i = 0; i < NSITE; i++) {
+    const double mass[3] = {cT.mass[0], cT.mass[1], cT.mass[1]};
+    const double rmO = 1.0 / mass[0], rmH = 1.0 / mass[1], rm[3] = {rmO, rmH, rmH};
+    double rx[3], ry[3], rz[3], vx[3], vy[3], vz[3];
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
         int g = g0 + i;
-        double mi = MolTopo<NSITE>::mass(i);
+        double mi = mass[i], yi = rm[i];
         rx[i] = d.x[g]; ry[i] = d.y[g]; rz[i] = d.z[g];
-        double axg = d.fx[g] * DTSQ2 / mi, ayg = d.fy[g] * DTSQ2 / mi, azg = d.fz[g] * DTSQ2 / mi;
+        double axg = div_by(d.fx[g] * DTSQ2, mi, yi), ayg = div_by(d.fy[g] * DTSQ2, mi, yi), azg = div_by(d.fz[g] * DTSQ2, mi, yi);
         d.ax[g] = axg; d.ay[g] = ayg; d.az[g] = azg;
         vx[i] = escale * (d.vx[g] + axg);
         vy[i] = escale * (d.vy[g] + ayg);
         vz[i] = escale * (d.vz[g] + azg);
     }
+    double rxab[3], ryab[3], rzab[3], den[3], iden[3];
+#pragma unroll
+    for (int b = 0; b < 3; b++) {
+        const int i = b, j = b == 2 ? 0 : b + 1;
+        rxab[b] = rx[i] - rx[j]; ryab[b] = ry[i] - ry[j]; rzab[b] = rz[i] - rz[j];
+        den[b] = (rm[i] + rm[j]) * cT.dsqw[b];
+        iden[b] = 1.0 / den[b];
+    }
     int it = 0;
     bool ldone = false;
     while (!ldone && it <= maxit) {
         ldone = true;
-        for (int b = 0; b < MolTopo<NSITE>::NB; b++) {
-            int i = MolTopo<NSITE>::bi(b), j = MolTopo<NSITE>::bj(b);
+#pragma unroll
+        for (int b = 0; b < 3; b++) {
+            const int i = b, j = b == 2 ? 0 : b + 1;
             double vxab = vx[i] - vx[j], vyab = vy[i] - vy[j], vzab = vz[i] - vz[j];
-            double rxab = rx[i] - rx[j], ryab = ry[i] - ry[j], rzab = rz[i] - rz[j];
-            double rvab = rxab * vxab + ryab * vyab + rzab * vzab;
-            double rma = 1.0 / MolTopo<NSITE>::mass(i), rmb = 1.0 / MolTopo<NSITE>::mass(j);
-            rvab = rvab / DT;
-            double gab = -rvab / ((rma + rmb) * MolTopo<NSITE>::dsq(b));
+            double rvab = rxab[b] * vxab + ryab[b] * vyab + rzab[b] * vzab;
+            double rma = rm[i], rmb = rm[j];
+            rvab = div_dt(rvab);
+            double gab = div_by(-rvab, den[b], iden[b]);
             if (fabs(gab) > tol) {
-                double dx = rxab * gab, dy = ryab * gab, dz = rzab * gab;
+                double dx = rxab[b] * gab, dy = ryab[b] * gab, dz = rzab[b] * gab;
                 vx[i] = vx[i] + rma * dx * DT; vy[i] = vy[i] + rma * dy * DT; vz[i] = vz[i] + rma * dz * DT;
                 vx[j] = vx[j] - rmb * dx * DT; vy[j] = vy[j] - rmb * dy * DT; vz[j] = vz[j] - rmb * dz * DT;
                 ldone = false;
@@ -458,7 +687,8 @@ __global__ void k_move_b(Dev d, const int *mols, int nm, double tol, int maxit) 
         }
         it++;
     }
-    for (int i = 0; i < NSITE; i++) {
+#pragma unroll
+    for (int i = 0; i < 3; i++) {
         int g = g0 + i;
         d.vx[g] = vx[i]; d.vy[g] = vy[i]; d.vz[g] = vz[i];
     }
@@ -590,6 +820,10 @@ void launch_isub(const Dev &d, int nsurf_sites, const int *surf_mols, int per, c
     if (per) k_isub_cfg<<<(nsurf_sites + 127) / 128, 128, 0, st>>>(d, nsurf_sites, surf_mols);
     else k_isub<<<(nsurf_sites + 31) / 32, 32, 0, st>>>(d, nsurf_sites, surf_mols);
 }
+static int move_blocks(int nw, int ns) {
+    const int w = nw <= MOVE_SPLIT_MAX ? WATERS_SPLIT : MOVE_BLOCK;
+    return (ns + SURF_MOLS - 1) / SURF_MOLS + (nw + w - 1) / w;
+}
 // fast = 0 (plain path): the FP64 sweeps above, dividing exactly as the
 // reference does; fast = 1 / 2 (mixed paths): the FP64 / FP32 sweeps of
 // k_constraint.cu.
@@ -597,15 +831,14 @@ void launch_move_a(const Dev &d, const int *wmols, int nw, const int *smols, int
                    double tol, int maxit, int fast, const ConstraintShape &sh, int chains, cudaStream_t st) {
     if (chains) {   // flexible chains: constraints on the waters only
         if (fast) launch_move_a32(d, nw, smols, 0, nmol, nsite, sh, st, tol, maxit, fast == 2, 1);
-        else if (nw) k_move_a<3><<<(nw + 127) / 128, 128, 0, st>>>(d, wmols, nw, tol, maxit);
+        else if (nw) k_move_a<<<move_blocks(nw, 0), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, 0, tol, maxit);
         if (ns) k_move_free_a<<<(ns * 16 + 127) / 128, 128, 0, st>>>(d, smols, ns);
         return;
     }
     if (fast) {
         launch_move_a32(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit, fast == 2, 0);
     } else {
-        if (ns) k_move_a_surf<<<(ns + SURF_BLOCK - 1) / SURF_BLOCK, SURF_BLOCK, 0, st>>>(d, smols, ns, tol, maxit);
-        if (nw) k_move_a<3><<<(nw + 127) / 128, 128, 0, st>>>(d, wmols, nw, tol, maxit);
+        if (nw + ns) k_move_a<<<move_blocks(nw, ns), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, ns, tol, maxit);
     }
 }
 void launch_eta(const Dev &d, int nrep, cudaStream_t st) { k_eta<<<nrep * ETA_BLOCKS, ETA_THREADS, 0, st>>>(d); }
@@ -613,15 +846,14 @@ void launch_move_b(const Dev &d, const int *wmols, int nw, const int *smols, int
                    int maxit, int fast, const ConstraintShape &sh, int chains, cudaStream_t st) {
     if (chains) {
         if (fast) launch_move_b32(d, nw, smols, 0, nmol, nsite, sh, st, tol, maxit, fast == 2, 1);
-        else if (nw) k_move_b<3><<<(nw + 127) / 128, 128, 0, st>>>(d, wmols, nw, tol, maxit);
+        else if (nw) k_move_b<<<move_blocks(nw, 0), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, 0, tol, maxit);
         if (ns) k_move_free_b<<<(ns * NCH + 255) / 256, 256, 0, st>>>(d, smols, ns);
         return;
     }
     if (fast) {
         launch_move_b32(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit, fast == 2, 0);
     } else {
-        if (ns) k_move_b_surf<<<(ns + SURF_BLOCK - 1) / SURF_BLOCK, SURF_BLOCK, 0, st>>>(d, smols, ns, tol, maxit);
-        if (nw) k_move_b<3><<<(nw + 127) / 128, 128, 0, st>>>(d, wmols, nw, tol, maxit);
+        if (nw + ns) k_move_b<<<move_blocks(nw, ns), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, ns, tol, maxit);
     }
 }
 void launch_init_accel(const Dev &d, int nsite, cudaStream_t st) {
