@@ -222,11 +222,15 @@ __device__ inline double cell_centre(const Dev &d, const Rep &r, int a, int i) {
     return t[i];
 }
 
+// fixed point of the FP64 pair field (see near_block64)
+constexpr double FIX_ONE = 4503599627370496.0;   // 2^52
+constexpr double FIX_REACH = 2.7;   // along an axis from a site to its cell's centre; beyond it the replica's items run in FP64
+
 // Slot positions of the step: the site's position (on the periodic preset
 // wrapped by the image it had at the last rebuild, so it stays beside its
-// frozen cell) and charge, FP64; on the mixed path also FP32 relative to the
-// cell centre.
-__global__ void k_gather(Dev d, int nslot, int ncell, int mixed) {
+// frozen cell) and charge, FP64; for the pair field also FP32 relative to the
+// cell centre (mixed) or fixed point (plain).
+__global__ void k_gather(Dev d, int nslot, int ncell, int mode) {
     griddep_wait();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) d.near_ctl[0] = 0;   // the pair field's work counter
@@ -242,10 +246,23 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mixed) {
         y -= (double)im.y * rr.rsd[1];
     }
     d.srt_pos[s] = make_double4(x, y, z, q);
-    if (mixed) {
-        const Rep r = rr;
-        int ix, iy, iz;
-        cell_xyz(r, c, ix, iy, iz);
+    const Rep r = rr;
+    int ix, iy, iz;
+    cell_xyz(r, c, ix, iy, iz);
+    if (mode == GATHER_PLAIN) {   // fixed point about the cell centre for the FP64 pair field
+        const double p[3] = {x, y, z};
+        const int ic[3] = {ix, iy, iz};
+        bool ok = true;
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            const double ca = cell_centre(d, r, a, ic[a]);
+            const bool in = fabs(p[a] - ca) < FIX_REACH && fabs(ca) < 1024.0;
+            d.srt_fix[s + a * (size_t)d.nsite] = in ? (__double2ll_rn(p[a] * FIX_ONE) - __double2ll_rn(ca * FIX_ONE)) << 7 : 0;
+            ok = ok && in;
+        }
+        if (!ok) d.near_far[d.crep[c]] = 1;   // cleared by the finish kernel
+    }
+    if (mode == GATHER_MIXED) {
         const float4 p = make_float4((float)(x - cell_centre(d, r, 0, ix)), (float)(y - cell_centre(d, r, 1, iy)),
                                      (float)(z - cell_centre(d, r, 2, iz)), (float)q);
         d.srt_pos32[s] = p;
@@ -255,9 +272,9 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mixed) {
     }
 }
 
-void launch_gather(const Dev &d, int nslot, int ncell, int mixed, cudaStream_t st) {
+void launch_gather(const Dev &d, int nslot, int ncell, int mode, cudaStream_t st) {
     launch_pdl(k_gather, dim3((nslot + 255) / 256 > 0 ? (nslot + 255) / 256 : 1), dim3(256), 0, st, d, nslot, ncell,
-               mixed);
+               mode);
 }
 
 // ------------------------------------------------------------------ solid harmonics
@@ -879,193 +896,239 @@ __device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, con
 
 // ---- FP64
 
-// GB300 issues an FP64 warp instruction in 16 cycles of an SM (2 FMA per SM
-// per cycle) and everything else 32 times as fast, so the FP64 pair loop
-// counts FP64 instructions alone: 15 for a Coulomb pair.  r^-3 comes from the
-// special-function unit's y ~ r^-1 (relative error below 2^-21): y^2 is exact
-// (48 bits), e = 1 - r^2 y^2 has one rounding, and r^-3 = y^3 (1 - e)^(-3/2) =
-// y^3 (1 + e (3/2 + 15/8 e)) up to 35/16 e^3 < 2^-61.  The conversions of r^2
-// to FP32 and of y to FP64 are bit moves on the integer pipe (GB300 converts
-// at its FP64 rate), and the cutoff is compared on the bits too.
-struct Rinv64 { double y2, e, i3; };   // y^2, 1 - r^2 y^2, r^-3
+// GB300 issues an FP64 warp instruction in 64 cycles of a scheduler, and an
+// integer or FP32 one in one or two.  So the FP64 pair loop does all but the
+// three force sums in integers: the coordinates are fixed point, the squared
+// distance, r^-3 and the conversions of the differences are formed from 64-bit
+// products, and a Coulomb pair takes 3 FP64 instructions and about 200 others
+// (15 FP64 instructions with r^-3 from one exact FP64 residual, 22 with two
+// Newton steps).  The integer and the FP64 pipe are then busy for 62 and 58 %
+// of the cycles.  FP64 pair field: 62,400 sites 7.14 -> 2.64 ms (10.5 with 22
+// instructions), 3,000 sites 317 -> 157 us.
+//
+// Coordinates: 2^-59 sigma relative to the partner's cell centre, from
+// positions and centres rounded to 2^-52 (exact for |x| >= 1), so a
+// difference carries at most that rounding.  r^2: units of 2^-56, truncated
+// within 3 of them.  r^-3: y ~ r^-1 from the special-function unit on r^2
+// scaled by a power of 4 to [1, 4), a little low; e = 1 - r^2 y^2 >= 0 exactly
+// (the product modulo 2^64 below its known top), r^-3 = y^3 (1 + e (3/2 + 15/8
+// e)) up to 35/16 e^3 < 2^-57, one rounding to FP64.  Against 80-bit
+// arithmetic over distances of 0.4 to 9 sigma: 0.7e-16 RMS (a plain FP64
+// evaluation: 1.2e-16).
+typedef unsigned long long u64;
+constexpr u64 FIX_NEAR2 = (u64)1 << 53;   // r^2 of 1/8: closer pairs are evaluated in FP64
 
-// r2 within 2^-100 .. 2^100 (the FP32 seed's range, with room for y^3)
-__device__ __forceinline__ bool rinv_plain(double r2) {
-    return (unsigned)(__double2hiint(r2) - ((1023 - 100) << 20)) < (200u << 20);
+// a difference (units of 2^-59) as FP64
+__device__ __forceinline__ double fix_to_double(long long v) {
+    const long long s = v >> 63;
+    const u64 u = (u64)((v ^ s) - s);
+    const unsigned uh = (unsigned)(u >> 32), ul = (unsigned)u;
+    const bool z = uh == 0;
+    const unsigned a = z ? ul : uh, b = z ? 0u : ul;
+    const int lz = __clz(a);
+    const unsigned mh = __funnelshift_l(b, a, lz), ml = b << (lz & 31);
+    const unsigned e = (unsigned)(1023 + 63 - 59 - 1 - lz - (z ? 32 : 0)) << 20;
+    unsigned hi = e + (mh >> 11);   // the leading bit adds 1 to the exponent
+    if (a == 0) hi = 0;
+    return __hiloint2double((int)(hi | ((unsigned)s & 0x80000000u)), (int)__funnelshift_r(ml, mh, 11));
 }
-__device__ __forceinline__ Rinv64 rinv64(double r2) {
-    // FP32 bits of r2 (truncated): exponent bias 1023 -> 127, mantissa's top 23 bits
-    const unsigned f = __funnelshift_l((unsigned)__double2loint(r2), (unsigned)__double2hiint(r2), 3) + 0x40000000u;
-    const unsigned b = __float_as_uint(rsqrt_ftz(__uint_as_float(f)));
-    const double y = __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
-    Rinv64 o;
-    o.y2 = y * y;
-    o.e = fma(-r2, o.y2, 1.0);
-    const double y3 = o.y2 * y;
-    o.i3 = fma(y3, o.e * fma(o.e, 1.875, 1.5), y3);
-    return o;
+// w 2^ex as FP64, w >= 2^32
+__device__ __forceinline__ double scale_to_double(u64 w, int ex) {
+    const int lz = __clz((unsigned)(w >> 32));
+    const u64 m = w << lz;
+    return __longlong_as_double((long long)(((u64)(1023 + 63 - 1 - lz + ex) << 52) + (m >> 11) + ((m >> 10) & 1)));
 }
-// any r2 (coincident or blown-up sites: infinities and NaN as 1 / r gives them)
-__device__ __noinline__ Rinv64 rinv64_any(double r2) {
-    const double i = 1.0 / sqrt(r2);
-    return {i * i, 0.0, i * i * i};
+__device__ __forceinline__ u64 fix_r2(long long x, long long y, long long z) {
+    const int hx = (int)(x >> 32), hy = (int)(y >> 32), hz = (int)(z >> 32);
+    const unsigned lx = (unsigned)x, ly = (unsigned)y, lz = (unsigned)z;
+    const u64 s = (u64)((long long)hx * hx) + (u64)((long long)hy * hy) + (u64)((long long)hz * hz);
+    const long long c = (long long)hx * (int)(lx >> 1) + (long long)hy * (int)(ly >> 1) + (long long)hz * (int)(lz >> 1);
+    const u64 q = (u64)__umulhi(lx, lx) + __umulhi(ly, ly) + __umulhi(lz, lz);
+    return (s << 2) + (u64)(c >> 28) + (q >> 30);
+}
+// r^-3 and, with LJ, r^-2 of r2 >= 2^32
+template <bool LJ>
+__device__ __forceinline__ void fix_inverse(u64 r2, double &i3, double &i2) {
+    const int lz = __clz((unsigned)(r2 >> 32)) & ~1;
+    const u64 n = r2 << lz;
+    const unsigned n1 = (unsigned)(n >> 32), n0 = (unsigned)n;
+    const float y = rsqrt_ftz(__uint2float_rn(n1));                      // 2^-15 / sqrt(n / 2^62)
+    const unsigned m = __float2uint_rz(y * (float)(70368744177664.0 * (1.0 - 1.5 / 4194304.0)));   // 2^31 y, low by 3.6e-7
+    const u64 mm = (u64)m * m, m2 = mm >> 12;                            // 2^62 y^2, exact; 2^50 y^2
+    const unsigned l = (unsigned)m2, h = (unsigned)(m2 >> 32);
+    const u64 t = (u64)n1 * l + (u64)n0 * h + __umulhi(n0, l) + ((u64)(n1 * h) << 32);   // 2^80 (1 - e), modulo 2^64
+    const u64 e = 0ull - t, e60 = e >> 20;                               // 2^80 e, 2^60 e
+    const unsigned e2 = __umulhi((unsigned)(e >> 32), (unsigned)(e >> 32));   // 2^64 e^2
+    const u64 m3 = (u64)(unsigned)(mm >> 32) * m + __umulhi((unsigned)mm, m);   // 2^61 y^3
+    i3 = scale_to_double(m3 + __umul64hi(m3, (e60 + (e60 >> 1) + ((e2 * 15u) >> 7)) << 4), -70 + 3 * (lz >> 1));
+    if constexpr (LJ) i2 = scale_to_double(mm + __umul64hi(mm, (e60 + (e2 >> 4)) << 4), -68 + lz);
+}
+
+// r^-3 and r^-2 of a close pair, in FP64
+__device__ __noinline__ double2 near_inverse(double x, double y, double z) {
+    const double r2 = fma(z, z, fma(y, y, x * x)), i = 1.0 / sqrt(r2);
+    return make_double2(i * i * i, i * i);
 }
 
 constexpr int NEAR_STAGE64 = 32;
 struct Stage64 {
-    double x[NEAR_STAGE64], y[NEAR_STAGE64], z[NEAR_STAGE64], q[NEAR_STAGE64];
+    long long x[NEAR_STAGE64], y[NEAR_STAGE64], z[NEAR_STAGE64];
+    double q[NEAR_STAGE64];
     int key[NEAR_STAGE64];
 };
-template <int K>
 struct Tgt64 {
-    double x[K], y[K], z[K], q[K];
-    int m[K], trow[K];
+    long long x, y, z;   // in the partner cell's frame
+    double q;            // charge * xpi
+    int m, trow;
 };
 
-// The pairs of one staged block (LJ and EXCL as in near_block32).
-template <int K, int LJ, bool EXCL>
-__device__ __forceinline__ void near_block64(const Tgt64<K> &t, const double (&qq)[K], const Stage64 &s, int n,
-                                             const double2 *ljt, double (&f)[K][3]) {
-    const long long rc2 = __double_as_longlong(RC * RC);   // positive doubles order as their bits
-#pragma unroll 2
+// One term of a pair: f += ft d
+__device__ __forceinline__ void near_sum64(double (&f)[3], double dx, double dy, double dz, double ft) {
+    f[0] = fma(dx, ft, f[0]); f[1] = fma(dy, ft, f[1]); f[2] = fma(dz, ft, f[2]);
+}
+// The LJ term of a pair within rc added to its Coulomb term (zero adds nothing)
+__device__ __forceinline__ double near_lj64(double ft, double2 p, bool in, double i3, double i2) {
+    const double i6 = i3 * i3;
+    return fma(((in ? p.x : 0.0) * i6) * fma(p.y, i6, -0.5), i2, ft);
+}
+
+// The pairs of one staged block.  LJ: 0 Coulomb of a run with one charge
+// (unscaled), 1 water-O partners with LJ, 2 any partners.  Partners of the
+// target's own molecule, and the target itself, are left out.
+template <int LJ>
+__device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const Stage64 &s, int n, const double2 *ljt,
+                                             double (&f)[3]) {
+    const u64 rc2 = (u64)(RC * RC * 72057594037927936.0);   // 2^56
+#pragma unroll 1
     for (int k = 0; k < n; k++) {
-        const double px = s.x[k], py = s.y[k], pz = s.z[k];
-        const int key = EXCL || LJ == 2 ? s.key[k] : 0;
-        double dx[K], dy[K], dz[K], r2[K];
-        bool out = false, same[K];
-#pragma unroll
-        for (int j = 0; j < K; j++) {
-            dx[j] = t.x[j] - px; dy[j] = t.y[j] - py; dz[j] = t.z[j] - pz;
-            r2[j] = fma(dz[j], dz[j], fma(dy[j], dy[j], dx[j] * dx[j]));
-            same[j] = EXCL && (key >> 5) == t.m[j];
-            out = out || !(same[j] || rinv_plain(r2[j]));
+        const long long x = t.x - s.x[k], y = t.y - s.y[k], z = t.z - s.z[k];
+        const int key = s.key[k];
+        const bool same = (key >> 5) == t.m;
+        const u64 r2 = fix_r2(x, y, z);
+        double i3, i2 = 0.0;
+        fix_inverse<LJ != 0>(r2, i3, i2);
+        const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
+        const bool close = r2 < FIX_NEAR2 && !same;
+        if (__any_sync(0xffffffffu, close)) {
+            if (close) {
+                const double2 v = near_inverse(dx, dy, dz);
+                i3 = v.x; i2 = v.y;
+            }
         }
-        Rinv64 v[K];
-#pragma unroll
-        for (int j = 0; j < K; j++) v[j] = rinv64(r2[j]);
-        if (__any_sync(0xffffffffu, out)) {
-#pragma unroll
-            for (int j = 0; j < K; j++)
-                if (!rinv_plain(r2[j])) v[j] = rinv64_any(r2[j]);
-        }
-        double ft[K];
-#pragma unroll
-        for (int j = 0; j < K; j++) ft[j] = same[j] ? 0.0 : v[j].i3;
+        double ft = same ? 0.0 : i3;
         if constexpr (LJ != 0) {
-            bool in[K], any = false;
-#pragma unroll
-            for (int j = 0; j < K; j++) {
-                in[j] = !same[j] && __double_as_longlong(r2[j]) <= rc2;
-                any = any || in[j];
-            }
-            any = __any_sync(0xffffffffu, any);
-#pragma unroll
-            for (int j = 0; j < K; j++) {
-                const double i3 = ft[j];
-                double c = qq[j];
-                if constexpr (LJ == 2) c *= s.q[k];
-                ft[j] = c * i3;
-                if (any) {   // a zero LJ term leaves the sum unchanged
-                    const double2 p = ljt[t.trow[j] + (LJ == 2 ? key & 31 : 0)];
-                    const double i6 = i3 * i3, i2 = fma(v[j].y2, fma(v[j].e, v[j].e, v[j].e), v[j].y2);
-                    ft[j] = fma(((in[j] ? p.x : 0.0) * i6) * fma(p.y, i6, -0.5), i2, ft[j]);
-                }
-            }
+            const bool in = !same && r2 <= rc2;
+            const double i = ft;
+            double c = qq;
+            if constexpr (LJ == 2) c *= s.q[k];
+            ft = c * i;
+            if (__any_sync(0xffffffffu, in)) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], in, i, i2);
         }
-#pragma unroll
-        for (int j = 0; j < K; j++) {
-            f[j][0] = fma(dx[j], ft[j], f[j][0]); f[j][1] = fma(dy[j], ft[j], f[j][1]); f[j][2] = fma(dz[j], ft[j], f[j][2]);
-        }
+        near_sum64(f, dx, dy, dz, ft);
     }
 }
 
-template <int K, int LJ, bool EXCL>
-__device__ __forceinline__ void near_run64(const Dev &d, const Tgt64<K> &t, int t0, int t1, const double2 *ljt,
-                                           double (&cell)[K][3], Stage64 &st, int lane) {
-    if (t0 >= t1) return;
-    double qq[K], f[K][3];
-    const double qr = d.srt_pos[t0].w;
-#pragma unroll
-    for (int j = 0; j < K; j++) { qq[j] = LJ == 2 ? t.q[j] : t.q[j] * qr; f[j][0] = f[j][1] = f[j][2] = 0.0; }
-    for (int b0 = t0; b0 < t1; b0 += NEAR_STAGE64) {
-        const int n = min(NEAR_STAGE64, t1 - b0);
-        __syncwarp();
-        if (lane < n) {
-            const double4 p = d.srt_pos[b0 + lane];
-            st.x[lane] = p.x; st.y[lane] = p.y; st.z[lane] = p.z;
-            if constexpr (LJ == 2) st.q[lane] = p.w;
-            if constexpr (EXCL || LJ == 2) st.key[lane] = d.srt_key[b0 + lane];
+// the same in FP64 throughout, from the FP64 positions: systems with a site
+// far from its cell (a state that is blowing up)
+template <int LJ>
+__device__ __noinline__ void near_run64_any(const Dev &d, double tx, double ty, double tz, const Tgt64 &t, double qq, int t0,
+                                            int t1, const double2 *ljt, double (&f)[3]) {
+    for (int k = t0; k < t1; k++) {
+        const double4 p = d.srt_pos[k];
+        const int key = d.srt_key[k];
+        const double dx = tx - p.x, dy = ty - p.y, dz = tz - p.z;
+        if ((key >> 5) == t.m) continue;
+        const double2 v = near_inverse(dx, dy, dz);
+        double ft = v.x;
+        if constexpr (LJ != 0) {
+            ft *= LJ == 2 ? qq * p.w : qq;
+            const bool in = fma(dz, dz, fma(dy, dy, dx * dx)) <= RC * RC;
+            if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], in, v.x, v.y);
         }
-        __syncwarp();
-        near_block64<K, LJ, EXCL>(t, qq, st, n, ljt, f);
+        near_sum64(f, dx, dy, dz, ft);
     }
-#pragma unroll
-    for (int j = 0; j < K; j++)
-#pragma unroll
-        for (int a = 0; a < 3; a++) cell[j][a] = LJ == 0 ? fma(qq[j], f[j][a], cell[j][a]) : cell[j][a] + f[j][a];
 }
 
-template <int K, bool PER>
-__device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, double *part, int c, int pr, int xo0,
-                                            int xo1, int first, int ni, int lane, Stage64 &st) {
+// One FP64 work item: the force of the partner cells xo0..xo1 of row pr on
+// the targets first..ni (at most 32), written to partial `part`.
+template <bool PER>
+__device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, double *part, int c, int pr, int xo0, int xo1,
+                                            int first, int ni, int lane, Stage64 &st) {
     const int dzc = pr / 3 - 1, dyc = pr % 3 - 1;
-    const int s0 = d.cstart[c];
-    const Rep &r = d.rep[d.crep[c]];
+    const int s0 = d.cstart[c], nslot = d.nsite, i = first + lane;
+    const int rep = d.crep[c];
+    const Rep &r = d.rep[rep];
     int ix, iy, iz;
     cell_xyz(r, c, ix, iy, iz);
     const int jy = iy + dyc, jz = iz + dzc, wy = PER ? wrap1(jy, r.nc[1]) : jy;
-    Tgt64<K> t;
-    double tx[K];
-    unsigned xm = 0;
-    const int rowsh = 3 * (dyc + 1) + 9 * (dzc + 1);
+    const bool far = d.near_far[rep] != 0;
     // a partner cell across a periodic face holds positions one box length
     // away, so the targets move by that length into its frame
     const double sy = (double)(jy - wy) * RS;
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-        const int i = first + lane + 32 * j;
-        tx[j] = t.y[j] = t.z[j] = 1e9;   // no site: far from every partner
-        t.q[j] = 0.0; t.m[j] = -2; t.trow[j] = NTYPE;
-        if (i < ni) {
-            const double4 p = d.srt_pos[s0 + i];
-            const int kk = d.srt_key[s0 + i];
-            tx[j] = p.x; t.y[j] = p.y - sy; t.z[j] = p.z; t.q[j] = p.w * XPI;
-            t.m[j] = kk >> 5; t.trow[j] = (kk & 31) * NTYPE;
-            xm |= ((unsigned)d.srt_xmask[s0 + i] >> rowsh) & 7u;
-        }
+    auto fixed = [](double v) { return __double2ll_rn(v * FIX_ONE); };
+    auto shift = [&](int a, int own, int cell, double box) {   // own cell's frame to the partner cell's
+        return (fixed(cell_centre(d, r, a, own)) - fixed(cell_centre(d, r, a, cell)) - fixed(box)) << 7;
+    };
+    const long long shy = shift(1, iy, wy, sy), shz = shift(2, iz, jz, 0.0);
+    Tgt64 t = {0, 5ll << 59, 0, 0.0, -2, NTYPE};   // no site: no molecule, water H (no LJ), clear of every partner
+    long long ox = 0;
+    if (i < ni) {
+        const long long *fp = d.srt_fix + s0 + i;
+        const int kk = d.srt_key[s0 + i];
+        ox = fp[0]; t.y = fp[nslot] + shy; t.z = fp[2 * (size_t)nslot] + shz;
+        t.q = d.srt_pos[s0 + i].w * XPI;
+        t.m = kk >> 5; t.trow = (kk & 31) * NTYPE;
     }
-    const unsigned excl = __reduce_or_sync(0xffffffffu, xm);
     const bool lj = first < d.cnh[c];
-    double row[K][3];
-#pragma unroll
-    for (int j = 0; j < K; j++) row[j][0] = row[j][1] = row[j][2] = 0.0;
+    const double qo = d.tq[0], qh = d.tq[1];
+    double row[3] = {0.0, 0.0, 0.0};
     for (int xo = xo0; xo <= xo1; xo++) {
         const int wx = PER ? wrap1(ix + xo, r.nc[0]) : ix + xo;
         const int cn = cell_index(r, wx, wy, jz);
-        const int t0 = d.cstart[cn], to = t0 + d.cno[cn], th = t0 + d.cnh[cn], t1 = d.cstart[cn + 1];
+        const int p0 = d.cstart[cn], po = p0 + d.cno[cn], ph = p0 + d.cnh[cn], p1 = d.cstart[cn + 1];
+        if (p0 == p1) continue;
         const double sx = (double)(ix + xo - wx) * RS;
-        double cell[K][3];
+        t.x = ox + shift(0, ix, wx, sx);
+        double cell[3] = {0.0, 0.0, 0.0};
+#pragma unroll 1
+        for (int g = 0; g < 3; g++) {   // water O, other LJ sites, water H
+            const int a = g == 0 ? p0 : g == 1 ? po : ph, b = g == 0 ? po : g == 1 ? ph : p1;
+            if (a == b) continue;
+            const bool one = g == 0 && lj;
+            const double qq = g == 1 ? t.q : t.q * (g ? qh : qo);
+            double f[3] = {0.0, 0.0, 0.0};
+            if (far) {
+                if (i < ni) {
+                    const double4 p = d.srt_pos[s0 + i];
+                    if (g == 1) near_run64_any<2>(d, p.x - sx, p.y - sy, p.z, t, qq, a, b, ljt, f);
+                    else if (one) near_run64_any<1>(d, p.x - sx, p.y - sy, p.z, t, qq, a, b, ljt, f);
+                    else near_run64_any<0>(d, p.x - sx, p.y - sy, p.z, t, qq, a, b, ljt, f);
+                }
+            } else {
+                for (int b0 = a; b0 < b; b0 += NEAR_STAGE64) {
+                    const int n = min(NEAR_STAGE64, b - b0);
+                    __syncwarp();
+                    if (lane < n) {
+                        const long long *fp = d.srt_fix + b0 + lane;
+                        st.x[lane] = fp[0]; st.y[lane] = fp[nslot]; st.z[lane] = fp[2 * (size_t)nslot];
+                        st.key[lane] = d.srt_key[b0 + lane];
+                        if (g == 1) st.q[lane] = d.srt_pos[b0 + lane].w;
+                    }
+                    __syncwarp();
+                    if (g == 1) near_block64<2>(t, qq, st, n, ljt, f);
+                    else if (one) near_block64<1>(t, qq, st, n, ljt, f);
+                    else near_block64<0>(t, qq, st, n, ljt, f);
+                }
+            }
 #pragma unroll
-        for (int j = 0; j < K; j++) { t.x[j] = tx[j] - sx; cell[j][0] = cell[j][1] = cell[j][2] = 0.0; }
-        const bool ex = (excl >> (xo + 1)) & 1u;
-        if (lj) near_run64<K, 1, true>(d, t, t0, to, ljt, cell, st, lane);
-        else if (ex) near_run64<K, 0, true>(d, t, t0, to, ljt, cell, st, lane);
-        else near_run64<K, 0, false>(d, t, t0, to, ljt, cell, st, lane);
-        near_run64<K, 2, true>(d, t, to, th, ljt, cell, st, lane);
-        if (ex) near_run64<K, 0, true>(d, t, th, t1, ljt, cell, st, lane);
-        else near_run64<K, 0, false>(d, t, th, t1, ljt, cell, st, lane);
-#pragma unroll
-        for (int j = 0; j < K; j++)
-#pragma unroll
-            for (int a = 0; a < 3; a++) row[j][a] += cell[j][a];
-    }
-#pragma unroll
-    for (int j = 0; j < K; j++) {
-        const int i = first + lane + 32 * j;
-        if (i < ni) {
-            double *o = part + 3 * (size_t)(s0 + i);
-            o[0] = row[j][0]; o[1] = row[j][1]; o[2] = row[j][2];
+            for (int k = 0; k < 3; k++) cell[k] = g == 1 || one ? cell[k] + f[k] : fma(qq, f[k], cell[k]);
         }
+#pragma unroll
+        for (int k = 0; k < 3; k++) row[k] += cell[k];
+    }
+    if (i < ni) {
+        double *o = part + 3 * (size_t)(s0 + i);
+        o[0] = row[0]; o[1] = row[1]; o[2] = row[2];
     }
 }
 
@@ -1079,8 +1142,9 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
 // A warp's first item is fixed: warp w of CTA b takes item w * grid + b.  All
 // CTAs wait together for the predecessor kernel, and taken from the counter
 // the first items went to the 20 to 32 warps of the SMs nearest to it: with
-// fewer items than warps the other SMs had none (3,000 sites in FP64: 3.2 ms,
-// 0.61 with the fixed first items, 0.32 with an item per cell as well).
+// fewer items than warps the other SMs had none (3,000 sites in FP64, with
+// 15 FP64 instructions a pair: 3.2 ms, 0.61 with the fixed first items, 0.32
+// with an item per cell as well).
 //
 // FP32, what bounds it: the FMA pipe and the registers that feed it.  A pair
 // of partners takes 11 paired instructions and two reciprocal square roots; a
@@ -1096,7 +1160,7 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
 // CTAs per SM: the FP32 loops want 110 to 146 registers, and one CTA more than
 // they leave room for spills into them (312,000 sites: 0.640 ms at 4 CTAs,
 // 0.736 at 5, 0.675 at 3; compensated, 41,600 sites: 0.164 ms at 3, 0.176 at
-// 4; FP64, 62,400 sites: 7.14 ms at 4, 7.25 at 5).
+// 4; FP64, 62,400 sites: 2.70 ms at 4, 3.00 at 3, 2.70 at 5, 2.76 at 6).
 constexpr int near_ctas(int mode) { return mode == 2 ? 3 : 4; }
 template <int MODE, bool PER>
 __global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, int nslot, int tile, int split) {
@@ -1143,8 +1207,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, i
                 if (e - first > 32) near_item32<2, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
                 else near_item32<1, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
             } else {
-                if (e - first > 32) near_item64<2, PER>(d, s_lj, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
-                else near_item64<1, PER>(d, s_lj, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
+                for (int f = first; f < e; f += 32) near_item64<PER>(d, s_lj, part, c, pr, xo0, xo1, f, min(f + 32, e), lane, s_stage[w]);
             }
         }
         k = __shfl_sync(0xffffffffu, next, 0);
@@ -1159,6 +1222,7 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms, int split)
     griddep_wait();
     typedef typename std::conditional<MIXED, float, double>::type R;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (!MIXED && s < d.nrep) d.near_far[s] = 0;   // for the next gather (fewer replicas than slots)
     if (s >= nslot || s >= d.cstart[ncell]) return;
     const int g = d.srt_site[s];
     const int c = d.sloc[g];

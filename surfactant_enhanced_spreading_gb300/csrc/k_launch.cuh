@@ -49,7 +49,9 @@ void upload_tables_force(const Tables &t, cudaStream_t st);
 void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st);
 // lists of the occupied boxes, and the packed multipoles cleared (with the cell lists, before launch_fma_build)
 void launch_far_lists(const Dev &d, int ncell, cudaStream_t st);
-void launch_gather(const Dev &d, int nslot, int ncell, int mixed, cudaStream_t st);
+// mode: the FP64 positions alone, or also what the context's pair field reads (its arrays exist by precision)
+constexpr int GATHER_FP64 = 0, GATHER_MIXED = 1, GATHER_PLAIN = 2;
+void launch_gather(const Dev &d, int nslot, int ncell, int mode, cudaStream_t st);
 // launch shape of the pair field (results do not depend on it)
 struct NearShape {
     int tile;   // target sites per work item: 32, 64 or (FP32 paths) 128

@@ -561,7 +561,7 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
         family(c, "water order");
         tstop(c, 5);
     }
-    launch_gather(d, c->nsite, c->ncell, mixed, c->st);
+    launch_gather(d, c->nsite, c->ncell, mixed ? GATHER_MIXED : GATHER_PLAIN, c->st);
     family(c, "gather");
     // graphite and intramolecular terms into the side forces (fside), on the
     // side stream beside the far-field build and the pair field on the mixed
@@ -708,7 +708,9 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&c->n_sm, cudaDevAttrMultiProcessorCount, dev);
         const int mixed = c->p.precision != SESP_PLAIN_FP64;
-        c->near.tile = 64;   // 128 (mixed paths) only where the autotuner measures it faster
+        // 128 (mixed paths) only where the autotuner measures it faster; the FP64
+        // items take 32 targets at a time anyway (3,000 sites: 231 us at 64, 157 at 32)
+        c->near.tile = c->p.precision == SESP_PLAIN_FP64 ? 32 : 64;
         c->near.grid = c->n_sm * near_resident_ctas(near_mode(c), c->chains);
         c->cshape.grid = c->n_sm;
     }
@@ -845,7 +847,8 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.ccount, C + 16 * (size_t)R + 3)) || (e = dalloc(c, &d.cfill, C)) || (e = dalloc(c, &d.sloc, N)) ||
         (e = dalloc(c, &d.sslot, N)) || (e = dalloc(c, &d.srt_site, N)) || (e = dalloc(c, &d.srt_pos, N)) ||
         (e = dalloc(c, &d.srt_pos32, N)) || (e = dalloc(c, &d.srt_meta, N)) || (e = dalloc(c, &d.srt_key, N)) ||
-        (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) ||
+        (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) || (e = dalloc(c, &d.srt_fix, c->p.precision == SESP_PLAIN_FP64 ? 3 * (size_t)N : 1)) ||
+        (e = dalloc(c, &d.near_far, R)) ||
         (e = dalloc(c, &d.pair_xyz, 3 * pair_max)) || (e = dalloc(c, &d.pair_key, pair_max)) || (e = dalloc(c, &d.crun, 8 * (size_t)C)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
         (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
         (e = dalloc(c, &d.near_items_tmp, near_items_max(N, C))) || (e = dalloc(c, &d.near_cls, near_items_max(N, C))) ||
@@ -1684,7 +1687,7 @@ int sesp_pair_counts(sesp_ctx *c, int64_t out[2]) {
     unsigned long long *dc = nullptr, h[2] = {0, 0};
     CK(cudaMalloc(&dc, sizeof h));
     cudaMemsetAsync(dc, 0, sizeof h, c->st);
-    launch_gather(c->d, c->nsite, c->ncell, 0, c->st);
+    launch_gather(c->d, c->nsite, c->ncell, GATHER_FP64, c->st);
     launch_count_pairs(c->d, c->ncell, dc, c->st);
     cudaMemcpyAsync(h, dc, sizeof h, cudaMemcpyDeviceToHost, c->st);
     cudaError_t err = cudaStreamSynchronize(c->st);
@@ -1788,7 +1791,7 @@ int sesp_energies(sesp_ctx *c, double out[8]) {
     std::vector<double> hs(3 * (size_t)N), hi(3 * (size_t)N), hm(3 * (size_t)(c->nsm + 1));
     err = cudaMemsetAsync(es, 0, 3 * sizeof(double) * N, c->st);
     if (err == cudaSuccess) {
-        launch_gather(c->d, c->nsite, c->ncell, 0, c->st);
+        launch_gather(c->d, c->nsite, c->ncell, GATHER_FP64, c->st);
         launch_energies(c->d, c->ncell, N, c->smols, c->nsm, c->chains, es, ei, em, c->st);
         err = cudaGetLastError();
     }
@@ -1894,7 +1897,7 @@ int sesp_energies_static(sesp_ctx *c, double out[8]) {
     double *tot = em + 3 * ((size_t)SESP_NOALLOC_MAX_SURF + 1);
     cudaError_t err = cudaMemsetAsync(es, 0, 3 * sizeof(double) * N, c->st);
     if (err == cudaSuccess) {
-        launch_gather(c->d, c->nsite, c->ncell, 0, c->st);
+        launch_gather(c->d, c->nsite, c->ncell, GATHER_FP64, c->st);
         launch_energies(c->d, c->ncell, N, c->smols, c->nsm, c->chains, es, ei, em, c->st);
         k_energy_totals<<<1, 32, 0, c->st>>>(es, ei, em, N, c->nsm, tot);
         err = cudaGetLastError();

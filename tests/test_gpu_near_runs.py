@@ -77,3 +77,36 @@ def test_cells_and_rows_give_the_same_bits(precision):
     assert batch.n > 40000 > small.n_sites
     fb = batch.force(True)
     assert np.array_equal(fb[:small.n_sites], E.Engine(small, precision).force(True))
+
+
+@pytest.mark.parametrize("precision,bar", [(E.PLAIN_FP64, 1e-10), (E.MIXED, 1e-5)])
+@pytest.mark.parametrize("drift", [0.5, 0.79, 0.81, 1.7, 40.0])
+def test_sites_that_leave_their_cells(drift, precision, bar):
+    """Frozen lists with every third molecule moved `drift` sigma along x: the
+    FP64 path's fixed-point coordinates reach 0.8 sigma past a cell's faces,
+    and a replica with a site beyond runs in FP64.  40 sigma stands for a
+    state that blows up."""
+    s = C.config_droplet(240, 4, cells=(8, 8, 8), seed=12)
+    pos = s.pos.copy()
+    pos[:3 * s.n_water].reshape(-1, 9)[::3, ::3] += drift
+    o, eng = O.Oracle(s), E.Engine(s, precision)
+    o.force(True, terms=E.T_NEAR)
+    eng.force(True, terms=E.T_NEAR)
+    o.set(0, pos)
+    eng.set_state(pos)
+    fo = o.force(False, terms=E.T_NEAR)
+    assert rel(eng.force(False, terms=E.T_NEAR), fo) < bar
+
+
+@pytest.mark.parametrize("r", [0.3, 0.35, 0.36, 0.5, 1.0, 2.0, 4.0, 5.25])
+def test_plain_pair_at_exact_distances(r):
+    """Two waters whose oxygens are r sigma apart along an axis: powers of two,
+    where the scaled distance of the FP64 path's integers meets the ends of
+    its range, and both sides of the distance below which it uses FP64."""
+    s = grid_waters(2, 3.0, seed=1)
+    wt = S.water_template() / S.SIGMA
+    pos = np.concatenate([wt, -wt]) + 0.25
+    pos[3:, 0] += r
+    s = dataclasses.replace(s, pos=pos)
+    fo = O.Oracle(s).force(True, terms=E.T_NEAR)
+    assert rel(E.Engine(s, E.PLAIN_FP64).force(True, terms=E.T_NEAR), fo) < 1e-13
