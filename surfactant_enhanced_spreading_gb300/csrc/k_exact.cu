@@ -70,6 +70,13 @@ __device__ inline int central_cell(const Dev &d, const Rep &r, int g) {
     return (ix < 0 || iy < 0 || iz < 0) ? -1 : cell_index(r, ix, iy, iz);
 }
 
+// the packed multipoles cleared for the coming far-field build (all threads of the launch)
+__device__ inline void clear_packed(const Dev &d) {
+    uint4 *p = (uint4 *)d.pk4;
+    for (size_t k = blockIdx.x * blockDim.x + threadIdx.x; k < d.pk_bytes / 16; k += (size_t)gridDim.x * blockDim.x)
+        p[k] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 // Re-key molecules (src/read_config.f90:44-175 and the delete/add pairs
 // src/delete_w1.f90:54-195, src/delete_s.f90:33-43; key site O for water,
 // 14 for surfactants) and locate every site in the cell it is Central in.
@@ -78,6 +85,7 @@ __device__ inline int central_cell(const Dev &d, const Rep &r, int g) {
 // Threads [0, nmol) take one molecule each (a water with its sites);
 // threads [nmol, nmol + nss) one surfactant site each.
 __global__ void k_locate(Dev d, int nmol, const int *smols, int nss) {
+    clear_packed(d);
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= nmol) {
         if (t - nmol >= nss) return;
@@ -716,6 +724,7 @@ __device__ inline int floor_div(int a, int b) { const int q = a / b; return (a %
 // molecules stay whole); a site outside the z range is in no cell.  The
 // molecule's key is the cell of its first site.
 __global__ void k_locate_cfg(Dev d, int nsite) {
+    clear_packed(d);
     const int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nsite) return;
     const int m = d.smol[g];

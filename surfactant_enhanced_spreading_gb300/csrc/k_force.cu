@@ -63,23 +63,91 @@ __device__ inline int block_exscan(int v, int *total) {
 // groups of four that hold n sites in up to five padded runs
 __host__ __device__ inline int pair_groups(int n) { return n > 0 ? (n + 15) >> 2 : 0; }
 
-// first slot of every cell, and the first group of its pair layout
-__global__ void k_scan(Dev d, int ncell) {
-    int per = (ncell + blockDim.x - 1) / blockDim.x;
-    int b = threadIdx.x * per, e = min(ncell, b + per);
-    int s = 0, q = 0;
-    for (int c = b; c < e; c++) { const int n = d.ccount[c]; s += n; q += pair_groups(n); }
-    int total, qtotal;
-    int acc = block_exscan(s, &total), qacc = block_exscan(q, &qtotal);
-    if (threadIdx.x == 0) d.cstart[ncell] = total;
-    for (int c = b; c < e; c++) {
-        const int n = d.ccount[c];
-        d.cstart[c] = acc; acc += n; d.cfill[c] = 0;
-        d.crun[8 * (size_t)c] = qacc; qacc += pair_groups(n);
+// A droplet occupies a ninth of the cells of its box (2,900 of 25,600 on the
+// 312,000-site configuration), so the cell sort, the work items and every
+// pass of the far field run over lists of the occupied boxes, rebuilt with
+// the cell lists: expansions of the others are neither formed nor read.  The
+// order of a list depends on timing and decides only which CTA takes which
+// box.  Far-field build, all boxes against occupied ones: 0.59 -> 0.15 ms
+// (312,000 sites), 0.83 -> 0.20 ms (eight replicas, 247,000 sites), FP64 1.68
+// -> 0.42 ms (62,400 sites).
+// fm_cnt: per replica, level (4, 3) and parity class the targets in fm_list;
+// then the occupied L4, L3 and L2 boxes in occ4, occ3 and occ2.
+__device__ __forceinline__ int *occ_counts(const Dev &d) { return d.fm_cnt + 16 * d.nrep; }
+// first list entry of a parity class: level 4's cells, then level 3's boxes
+__device__ __forceinline__ int class_list(const Rep &r, int level, int cls, int ncell) {
+    const int n = r.nc[0] * r.nc[1] * r.nc[2];
+    return level == 4 ? r.cell0 + cls * (n / 8) : ncell + r.l3_0 + cls * (n / 64);
+}
+
+// cell c's entries in the lists of occupied boxes (and those of the L3 and L2
+// boxes it is the corner of)
+__device__ inline void occupied_boxes(const Dev &d, int c, int ncell) {
+    const int q = d.crep[c];
+    const Rep &r = d.rep[q];
+    int x, y, z;
+    cell_xyz(r, c, x, y, z);
+    int *occ = occ_counts(d);
+    auto target = [&](int level, int bx, int by, int bz) {
+        const int div = level == 4 ? 2 : 4, cls = (bx & 1) + 2 * (by & 1) + 4 * (bz & 1);
+        const int k = atomicAdd(&d.fm_cnt[16 * q + (level == 4 ? 0 : 8) + cls], 1);
+        d.fm_list[class_list(r, level, cls, ncell) + k] =
+            (bx >> 1) + r.nc[0] / div * ((by >> 1) + r.nc[1] / div * (bz >> 1));
+    };
+    auto sites = [&](int w) {   // whether the w^3 cells from c hold a site
+        int n = 0;
+        for (int k = 0; k < w; k++)
+            for (int j = 0; j < w; j++)
+                for (int i = 0; i < w; i++) n |= d.ccount[c + i + r.nc[0] * (j + r.nc[1] * k)];
+        return n > 0;
+    };
+    if (d.ccount[c] > 0) {
+        d.occ4[atomicAdd(&occ[0], 1)] = c;
+        target(4, x, y, z);
     }
+    if ((x | y | z) & 1) return;
+    const int b3 = r.l3_0 + x / 2 + r.nc[0] / 2 * (y / 2 + r.nc[1] / 2 * (z / 2));
+    const bool o3 = sites(2);
+    d.has3[b3] = o3;
+    if (o3) {
+        d.occ3[atomicAdd(&occ[1], 1)] = b3;
+        target(3, x / 2, y / 2, z / 2);
+    }
+    if ((x | y | z) & 3) return;
+    const int b2 = r.l2_0 + x / 4 + r.nr[0] * (y / 4 + r.nr[1] * (z / 4));
+    const bool o2 = sites(4);
+    d.has2[b2] = o2;
+    if (o2) d.occ2[atomicAdd(&occ[2], 1)] = b2;
+}
+
+// First slot of every cell, the first group of its pair layout, and the lists
+// of occupied boxes.  A CTA takes 1,024 cells and adds up the counts before
+// them itself (coalesced; nothing waits on another CTA).  One CTA scanning all
+// cells in strided runs took 49 us on 25,600 cells.
+constexpr int SCAN_CELLS = 1024;
+__global__ void __launch_bounds__(SCAN_CELLS) k_scan(Dev d, int ncell) {
+    griddep_wait();
+    const int c0 = blockIdx.x * SCAN_CELLS, c = c0 + threadIdx.x;
+    int s = 0, q = 0;
+    for (int k = threadIdx.x; k < c0; k += SCAN_CELLS) { const int n = d.ccount[k]; s += n; q += pair_groups(n); }
+    int sites0, groups0, t;
+    block_exscan(s, &sites0);
+    block_exscan(q, &groups0);
+    const int n = c < ncell ? d.ccount[c] : 0;
+    const int slot = sites0 + block_exscan(n, &t), group = groups0 + block_exscan(pair_groups(n), &t);
+    if (c >= ncell) return;
+    d.cstart[c] = slot;
+    if (c == ncell - 1) d.cstart[ncell] = slot + n;
+    d.cfill[c] = 0;
+    int *run = d.crun + 8 * (size_t)c;
+    *(int4 *)run = make_int4(group, 0, 0, 0);   // the runs of an empty cell; the sort writes the others'
+    *(int4 *)(run + 4) = make_int4(0, 0, 0, 0);
+    if (n == 0) d.cnh[c] = d.cno[c] = 0;
+    occupied_boxes(d, c, ncell);
 }
 
 __global__ void k_scatter(Dev d, int nsite) {
+    griddep_wait();
     int g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= nsite) return;
     int c = d.sloc[g];
@@ -124,18 +192,17 @@ __device__ int molecule_cells(const Dev &d, int c, int v) {
 // before the others in theirs, so that a neighbour cell's same-molecule test
 // is needed in a run's second part only (a fifth of its sites).  The FP32
 // paths' pair layout holds the same order with every run padded to fours.
-__global__ void k_sort_cells(Dev d) {
+__global__ void __launch_bounds__(256) k_sort_cells(Dev d) {
+    griddep_wait();
     __shared__ unsigned buf[SORT_CAP];
     __shared__ int xm[SORT_CAP];
     __shared__ int cnt[5];
-    int c = blockIdx.x;
-    int s0 = d.cstart[c], n = d.cstart[c + 1] - s0;
+    const int nocc = occ_counts(d)[0];
+    for (int ci = blockIdx.x; ci < nocc; ci += gridDim.x) {
+    const int c = d.occ4[ci];
+    const int s0 = d.cstart[c], n = d.cstart[c + 1] - s0;
     int *run = d.crun + 8 * (size_t)c;
-    if (n == 0) {
-        if (threadIdx.x < 5) run[1 + threadIdx.x] = 0;
-        if (threadIdx.x == 0) d.cnh[c] = d.cno[c] = 0;
-        return;
-    }
+    __syncthreads();   // the previous cell is done with the shared arrays
     if (threadIdx.x < 5) cnt[threadIdx.x] = 0;
     if (threadIdx.x == 0) atomicMax(&d.counters[3], (unsigned long long)n);
     __syncthreads();
@@ -149,6 +216,7 @@ __global__ void k_sort_cells(Dev d) {
         d.srt_key[s0 + slot] = key;
         d.srt_xmask[s0 + slot] = mask;
         d.srt_pair[s0 + slot] = 4 * run[0] + pair;
+        d.srt_cell[s0 + slot] = c;
         keys[pair] = key;
     };
     auto pad = [&](int pair) {   // no molecule, kind 0, far away
@@ -168,7 +236,7 @@ __global__ void k_sort_cells(Dev d) {
             run[1] = run[2] = 0;
             run[3] = run[4] = run[5] = (n + 3) >> 2;
         }
-        return;
+        continue;
     }
     for (int t = threadIdx.x; t < n; t += blockDim.x) {
         const int v = d.srt_site[s0 + t], ty = d.ptype[v], mask = molecule_cells(d, c, v);
@@ -200,19 +268,13 @@ __global__ void k_sort_cells(Dev d) {
             if (cls == a) { f = first[a]; q = quad[a]; }
         place(rank, (int)(k & ((1u << SORT_SHIFT) - 1)), xm[t], 4 * q + rank - f);
     }
+    }
 }
 
 void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st) {
-    k_scan<<<1, 1024, 0, st>>>(d, ncell);
-    k_scatter<<<(nsite + 255) / 256, 256, 0, st>>>(d, nsite);
-    k_sort_cells<<<ncell, 256, 0, st>>>(d);
-}
-
-// the occupied boxes of the far field (its counts are cleared with the cell counts)
-__global__ void k_far_lists(Dev d, int ncell);
-void launch_far_lists(const Dev &d, int ncell, cudaStream_t st) {
-    cudaMemsetAsync(d.pk4, 0, d.pk_bytes, st);   // class-packed multipoles of both levels
-    k_far_lists<<<(ncell + 127) / 128, 128, 0, st>>>(d, ncell);
+    launch_pdl(k_scan, dim3((ncell + SCAN_CELLS - 1) / SCAN_CELLS), dim3(SCAN_CELLS), 0, st, d, ncell);
+    launch_pdl(k_scatter, dim3((nsite + 255) / 256 > 0 ? (nsite + 255) / 256 : 1), dim3(256), 0, st, d, nsite);
+    launch_pdl(k_sort_cells, dim3(min(ncell, 152 * 8)), dim3(256), 0, st, d);
 }
 
 // ------------------------------------------------------------------ gather
@@ -236,9 +298,9 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mode) {
     if (s == 0) d.near_ctl[0] = 0;   // the pair field's work counter
     if (s >= nslot || s >= d.cstart[ncell]) return;
     int g = d.srt_site[s];
+    const int c = d.srt_cell[s];
     double x = d.x[g], y = d.y[g], z = d.z[g];
     double q = d.tq[d.ptype[g]];
-    const int c = d.sloc[g];
     const Rep &rr = d.rep[d.crep[c]];
     if (rr.per) {
         const short2 im = d.simg[g];
@@ -429,114 +491,84 @@ __device__ __forceinline__ void row_x(const Rep &r, int ix, int &jx0, int &jx1) 
     else { jx0 = ix > 0 ? ix - 1 : 0; jx1 = ix + 1 < r.nc[0] ? ix + 1 : r.nc[0] - 1; }
 }
 
-__global__ void k_near_items_count(Dev d, int ncell, int tile) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    const int ni = d.cstart[c + 1] - d.cstart[c];
-    int n = 0;
-    if (ni > 0) {
-        const Rep r = d.rep[d.crep[c]];
-        int ix, iy, iz;
-        cell_xyz(r, c, ix, iy, iz);
-        int jx0, jx1;
-        row_x(r, ix, jx0, jx1);
-        n = __popc(near_row_mask(r, iy, iz)) * near_chunks(d.cnh[c], ni, tile) * (d.near_split ? jx1 - jx0 + 1 : 1);
-    }
-    d.near_icount[c] = n;
-}
-
-// exclusive scan of the item counts in place (one block), total to near_ctl[1]
-__global__ void k_near_items_scan(Dev d, int ncell) {
-    const int per = (ncell + blockDim.x - 1) / blockDim.x;
-    const int b = threadIdx.x * per, e = min(ncell, b + per);
-    int s = 0;
-    for (int c = b; c < e; c++) s += d.near_icount[c];
-    int total;
-    int acc = block_exscan(s, &total);
-    if (threadIdx.x == 0) d.near_ctl[1] = total;
-    for (int c = b; c < e; c++) { int v = d.near_icount[c]; d.near_icount[c] = acc; acc += v; }
-}
-
-// the work items of one cell, counted per cost class in the block's histogram
-__device__ inline void near_items_fill_cell(const Dev &d, int c, int ni, int tile, int *hist) {
-    const Rep r = d.rep[d.crep[c]];
+// The work items of one cell by its warp, lane p its part p (a row, or with
+// near_split a cell): emit(cost class, item) for every chunk of a part with
+// partners; near_mask gets the parts that have any.  The cost class is
+// floor(log2(targets x partners)).
+template <typename F>
+__device__ __forceinline__ void near_cell_items(const Dev &d, int c, int tile, bool mask, F emit) {
+    const int lane = threadIdx.x & 31;
+    const Rep &r = d.rep[d.crep[c]];
     int ix, iy, iz;
     cell_xyz(r, c, ix, iy, iz);
-    const int mask = near_row_mask(r, iy, iz);
-    const int nh = d.cnh[c], nch = near_chunks(nh, ni, tile);
-    int jx0, jx1;
-    row_x(r, ix, jx0, jx1);
-    int k = d.near_icount[c];
-    const int step = d.near_split ? 1 : jx1 - jx0 + 1;   // cells of an item
-    for (int pr = 0; pr < 9; pr++) {
-        if (!(mask >> pr & 1)) continue;
-        for (int x0 = jx0; x0 <= jx1; x0 += step) {
-            int npart = 0;
-            for (int jx = x0; jx < x0 + step; jx++) {
-                const int cn = shell_cell(r, jx, iy + pr % 3 - 1, iz + pr / 3 - 1);
-                npart += d.cstart[cn + 1] - d.cstart[cn];
-            }
-            const int p = d.near_split ? 3 * pr + x0 - ix + 1 : pr;
-            for (int ch = 0; ch < nch; ch++) {
-                int tb, te;
-                near_chunk(nh, ni, tile, ch, tb, te);
-                const int cls = 31 - __clz((te - tb) * npart + 1);
-                d.near_items_tmp[k] = make_int2(c, p << 24 | ch);
-                d.near_cls[k] = cls;
-                atomicAdd(&hist[cls], 1);
-                k++;
-            }
+    int x0, x1;
+    row_x(r, ix, x0, x1);
+    const int pr = d.near_split ? lane / 3 : lane;
+    if (d.near_split) {
+        const int jx = ix + lane % 3 - 1;
+        x0 = max(x0, jx); x1 = min(x1, jx);
+    }
+    int npart = 0;
+    if (pr < 9 && (near_row_mask(r, iy, iz) >> pr & 1))
+        for (int jx = x0; jx <= x1; jx++) {
+            const int cn = shell_cell(r, jx, iy + pr % 3 - 1, iz + pr / 3 - 1);
+            npart += d.cstart[cn + 1] - d.cstart[cn];
         }
+    if (mask) {
+        const unsigned m = __ballot_sync(0xffffffffu, npart > 0);
+        if (lane == 0) d.near_mask[c] = (int)m;
+    }
+    if (npart == 0) return;
+    const int ni = d.cstart[c + 1] - d.cstart[c], nh = d.cnh[c], nch = near_chunks(nh, ni, tile);
+    for (int ch = 0; ch < nch; ch++) {
+        int tb, te;
+        near_chunk(nh, ni, tile, ch, tb, te);
+        emit(31 - __clz((te - tb) * npart + 1), make_int2(c, lane << 24 | ch));
     }
 }
 
-// Items in cell order into near_items_tmp, each with a cost class:
-// floor(log2(targets x partners in its row)).
-__global__ void k_near_items_fill(Dev d, int ncell, int tile) {
-    __shared__ int hist[32];   // the block's items per class, added to the global counts once
+// items per cost class
+__global__ void __launch_bounds__(256) k_near_items_count(Dev d, int tile) {
+    griddep_wait();
+    __shared__ int hist[32];
     if (threadIdx.x < 32) hist[threadIdx.x] = 0;
     __syncthreads();
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    const int ni = c < ncell ? d.cstart[c + 1] - d.cstart[c] : 0;
-    if (ni > 0) near_items_fill_cell(d, c, ni, tile, hist);
+    const int nocc = occ_counts(d)[0], nw = blockDim.x >> 5;
+    for (int ci = blockIdx.x * nw + (threadIdx.x >> 5); ci < nocc; ci += gridDim.x * nw)
+        near_cell_items(d, d.occ4[ci], tile, true, [&](int cls, int2) { atomicAdd(&hist[cls], 1); });
     __syncthreads();
     if (threadIdx.x < 32 && hist[threadIdx.x]) atomicAdd(&d.near_ctl[2 + threadIdx.x], hist[threadIdx.x]);
 }
 
-// start of each cost class in the final order, most expensive class first
-__global__ void k_near_items_classes(Dev d) {
-    if (threadIdx.x != 0) return;
-    int *bcount = d.near_ctl + 2, *bnext = d.near_ctl + 34;
-    int acc = 0;
-    for (int b = 31; b >= 0; b--) { bnext[b] = acc; acc += bcount[b]; }
-}
-
-// Items into near_items by class.  Within a class the order depends on
-// thread timing; it only decides which warp takes which item first, and every
-// item's arithmetic is the same whatever its position.
-__global__ void k_near_items_place(Dev d) {
-    __shared__ int cnt[32], base[32];   // the block's items per class and their reserved range
+// Items into near_items, most expensive class first.  Within a class the
+// order depends on thread timing; it only decides which warp takes which item
+// first, and every item's arithmetic is the same whatever its position.
+__global__ void __launch_bounds__(256) k_near_items_place(Dev d, int tile) {
+    griddep_wait();
+    __shared__ int cnt[32], next[32];   // the CTA's items per class; the next place of each
     if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
     __syncthreads();
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    int cls = -1, rank = 0;
-    if (k < d.near_ctl[1]) {
-        cls = d.near_cls[k];
-        rank = atomicAdd(&cnt[cls], 1);
+    const int nocc = occ_counts(d)[0], nw = blockDim.x >> 5, first = blockIdx.x * nw + (threadIdx.x >> 5);
+    for (int ci = first; ci < nocc; ci += gridDim.x * nw)
+        near_cell_items(d, d.occ4[ci], tile, false, [&](int cls, int2) { atomicAdd(&cnt[cls], 1); });
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        int start = 0;   // items of the more expensive classes
+        for (int b = threadIdx.x + 1; b < 32; b++) start += d.near_ctl[2 + b];
+        next[threadIdx.x] = cnt[threadIdx.x] ? start + atomicAdd(&d.near_ctl[34 + threadIdx.x], cnt[threadIdx.x]) : 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) d.near_ctl[1] = start + d.near_ctl[2];
     }
     __syncthreads();
-    if (threadIdx.x < 32 && cnt[threadIdx.x]) base[threadIdx.x] = atomicAdd(&d.near_ctl[34 + threadIdx.x], cnt[threadIdx.x]);
-    __syncthreads();
-    if (cls >= 0) d.near_items[base[cls] + rank] = d.near_items_tmp[k];
+    for (int ci = first; ci < nocc; ci += gridDim.x * nw)
+        near_cell_items(d, d.occ4[ci], tile, false, [&](int cls, int2 item) { d.near_items[atomicAdd(&next[cls], 1)] = item; });
 }
 
-void launch_near_items(const Dev &d, int ncell, int nitems_max, int tile, cudaStream_t st) {
+// (the lists of the last rebuild must be in place)
+void launch_near_items(const Dev &d, int ncell, int tile, cudaStream_t st) {
     cudaMemsetAsync(d.near_ctl + 2, 0, 64 * sizeof(int), st);
-    k_near_items_count<<<(ncell + 255) / 256, 256, 0, st>>>(d, ncell, tile);
-    k_near_items_scan<<<1, 1024, 0, st>>>(d, ncell);
-    k_near_items_fill<<<(ncell + 255) / 256, 256, 0, st>>>(d, ncell, tile);
-    k_near_items_classes<<<1, 32, 0, st>>>(d);
-    k_near_items_place<<<(nitems_max + 255) / 256, 256, 0, st>>>(d);
+    const dim3 g(min((ncell + 7) / 8, 152 * 4)), b(256);
+    k_near_items_count<<<g, b, 0, st>>>(d, tile);
+    launch_pdl(k_near_items_place, g, b, 0, st, d, tile);
 }
 
 // One partner's force on a target site (src/evalw1w1n.f90:86-104 form):
@@ -1224,11 +1256,7 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms, int split)
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (!MIXED && s < d.nrep) d.near_far[s] = 0;   // for the next gather (fewer replicas than slots)
     if (s >= nslot || s >= d.cstart[ncell]) return;
-    const int g = d.srt_site[s];
-    const int c = d.sloc[g];
-    const Rep r = d.rep[d.crep[c]];
-    int ix, iy, iz;
-    cell_xyz(r, c, ix, iy, iz);
+    const int c = d.srt_cell[s];
     // FP32 partials summed in FP32 on the mixed path (one conversion to FP64
     // per component), FP64 on the plain path (COMP: compensated FP32 sums, as
     // in the pair field)
@@ -1238,26 +1266,29 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms, int split)
         else sum += v;
     };
     if (terms & SESP_T_NEAR) {
-        const int mask = near_row_mask(r, iy, iz);
+        // the parts (rows, or cells of rows) with partners; no item wrote the others
+        const int mask = d.near_mask[c];
         const R *part = (const R *)d.near_part + 3 * (size_t)s;
         const size_t stride = 3 * (size_t)nslot;
-        int x0, x1;
-        row_x(r, ix, x0, x1);
-        for (int pr = 0; pr < 9; pr++) {
-            if (!(mask >> pr & 1)) continue;
-            R v[3];
-            if (split) {
+        if (split) {
+            for (int pr = 0; pr < 9; pr++) {
+                if (!(mask >> (3 * pr) & 7)) continue;
                 R rs[3] = {0, 0, 0}, re[3] = {0, 0, 0};
-                for (int xo = x0 - ix; xo <= x1 - ix; xo++) {
-                    const R *p = part + (size_t)(3 * pr + xo + 1) * stride;
-                    for (int a = 0; a < 3; a++) add(rs[a], re[a], p[a]);
-                }
-                for (int a = 0; a < 3; a++) v[a] = rs[a] - re[a];
-            } else {
-                const R *p = part + (size_t)pr * stride;
-                for (int a = 0; a < 3; a++) v[a] = p[a];
+#pragma unroll
+                for (int xo = 0; xo < 3; xo++)
+                    if (mask >> (3 * pr + xo) & 1) {
+                        const R *p = part + (size_t)(3 * pr + xo) * stride;
+                        for (int a = 0; a < 3; a++) add(rs[a], re[a], p[a]);
+                    }
+                for (int a = 0; a < 3; a++) add(fs[a], es[a], rs[a] - re[a]);
             }
-            for (int a = 0; a < 3; a++) add(fs[a], es[a], v[a]);
+        } else {
+#pragma unroll
+            for (int pr = 0; pr < 9; pr++)
+                if (mask >> pr & 1) {
+                    const R *p = part + (size_t)pr * stride;
+                    for (int a = 0; a < 3; a++) add(fs[a], es[a], p[a]);
+                }
         }
     }
     R fx = fs[0] - es[0], fy = fs[1] - es[1], fz = fs[2] - es[2];
@@ -1271,6 +1302,9 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms, int split)
             const float4 p = d.srt_pos32[s];
             x = p.x; y = p.y; z = p.z; q = p.w * (float)XPI;
         } else {
+            const Rep &r = d.rep[d.crep[c]];
+            int ix, iy, iz;
+            cell_xyz(r, c, ix, iy, iz);
             const double4 pd = d.srt_pos[s];
             x = pd.x - cell_centre(d, r, 0, ix); y = pd.y - cell_centre(d, r, 1, iy); z = pd.z - cell_centre(d, r, 2, iz);
             q = pd.w * XPI;
@@ -1315,64 +1349,6 @@ void launch_near(const Dev &d, int ncell, int nslot, int mode, int terms, const 
 }
 
 // ------------------------------------------------------------------ multipoles
-
-// A droplet occupies a ninth of the cells of its box (2,900 of 25,600 on the
-// 312,000-site configuration), so every pass of the far field runs over lists
-// of the occupied boxes, rebuilt with the cell lists: expansions of the others
-// are neither formed nor read.  The order of a list depends on timing and
-// decides only which CTA takes which box.  Far-field build, all boxes against
-// occupied ones: 0.59 -> 0.15 ms (312,000 sites), 0.83 -> 0.20 ms (eight
-// replicas, 247,000 sites), FP64 1.68 -> 0.42 ms (62,400 sites).
-// fm_cnt: per replica, level (4, 3) and parity class the targets in fm_list;
-// then the occupied L4, L3 and L2 boxes in occ4, occ3 and occ2.
-__device__ __forceinline__ int *occ_counts(const Dev &d) { return d.fm_cnt + 16 * d.nrep; }
-// first list entry of a parity class: level 4's cells, then level 3's boxes
-__device__ __forceinline__ int class_list(const Rep &r, int level, int cls, int ncell) {
-    const int n = r.nc[0] * r.nc[1] * r.nc[2];
-    return level == 4 ? r.cell0 + cls * (n / 8) : ncell + r.l3_0 + cls * (n / 64);
-}
-
-__global__ void k_far_lists(Dev d, int ncell) {
-    const int c = blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= ncell) return;
-    const int q = d.crep[c];
-    const Rep &r = d.rep[q];
-    int x, y, z;
-    cell_xyz(r, c, x, y, z);
-    int *occ = occ_counts(d);
-    auto target = [&](int level, int bx, int by, int bz) {
-        const int div = level == 4 ? 2 : 4, cls = (bx & 1) + 2 * (by & 1) + 4 * (bz & 1);
-        const int k = atomicAdd(&d.fm_cnt[16 * q + (level == 4 ? 0 : 8) + cls], 1);
-        d.fm_list[class_list(r, level, cls, ncell) + k] =
-            (bx >> 1) + r.nc[0] / div * ((by >> 1) + r.nc[1] / div * (bz >> 1));
-    };
-    auto sites = [&](int w) {   // sites in the w^3 cells from c (rows along x are contiguous slots)
-        int n = 0;
-        for (int k = 0; k < w; k++)
-            for (int j = 0; j < w; j++) {
-                const int s = c + r.nc[0] * (j + r.nc[1] * k);
-                n += d.cstart[s + w] - d.cstart[s];
-            }
-        return n;
-    };
-    if (d.cstart[c + 1] > d.cstart[c]) {
-        d.occ4[atomicAdd(&occ[0], 1)] = c;
-        target(4, x, y, z);
-    }
-    if ((x | y | z) & 1) return;
-    const int b3 = r.l3_0 + x / 2 + r.nc[0] / 2 * (y / 2 + r.nc[1] / 2 * (z / 2));
-    const bool o3 = sites(2) > 0;
-    d.has3[b3] = o3;
-    if (o3) {
-        d.occ3[atomicAdd(&occ[1], 1)] = b3;
-        target(3, x / 2, y / 2, z / 2);
-    }
-    if ((x | y | z) & 3) return;
-    const int b2 = r.l2_0 + x / 4 + r.nr[0] * (y / 4 + r.nr[1] * (z / 4));
-    const bool o2 = sites(4) > 0;
-    d.has2[b2] = o2;
-    if (o2) d.occ2[atomicAdd(&occ[2], 1)] = b2;
-}
 
 template <typename R>
 struct C2 {

@@ -47,8 +47,6 @@ void init_constraint_kernels();   // shared-memory limits of the constraint laun
 // k_force.cu
 void upload_tables_force(const Tables &t, cudaStream_t st);
 void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st);
-// lists of the occupied boxes, and the packed multipoles cleared (with the cell lists, before launch_fma_build)
-void launch_far_lists(const Dev &d, int ncell, cudaStream_t st);
 // mode: the FP64 positions alone, or also what the context's pair field reads (its arrays exist by precision)
 constexpr int GATHER_FP64 = 0, GATHER_MIXED = 1, GATHER_PLAIN = 2;
 void launch_gather(const Dev &d, int nslot, int ncell, int mode, cudaStream_t st);
@@ -57,7 +55,7 @@ struct NearShape {
     int tile;   // target sites per work item: 32, 64 or (FP32 paths) 128
     int grid;   // CTAs of the persistent kernel
 };
-void launch_near_items(const Dev &d, int ncell, int nitems_max, int tile, cudaStream_t st);
+void launch_near_items(const Dev &d, int ncell, int tile, cudaStream_t st);
 // mode: 0 FP64, 1 FP32, 2 FP32 with compensated sums; per: the periodic preset's kernels
 int near_resident_ctas(int mode, int per);
 int near_max_ctas_per_sm(int mode, int per);

@@ -429,7 +429,7 @@ struct sesp_ctx {
     // beside the far-field build and the pair field (fork after the gather,
     // join before the site forces)
     cudaStream_t st2 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_eta = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_eta = nullptr, ev_list = nullptr;
     NearShape near = {64, 0};   // pair-field launch shape (autotuned or set; results do not depend on it)
     ConstraintShape cshape = {0, 4, 1};   // constraint halves of the mixed paths (likewise)
     int n_sm = 0;               // streaming multiprocessors of the device
@@ -541,24 +541,29 @@ void family(sesp_ctx *c, const char *name) {
 void seq_force(sesp_ctx *c, int rebuild, int terms) {
     const Dev &d = c->d;
     const int mixed = c->p.precision != SESP_PLAIN_FP64;
+    const bool fork = mixed && !c->timing && !c->sync_check;
     if (rebuild) {
         tstart(c, 5);
         // sites per cell, then the far field's counts
         cudaMemsetAsync(d.ccount, 0, sizeof(int) * (c->ncell + 16 * c->nrep + 3), c->st);
         launch_locate(d, c->nmol, c->smols, c->nsm * c->ssite, c->chains, c->nsite, c->st);
         family(c, "locate");
+        // lists that need no sorted slots, on the side stream that reads them
+        const cudaStream_t ls = fork ? c->st2 : c->st;
+        if (fork) {
+            cudaEventRecord(c->ev_list, c->st);
+            cudaStreamWaitEvent(c->st2, c->ev_list, 0);
+        }
+        launch_isub(d, c->nsm * c->ssite, c->smols, c->chains, ls);
+        family(c, "isub");
+        launch_graphite_list(d, c->nsite, ls);
+        family(c, "graphite list");
+        if (mixed) launch_water_order(d, c->wmols, c->nwm, ls);
+        family(c, "water order");
         launch_sort(d, c->nsite, c->ncell, c->st);
         family(c, "cell sort");
-        launch_far_lists(d, c->ncell, c->st);
-        family(c, "far-field lists");
-        launch_near_items(d, c->ncell, (int)near_items_max(c->nsite, c->ncell), c->near.tile, c->st);
+        launch_near_items(d, c->ncell, c->near.tile, c->st);
         family(c, "near-field items");
-        launch_isub(d, c->nsm * c->ssite, c->smols, c->chains, c->st);
-        family(c, "isub");
-        launch_graphite_list(d, c->nsite, c->st);
-        family(c, "graphite list");
-        if (mixed) launch_water_order(d, c->wmols, c->nwm, c->st);
-        family(c, "water order");
         tstop(c, 5);
     }
     launch_gather(d, c->nsite, c->ncell, mixed ? GATHER_MIXED : GATHER_PLAIN, c->st);
@@ -568,7 +573,6 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
     // paths; in order on the main stream on the plain path (its FP64 pair
     // field beside them ran a batched step at 581 ms against 259 ms in order)
     // and when kernels are timed or checked one by one
-    const bool fork = mixed && !c->timing && !c->sync_check;
     if (fork) {
         cudaEventRecord(c->ev_fork, c->st);
         cudaStreamWaitEvent(c->st2, c->ev_fork, 0);
@@ -696,7 +700,8 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
         cudaStreamCreateWithFlags(&c->st2, cudaStreamNonBlocking) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_eta, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_eta, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_list, cudaEventDisableTiming) != cudaSuccess) {
         delete c;
         return fail(SESP_ECUDA, "stream");
     }
@@ -738,6 +743,7 @@ int sesp_destroy(sesp_ctx *c) {
     cudaEventDestroy(c->ev_fork);
     cudaEventDestroy(c->ev_join);
     cudaEventDestroy(c->ev_eta);
+    cudaEventDestroy(c->ev_list);
     cudaStreamDestroy(c->st2);
     cudaStreamDestroy(c->st);
     delete c;
@@ -851,8 +857,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.near_far, R)) ||
         (e = dalloc(c, &d.pair_xyz, 3 * pair_max)) || (e = dalloc(c, &d.pair_key, pair_max)) || (e = dalloc(c, &d.crun, 8 * (size_t)C)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
         (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
-        (e = dalloc(c, &d.near_items_tmp, near_items_max(N, C))) || (e = dalloc(c, &d.near_cls, near_items_max(N, C))) ||
-        (e = dalloc(c, &d.near_icount, C + 1)) || (e = dalloc(c, &d.near_ctl, 66)) ||
+        (e = dalloc(c, &d.near_mask, C)) || (e = dalloc(c, &d.srt_cell, N)) || (e = dalloc(c, &d.near_ctl, 66)) ||
         (e = dalloc(c, &d.isub, (size_t)c->ssite * nsm)) || (e = dalloc(c, &d.O4, (size_t)LP * C)) ||
         (e = dalloc(c, &d.L4, (size_t)LP * C)) || (e = dalloc(c, &d.L4f, (size_t)LP * C)) ||
         (e = dalloc(c, &d.fside, 3 * (size_t)N)) || (e = dalloc(c, &d.stage, 12 * (size_t)N)) ||
@@ -1528,7 +1533,7 @@ int sesp_set_tuning(sesp_ctx *c, int tile, int ctas_per_sm) {
     if (set_device(c)) return SESP_ECUDA;
     const bool retile = tile != c->near.tile;
     c->near = {tile, c->n_sm * ctas_per_sm};
-    if (retile && c->have_force) launch_near_items(c->d, c->ncell, (int)near_items_max(c->nsite, c->ncell), tile, c->st);   // items of the current lists
+    if (retile && c->have_force) launch_near_items(c->d, c->ncell, tile, c->st);   // items of the current lists
     drop_graphs(c);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(c->st));
@@ -1646,7 +1651,7 @@ int sesp_autotune(sesp_ctx *c, int out[3]) {
         if (tile == 128 && !mixed) continue;
         const int mx = near_resident_ctas(near_mode(c), c->chains);
         const int cands[4] = {mx, (3 * mx) / 4, mx / 2, mx / 4};
-        launch_near_items(c->d, c->ncell, (int)near_items_max(c->nsite, c->ncell), tile, c->st);
+        launch_near_items(c->d, c->ncell, tile, c->st);
         for (int k = 0; k < 4; k++) {
             const int cps = cands[k];
             if (cps < 1 || (k > 0 && cps == cands[k - 1])) continue;
@@ -1667,7 +1672,7 @@ int sesp_autotune(sesp_ctx *c, int out[3]) {
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     c->near = pick;
-    launch_near_items(c->d, c->ncell, (int)near_items_max(c->nsite, c->ncell), pick.tile, c->st);
+    launch_near_items(c->d, c->ncell, pick.tile, c->st);
     if (mixed && c->nsm > 0 && !c->chains)   // flexible chains have no constraint sweeps to shape
         if (int e = tune_constraints(c)) return e;
     drop_graphs(c);

@@ -174,6 +174,7 @@ struct Dev {
     int *crun, *srt_pair;
     int2 *srt_meta;      // molecule, type
     int *srt_key;        // molecule << 5 | type
+    int *srt_cell;       // the slot's cell
     int *srt_xmask;      // per slot: bit dx + 3 dy + 9 dz (each offset + 1) set when the cell at that
                          // offset from the slot's own holds a site of the slot's molecule (itself
                          // included), so the pair loop tests same-molecule partners there only
@@ -181,9 +182,7 @@ struct Dev {
     double *near_part;   // partial near forces [9 rows, or 27 cells with near_split][3 * nslot] (float on the mixed path)
     int near_split;      // pair-field items are single partner cells, not rows of three
     int2 *near_items;    // near-field work items (cell, row << 24 | chunk), most expensive first
-    int2 *near_items_tmp;   // the same in cell order
-    int *near_cls;       // cost class of each item in cell order
-    int *near_icount;    // per cell: item count, then first item
+    int *near_mask;      // per occupied cell: its parts (rows or cells) that have partners
     int *near_ctl;       // [0] items taken past each warp's first in the running launch, [1] item count,
                          // [2..33] items per cost class, [34..65] next slot per class
     // graphite columns of the bottom layer

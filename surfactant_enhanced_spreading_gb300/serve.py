@@ -114,10 +114,10 @@ def estimate_bytes(system: S.System) -> int:
     # pair field: partials of 9 rows, or of 27 cells in small contexts; its
     # work items and the padded partner layout
     parts = 27 if n <= 40000 else 9
-    per_site = 12 * 8 + 1 + 4 * 4 + 32 + 16 + 8 + 4 + 3 * 8 + parts * 3 * 8 + 6 + 3 * 8 + 12 * 8 + 4 + 16 + 24 + parts * 20 / 32
+    per_site = 12 * 8 + 1 + 4 * 4 + 32 + 16 + 8 + 4 + 3 * 8 + parts * 3 * 8 + 6 + 3 * 8 + 12 * 8 + 4 + 16 + 24 + parts * 8 / 32 + 4
     per_mol = 5 * 4 + 2 * 8 + 4 + 4 + 2 * 4 + 2   # incl. the constraint halves' water lists and sweep counts
     cz = 25 * 16
-    cells = ncell * (8 * 4 + 2 * cz + 4 + 32 + 25 * 8) + min(n, ncell) * (parts * 40 + 4 * 64) + n3 * (13 + 2 * cz) + n2 * (9 + 2 * cz) + 80
+    cells = ncell * (8 * 4 + 2 * cz + 4 + 32 + 25 * 8) + min(n, ncell) * (parts * 16 + 4 * 64) + n3 * (13 + 2 * cz) + n2 * (9 + 2 * cz) + 80
     ops = (w2 ** 3 + 4 * 8) * 15 * 25 * 16 + w2 ** 3 * 45 * 24
     # real-form M2L at L4 and L3: operators, class-packed multipoles, partial
     # sums of 21 offset groups (FP64 sizes: an upper bound)
