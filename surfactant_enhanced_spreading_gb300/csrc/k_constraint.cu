@@ -372,6 +372,27 @@ inline double wk_host(const double *rm, int b, int c) {
 // s_kb: +1 if site k is bond b's first site, -1 if its second, else 0
 __device__ __forceinline__ double wsgn(int k, int b) { return k == wbi(b) ? 1.0 : (k == wbj(b) ? -1.0 : 0.0); }
 
+// |x| > t and not NaN
+__device__ __forceinline__ bool gt_abs_num(double x, double t) {
+    const long long a = __double_as_longlong(x) & 0x7fffffffffffffffLL;
+    return a > __double_as_longlong(t) && a <= 0x7ff0000000000000LL;
+}
+// FP64 to FP32 (truncated; below FP32's normal range 0) and back as bit moves
+// on the integer pipe: GB300 converts at its FP64 rate, 64 cycles a warp
+// instruction against about 14 for these.  With them and fused predictors a
+// water's SHAKE half takes 185 FP64 instructions, not 258 (100,000 waters: 79
+// -> 67 us; RATTLE 50 -> 43)
+__device__ __forceinline__ float to32(double v) {
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
+    const unsigned a = hi & 0x7fffffffu;
+    const unsigned f = __funnelshift_l(lo, a, 3) + 0x40000000u;   // exponent bias 1023 -> 127
+    return __uint_as_float(a < 897u << 20 ? 0u : (f & 0x7fffffffu) | (hi & 0x80000000u));
+}
+__device__ __forceinline__ double to64(float v) {   // (0 becomes 2^-127)
+    const unsigned f = __float_as_uint(v);
+    return __hiloint2double((int)((((f & 0x7fffffffu) >> 3) + 0x38000000u) | (f & 0x80000000u)), (int)(f << 29));
+}
+
 __device__ __forceinline__ void inv3f(const float (&A)[3][3], float (&B)[3][3]) {
     B[0][0] = A[1][1] * A[2][2] - A[1][2] * A[2][1];
     B[0][1] = A[0][2] * A[2][1] - A[0][1] * A[2][2];
@@ -415,8 +436,9 @@ __device__ __forceinline__ void water_step32(const float (&Ji)[3][3], const floa
 // the FP32 residual's resolution)
 constexpr int WMAT_FP32_STEPS = 8;
 
-// SHAKE half of one water in matrix form; returns the Newton steps it ran
-__device__ __forceinline__ int water_a_mat(const Dev &d, int m, double tol, int maxit) {
+// SHAKE half of one water in matrix form (thr: 2 tol d^2 per bond); returns
+// the Newton steps it ran
+__device__ __forceinline__ int water_a_mat(const Dev &d, int m, const double (&thr)[3], int maxit) {
     const int g0 = d.mfirst[m];
     const double escale = __dsub_rn(1.0, __dmul_rn(d.eta[d.mrep[m]], DT) * 0.5);
     // (the velocity predictor is formed again at the end from the state, so
@@ -430,25 +452,24 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, double tol, int 
         r[i][0] = d.x[g]; r[i][1] = d.y[g]; r[i][2] = d.z[g];
         ke0 = __dadd_rn(ke0, __dmul_rn(cF.mass64[wkind(i)],
                                        __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz))));
-        p[i][0] = pred_a(r[i][0], vx, ax, escale);
-        p[i][1] = pred_a(r[i][1], vy, ay, escale);
-        p[i][2] = pred_a(r[i][2], vz, az, escale);
+        p[i][0] = r[i][0] + fma(vx, escale, ax);
+        p[i][1] = r[i][1] + fma(vy, escale, ay);
+        p[i][2] = r[i][2] + fma(vz, escale, az);
     }
-    double R[3][3], P[3][3], D0[3], thr[3];
+    double R[3][3], P[3][3], D0[3];
 #pragma unroll
     for (int b = 0; b < 3; b++) {
         const int i = wbi(b), j = wbj(b);
 #pragma unroll
         for (int a = 0; a < 3; a++) { R[b][a] = r[i][a] - r[j][a]; P[b][a] = p[i][a] - p[j][a]; }
         D0[b] = cF.dsq64_w[b] - (P[b][0] * P[b][0] + P[b][1] * P[b][1] + P[b][2] * P[b][2]);
-        thr[b] = cF.dsq64_w[b] * (2.0 * tol);
     }
     // the Jacobian and its inverse in FP32: they only steer the steps
     float R32[3][3], P32[3][3], J[3][3], Ji[3][3];
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
-        for (int a = 0; a < 3; a++) { R32[b][a] = (float)R[b][a]; P32[b][a] = (float)P[b][a]; }
+        for (int a = 0; a < 3; a++) { R32[b][a] = to32(R[b][a]); P32[b][a] = to32(P[b][a]); }
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -459,8 +480,8 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, double tol, int 
     // tolerance (its rounding, ~1e-9 of d^2 ~ 0.1, is about the tolerance
     // band itself, so these only bring the corrections near the answer)
     float c32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    const float D0f[3] = {(float)D0[0], (float)D0[1], (float)D0[2]};
-    const float thrf[3] = {(float)thr[0], (float)thr[1], (float)thr[2]};
+    const float D0f[3] = {to32(D0[0]), to32(D0[1]), to32(D0[2])};
+    const float thrf[3] = {to32(thr[0]), to32(thr[1]), to32(thr[2])};
     int it = 0;
     for (int k32 = 0; k32 < WMAT_FP32_STEPS && it <= maxit; k32++) {
         float f[3];
@@ -485,7 +506,7 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, double tol, int 
 #pragma unroll
     for (int k = 0; k < 3; k++)
 #pragma unroll
-        for (int a = 0; a < 3; a++) cc[k][a] = (double)c32[k][a];
+        for (int a = 0; a < 3; a++) cc[k][a] = to64(c32[k][a]);
     // the tolerance test in FP64, as the reference's; a failed test takes
     // one more step from the FP64 residual (solved in FP32: it is small)
     bool done = false;
@@ -502,23 +523,22 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, double tol, int 
                 q += cd * (cd + 2.0 * P[b][a]);
             }
             f[b] = D0[b] - q;   // d^2 - |P_b + c_i - c_j|^2
-            done = done && !(fabs(f[b]) > thr[b]);
+            done = done && !gt_abs_num(f[b], thr[b]);
         }
         if (done) break;
-        float f32[3] = {(float)f[0], (float)f[1], (float)f[2]}, d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        float f32[3] = {to32(f[0]), to32(f[1]), to32(f[2])}, d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
         water_step32(Ji, R32, f32, d32);
 #pragma unroll
         for (int k = 0; k < 3; k++)
 #pragma unroll
-            for (int a = 0; a < 3; a++) cc[k][a] += (double)d32[k][a];
+            for (int a = 0; a < 3; a++) cc[k][a] += to64(d32[k][a]);
         it++;
     }
     double ke1 = 0.0;
 #pragma unroll
     for (int i = 0; i < 3; i++) {
         const int g = g0 + i;
-        const double v0 = vel_a(d.vx[g], d.ax[g], escale), v1 = vel_a(d.vy[g], d.ay[g], escale),
-                     v2 = vel_a(d.vz[g], d.az[g], escale);
+        const double v0 = fma(d.vx[g], escale, d.ax[g]), v1 = fma(d.vy[g], escale, d.ay[g]), v2 = fma(d.vz[g], escale, d.az[g]);
         d.x[g] = p[i][0] + cc[i][0]; d.y[g] = p[i][1] + cc[i][1]; d.z[g] = p[i][2] + cc[i][2];
         const double vx = v0 + cc[i][0], vy = v1 + cc[i][1], vz = v2 + cc[i][2];
         d.vx[g] = vx; d.vy[g] = vy; d.vz[g] = vz;
@@ -557,7 +577,7 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
-        for (int c = 0; c < 3; c++) R32[b][c] = (float)R[b][c];
+        for (int c = 0; c < 3; c++) R32[b][c] = to32(R[b][c]);
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -574,11 +594,11 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
             const int i = wbi(b), j = wbj(b);
             rv[b] = R[b][0] * (v[i][0] - v[j][0]) + R[b][1] * (v[i][1] - v[j][1]) + R[b][2] * (v[i][2] - v[j][2]);
             // RATTLE's test: -(R.V / dt) / ((1/m_i + 1/m_j) d^2)
-            done = done && !(fabs(cF.fb64_w[b] * rv[b]) > tol);
+            done = done && !gt_abs_num(cF.fb64_w[b] * rv[b], tol);
         }
         if (done) break;
         // A h = -R.V in FP32 (R.V is small: the rounding of h is far below the tolerance)
-        float rv32[3] = {(float)rv[0], (float)rv[1], (float)rv[2]}, d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        float rv32[3] = {to32(rv[0]), to32(rv[1]), to32(rv[2])}, d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
         float h[3];
 #pragma unroll
         for (int b = 0; b < 3; b++) h[b] = -(Ai[b][0] * rv32[0] + Ai[b][1] * rv32[1] + Ai[b][2] * rv32[2]);
@@ -586,7 +606,7 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
 #pragma unroll
         for (int k = 0; k < 3; k++)
 #pragma unroll
-            for (int a = 0; a < 3; a++) v[k][a] += (double)d32[k][a];
+            for (int a = 0; a < 3; a++) v[k][a] += to64(d32[k][a]);
         it++;
     }
 #pragma unroll
@@ -723,76 +743,90 @@ __device__ __forceinline__ double tri_sum(double v, int base) {
     return (v0 + v1) + v2;
 }
 
-// The wavefront for FP64 corrections with each bond split over 3 lanes, one
-// per Cartesian component: lane 12 q + 3 w + k works on component k of
-// wavefront lane w of molecule q (q < 2; lanes 24..31 idle).  Every FP64
-// warp instruction costs the same whatever its active lanes, so splitting
-// the components takes a SHAKE bond from 25 to 18 FP64 warp instructions
-// (9 to 6 for a bond within tolerance) and a RATTLE bond from 12 to 7; the
-// two dot products go over shuffles.  Returns a ballot whose bit 12 q is set
-// if molecule q ran out of sweeps.
+// The wavefront for FP64 corrections, one molecule at a time with each bond
+// split over 3 lanes, one per Cartesian component.  Every FP64 warp
+// instruction costs the same whatever its active lanes (64 cycles of a
+// scheduler), so a step costs the same for one bond as for ten, and what
+// counts is the number of steps.  A bond has a fixed place in its sweep, so
+// that sweeps follow each other at a lag of 4 steps and not 8 (TAU: a sweep's
+// bonds 0..22 at steps 0..22, the second branch of site 17, bonds 23..26,
+// beside the first at 19..22, bond 27 at 23): of two bonds that share a site
+// the later in the reference's order comes 1 to 3 steps after the other, so
+// every site sees the sequential order's updates.  Six sweeps are in flight,
+// seven bonds a step: lane 3 u + k is component k of the main line of sweep u
+// (mod 6) for u < 6, and of the second branch for u = 6.  S sweeps take 4 S +
+// 20 steps (8 S + 20 at a lag of 8, which ran two molecules in a warp).
+// Splitting the components takes a SHAKE bond from 25 to 18 FP64 warp
+// instructions (9 to 6 for a bond within tolerance) and a RATTLE bond from 12
+// to 7; the two dot products go over shuffles.  Returns a ballot whose bit
+// 12 q is set if molecule q ran out of sweeps.
+constexpr int TAU_LAG = 4, TAU_END = 23, TAU_LINES = 6;
 template <bool SHAKE>
 __device__ __forceinline__ unsigned surf_wavefront3(const Dev &d, MolSmem<double, SHAKE ? 16 : 11> *sms, int n,
                                                     double tol, int maxit) {
     const int lane = threadIdx.x & 31;
-    const int q = lane < 24 ? lane / 12 : 0, r = lane - 12 * q, w = lane < 24 ? r / 3 : 0, k = lane < 24 ? r % 3 : 0;
-    const int base = lane - k;
-    const unsigned gmask = 0xFFFu << (12 * q);
-    MolSmem<double, SHAKE ? 16 : 11> &sm = sms[q < n ? q : 0];
-    double *rec = &sm.rec[0][0];
-    int kmine = w;
-    bool changed = false, done = lane >= 24 || q >= n, fail = false;
-    for (int t = 0;; t++) {
-        bool clean = false, last = false;
-        const int b = t - WF_LAG * kmine;
-        const bool valid = !done && kmine <= maxit && b >= 0 && b < NBOND;
-        const int sb = skew8(valid ? b : 0), i = valid ? sbi32(b) : 0, si = skew8(i), sj = skew8(valid ? b + 1 : 0);
-        double ci = 0.0, cj = 0.0, dx = 0.0, pr = 0.0;
-        if (valid) {
-            ci = sm.sc[k][si];
-            cj = sm.sc[k][sj];
-            dx = ci - cj;
-            pr = SHAKE ? dx * (dx + rec[k * SK + sb]) : rec[k * SK + sb] * dx;   // c_k (c_k + 2P_k)  /  -fb R_k c_k
-        }
-        const double sum = tri_sum(pr, base);
-        double gab = 0.0;
-        bool act = false;
-        if constexpr (SHAKE) {
-            const double diffsq = valid ? rec[12 * SK + sb] - sum : 0.0;   // D0 - c.(c + 2P)
-            act = valid && gt_abs(diffsq, rec[14 * SK + sb]);
-            if (__any_sync(FULL, act)) {   // the step only when some bond of the warp is corrected
-                const double tk = valid ? rec[(3 + k) * SK + sb] * dx : 0.0;
-                const double tt = tri_sum(tk, base);
-                const double y0 = valid ? rec[13 * SK + sb] : 0.0;
-                const double t2 = tt * tt;
-                const double ya = fma(-y0, tt, y0), yb = fma(tt, tt, 1.0), yc = fma(t2, t2, 1.0);
-                gab = (diffsq * ya) * (yb * yc);
+    const int u = lane / 3, k = lane - 3 * u, base = min(3 * u, 29);
+    const bool line = u < TAU_LINES, branch = u == TAU_LINES;
+    unsigned failed = 0;
+    if (maxit < 0) return 0x1001u;   // no sweep allowed
+    for (int q = 0; q < n; q++) {
+        MolSmem<double, SHAKE ? 16 : 11> &sm = sms[q];
+        double *rec = &sm.rec[0][0];
+        int kmine = line ? u : 0;   // the lane's current sweep
+        bool changed = false, branch_changed = false;   // in it; on its second branch (kept one step for the main line)
+        for (int t = 0;; t++) {
+            const int tau = t - TAU_LAG * kmine;
+            const bool valid = kmine <= maxit && (line ? tau >= 0 : branch && tau >= 19 && tau <= 22);
+            const int b = valid ? (branch ? tau + 4 : tau == TAU_END ? NBOND - 1 : tau) : 0;
+            const int sb = skew8(b), i = sbi32(b), si = skew8(i), sj = skew8(b + 1);
+            double ci = 0.0, cj = 0.0, dx = 0.0, pr = 0.0;
+            if (valid) {
+                ci = sm.sc[k][si];
+                cj = sm.sc[k][sj];
+                dx = ci - cj;
+                pr = SHAKE ? dx * (dx + rec[k * SK + sb]) : rec[k * SK + sb] * dx;   // c_k (c_k + 2P_k)  /  -fb R_k c_k
             }
-        } else {
-            gab = valid ? rec[9 * SK + sb] + sum : 0.0;   // -fb R.(V + c)
-            act = valid && gt_abs(gab, tol);
-        }
-        if (act) {
-            const int fa = SHAKE ? 6 : 3, fb = SHAKE ? 9 : 6;
-            sm.sc[k][si] = fma(rec[(fa + k) * SK + sb], gab, ci);
-            sm.sc[k][sj] = fma(-rec[(fb + k) * SK + sb], gab, cj);
-            changed = true;
-        }
-        if (valid && b == NBOND - 1) {
-            clean = !changed;
-            last = changed && kmine == maxit;
-            changed = false;
-            kmine += WF_LANES;
+            const double sum = tri_sum(pr, base);
+            double gab = 0.0;
+            bool act = false;
+            if constexpr (SHAKE) {
+                const double diffsq = valid ? rec[12 * SK + sb] - sum : 0.0;   // D0 - c.(c + 2P)
+                act = valid && gt_abs(diffsq, rec[14 * SK + sb]);
+                if (__any_sync(FULL, act)) {   // the step only when some bond of the warp is corrected
+                    const double tk = valid ? rec[(3 + k) * SK + sb] * dx : 0.0;
+                    const double tt = tri_sum(tk, base);
+                    const double y0 = valid ? rec[13 * SK + sb] : 0.0;
+                    const double t2 = tt * tt;
+                    const double ya = fma(-y0, tt, y0), yb = fma(tt, tt, 1.0), yc = fma(t2, t2, 1.0);
+                    gab = (diffsq * ya) * (yb * yc);
+                }
+            } else {
+                gab = valid ? rec[9 * SK + sb] + sum : 0.0;   // -fb R.(V + c)
+                act = valid && gt_abs(gab, tol);
+            }
+            if (act) {
+                const int fa = SHAKE ? 6 : 3, fb = SHAKE ? 9 : 6;
+                sm.sc[k][si] = fma(rec[(fa + k) * SK + sb], gab, ci);
+                sm.sc[k][sj] = fma(-rec[(fb + k) * SK + sb], gab, cj);
+                changed = true;
+            }
+            // a sweep ends with its main line; the branch's flag dates from the step before
+            const bool ends = line && valid && tau == TAU_END;
+            const bool bc = __any_sync(FULL, branch && branch_changed);
+            const unsigned clean = __ballot_sync(FULL, ends && !changed && !bc);
+            const unsigned last = __ballot_sync(FULL, ends && kmine == maxit);
+            if (ends) { changed = false; kmine += TAU_LINES; }
+            if (branch && tau == 22) { branch_changed = changed; changed = false; kmine++; }
+            __syncwarp();
+            if (clean) break;
+            if (last) {
+                failed |= 1u << (12 * q);
+                break;
+            }
         }
         __syncwarp();
-        const unsigned bc = __ballot_sync(FULL, clean), bl = __ballot_sync(FULL, last);
-        if (!done) {
-            if (bc & gmask) done = true;
-            else if (bl & gmask) { done = true; fail = true; }
-        }
-        if (__all_sync(FULL, done)) break;
     }
-    return __ballot_sync(FULL, fail && r == 0 && lane < 24);
+    return failed;
 }
 
 // whether molecule g of the warp ran out of sweeps, from the wavefront's ballot
@@ -989,6 +1023,20 @@ __device__ __forceinline__ bool mol_ok(const Dev &d, const CPlan &p, int m, int 
     return g0 >= 0 && g0 + nsites <= p.nsite;
 }
 
+// A warp's next item of 32 waters.  Its first is fixed (`mine`, below
+// `reserved`), the others come from the queue: taken from the queue, the
+// first items all went to the warps of the SMs nearest to the counter, as
+// every CTA starts at once when the predecessor kernel ends.  SHAKE / RATTLE
+// halves (us): 120 surfactants with 3,001 waters 106 / 71 -> 61 / 47, 200 with
+// 20,000 waters 114 / 73 -> 97 / 63, 20,000 waters in matrix form 51 / 36 -> 41
+// / 25.
+__device__ __forceinline__ unsigned water_item(const CPlan &p, int lane, bool first, unsigned mine, unsigned reserved) {
+    if (first) return mine;
+    unsigned item = 0;
+    if (lane == 0) item = atomicAdd(&p.ctl[1], 1u) + reserved;
+    return __shfl_sync(FULL, item, 0);
+}
+
 template <typename C, bool SHAKE>
 __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double tol, int maxit) {
     griddep_wait();
@@ -1016,10 +1064,12 @@ __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double
     }
     // the other warps of a surfactant CTA stay idle, so its chains keep the SM's FP64 pipe
     if (!surf_cta || warp < p.s_warps) {
-        for (;;) {
-            unsigned item = 0;
-            if (lane == 0) item = atomicAdd(&p.ctl[1], 1u);
-            item = __shfl_sync(FULL, item, 0);
+        // (FP32 sweeps are no FP64 queue: 5,000 waters ran 51 us from the
+        // counter alone, 58 spread over all SMs)
+        const double thr[3] = {cF.dsq64_w[0] * (2.0 * tol), cF.dsq64_w[1] * (2.0 * tol), cF.dsq64_w[2] * (2.0 * tol)};
+        const unsigned free_ctas = sizeof(C) == 8 ? gridDim.x - p.n_scta : 0;
+        for (bool first = !surf_cta && free_ctas;; first = false) {
+            const unsigned item = water_item(p, lane, first, warp * free_ctas + blockIdx.x - p.n_scta, CW * free_ctas);
             const long long t0 = 32LL * item;
             if (t0 >= p.nw) break;
             const int t = (int)t0 + lane;
@@ -1031,7 +1081,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double
                 }
                 int sweeps;
                 if (std::is_same<C, double>::value && p.mat)
-                    sweeps = SHAKE ? water_a_mat(d, m, tol, maxit) : water_b_mat(d, m, tol, maxit);
+                    sweeps = SHAKE ? water_a_mat(d, m, thr, maxit) : water_b_mat(d, m, tol, maxit);
                 else
                     sweeps = SHAKE ? water_a<C>(d, m, tol, maxit) : water_b<C>(d, m, tol, maxit);
                 p.wsw[m] = (uint8_t)(sweeps < 255 ? sweeps : 255);
@@ -1056,10 +1106,12 @@ template <bool SHAKE>
 __global__ void __launch_bounds__(CW_THREADS) k_water_mat(Dev d, CPlan p, double tol, int maxit) {
     griddep_wait();
     const int lane = threadIdx.x & 31;
-    for (;;) {
-        unsigned item = 0;
-        if (lane == 0) item = atomicAdd(&p.ctl[1], 1u);
-        item = __shfl_sync(FULL, item, 0);
+    // the CTAs of one SM start on different schedulers (a scheduler's FP64
+    // unit takes 64 cycles an instruction)
+    const double thr[3] = {cF.dsq64_w[0] * (2.0 * tol), cF.dsq64_w[1] * (2.0 * tol), cF.dsq64_w[2] * (2.0 * tol)};
+    const unsigned rank = (threadIdx.x / 32 + CW - blockIdx.x / GB300_SMS % CW) % CW;
+    for (bool first = true;; first = false) {
+        const unsigned item = water_item(p, lane, first, rank * gridDim.x + blockIdx.x, CW * gridDim.x);
         const long long t0 = 32LL * item;
         if (t0 >= p.nw) break;
         const int t = (int)t0 + lane;
@@ -1069,7 +1121,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_water_mat(Dev d, CPlan p, double
                 atomicAdd(&d.counters[7], 1ull);
                 continue;
             }
-            const int sweeps = SHAKE ? water_a_mat(d, m, tol, maxit) : water_b_mat(d, m, tol, maxit);
+            const int sweeps = SHAKE ? water_a_mat(d, m, thr, maxit) : water_b_mat(d, m, tol, maxit);
             p.wsw[m] = (uint8_t)(sweeps < 255 ? sweeps : 255);
         }
     }

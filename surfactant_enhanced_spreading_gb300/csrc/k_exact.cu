@@ -200,21 +200,23 @@ __device__ __forceinline__ double div_dt(double a) {
 
 // The plain path's surfactants: the Gauss-Seidel sweeps over 28 bonds of
 // src/move_surfactant_a.f90:36-134 and src/move_surfactant_b.f90:30-118, bit
-// for bit, as a wavefront.  Sweep k takes bond b in step 8 k + b, on the k-th
-// (mod 4) of four groups of three lanes, one lane per component.  Bonds that
-// share a site are at most 7 apart in the reference's order, so when sweep k
-// takes bond b, sweep k - 1 has done every bond that shares a site with it and
-// is at b + 8, which shares none: each site sees the sequential order's
-// updates.  Once a sweep has changed nothing, neither have the later ones
-// under way.  A sum over components is formed by every lane in the
-// reference's order from its neighbours' products.
+// for bit, as a wavefront of one molecule per warp.  A bond has a fixed step
+// within its sweep (SURF_TAU), sweeps follow each other 4 steps apart, and of
+// two bonds that share a site the later in the reference's order comes 1 to 3
+// steps after the other: each site sees the sequential order's updates.  Six
+// sweeps are in flight, seven bonds a step, three lanes each (one per
+// component): lane 3 u + a has the main line of sweep u (mod 6), bonds 0..22
+// and 27, for u < 6, and the second branch of site 17, bonds 23..26, for u =
+// 6.  Once a sweep has changed nothing, neither have the later ones under
+// way.  A sum over components is formed by every lane in the reference's
+// order from its neighbours' products.
 // Bound by FP64 issue and latency along one molecule's steps (a step of a
 // correcting bond is 32 FP64 warp instructions; a thread per molecule took 52,
 // in sequence over all sweeps, and spilled): 12 surfactants with 701 waters,
-// SHAKE 280 -> 75 us, RATTLE 571 -> 149 us.
-constexpr int SURF_MOLS = 2;   // molecules of a warp, 12 lanes each
+// SHAKE 280 -> 60 us, RATTLE 571 -> 144 us (75 and 149 with sweeps 8 apart;
+// the waters bound them now).
 struct SurfShared {
-    double p[SURF_MOLS][NSURF][3], v[SURF_MOLS][NSURF][3], r[SURF_MOLS][NBOND][3], ke[SURF_MOLS][NSURF];
+    double p[NSURF][3], v[NSURF][3], r[NBOND][3], ke[NSURF];
     double m[NSURF], rm[NSURF], c0[NBOND], c1[NBOND], c2[NBOND];   // masses and their reciprocals; per-bond constants
     int i[NBOND], j[NBOND];
 };
@@ -226,47 +228,45 @@ __device__ __forceinline__ double sum3(double v, int first) {
     return a + b + c;
 }
 
-// Runs the sweeps of the warp's molecules; act(b, on) takes bond b for the
-// lane's group (every lane calls it; `on`: the group has a bond in this step)
-// and says whether it corrected it.  True if the lane's molecule met the
-// tolerance within maxit + 1 sweeps.
+// Runs a molecule's sweeps; act(b, on) takes bond b for the lane's group
+// (every lane calls it; `on`: the group has a bond in this step) and says
+// whether it corrected it.  True if the tolerance was met within maxit + 1
+// sweeps.
+constexpr int SURF_LAG = 4, SURF_END = 23, SURF_LINES = 6;
 template <typename F>
-__device__ __forceinline__ bool surf_sweeps(int slot, unsigned mol, bool mine, int maxit, F act) {
-    bool ok = false, done = !mine || maxit < 0, dirty = false;
-    int sweep = slot;
-    for (int step = 0; __any_sync(0xffffffffu, !done); step++) {
-        int b = step - 8 * sweep;
-        if (b == NBOND) { sweep += 4; b -= 32; }   // this group's next sweep starts in 4 steps
-        const bool on = !done && b >= 0 && sweep <= maxit;
-        if (b == 0) dirty = false;
-        if (act(on ? b : 0, on)) dirty = true;
+__device__ __forceinline__ bool surf_sweeps(int u, int maxit, F act) {
+    if (maxit < 0) return false;
+    const bool line = u < SURF_LINES, branch = u == SURF_LINES;
+    int sweep = line ? u : 0;
+    bool dirty = false, branch_dirty = false;   // in the lane's sweep; on its second branch (kept one step)
+    for (int step = 0;; step++) {
+        const int tau = step - SURF_LAG * sweep;
+        const bool on = sweep <= maxit && (line ? tau >= 0 : branch && tau >= 19 && tau <= 22);
+        const int b = on ? (branch ? tau + 4 : tau == SURF_END ? NBOND - 1 : tau) : 0;
+        if (act(b, on)) dirty = true;
+        const bool ends = line && on && tau == SURF_END;
+        const bool bd = __any_sync(0xffffffffu, branch && branch_dirty);
+        const unsigned clean = __ballot_sync(0xffffffffu, ends && !dirty && !bd);
+        const unsigned out = __ballot_sync(0xffffffffu, ends && sweep == maxit);
+        if (ends) { dirty = false; sweep += SURF_LINES; }
+        if (branch && tau == 22) { branch_dirty = dirty; dirty = false; sweep++; }
         __syncwarp();
-        const bool ends = on && b == NBOND - 1;
-        const unsigned clean = __ballot_sync(0xffffffffu, ends && !dirty) & mol;
-        const unsigned out = __ballot_sync(0xffffffffu, ends && sweep == maxit) & mol;
-        if (!done && clean) ok = done = true;
-        else if (!done && out) done = true;
+        if (clean) return true;
+        if (out) return false;
     }
-    return ok;
 }
 
-// which molecule of the warp, sweep slot and component a lane has
+// which group and component a lane has
 struct SurfLane {
-    int lane, mo, l, slot, a, first;
-    unsigned mol;
-    bool in;
+    int lane, u, a, first;
     __device__ SurfLane() {
         lane = threadIdx.x & 31;
-        mo = lane >= 12 && lane < 24;
-        in = lane < 12 * SURF_MOLS;
-        l = in ? lane - 12 * mo : lane - 24;   // 0..11 (0..7 past the molecules)
-        slot = l / 3; a = l % 3;
+        u = lane / 3; a = lane % 3;
         first = min(lane - a, 29);
-        mol = in ? 0xfffu << (12 * mo) : 0u;
     }
 };
 
-__device__ void surf_move_a(const Dev &d, const int *mols, int nm, double tol, int maxit, SurfShared &s, int block) {
+__device__ void surf_move_a(const Dev &d, const int *mols, double tol, int maxit, SurfShared &s, int block) {
     const SurfLane L;
     for (int k = L.lane; k < NSURF; k += 32) { s.m[k] = cT.mass[2 + k]; s.rm[k] = 1.0 / cT.mass[2 + k]; }
     for (int b = L.lane; b < NBOND; b += 32) {
@@ -276,68 +276,63 @@ __device__ void surf_move_a(const Dev &d, const int *mols, int nm, double tol, i
         s.c1[b] = cT.dsqs[b] * (2.0 * tol);
         s.c2[b] = 2.0 * (1.0 / cT.mass[2 + i] + 1.0 / cT.mass[2 + j]);
     }
-    const int t = block * SURF_MOLS + L.mo;
-    const bool mine = L.in && t < nm;
-    const int m = mine ? mols[t] : 0, g0 = mine ? d.mfirst[m] : 0;
-    const double escale = mine ? 1.0 - d.eta[d.mrep[m]] * DT / 2.0 : 1.0;
+    const int m = mols[block], g0 = d.mfirst[m];
+    const double escale = 1.0 - d.eta[d.mrep[m]] * DT / 2.0;
     double *const xs[3] = {d.x, d.y, d.z}, *const vs[3] = {d.vx, d.vy, d.vz}, *const as[3] = {d.ax, d.ay, d.az};
-    auto each = [&](auto f) {   // every (site, component) of the molecule over its 12 lanes
-        if (mine)
-            for (int k = L.l; k < 3 * NSURF; k += 12) f(k / 3, k % 3);
+    auto each = [&](auto f) {   // every (site, component)
+        for (int k = L.lane; k < 3 * NSURF; k += 32) f(k / 3, k % 3);
         __syncwarp();
     };
     auto kinetic = [&]() {   // sum of m v^2 in site order
-        if (mine)
-            for (int k = L.l; k < NSURF; k += 12) {
-                const double vx = s.v[L.mo][k][0], vy = s.v[L.mo][k][1], vz = s.v[L.mo][k][2];
-                s.ke[L.mo][k] = s.m[k] * (vx * vx + vy * vy + vz * vz);
-            }
+        for (int k = L.lane; k < NSURF; k += 32) {
+            const double vx = s.v[k][0], vy = s.v[k][1], vz = s.v[k][2];
+            s.ke[k] = s.m[k] * (vx * vx + vy * vy + vz * vz);
+        }
         __syncwarp();
         double sum = 0.0;
-        if (mine && L.l == 0)
-            for (int k = 0; k < NSURF; k++) sum += s.ke[L.mo][k];
+        if (L.lane == 0)
+            for (int k = 0; k < NSURF; k++) sum += s.ke[k];
         __syncwarp();
         return sum;
     };
-    each([&](int k, int a) { s.p[L.mo][k][a] = xs[a][g0 + k]; s.v[L.mo][k][a] = vs[a][g0 + k]; });
+    each([&](int k, int a) { s.p[k][a] = xs[a][g0 + k]; s.v[k][a] = vs[a][g0 + k]; });
     const double ke0 = kinetic();
-    if (mine)
-        for (int k = L.l; k < 3 * NBOND; k += 12) {
-            const int b = k / 3, a = k % 3;
-            s.r[L.mo][b][a] = s.p[L.mo][s.i[b]][a] - s.p[L.mo][s.j[b]][a];
-        }
+    for (int k = L.lane; k < 3 * NBOND; k += 32) {
+        const int b = k / 3, a = k % 3;
+        s.r[b][a] = s.p[s.i[b]][a] - s.p[s.j[b]][a];
+    }
     __syncwarp();
     each([&](int k, int a) {
-        const double v = s.v[L.mo][k][a], acc = as[a][g0 + k];
-        s.p[L.mo][k][a] = s.p[L.mo][k][a] + v * escale + acc;
-        s.v[L.mo][k][a] = v * escale + acc;
+        const double v = s.v[k][a], acc = as[a][g0 + k];
+        s.p[k][a] = s.p[k][a] + v * escale + acc;
+        s.v[k][a] = v * escale + acc;
     });
-    const bool ok = surf_sweeps(L.slot, L.mol, mine, maxit, [&](int b, bool on) {
-        const int i = s.i[b], j = s.j[b], a = L.a, mo = L.mo;
-        const double p = s.p[mo][i][a] - s.p[mo][j][a];
+    const bool ok = surf_sweeps(L.u, maxit, [&](int b, bool on) {
+        const int i = s.i[b], j = s.j[b], a = L.a;
+        const double p = s.p[i][a] - s.p[j][a];
         const double diffsq = s.c0[b] - sum3(p * p, L.first);
         const bool cor = on && fabs(diffsq) > s.c1[b];
         if (__any_sync(0xffffffffu, cor)) {
-            const double r = s.r[mo][b][a], rpab = sum3(r * p, L.first);
+            const double r = s.r[b][a], rpab = sum3(r * p, L.first);
             const double gab = diffsq / (s.c2[b] * rpab);
             if (cor) {
                 const double dx = r * gab, di = s.rm[i] * dx, dj = s.rm[j] * dx;
-                s.p[mo][i][a] = s.p[mo][i][a] + di; s.p[mo][j][a] = s.p[mo][j][a] - dj;
-                s.v[mo][i][a] = s.v[mo][i][a] + di; s.v[mo][j][a] = s.v[mo][j][a] - dj;
+                s.p[i][a] = s.p[i][a] + di; s.p[j][a] = s.p[j][a] - dj;
+                s.v[i][a] = s.v[i][a] + di; s.v[j][a] = s.v[j][a] - dj;
             }
         }
         return cor;
     });
-    each([&](int k, int a) { xs[a][g0 + k] = s.p[L.mo][k][a]; vs[a][g0 + k] = s.v[L.mo][k][a]; });
+    each([&](int k, int a) { xs[a][g0 + k] = s.p[k][a]; vs[a][g0 + k] = s.v[k][a]; });
     const double ke1 = kinetic();
-    if (mine && L.l == 0) {
+    if (L.lane == 0) {
         d.ke[2 * m] = ke0;
         d.ke[2 * m + 1] = ke1;
         if (!ok) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
     }
 }
 
-__device__ void surf_move_b(const Dev &d, const int *mols, int nm, double tol, int maxit, SurfShared &s, int block) {
+__device__ void surf_move_b(const Dev &d, const int *mols, double tol, int maxit, SurfShared &s, int block) {
     const SurfLane L;
     for (int k = L.lane; k < NSURF; k += 32) { s.m[k] = cT.mass[2 + k]; s.rm[k] = 1.0 / cT.mass[2 + k]; }
     for (int b = L.lane; b < NBOND; b += 32) {
@@ -346,44 +341,39 @@ __device__ void surf_move_b(const Dev &d, const int *mols, int nm, double tol, i
         s.c0[b] = (1.0 / cT.mass[2 + i] + 1.0 / cT.mass[2 + j]) * cT.dsqs[b];
         s.c1[b] = 1.0 / s.c0[b];
     }
-    const int t = block * SURF_MOLS + L.mo;
-    const bool mine = L.in && t < nm;
-    const int m = mine ? mols[t] : 0, g0 = mine ? d.mfirst[m] : 0;
-    const double escale = mine ? 2.0 / (2.0 + d.eta[d.mrep[m]] * DT) : 1.0;
+    const int m = mols[block], g0 = d.mfirst[m];
+    const double escale = 2.0 / (2.0 + d.eta[d.mrep[m]] * DT);
     double *const xs[3] = {d.x, d.y, d.z}, *const vs[3] = {d.vx, d.vy, d.vz}, *const as[3] = {d.ax, d.ay, d.az};
     double *const fs[3] = {d.fx, d.fy, d.fz};
     __syncwarp();   // the constants are in place
-    if (mine)
-        for (int k = L.l; k < 3 * NSURF; k += 12) {
-            const int n = k / 3, a = k % 3;
-            const double acc = div_by(fs[a][g0 + n] * DTSQ2, s.m[n], s.rm[n]);
-            as[a][g0 + n] = acc;
-            s.p[L.mo][n][a] = xs[a][g0 + n];
-            s.v[L.mo][n][a] = escale * (vs[a][g0 + n] + acc);
-        }
+    for (int k = L.lane; k < 3 * NSURF; k += 32) {
+        const int n = k / 3, a = k % 3;
+        const double acc = div_by(fs[a][g0 + n] * DTSQ2, s.m[n], s.rm[n]);
+        as[a][g0 + n] = acc;
+        s.p[n][a] = xs[a][g0 + n];
+        s.v[n][a] = escale * (vs[a][g0 + n] + acc);
+    }
     __syncwarp();
-    if (mine)
-        for (int k = L.l; k < 3 * NBOND; k += 12) {
-            const int b = k / 3, a = k % 3;
-            s.r[L.mo][b][a] = s.p[L.mo][s.i[b]][a] - s.p[L.mo][s.j[b]][a];
-        }
+    for (int k = L.lane; k < 3 * NBOND; k += 32) {
+        const int b = k / 3, a = k % 3;
+        s.r[b][a] = s.p[s.i[b]][a] - s.p[s.j[b]][a];
+    }
     __syncwarp();
-    const bool ok = surf_sweeps(L.slot, L.mol, mine, maxit, [&](int b, bool on) {
-        const int i = s.i[b], j = s.j[b], a = L.a, mo = L.mo;
-        const double r = s.r[mo][b][a], v = s.v[mo][i][a] - s.v[mo][j][a];
+    const bool ok = surf_sweeps(L.u, maxit, [&](int b, bool on) {
+        const int i = s.i[b], j = s.j[b], a = L.a;
+        const double r = s.r[b][a], v = s.v[i][a] - s.v[j][a];
         const double rvab = div_dt(sum3(r * v, L.first));
         const double gab = div_by(-rvab, s.c0[b], s.c1[b]);
         const bool cor = on && fabs(gab) > tol;
         if (cor) {
             const double dx = r * gab;
-            s.v[mo][i][a] = s.v[mo][i][a] + s.rm[i] * dx * DT;
-            s.v[mo][j][a] = s.v[mo][j][a] - s.rm[j] * dx * DT;
+            s.v[i][a] = s.v[i][a] + s.rm[i] * dx * DT;
+            s.v[j][a] = s.v[j][a] - s.rm[j] * dx * DT;
         }
         return cor;
     });
-    if (mine)
-        for (int k = L.l; k < 3 * NSURF; k += 12) vs[k % 3][g0 + k / 3] = s.v[L.mo][k / 3][k % 3];
-    if (mine && L.l == 0 && !ok) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
+    for (int k = L.lane; k < 3 * NSURF; k += 32) vs[k % 3][g0 + k / 3] = s.v[k / 3][k % 3];
+    if (L.lane == 0 && !ok) { d.mfail[m] += 1; atomicAdd(&d.counters[0], 1ull); }
 }
 
 // A water over three lanes, one per component: the same operations in the
@@ -513,9 +503,9 @@ __device__ void water_split_b(const Dev &d, const int *mols, int nm, double tol,
 __global__ void __launch_bounds__(MOVE_BLOCK) k_move_a(Dev d, const int *mols, int nm, const int *smols, int ns, double tol,
                                                       int maxit) {
     __shared__ SurfShared surf;
-    const int sb = (ns + SURF_MOLS - 1) / SURF_MOLS;
+    const int sb = ns;
     if ((int)blockIdx.x < sb) {
-        surf_move_a(d, smols, ns, tol, maxit, surf, blockIdx.x);
+        surf_move_a(d, smols, tol, maxit, surf, blockIdx.x);
         return;
     }
     if (nm <= MOVE_SPLIT_MAX) {
@@ -637,9 +627,9 @@ __global__ void __launch_bounds__(ETA_THREADS) k_eta(Dev d) {
 __global__ void __launch_bounds__(MOVE_BLOCK) k_move_b(Dev d, const int *mols, int nm, const int *smols, int ns, double tol,
                                                       int maxit) {
     __shared__ SurfShared surf;
-    const int sb = (ns + SURF_MOLS - 1) / SURF_MOLS;
+    const int sb = ns;
     if ((int)blockIdx.x < sb) {
-        surf_move_b(d, smols, ns, tol, maxit, surf, blockIdx.x);
+        surf_move_b(d, smols, tol, maxit, surf, blockIdx.x);
         return;
     }
     if (nm <= MOVE_SPLIT_MAX) {
@@ -831,7 +821,7 @@ void launch_isub(const Dev &d, int nsurf_sites, const int *surf_mols, int per, c
 }
 static int move_blocks(int nw, int ns) {
     const int w = nw <= MOVE_SPLIT_MAX ? WATERS_SPLIT : MOVE_BLOCK;
-    return (ns + SURF_MOLS - 1) / SURF_MOLS + (nw + w - 1) / w;
+    return ns + (nw + w - 1) / w;
 }
 // fast = 0 (plain path): the FP64 sweeps above, dividing exactly as the
 // reference does; fast = 1 / 2 (mixed paths): the FP64 / FP32 sweeps of

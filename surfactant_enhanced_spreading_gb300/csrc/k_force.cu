@@ -1171,7 +1171,7 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
 // finish kernel adds the cells of a row and the 9 rows in a fixed order.
 // Which warp takes which item does not change any arithmetic, so results are
 // bit-reproducible.
-// A warp's first item is fixed: warp w of CTA b takes item w * grid + b.  All
+// A warp's first item is fixed (w * grid + b for warp w of CTA b, w rotated).  All
 // CTAs wait together for the predecessor kernel, and taken from the counter
 // the first items went to the 20 to 32 warps of the SMs nearest to it: with
 // fewer items than warps the other SMs had none (3,000 sites in FP64, with
@@ -1212,7 +1212,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, i
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const int nitems = d.near_ctl[1];
-    int k = w * gridDim.x + blockIdx.x;
+    int k = (w + NW - blockIdx.x / GB300_SMS % NW) % NW * gridDim.x + blockIdx.x;   // the CTAs of one SM start on different schedulers
     while (k < nitems) {
         const int2 item = d.near_items[k];
         int next = 0;   // the next item's number, asked for before this one's work

@@ -44,6 +44,7 @@ inline cudaError_t launch_pdl(void (*k)(K...), dim3 grid, dim3 block, size_t sme
     return cudaLaunchKernelEx(&cfg, k, std::forward<A>(args)...);
 }
 
+constexpr int GB300_SMS = 152;
 constexpr int P = 4;
 constexpr int LP = 25;        // (P+1)^2 coefficients
 constexpr int LPH = 15;       // coefficients with m >= 0
