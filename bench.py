@@ -43,11 +43,10 @@ FLOPS_LJ_EXTRA = 11   # added when the pair is LJ-active within rc
 FLOPS_L2P = 25 * 40   # local-expansion force per site
 # kernels launched per step on the configuration preset's mixed path (gather;
 # graphite and chain terms on the side stream; pair field + finish; site
-# forces; waters' constraint half, chains' half and the eta update for
-# move_a; the two constraint halves for move_b) and per rebuild step (cell
-# location, sort 3, work items 5, correction masks, graphite list, water
-# order 3, P2M, 2 M2M, multipole packing, 2 M2L, 2 L2L)
-LAUNCHES_STEP, LAUNCHES_REBUILD = 11, 22
+# forces; SHAKE half and eta update; RATTLE half) and per rebuild step (cell
+# location, sort 3, work items 2, correction masks, graphite list, water
+# order 3, P2M, 2 M2M, 2 M2L, 2 L2L)
+LAUNCHES_STEP, LAUNCHES_REBUILD = 9, 18
 
 
 def parse(argv=None):

@@ -1012,7 +1012,8 @@ struct CPlan {
     int s_warps;        // surfactant warps in each of them
     int mpw;            // surfactants per warp (groups of 4 lanes), 1..MPW
     int nmol, nsite;    // bounds every listed molecule is checked against
-    int mat;            // waters in matrix form (configuration preset, FP64 corrections)
+    const int *chains;  // flexible chains advanced by the same launch (k_water_mat)
+    int nch;
 };
 
 // a listed molecule with its nsites sites inside the state arrays; a list
@@ -1066,7 +1067,6 @@ __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double
     if (!surf_cta || warp < p.s_warps) {
         // (FP32 sweeps are no FP64 queue: 5,000 waters ran 51 us from the
         // counter alone, 58 spread over all SMs)
-        const double thr[3] = {cF.dsq64_w[0] * (2.0 * tol), cF.dsq64_w[1] * (2.0 * tol), cF.dsq64_w[2] * (2.0 * tol)};
         const unsigned free_ctas = sizeof(C) == 8 ? gridDim.x - p.n_scta : 0;
         for (bool first = !surf_cta && free_ctas;; first = false) {
             const unsigned item = water_item(p, lane, first, warp * free_ctas + blockIdx.x - p.n_scta, CW * free_ctas);
@@ -1079,11 +1079,7 @@ __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double
                     atomicAdd(&d.counters[7], 1ull);
                     continue;
                 }
-                int sweeps;
-                if (std::is_same<C, double>::value && p.mat)
-                    sweeps = SHAKE ? water_a_mat(d, m, thr, maxit) : water_b_mat(d, m, tol, maxit);
-                else
-                    sweeps = SHAKE ? water_a<C>(d, m, tol, maxit) : water_b<C>(d, m, tol, maxit);
+                const int sweeps = SHAKE ? water_a<C>(d, m, tol, maxit) : water_b<C>(d, m, tol, maxit);
                 p.wsw[m] = (uint8_t)(sweeps < 255 ? sweeps : 255);
             }
         }
@@ -1097,11 +1093,54 @@ __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double
     }
 }
 
+// Two flexible chains (SHAKE half) or 32 beads (RATTLE half) by a warp: the
+// operations of k_move_free_a and k_move_free_b, in their order.
+__device__ __forceinline__ void chains_a(const Dev &d, const CPlan &p, int pair, int lane) {
+    const int q = 2 * pair + (lane >> 4), i = lane & 15;
+    double ke0 = 0.0, ke1 = 0.0;
+    int m = 0;
+    if (q < p.nch) m = p.chains[q];
+    if (q < p.nch && i < NCH) {
+        const int g = d.mfirst[m] + i;
+        const double escale = __dsub_rn(1.0, __dmul_rn(d.eta[d.mrep[m]], DT) * 0.5), mi = d.tmass[d.ptype[g]];
+        const double vx = d.vx[g], vy = d.vy[g], vz = d.vz[g], ax = d.ax[g], ay = d.ay[g], az = d.az[g];
+        ke0 = __dmul_rn(mi, __dadd_rn(__dadd_rn(__dmul_rn(vx, vx), __dmul_rn(vy, vy)), __dmul_rn(vz, vz)));
+        d.x[g] = pred_a(d.x[g], vx, ax, escale);
+        d.y[g] = pred_a(d.y[g], vy, ay, escale);
+        d.z[g] = pred_a(d.z[g], vz, az, escale);
+        const double ux = vel_a(vx, ax, escale), uy = vel_a(vy, ay, escale), uz = vel_a(vz, az, escale);
+        d.vx[g] = ux; d.vy[g] = uy; d.vz[g] = uz;
+        ke1 = __dmul_rn(mi, __dadd_rn(__dadd_rn(__dmul_rn(ux, ux), __dmul_rn(uy, uy)), __dmul_rn(uz, uz)));
+    }
+    for (int o = 8; o > 0; o >>= 1) {
+        ke0 = __dadd_rn(ke0, __shfl_xor_sync(FULL, ke0, o));
+        ke1 = __dadd_rn(ke1, __shfl_xor_sync(FULL, ke1, o));
+    }
+    if (q < p.nch && i == 0) {
+        d.ke[2 * m] = ke0;
+        d.ke[2 * m + 1] = ke1;
+    }
+}
+__device__ __forceinline__ void chains_b(const Dev &d, const CPlan &p, int item, int lane) {
+    const int t = 32 * item + lane;
+    if (t >= p.nch * NCH) return;
+    const int m = p.chains[t / NCH], g = d.mfirst[m] + t % NCH;
+    const double escale = __ddiv_rn(2.0, __dadd_rn(2.0, __dmul_rn(d.eta[d.mrep[m]], DT))), mi = d.tmass[d.ptype[g]];
+    const double ax = __ddiv_rn(__dmul_rn(d.fx[g], DTSQ2), mi), ay = __ddiv_rn(__dmul_rn(d.fy[g], DTSQ2), mi),
+                 az = __ddiv_rn(__dmul_rn(d.fz[g], DTSQ2), mi);
+    d.ax[g] = ax; d.ay[g] = ay; d.az[g] = az;
+    d.vx[g] = __dmul_rn(escale, __dadd_rn(d.vx[g], ax));
+    d.vy[g] = __dmul_rn(escale, __dadd_rn(d.vy[g], ay));
+    d.vz[g] = __dmul_rn(escale, __dadd_rn(d.vz[g], az));
+}
+
 // Configuration preset, mixed path: its chains carry no constraints, so the
 // half is the water queue of k_constrain alone (matrix form), in a kernel
 // without the surfactant wavefront's registers and shared memory: several
 // CTAs per SM instead of one, to hide the FP64 latency of the per-water
-// chains.  Same queue, same per-water arithmetic, same counter reset.
+// chains.  Same queue, same per-water arithmetic, same counter reset.  The
+// flexible chains are the queue's last items (a launch of their own took 6 us
+// of the SHAKE half and 8 of the RATTLE half).
 template <bool SHAKE>
 __global__ void __launch_bounds__(CW_THREADS) k_water_mat(Dev d, CPlan p, double tol, int maxit) {
     griddep_wait();
@@ -1113,7 +1152,13 @@ __global__ void __launch_bounds__(CW_THREADS) k_water_mat(Dev d, CPlan p, double
     for (bool first = true;; first = false) {
         const unsigned item = water_item(p, lane, first, rank * gridDim.x + blockIdx.x, CW * gridDim.x);
         const long long t0 = 32LL * item;
-        if (t0 >= p.nw) break;
+        if (t0 >= p.nw) {
+            const int k = (int)(item - (p.nw + 31) / 32);
+            if (k >= (SHAKE ? (p.nch + 1) / 2 : (p.nch * NCH + 31) / 32)) break;
+            if constexpr (SHAKE) chains_a(d, p, k, lane);
+            else chains_b(d, p, k, lane);
+            continue;
+        }
         const int t = (int)t0 + lane;
         if (t < p.nw) {
             const int m = p.wlist[t];
@@ -1232,9 +1277,10 @@ constexpr size_t surf_smem(int s_warps, int mpw) {
 
 template <typename C, bool SHAKE>
 void launch_constrain_t(const Dev &d, const int *smols, int ns, int nw, int nmol, int nsite, const ConstraintShape &sh,
-                        double tol, int maxit, cudaStream_t st, int mat) {
+                        double tol, int maxit, cudaStream_t st, int mat, const int *chains = nullptr, int nch = 0) {
     CPlan p;
-    p.mat = mat;
+    p.chains = chains;
+    p.nch = nch;
     p.smols = smols;
     p.wlist = SHAKE ? d.wlist_a : d.wlist_b;
     p.wsw = SHAKE ? d.wsw_a : d.wsw_b;
@@ -1248,7 +1294,7 @@ void launch_constrain_t(const Dev &d, const int *smols, int ns, int nw, int nmol
     const int groups = (ns + p.mpw - 1) / p.mpw;
     const int need = (groups + p.s_warps - 1) / p.s_warps;
     p.n_scta = ns ? (need < sh.grid ? need : sh.grid) : 0;
-    if (std::is_same<C, double>::value && mat && ns == 0) {
+    if (mat) {
         // waters only, in matrix form: as many CTAs per SM as fit
         const int occ = g_water_mat_ctas[SHAKE ? 1 : 0] > 0 ? g_water_mat_ctas[SHAKE ? 1 : 0] : 1;
         launch_pdl(k_water_mat<SHAKE>, dim3(sh.grid * occ), dim3(CW_THREADS), 0, st, d, p, tol, maxit);
@@ -1274,17 +1320,25 @@ void init_constraint_kernels() {
 
 // fp32: 1 for FP32 sweeps, 0 for FP64 sweeps
 void launch_move_a32(const Dev &d, int nw, const int *smols, int ns, int nmol, int nsite, const ConstraintShape &sh,
-                     cudaStream_t st, double tol, int maxit, int fp32, int mat) {
+                     cudaStream_t st, double tol, int maxit, int fp32) {
     if (!nw && !ns) return;
     if (fp32) launch_constrain_t<float, true>(d, smols, ns, nw, nmol, nsite, sh, tol, maxit, st, 0);
-    else launch_constrain_t<double, true>(d, smols, ns, nw, nmol, nsite, sh, tol, maxit, st, mat);
+    else launch_constrain_t<double, true>(d, smols, ns, nw, nmol, nsite, sh, tol, maxit, st, 0);
+}
+void launch_move_a_mat(const Dev &d, int nw, const int *chains, int nch, int nmol, int nsite, const ConstraintShape &sh,
+                       cudaStream_t st, double tol, int maxit) {
+    if (nw || nch) launch_constrain_t<double, true>(d, nullptr, 0, nw, nmol, nsite, sh, tol, maxit, st, 1, chains, nch);
 }
 
 void launch_move_b32(const Dev &d, int nw, const int *smols, int ns, int nmol, int nsite, const ConstraintShape &sh,
-                     cudaStream_t st, double tol, int maxit, int fp32, int mat) {
+                     cudaStream_t st, double tol, int maxit, int fp32) {
     if (!nw && !ns) return;
     if (fp32) launch_constrain_t<float, false>(d, smols, ns, nw, nmol, nsite, sh, tol, maxit, st, 0);
-    else launch_constrain_t<double, false>(d, smols, ns, nw, nmol, nsite, sh, tol, maxit, st, mat);
+    else launch_constrain_t<double, false>(d, smols, ns, nw, nmol, nsite, sh, tol, maxit, st, 0);
+}
+void launch_move_b_mat(const Dev &d, int nw, const int *chains, int nch, int nmol, int nsite, const ConstraintShape &sh,
+                       cudaStream_t st, double tol, int maxit) {
+    if (nw || nch) launch_constrain_t<double, false>(d, nullptr, 0, nw, nmol, nsite, sh, tol, maxit, st, 1, chains, nch);
 }
 
 void launch_water_order(const Dev &d, const int *wmols, int nw, cudaStream_t st) {

@@ -829,13 +829,17 @@ static int move_blocks(int nw, int ns) {
 void launch_move_a(const Dev &d, const int *wmols, int nw, const int *smols, int ns, int nrep, int nmol, int nsite,
                    double tol, int maxit, int fast, const ConstraintShape &sh, int chains, cudaStream_t st) {
     if (chains) {   // flexible chains: constraints on the waters only
-        if (fast) launch_move_a32(d, nw, smols, 0, nmol, nsite, sh, st, tol, maxit, fast == 2, 1);
+        if (fast && fast != 2) {
+            launch_move_a_mat(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit);
+            return;
+        }
+        if (fast) launch_move_a32(d, nw, smols, 0, nmol, nsite, sh, st, tol, maxit, 1);
         else if (nw) k_move_a<<<move_blocks(nw, 0), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, 0, tol, maxit);
         if (ns) k_move_free_a<<<(ns * 16 + 127) / 128, 128, 0, st>>>(d, smols, ns);
         return;
     }
     if (fast) {
-        launch_move_a32(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit, fast == 2, 0);
+        launch_move_a32(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit, fast == 2);
     } else {
         if (nw + ns) k_move_a<<<move_blocks(nw, ns), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, ns, tol, maxit);
     }
@@ -844,13 +848,17 @@ void launch_eta(const Dev &d, int nrep, cudaStream_t st) { k_eta<<<nrep * ETA_BL
 void launch_move_b(const Dev &d, const int *wmols, int nw, const int *smols, int ns, int nmol, int nsite, double tol,
                    int maxit, int fast, const ConstraintShape &sh, int chains, cudaStream_t st) {
     if (chains) {
-        if (fast) launch_move_b32(d, nw, smols, 0, nmol, nsite, sh, st, tol, maxit, fast == 2, 1);
+        if (fast && fast != 2) {
+            launch_move_b_mat(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit);
+            return;
+        }
+        if (fast) launch_move_b32(d, nw, smols, 0, nmol, nsite, sh, st, tol, maxit, 1);
         else if (nw) k_move_b<<<move_blocks(nw, 0), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, 0, tol, maxit);
         if (ns) k_move_free_b<<<(ns * NCH + 255) / 256, 256, 0, st>>>(d, smols, ns);
         return;
     }
     if (fast) {
-        launch_move_b32(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit, fast == 2, 0);
+        launch_move_b32(d, nw, smols, ns, nmol, nsite, sh, st, tol, maxit, fast == 2);
     } else {
         if (nw + ns) k_move_b<<<move_blocks(nw, ns), MOVE_BLOCK, 0, st>>>(d, wmols, nw, smols, ns, tol, maxit);
     }

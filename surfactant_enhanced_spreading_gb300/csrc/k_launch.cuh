@@ -32,12 +32,16 @@ void launch_eta(const Dev &d, int nrep, cudaStream_t st);
 // k_constraint.cu (mixed paths: FP64 or FP32 sweeps); false if the uploaded
 // bond graph is not the one the kernels are specialised for
 bool upload_tables_fast(const Tables &t, cudaStream_t st);
-// mat: waters as the 3 x 3 system of their constraints (matrix SHAKE /
-// RATTLE; the configuration preset's FP64 corrections)
 void launch_move_a32(const Dev &d, int nw, const int *smols, int ns, int nmol, int nsite, const ConstraintShape &sh,
-                     cudaStream_t st, double tol, int maxit, int fp32, int mat);
+                     cudaStream_t st, double tol, int maxit, int fp32);
 void launch_move_b32(const Dev &d, int nw, const int *smols, int ns, int nmol, int nsite, const ConstraintShape &sh,
-                     cudaStream_t st, double tol, int maxit, int fp32, int mat);
+                     cudaStream_t st, double tol, int maxit, int fp32);
+// the configuration preset's: waters as the 3 x 3 system of their constraints
+// (matrix SHAKE / RATTLE, FP64 corrections), and its flexible chains
+void launch_move_a_mat(const Dev &d, int nw, const int *chains, int nch, int nmol, int nsite, const ConstraintShape &sh,
+                       cudaStream_t st, double tol, int maxit);
+void launch_move_b_mat(const Dev &d, int nw, const int *chains, int nch, int nmol, int nsite, const ConstraintShape &sh,
+                       cudaStream_t st, double tol, int maxit);
 // reorders the halves' water lists by the sweeps of their last call (at list rebuilds)
 void launch_water_order(const Dev &d, const int *wmols, int nw, cudaStream_t st);
 int constraint_max_surf_warps();
