@@ -970,30 +970,57 @@ __device__ __forceinline__ double scale_to_double(u64 w, int ex) {
     const u64 m = w << lz;
     return __longlong_as_double((long long)(((u64)(1023 + 63 - 1 - lz + ex) << 52) + (m >> 11) + ((m >> 10) & 1)));
 }
-__device__ __forceinline__ u64 fix_r2(long long x, long long y, long long z) {
-    const int hx = (int)(x >> 32), hy = (int)(y >> 32), hz = (int)(z >> 32);
-    const unsigned lx = (unsigned)x, ly = (unsigned)y, lz = (unsigned)z;
-    const u64 s = (u64)((long long)hx * hx) + (u64)((long long)hy * hy) + (u64)((long long)hz * hz);
-    const long long c = (long long)hx * (int)(lx >> 1) + (long long)hy * (int)(ly >> 1) + (long long)hz * (int)(lz >> 1);
-    const u64 q = (u64)__umulhi(lx, lx) + __umulhi(ly, ly) + __umulhi(lz, lz);
-    return (s << 2) + (u64)(c >> 28) + (q >> 30);
+// a difference's halves: h 2^32 + 2 l, with l signed (its low 7 bits are zero)
+struct Fix {
+    int h, l;
+    __device__ __forceinline__ explicit Fix(long long v) : h((int)(v >> 32) + (int)((unsigned)v >> 31)), l((int)(unsigned)v >> 1) {}
+};
+// (l^2 is left out, three units at most, and its mean is in the constant)
+__device__ __forceinline__ u64 fix_r2(const Fix &x, const Fix &y, const Fix &z) {
+    const u64 s = (u64)((long long)x.h * x.h) + (u64)((long long)y.h * y.h) + (u64)((long long)z.h * z.h);
+    const long long c = (long long)x.h * x.l + (long long)y.h * y.l + (long long)z.h * z.l + 3ll * (1 << 27);
+    return (s << 2) + (u64)(c >> 28);
 }
-// r^-3 and, with LJ, r^-2 of r2 >= 2^32
-template <bool LJ>
-__device__ __forceinline__ void fix_inverse(u64 r2, double &i3, double &i2) {
-    const int lz = __clz((unsigned)(r2 >> 32)) & ~1;
-    const u64 n = r2 << lz;
+// r^-3 of r2 >= 2^53 as w 2^(3 lz / 2 - 70), and what r^-2 takes
+struct FixInv {
+    u64 w, mm, e60;
+    unsigned e2;
+    int lz;
+};
+__device__ __forceinline__ FixInv fix_inverse(u64 r2) {
+    FixInv v;
+    v.lz = __clz((unsigned)(r2 >> 32) | 1u << 21) & ~1;
+    const u64 n = r2 << v.lz;
     const unsigned n1 = (unsigned)(n >> 32), n0 = (unsigned)n;
     const float y = rsqrt_ftz(__uint2float_rn(n1));                      // 2^-15 / sqrt(n / 2^62)
     const unsigned m = __float2uint_rz(y * (float)(70368744177664.0 * (1.0 - 1.5 / 4194304.0)));   // 2^31 y, low by 3.6e-7
-    const u64 mm = (u64)m * m, m2 = mm >> 12;                            // 2^62 y^2, exact; 2^50 y^2
+    v.mm = (u64)m * m;                                                   // 2^62 y^2, exact
+    const u64 m2 = v.mm >> 12;                                           // 2^50 y^2
     const unsigned l = (unsigned)m2, h = (unsigned)(m2 >> 32);
     const u64 t = (u64)n1 * l + (u64)n0 * h + __umulhi(n0, l) + ((u64)(n1 * h) << 32);   // 2^80 (1 - e), modulo 2^64
-    const u64 e = 0ull - t, e60 = e >> 20;                               // 2^80 e, 2^60 e
-    const unsigned e2 = __umulhi((unsigned)(e >> 32), (unsigned)(e >> 32));   // 2^64 e^2
-    const u64 m3 = (u64)(unsigned)(mm >> 32) * m + __umulhi((unsigned)mm, m);   // 2^61 y^3
-    i3 = scale_to_double(m3 + __umul64hi(m3, (e60 + (e60 >> 1) + ((e2 * 15u) >> 7)) << 4), -70 + 3 * (lz >> 1));
-    if constexpr (LJ) i2 = scale_to_double(mm + __umul64hi(mm, (e60 + (e2 >> 4)) << 4), -68 + lz);
+    const u64 e = 0ull - t;                                              // 2^80 e
+    v.e60 = e >> 20;
+    v.e2 = __umulhi((unsigned)(e >> 32), (unsigned)(e >> 32));           // 2^64 e^2
+    const u64 m3 = (u64)(unsigned)(v.mm >> 32) * m + __umulhi((unsigned)v.mm, m);   // 2^61 y^3
+    const u64 k = (v.e60 + (v.e60 >> 1) + ((v.e2 * 15u) >> 7)) << 4;     // 2^64 e (3/2 + 15/8 e) < 2^46
+    const unsigned kh = (unsigned)(k >> 32), kl = (unsigned)k, mh = (unsigned)(m3 >> 32), ml = (unsigned)m3;
+    v.w = m3 + (u64)mh * kh + (((u64)mh * kl + (u64)ml * kh) >> 32);
+    return v;
+}
+// r^-3 in units of 2^-57, to nearest: h 2^31 + l
+struct FixTerm {
+    int h, l;
+    __device__ __forceinline__ explicit FixTerm(const FixInv &v) {
+        const int k = v.lz + (v.lz >> 1);   // 3 lz / 2 <= 15
+        const u64 w = (v.w + (4096u >> k)) << 2;
+        const unsigned wh = (unsigned)(w >> 32), t0 = __funnelshift_r((unsigned)w, wh, 15 - k), t1 = wh >> (15 - k);
+        h = (int)__funnelshift_l(t0, t1, 1); l = (int)(t0 & 0x7fffffffu);
+    }
+};
+// a += the product of a difference and r^-3, in units of 2^-53, to nearest
+__device__ __forceinline__ void fix_add(long long &a, const Fix &x, const FixTerm &t) {
+    const long long c = (long long)x.h * t.l + (long long)x.l * t.h + (1 << 30);
+    a += (long long)x.h * t.h + (c >> 31);
 }
 
 // r^-3 and r^-2 of a close pair, in FP64
@@ -1024,39 +1051,53 @@ __device__ __forceinline__ double near_lj64(double ft, double2 p, bool in, doubl
     return fma(((in ? p.x : 0.0) * i6) * fma(p.y, i6, -0.5), i2, ft);
 }
 
-// The pairs of one staged block.  LJ: 0 Coulomb of a run with one charge
-// (unscaled), 1 water-O partners with LJ, 2 any partners.  Partners of the
-// target's own molecule, and the target itself, are left out.
+// The pairs of one staged block.  LJ: 0 Coulomb of a run with one charge, 1
+// water-O partners with LJ, 2 any partners.  Partners of the target's own
+// molecule, and the target itself, are left out.  S: the unscaled Coulomb sum
+// of runs with one charge; f: all else, scaled except with LJ 0.
 template <int LJ>
 __device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const Stage64 &s, int n, const double2 *ljt,
-                                             double (&f)[3]) {
+                                             double (&S)[3], double (&f)[3]) {
     const u64 rc2 = (u64)(RC * RC * 72057594037927936.0);   // 2^56
+    long long a[3] = {0, 0, 0};   // at most 32 terms of 8 (2^56)
 #pragma unroll 1
     for (int k = 0; k < n; k++) {
         const long long x = t.x - s.x[k], y = t.y - s.y[k], z = t.z - s.z[k];
         const int key = s.key[k];
         const bool same = (key >> 5) == t.m;
-        const u64 r2 = fix_r2(x, y, z);
-        double i3, i2 = 0.0;
-        fix_inverse<LJ != 0>(r2, i3, i2);
-        const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
-        const bool close = r2 < FIX_NEAR2 && !same;
-        if (__any_sync(0xffffffffu, close)) {
-            if (close) {
-                const double2 v = near_inverse(dx, dy, dz);
-                i3 = v.x; i2 = v.y;
+        const Fix X(x), Y(y), Z(z);
+        const u64 r2 = fix_r2(X, Y, Z);
+        const FixInv v = fix_inverse(r2);
+        const bool close = r2 < FIX_NEAR2;
+        if constexpr (LJ != 2) {
+            FixTerm w(v);
+            if (same || close) w.h = w.l = 0;
+            fix_add(a[0], X, w); fix_add(a[1], Y, w); fix_add(a[2], Z, w);
+        }
+        const bool cl = close && !same, in = LJ != 0 && !same && r2 <= rc2;
+        if (LJ == 2 || __any_sync(0xffffffffu, cl || in)) {
+            const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
+            double i3 = 0.0, i2 = 0.0;
+            if (LJ != 0) {
+                i3 = scale_to_double(v.w, -70 + 3 * (v.lz >> 1));
+                i2 = scale_to_double(v.mm + __umul64hi(v.mm, (v.e60 + (v.e2 >> 4)) << 4), -68 + v.lz);
             }
+            if (cl) {
+                const double2 u = near_inverse(dx, dy, dz);
+                i3 = u.x; i2 = u.y;
+            }
+            double ft;
+            if constexpr (LJ == 0) ft = cl ? i3 : 0.0;
+            if constexpr (LJ == 1) ft = cl ? qq * i3 : 0.0;
+            if constexpr (LJ == 2) ft = same ? 0.0 : qq * s.q[k] * i3;
+            if constexpr (LJ != 0)
+                if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], in, i3, i2);
+            near_sum64(f, dx, dy, dz, ft);
         }
-        double ft = same ? 0.0 : i3;
-        if constexpr (LJ != 0) {
-            const bool in = !same && r2 <= rc2;
-            const double i = ft;
-            double c = qq;
-            if constexpr (LJ == 2) c *= s.q[k];
-            ft = c * i;
-            if (__any_sync(0xffffffffu, in)) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], in, i, i2);
-        }
-        near_sum64(f, dx, dy, dz, ft);
+    }
+    if constexpr (LJ != 2) {
+#pragma unroll
+        for (int b = 0; b < 3; b++) S[b] = fma((double)a[b], 0x1p-53, S[b]);
     }
 }
 
@@ -1128,7 +1169,7 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
             if (a == b) continue;
             const bool one = g == 0 && lj;
             const double qq = g == 1 ? t.q : t.q * (g ? qh : qo);
-            double f[3] = {0.0, 0.0, 0.0};
+            double S[3] = {0.0, 0.0, 0.0}, f[3] = {0.0, 0.0, 0.0};
             if (far) {
                 if (i < ni) {
                     const double4 p = d.srt_pos[s0 + i];
@@ -1147,13 +1188,13 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
                         if (g == 1) st.q[lane] = d.srt_pos[b0 + lane].w;
                     }
                     __syncwarp();
-                    if (g == 1) near_block64<2>(t, qq, st, n, ljt, f);
-                    else if (one) near_block64<1>(t, qq, st, n, ljt, f);
-                    else near_block64<0>(t, qq, st, n, ljt, f);
+                    if (g == 1) near_block64<2>(t, qq, st, n, ljt, S, f);
+                    else if (one) near_block64<1>(t, qq, st, n, ljt, S, f);
+                    else near_block64<0>(t, qq, st, n, ljt, S, f);
                 }
             }
 #pragma unroll
-            for (int k = 0; k < 3; k++) cell[k] = g == 1 || one ? cell[k] + f[k] : fma(qq, f[k], cell[k]);
+            for (int k = 0; k < 3; k++) cell[k] = g == 1 || one ? cell[k] + fma(qq, S[k], f[k]) : fma(qq, S[k] + f[k], cell[k]);
         }
 #pragma unroll
         for (int k = 0; k < 3; k++) row[k] += cell[k];
