@@ -543,7 +543,7 @@ void family(sesp_ctx *c, const char *name) {
 void seq_force(sesp_ctx *c, int rebuild, int terms) {
     const Dev &d = c->d;
     const int mixed = c->p.precision != SESP_PLAIN_FP64;
-    const bool fork = mixed && !c->timing && !c->sync_check;
+    const bool fork = !c->timing && !c->sync_check;
     if (rebuild) {
         tstart(c, 5);
         // sites per cell, then the far field's counts
@@ -571,10 +571,11 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
     launch_gather(d, c->nsite, c->ncell, mixed ? GATHER_MIXED : GATHER_PLAIN, c->st);
     family(c, "gather");
     // graphite and intramolecular terms into the side forces (fside), on the
-    // side stream beside the far-field build and the pair field on the mixed
-    // paths; in order on the main stream on the plain path (its FP64 pair
-    // field beside them ran a batched step at 581 ms against 259 ms in order)
-    // and when kernels are timed or checked one by one
+    // side stream beside the far-field build and the pair field; in order on
+    // the main stream when kernels are timed or checked one by one.  (On the
+    // plain path they are FP64 work beside an integer pair field: steps of
+    // 3,000 sites 457 us in order, 423 beside; reference droplet of
+    // 2,451 sites 439 and 364; 62,400 sites 2,757 and 2,569.)
     if (fork) {
         cudaEventRecord(c->ev_fork, c->st);
         cudaStreamWaitEvent(c->st2, c->ev_fork, 0);
@@ -1473,9 +1474,9 @@ static int launch_steps(sesp_ctx *c, int kb0, int nsteps) {
             if (!ge) {
                 cudaGraph_t g;
                 CK(cudaStreamBeginCapture(c->st, cudaStreamCaptureModeThreadLocal));
-                // on the mixed paths the force call forks its side stream and
-                // joins it before the site forces, which also joins the eta update
-                seq_move_a(c, c->p.precision != SESP_PLAIN_FP64);
+                // the force call forks its side stream and joins it before
+                // the site forces, which also joins the eta update
+                seq_move_a(c, true);
                 seq_force(c, rb, SESP_T_ALL);
                 seq_move_b(c);
                 CK(cudaStreamEndCapture(c->st, &g));
