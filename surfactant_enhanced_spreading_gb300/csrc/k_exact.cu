@@ -177,6 +177,10 @@ constexpr int WATERS_SPLIT = 10;                       // waters of a warp with 
 constexpr int MOVE_SPLIT_MAX = WATERS_SPLIT * 4 * 152;
 constexpr int MOVE_BLOCK = 32;
 
+// a rare division as a call: inlined, the compiler runs it beside the common
+// path for every operand and selects
+__device__ __noinline__ double div_call(double a, double b) { return a / b; }
+
 // a / b, correctly rounded, from y = 1 / b correctly rounded (P. Markstein,
 // IBM J. Res. Dev. 34, 111 (1990)): the first step brings the quotient within
 // an ulp, the second rounds it.  Infinities and NaN take the division.
@@ -184,7 +188,7 @@ __device__ __forceinline__ double div_by(double a, double b, double y) {
     double q = a * y;
     q = fma(fma(-q, b, a), y, q);
     q = fma(fma(-q, b, a), y, q);
-    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = a / b;
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = div_call(a, b);
     return q;
 }
 
@@ -194,7 +198,7 @@ __device__ __forceinline__ double div_dt(double a) {
     constexpr double y = 1.0 / DT;
     double q = a * y;
     q = fma(fma(-q, DT, a), y, q);
-    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = a / DT;
+    if ((__double2hiint(q) & 0x7ff00000) == 0x7ff00000) q = div_call(a, DT);
     return q;
 }
 

@@ -863,7 +863,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.near_far, R)) ||
         (e = dalloc(c, &d.pair_xyz, 3 * pair_max)) || (e = dalloc(c, &d.pair_key, pair_max)) || (e = dalloc(c, &d.crun, 8 * (size_t)C)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
         (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
-        (e = dalloc(c, &d.near_mask, C)) || (e = dalloc(c, &d.srt_cell, N)) || (e = dalloc(c, &d.near_ctl, 66)) ||
+        (e = dalloc(c, &d.near_mask, C)) || (e = dalloc(c, &d.srt_cell, N)) || (e = dalloc(c, &d.near_ctl, 2 + 2 * NEAR_CLASSES)) ||
         (e = dalloc(c, &d.isub, (size_t)c->ssite * nsm)) || (e = dalloc(c, &d.O4, (size_t)LP * C)) ||
         (e = dalloc(c, &d.L4, (size_t)LP * C)) || (e = dalloc(c, &d.L4f, (size_t)LP * C)) ||
         (e = dalloc(c, &d.fside, 3 * (size_t)N)) || (e = dalloc(c, &d.stage, 12 * (size_t)N)) ||
@@ -1279,7 +1279,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         CK(cudaMemcpyAsync(d.ggrp_z, ggrp_z.data(), ggrp_z.size() * sizeof(float2), cudaMemcpyHostToDevice, c->st));
     }
     CK(cudaMemcpyAsync(d.ljt, ljt.data(), ljt.size() * sizeof(double2), cudaMemcpyHostToDevice, c->st));
-    CK(cudaMemsetAsync(d.near_ctl, 0, 66 * sizeof(int), c->st));   // no near-field items before the first rebuild
+    CK(cudaMemsetAsync(d.near_ctl, 0, (2 + 2 * NEAR_CLASSES) * sizeof(int), c->st));   // no near-field items before the first rebuild
     CK(cudaStreamSynchronize(c->st));
     c->uploaded = true;
     c->have_force = false;

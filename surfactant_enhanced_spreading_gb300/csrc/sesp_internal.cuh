@@ -75,6 +75,7 @@ constexpr double DTSQ2 = 0.00127362 * 0.00127362 / 2.0;
 constexpr int M2C_NOFF = 189; // M2L offsets of a cell (6^3 - 3^3 for its parity class)
 constexpr int M2C_LD = 28;    // padded output stride of a real M2L operator row
 constexpr int M2C_W = 4;      // warps of an M2L CTA, 64 targets each (2 per lane)
+constexpr int NEAR_CLASSES = 64;   // cost classes of the pair field's items
 constexpr int M2C_FEW = 16;   // targets of a tile that are taken one per warp
 constexpr int M2C_TILE = 64 * M2C_W, M2C_TILE64 = M2C_FEW;   // targets of a tile, FP32 and FP64
 constexpr int M2C_GROUPS = 21; // offset groups of an M2L work item, 9 offsets each (partial sums added in group order)
@@ -185,7 +186,7 @@ struct Dev {
     int2 *near_items;    // near-field work items (cell, row << 24 | chunk), most expensive first
     int *near_mask;      // per occupied cell: its parts (rows or cells) that have partners
     int *near_ctl;       // [0] items taken past each warp's first in the running launch, [1] item count,
-                         // [2..33] items per cost class, [34..65] next slot per class
+                         // [2..) items per cost class, [2 + NEAR_CLASSES..) next slot per class
     // graphite columns of the bottom layer
     int *gcol_start;
     double4 *gpos;
