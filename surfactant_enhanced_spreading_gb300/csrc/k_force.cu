@@ -1690,8 +1690,12 @@ __device__ __forceinline__ void m2l_acc_s(const C2<R> *__restrict__ H, const S *
 // multipoles, whose zero margin of 2 stands for the cells outside the box.
 // Each offset group writes its partial sums; k_l2l adds the groups in a
 // fixed order.
+// Tiles of a few targets are bound by latency: the sources of a chunk's offsets
+// are read together, beside its operators, which come in 16-byte words (far
+// field of a rebuild, us: 3,000 sites 58 -> 49, 21,400 sites 83 -> 75, 312,000
+// sites 142 -> 133, 62,400 sites in FP64 418 -> 396).
 
-constexpr int M2C_CH = 4;   // operators staged per chunk
+constexpr int M2C_CH = 3;   // operators staged per chunk (a group is nine offsets)
 
 // FP32 rows in Blackwell's paired arithmetic: the operator row's outputs
 // (o, o + 1) against one target's input, one fma.rn.f32x2 for both outputs
@@ -1757,9 +1761,11 @@ __global__ void __launch_bounds__(32 * M2C_W) k_m2l_cls(Dev d, int ncell) {
     auto stage = [&](int c0) {   // the operators of offsets c0.. of the group; returns how many
         const int nch = min(M2C_CH, k1 - c0);
         __syncthreads();
-        for (int idx = threadIdx.x; idx < nch * LP * M2C_LD; idx += blockDim.x) {
-            const int kk = idx / (LP * M2C_LD);
-            sop[idx] = rop[(size_t)offs[c0 + kk] * (LP * M2C_LD) + (idx - kk * (LP * M2C_LD))];
+        constexpr int NV = LP * M2C_LD * sizeof(R) / 16;   // 16-byte words of an operator
+        static_assert(LP * M2C_LD * sizeof(R) % 16 == 0, "operators are copied in 16-byte words");
+        for (int idx = threadIdx.x; idx < nch * NV; idx += blockDim.x) {
+            const int kk = idx / NV;
+            ((uint4 *)sop)[idx] = ((const uint4 *)rop)[(size_t)offs[c0 + kk] * NV + (idx - kk * NV)];
         }
         __syncthreads();
         return nch;
@@ -1780,20 +1786,28 @@ __global__ void __launch_bounds__(32 * M2C_W) k_m2l_cls(Dev d, int ncell) {
             at[j] = pidx(list[min(w + M2C_W * j, cnt - 1)]);
         }
         for (int c0 = k0; c0 < k1; c0 += M2C_CH) {
+            // the sources of the chunk's offsets, all under way beside the operators
+            R v[M2C_CH][NT];
+#pragma unroll
+            for (int kk = 0; kk < M2C_CH; kk++)
+                if (c0 + kk < k1) {
+                    const R *src = src_of(c0 + kk) + (size_t)min(lane, LP - 1) * vol;
+#pragma unroll
+                    for (int j = 0; j < NT; j++)
+                        if (w + M2C_W * j < cnt) v[kk][j] = src[at[j]];
+                }
             const int nch = stage(c0);
-            for (int kk = 0; kk < nch; kk++) {
-                const R *src = src_of(c0 + kk) + (size_t)min(lane, LP - 1) * vol;
-                const R *op = sop + kk * LP * M2C_LD + min(lane, LP - 1);
-                R v[NT];
 #pragma unroll
-                for (int j = 0; j < NT; j++)
-                    if (w + M2C_W * j < cnt) v[j] = src[at[j]];
+            for (int kk = 0; kk < M2C_CH; kk++)
+                if (kk < nch) {
+                    const R *op = sop + kk * LP * M2C_LD + min(lane, LP - 1);
 #pragma unroll
-                for (int j = 0; j < NT; j++)
-                    if (w + M2C_W * j < cnt)
+                    for (int j = 0; j < NT; j++)
+                        if (w + M2C_W * j < cnt)
 #pragma unroll
-                        for (int i = 0; i < LP; i++) acc[j] = fma(op[i * M2C_LD], __shfl_sync(0xffffffffu, v[j], i), acc[j]);
-            }
+                            for (int i = 0; i < LP; i++)
+                                acc[j] = fma(op[i * M2C_LD], __shfl_sync(0xffffffffu, v[kk][j], i), acc[j]);
+                }
         }
         if (lane < LP)
 #pragma unroll
