@@ -466,10 +466,13 @@ int dalloc(sesp_ctx *c, T **p, size_t n) {
 
 // Systems up to this size run the pair field with one work item per partner
 // cell (27 partials per site) instead of per row of three (9): a small system
-// has too few rows to fill the GPU (us per call, rows against cells: 3,000
-// sites 30.9 / 26.6, FP64 614 / 317; 21,400 sites 69.2 / 63.6; 62,400 sites
-// 142.6 / 150.7).
-constexpr int NEAR_SPLIT_MAX = 40000;
+// has too few rows to fill the GPU.  The field alone gains up to 45,000 sites
+// (us, rows against cells: 3,000 sites 30.9 / 26.6, FP64 614 / 317; 21,400
+// sites 64.9 / 57.1; 62,400 sites 142.6 / 150.7), a step with the graphite and
+// chain kernels beside it up to 15,000 (16,450 sites 162.8 / 164.1, 21,400
+// sites 96.5 / 99.7, 38,700 sites 131.8 / 139.4; FP64 36,600 sites 1,421 /
+// 1,445).
+constexpr int NEAR_SPLIT_MAX = 20000;
 // work items of the pair field: 9 rows (or 27 cells) x the chunks of every
 // occupied cell (LJ-carrying sites and water H, each rounded up to 32s)
 size_t near_items_max(int nsite, int ncell) {

@@ -113,7 +113,7 @@ def estimate_bytes(system: S.System) -> int:
     w2 = 2 * d2 + 1
     # pair field: partials of 9 rows, or of 27 cells in small contexts; its
     # work items and the padded partner layout
-    parts = 27 if n <= 40000 else 9
+    parts = 27 if n <= 20000 else 9
     per_site = 12 * 8 + 1 + 4 * 4 + 32 + 16 + 8 + 4 + 3 * 8 + parts * 3 * 8 + 6 + 3 * 8 + 12 * 8 + 4 + 16 + 24 + parts * 8 / 32 + 4
     per_mol = 5 * 4 + 2 * 8 + 4 + 4 + 2 * 4 + 2   # incl. the constraint halves' water lists and sweep counts
     cz = 25 * 16
