@@ -431,7 +431,7 @@ struct sesp_ctx {
     // beside the far-field build and the pair field (fork after the gather,
     // join before the site forces)
     cudaStream_t st2 = nullptr;
-    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_eta = nullptr, ev_list = nullptr;
+    cudaEvent_t ev_fork = nullptr, ev_join = nullptr, ev_eta = nullptr, ev_list = nullptr, ev_items = nullptr;
     NearShape near = {64, 0};   // pair-field launch shape (autotuned or set; results do not depend on it)
     ConstraintShape cshape = {0, 4, 1};   // constraint halves of the mixed paths (likewise)
     int n_sm = 0;               // streaming multiprocessors of the device
@@ -567,8 +567,14 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
         family(c, "water order");
         launch_sort(d, c->nsite, c->ncell, c->st);
         family(c, "cell sort");
-        launch_near_items(d, c->ncell, c->near.tile, c->st);
+        // the pair field's items, beside the far-field build
+        if (fork) {
+            cudaEventRecord(c->ev_list, c->st);
+            cudaStreamWaitEvent(c->st2, c->ev_list, 0);
+        }
+        launch_near_items(d, c->ncell, c->near.tile, ls);
         family(c, "near-field items");
+        if (fork) cudaEventRecord(c->ev_items, c->st2);
         tstop(c, 5);
     }
     launch_gather(d, c->nsite, c->ncell, mixed ? GATHER_MIXED : GATHER_PLAIN, c->st);
@@ -592,6 +598,7 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
         family(c, "far-field build");
         tstop(c, 6);
     }
+    if (rebuild && fork) cudaStreamWaitEvent(c->st, c->ev_items, 0);
     tstart(c, 0);
     launch_near(d, c->ncell, c->nsite, near_mode(c), terms, c->near, c->st, false, c->chains);
     family(c, "near field");
@@ -708,6 +715,7 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_eta, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_list, cudaEventDisableTiming) != cudaSuccess ||
+        cudaEventCreateWithFlags(&c->ev_items, cudaEventDisableTiming) != cudaSuccess ||
         cudaHostAlloc(&c->host_values, HOST_VALUES * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
         cudaHostGetDevicePointer((void **)&c->host_values_dev, c->host_values, 0) != cudaSuccess) {
         delete c;
@@ -752,6 +760,7 @@ int sesp_destroy(sesp_ctx *c) {
     cudaEventDestroy(c->ev_join);
     cudaEventDestroy(c->ev_eta);
     cudaEventDestroy(c->ev_list);
+    cudaEventDestroy(c->ev_items);
     cudaStreamDestroy(c->st2);
     cudaStreamDestroy(c->st);
     cudaFreeHost(c->host_values);
