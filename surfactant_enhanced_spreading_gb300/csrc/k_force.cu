@@ -1593,7 +1593,7 @@ __global__ void __launch_bounds__(128) k_m2m(Dev d, const OP *ops, int level) {
 // group order.  L4 is kept in FP64 (energies) with an FP32 copy for the mixed
 // path's L2P.
 template <typename R, typename OP>
-__global__ void __launch_bounds__(128) k_l2l(Dev d, const OP *ops, int level, int G) {
+__global__ void __launch_bounds__(128) k_l2l(Dev d, const OP *ops, int level) {
     griddep_wait();
     const int *list = level == 3 ? d.occ3 : d.occ4;
     const int nocc = occ_counts(d)[level == 3 ? 1 : 0];
@@ -1616,14 +1616,18 @@ __global__ void __launch_bounds__(128) k_l2l(Dev d, const OP *ops, int level, in
         const int cx = l % nc[0], cy = (l / nc[0]) % nc[1], cz = l / (nc[0] * nc[1]);
         const int ch = (cx & 1) + 2 * (cy & 1) + 4 * (cz & 1);
         const int pi = base_p + cx / 2 + np[0] * (cy / 2 + np[1] * (cz / 2));
+        // the groups' partial sums, all under way beside the parent's expansion
+        // (loads of seven at a time after it: a rebuild 5 us slower)
+        R pre = 0, pim = 0, gr[M2C_GROUPS], gi[M2C_GROUPS];
+        const R *pb = part + (size_t)b * M2C_GROUPS * LP, *qb = pb + (k > 0 ? LPH + o - (j + 1) : o);
+#pragma unroll
+        for (int g = 0; g < M2C_GROUPS; g++) { gr[g] = pb[g * LP + o]; gi[g] = qb[g * LP]; }
         R re = 0, im = 0;
         apply_op_r<R>(ops + ((size_t)ch * LPH + o) * LP, Lp + (size_t)pi * LP, re, im);
-        R pre = 0, pim = 0;
-        const R *pb = part + (size_t)b * G * LP;
-#pragma unroll 7
-        for (int g = 0; g < G; g++) {
-            pre += pb[g * LP + o];
-            if (k > 0) pim += pb[g * LP + LPH + o - (j + 1)];
+#pragma unroll
+        for (int g = 0; g < M2C_GROUPS; g++) {
+            pre += gr[g];
+            if (k > 0) pim += gi[g];
         }
         if (level == 3) {
             store_jk((C2<R> *)d.L3 + (size_t)b * LP, o, re + pre, im + pim);
@@ -1736,7 +1740,8 @@ __global__ void __launch_bounds__(32 * M2C_W) k_m2l_cls(Dev d, int ncell) {
     if (cnt <= 0) return;
     const Rep r = d.rep[q];
     const int *list = d.fm_list + class_list(r, level, cls, ncell) + t0;
-    const int G = d.m2c_groups, g = blockIdx.y;
+    constexpr int G = M2C_GROUPS;
+    const int g = blockIdx.y;
     const int k0 = g * M2C_NOFF / G, k1 = (g + 1) * M2C_NOFF / G;
     const int div = level == 4 ? 2 : 4;   // class grid = nc / div
     const int h0 = r.nc[0] / div, h1 = r.nc[1] / div;
@@ -1935,10 +1940,10 @@ void fma_build(const Dev &d, int ncell, int n3, int n2, int3 d2, const OP *m43, 
     launch_pdl(k_p2m<R>, dim3(min(ncell, GRID)), dim3(64), 0, st, d);
     launch_pdl(k_m2m<R, OP>, dim3(min(n3, GRID)), dim3(128), 0, st, d, m43, 3);
     launch_pdl(k_m2m<R, OP>, dim3(n2), dim3(128), 0, st, d, m32, 2);
-    launch_pdl(k_m2l_cls<R>, dim3(d.m2c_nitems, d.m2c_groups), dim3(32 * M2C_W), m2c_smem<R>(), st, d, ncell);
+    launch_pdl(k_m2l_cls<R>, dim3(d.m2c_nitems, M2C_GROUPS), dim3(32 * M2C_W), m2c_smem<R>(), st, d, ncell);
     launch_pdl(k_m2l_all<R>, dim3(n2), dim3(256), 0, st, d, h2, hper, cf, d2);
-    launch_pdl(k_l2l<R, OP>, dim3(min((n3 + 3) / 4, GRID)), dim3(128), 0, st, d, l23, 3, d.m2c_groups);
-    launch_pdl(k_l2l<R, OP>, dim3(min((ncell + 3) / 4, GRID)), dim3(128), 0, st, d, l34, 4, d.m2c_groups);
+    launch_pdl(k_l2l<R, OP>, dim3(min((n3 + 3) / 4, GRID)), dim3(128), 0, st, d, l23, 3);
+    launch_pdl(k_l2l<R, OP>, dim3(min((ncell + 3) / 4, GRID)), dim3(128), 0, st, d, l34, 4);
 }
 
 void launch_fma_build(const Dev &d, int ncell, int n3, int n2, int mixed, int3 d2, cudaStream_t st) {

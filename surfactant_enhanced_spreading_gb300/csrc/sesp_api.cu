@@ -909,15 +909,14 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
                     m2c_items.push_back(make_int4(lev << 28 | q, cls, t0, std::min(tile, ncls - t0)));
         }
     d.m2c_nitems = (int)m2c_items.size();
-    d.m2c_groups = M2C_GROUPS;
     {
         char *p4 = nullptr, *q4 = nullptr, *q3 = nullptr, *o4 = nullptr, *o3 = nullptr;
         if ((e = dalloc(c, &o4, (size_t)343 * LP * M2C_LD * rsz)) || (e = dalloc(c, &o3, (size_t)343 * LP * M2C_LD * rsz)) ||
             (e = dalloc(c, &p4, (npk4 + npk3) * rsz)) ||
             (e = dalloc(c, &d.fm_list, (size_t)C + n3)) || (e = dalloc(c, &d.occ4, C)) || (e = dalloc(c, &d.occ3, n3)) ||
             (e = dalloc(c, &d.occ2, n2)) || (e = dalloc(c, &d.has3, n3)) || (e = dalloc(c, &d.has2, n2)) ||
-            (e = dalloc(c, &q4, (size_t)d.m2c_groups * LP * C * rsz)) ||
-            (e = dalloc(c, &q3, (size_t)d.m2c_groups * LP * n3 * rsz)) ||
+            (e = dalloc(c, &q4, (size_t)M2C_GROUPS * LP * C * rsz)) ||
+            (e = dalloc(c, &q3, (size_t)M2C_GROUPS * LP * n3 * rsz)) ||
             (e = dalloc(c, &d.m2c_items, m2c_items.size())) || (e = dalloc(c, &d.m2c_off, (size_t)8 * M2C_NOFF)))
             return e;
         d.rop4 = o4; d.rop3 = o3; d.pk4 = p4; d.pk3 = p4 + npk4 * rsz; d.pk_bytes = (npk4 + npk3) * rsz; d.fm_cnt = d.ccount + C; d.part4 = q4; d.part3 = q3;

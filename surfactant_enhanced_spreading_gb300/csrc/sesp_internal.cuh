@@ -229,7 +229,7 @@ struct Dev {
     void *part4, *part3;
     int4 *m2c_items;     // work items: (level << 28 | replica, class, first target, targets)
     int *m2c_off;        // per class its 189 offsets, (dx + 3) + 7 (dy + 3) + 49 (dz + 3)
-    int m2c_nitems, m2c_groups;
+    int m2c_nitems;
     // occupied boxes: class targets and their counts, boxes per level, flags (see k_far_lists)
     int *fm_list, *fm_cnt, *occ4, *occ3, *occ2;
     uint8_t *has3, *has2;
