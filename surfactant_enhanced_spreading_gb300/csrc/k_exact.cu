@@ -171,8 +171,9 @@ __global__ void k_isub(Dev d, int nsurf_sites, const int *surf_mol_of) {
 // takes three lanes, one per component (26 FP64 instructions a corrected SHAKE
 // bond, 46 with a lane per water; more waters than that are bound by the sum
 // over all of them, which a lane per water keeps smaller).  1,000 waters at
-// tolerance 1e-8: SHAKE 204 -> 109 us, RATTLE 218 -> 187 us; 20,000 waters
-// (a lane each) 381 -> 252 and 417 -> 346 us.
+// tolerance 1e-8: SHAKE 204 -> 109 us, RATTLE 218 -> 98 us (187 with the
+// division of infinities inlined); 20,000 waters (a lane each) 381 -> 254 and
+// 417 -> 244 us (346).
 constexpr int WATERS_SPLIT = 10;                       // waters of a warp with three lanes each
 constexpr int MOVE_SPLIT_MAX = WATERS_SPLIT * 4 * 152;
 constexpr int MOVE_BLOCK = 32;
@@ -217,8 +218,8 @@ __device__ __forceinline__ double div_dt(double a) {
 // Bound by FP64 issue and latency along one molecule's steps (a step of a
 // correcting bond is 32 FP64 warp instructions; a thread per molecule took 52,
 // in sequence over all sweeps, and spilled): 12 surfactants with 701 waters,
-// SHAKE 280 -> 60 us, RATTLE 571 -> 144 us (75 and 149 with sweeps 8 apart;
-// the waters bound them now).
+// SHAKE 280 -> 60 us, RATTLE 571 -> 58 us (75 and 149 with sweeps 8 apart and
+// the division of infinities inlined; the waters bound them now).
 struct SurfShared {
     double p[NSURF][3], v[NSURF][3], r[NBOND][3], ke[NSURF];
     double m[NSURF], rm[NSURF], c0[NBOND], c1[NBOND], c2[NBOND];   // masses and their reciprocals; per-bond constants

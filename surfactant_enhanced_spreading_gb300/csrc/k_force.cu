@@ -1,16 +1,18 @@
 // Force kernels of the GB300 engine: cell sort, the full-shell short-range
-// pair kernel (FP64, or FP32 with compensated accumulation) with the local
-// expansion force fused into its epilogue, the order-4 multipole passes,
-// walls, graphite and the surfactant intramolecular terms.
+// pair kernel (fixed point with FP64, FP32, or FP32 with compensated
+// accumulation) and the kernel that adds its partials and the local expansion's
+// force, the order-4 multipole passes, walls, graphite and the surfactant
+// intramolecular terms.
 //
 // The reference splits its short-range work into 39 list kernels
 // (src/eval[wS]*.f90) over "Central" and "26" lists built every 10 steps
 // (src/build*.f90).  Together they give every site the Coulomb force of all
 // sites of other molecules that sit in the 27 cells around its own cell, plus
 // the LJ force within rc for the site kinds that carry LJ.  Here that rule is
-// one kernel: one CTA per cell, the 27 neighbour cells staged through shared
-// memory, each thread accumulating the full force on its own site (no
-// third-law scatter, no atomics, so results are bit-reproducible).
+// one kernel: a warp takes up to 64 sites of a cell and the partners of a row
+// of three neighbouring cells (or of one), staged through its shared memory,
+// and each lane accumulates the force on its own sites (no third-law scatter,
+// no atomics, so results are bit-reproducible).
 #include "k_launch.cuh"
 
 namespace sesp {
@@ -955,24 +957,31 @@ __device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, con
 // ---- FP64
 
 // GB300 issues an FP64 warp instruction in 64 cycles of a scheduler, and an
-// integer or FP32 one in one or two.  So the FP64 pair loop does all but the
-// three force sums in integers: the coordinates are fixed point, the squared
-// distance, r^-3 and the conversions of the differences are formed from 64-bit
-// products, and a Coulomb pair takes 3 FP64 instructions and about 200 others
-// (15 FP64 instructions with r^-3 from one exact FP64 residual, 22 with two
-// Newton steps).  The integer and the FP64 pipe are then busy for 62 and 58 %
-// of the cycles.  FP64 pair field: 62,400 sites 7.14 -> 2.64 ms (10.5 with 22
-// instructions), 3,000 sites 317 -> 157 us.
+// integer or FP32 one in one or two.  So a Coulomb pair has none: the
+// coordinates are fixed point, the squared distance, r^-3 and the force terms
+// are formed from 64-bit products, and the terms of up to 32 partners are added
+// as integers.  FP64 enters once a block, for LJ terms (a ninth of the pairs),
+// partners with charges of their own and close pairs.  About 157 instructions
+// a pair with LJ's share; the heavy half of the FMA pipe (64-bit products) is
+// busy for 63 % of the cycles, the integer pipe 57, FP64 23.  FP64 pair field of
+// 62,400 sites, ms: 10.5 with 22 FP64 instructions a pair (two Newton steps),
+// 7.14 with 15 (r^-3 from one exact FP64 residual), 2.64 with the three force
+// sums alone, 1.98 now, and 1.80 with items ordered by a warp's cost; 3,000
+// sites 3.2, 0.317, 0.158, 0.136, 0.119.
 //
 // Coordinates: 2^-59 sigma relative to the partner's cell centre, from
 // positions and centres rounded to 2^-52 (exact for |x| >= 1), so a
-// difference carries at most that rounding.  r^2: units of 2^-56, truncated
-// within 3 of them.  r^-3: y ~ r^-1 from the special-function unit on r^2
+// difference carries at most that rounding.  r^2: units of 2^-56, within 2.5 of
+// them.  r^-3: y ~ r^-1 from the special-function unit on r^2
 // scaled by a power of 4 to [1, 4), a little low; e = 1 - r^2 y^2 >= 0 exactly
 // (the product modulo 2^64 below its known top), r^-3 = y^3 (1 + e (3/2 + 15/8
-// e)) up to 35/16 e^3 < 2^-57, one rounding to FP64.  Against 80-bit
-// arithmetic over distances of 0.4 to 9 sigma: 0.7e-16 RMS (a plain FP64
-// evaluation: 1.2e-16).
+// e)) up to 35/16 e^3 < 2^-57, then one rounding: to units of 2^-57 for the
+// Coulomb terms, to FP64 for the others (against 80-bit arithmetic over
+// distances of 0.4 to 9 sigma 0.7e-16 RMS; a plain FP64 evaluation 1.2e-16).
+// Terms: units of 2^-53, within one of them; an FP64 sum of 30 terms of a
+// cell, which reaches 4 to 8, rounds each of the last ones to 2^-51.  Force of
+// 62,400 sites against a 64-bit reference, two draws: 5.2e-15 and 1.2e-14 RMS,
+// with FP64 arithmetic 7.3e-15 and 1.3e-14.
 typedef unsigned long long u64;
 constexpr u64 FIX_NEAR2 = (u64)1 << 53;   // r^2 of 1/8: closer pairs are evaluated in FP64
 
@@ -1246,20 +1255,20 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
 // with an item per cell as well).
 //
 // FP32, what bounds it: the FMA pipe and the registers that feed it.  A pair
-// of partners takes 11 paired instructions and two reciprocal square roots; a
-// loop of nothing else runs 2.85 T pairs/s (three-operand paired FMAs issue
-// at 0.6 of the rate of two-operand ones), which is 0.42 ms for the 1.19 G
-// pairs of the 312,000-site configuration.  Lanes without a target (14 %) and
-// LJ (a ninth of the pairs, at three times the cost) make it 0.53; measured
-// 0.64, and 0.72 with two targets per pair register, LJ arithmetic on water-H
-// targets, and partners staged 32 at a time.
+// of partners takes 11 paired instructions and two reciprocal square roots
+// (three-operand paired FMAs issue at 0.6 of the rate of two-operand ones).  Of
+// the 0.625 ms of the 312,000-site configuration (1.19 G pairs, 18 % more with
+// lanes and partners that pad), plain Coulomb runs take 0.35 at 3.3 T pairs/s,
+// LJ and excluded pairs, a fifth of all, 0.14, and all else (staging, run ends,
+// items) 0.14: 83 M of 476 M instructions.  0.72 ms with two targets per pair
+// register, LJ arithmetic on water-H targets, and partners staged 32 at a time.
 // MODE 0: FP64; 1: FP32 positions relative to the cell centres, FP32 pair
 // terms; 2: FP32 with compensated (Kahan) sums (SESP_MIXED_COMP).
 // PER: the periodic preset's instantiation (rows wrap around x and y)
 // CTAs per SM: the FP32 loops want 110 to 146 registers, and one CTA more than
 // they leave room for spills into them (312,000 sites: 0.640 ms at 4 CTAs,
 // 0.736 at 5, 0.675 at 3; compensated, 41,600 sites: 0.164 ms at 3, 0.176 at
-// 4; FP64, 62,400 sites: 2.70 ms at 4, 3.00 at 3, 2.70 at 5, 2.76 at 6).
+// 4; FP64, 62,400 sites: 1.98 ms at 4, 2.02 at 5).
 constexpr int near_ctas(int mode) { return mode == 2 ? 3 : 4; }
 template <int MODE, bool PER>
 __global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, int nslot, int tile, int split) {
