@@ -410,6 +410,12 @@ void op_l2l(double x, double y, double z, double2 *op) {
 // ------------------------------------------------------------------ context
 
 constexpr int HOST_VALUES = 256;   // doubles of a context's mapped result buffer
+// Contexts up to this size pass their state through mapped host memory, which
+// the transposing kernel reads and writes itself: no copies, one launch.  The
+// host's own copy to and from it costs more beyond (us, copies / mapped; three
+// arrays in, three out: 900 sites 29 / 25, 43 / 20; 3,000 sites 49 / 29,
+// 41 / 26; 12,000 sites 53 / 59, 47 / 54; 60,000 sites 78 / 310, 73 / 315).
+constexpr int HOST_STATE_MAX = 4096;
 
 struct sesp_ctx {
     sesp_params p;
@@ -447,6 +453,8 @@ struct sesp_ctx {
     bool t_rec[8] = {false};
     // mapped host memory that kernels write a few results to (one per replica)
     double *host_values = nullptr, *host_values_dev = nullptr;
+    // mapped host staging of the state (12 values per site), up to HOST_STATE_MAX sites
+    double *host_state = nullptr, *host_state_dev = nullptr;
 };
 
 namespace {
@@ -484,6 +492,8 @@ void free_state(sesp_ctx *c) {
         if (g) { cudaGraphExecDestroy(g); g = nullptr; }
     for (void *q : c->allocs) cudaFree(q);
     c->allocs.clear();
+    cudaFreeHost(c->host_state);
+    c->host_state = c->host_state_dev = nullptr;
     c->bytes = 0;
     c->uploaded = false;
     c->have_force = false;
@@ -891,6 +901,13 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         return e;
     const int w2x = 2 * d2.x + 1, w2y = 2 * d2.y + 1, w2z = 2 * d2.z + 1;
     const size_t nh2 = (size_t)w2x * w2y * w2z * NHARM;
+    if (N <= HOST_STATE_MAX &&
+        (cudaHostAlloc(&c->host_state, 12 * (size_t)N * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
+         cudaHostGetDevicePointer((void **)&c->host_state_dev, c->host_state, 0) != cudaSuccess)) {
+        cudaGetLastError();   // none to be had: the state goes by copies
+        cudaFreeHost(c->host_state);
+        c->host_state = c->host_state_dev = nullptr;
+    }
     lap("allocation");
     // real-form M2L at L4 and L3: work items (tiles of targets) of one parity
     // class, each split into M2C_GROUPS offset groups (a constant, so a
@@ -1355,55 +1372,70 @@ int sesp_set_eta_batch(sesp_ctx *c, const double *eta) {
     return 0;
 }
 
-// (3, n) site-major host arrays <-> the device's x / y / z arrays: one
-// contiguous copy per array through a device staging buffer, transposed by
-// a kernel (array k of the staging buffer at k * 3n: positions, velocities,
-// accelerations, forces)
+// (3, n) site-major host arrays <-> the device's x / y / z arrays, array k of
+// the staging buffer at k * 3n (positions, velocities, accelerations, forces).
+// One thread per element: the staging side, which may be host memory, is read
+// and written contiguously.
 __global__ void k_state_io(Dev d, double *stage, int n, int mask, int unpack) {
-    const int g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= n) return;
-    double *soa[4][3] = {{d.x, d.y, d.z}, {d.vx, d.vy, d.vz}, {d.ax, d.ay, d.az}, {d.fx, d.fy, d.fz}};
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 3 * n) return;
+    const int g = e / 3, a = e - 3 * g;
+    double *const soa[4][3] = {{d.x, d.y, d.z}, {d.vx, d.vy, d.vz}, {d.ax, d.ay, d.az}, {d.fx, d.fy, d.fz}};
+#pragma unroll
     for (int k = 0; k < 4; k++) {
         if (!(mask >> k & 1)) continue;
-        double *aos = stage + (size_t)k * 3 * n + 3 * (size_t)g;
-        for (int a = 0; a < 3; a++) {
-            if (unpack) soa[k][a][g] = aos[a];
-            else aos[a] = soa[k][a][g];
-        }
+        double *p = a == 0 ? soa[k][0] : a == 1 ? soa[k][1] : soa[k][2];
+        double *aos = stage + (size_t)k * 3 * n + e;
+        if (unpack) p[g] = *aos;
+        else *aos = p[g];
     }
 }
+
+namespace {
+
+// State between the caller's arrays (null: left out) and the device.  Up to
+// HOST_STATE_MAX sites the kernel reads or writes the context's mapped buffer;
+// above, one copy per array through device staging.
+int state_io(sesp_ctx *c, double *const arr[4], int unpack) {
+    const int N = c->nsite;
+    const size_t n3 = 3 * (size_t)N, bytes = n3 * sizeof(double);
+    const bool mapped = c->host_state != nullptr;
+    int mask = 0;
+    for (int k = 0; k < 4; k++) mask |= arr[k] ? 1 << k : 0;
+    if (!mask) return 0;
+    if (unpack)
+        for (int k = 0; k < 4; k++) {
+            if (!arr[k]) continue;
+            if (mapped) memcpy(c->host_state + k * n3, arr[k], bytes);
+            else CK(cudaMemcpyAsync(c->d.stage + k * n3, arr[k], bytes, cudaMemcpyHostToDevice, c->st));
+        }
+    k_state_io<<<(unsigned)((n3 + 255) / 256), 256, 0, c->st>>>(c->d, mapped ? c->host_state_dev : c->d.stage, N, mask, unpack);
+    CK(cudaGetLastError());
+    if (unpack) return 0;
+    if (!mapped)
+        for (int k = 0; k < 4; k++)
+            if (arr[k]) CK(cudaMemcpyAsync(arr[k], c->d.stage + k * n3, bytes, cudaMemcpyDeviceToHost, c->st));
+    CK(cudaStreamSynchronize(c->st));
+    if (mapped)
+        for (int k = 0; k < 4; k++)
+            if (arr[k]) memcpy(arr[k], c->host_state + k * n3, bytes);
+    return 0;
+}
+
+}  // namespace
 
 int sesp_download_state(sesp_ctx *c, double *pos, double *vel, double *acc) {
     if (int e = check_ctx(c, true)) return e;
     if (set_device(c)) return SESP_ECUDA;
-    const int N = c->nsite;
-    double *outs[3] = {pos, vel, acc};
-    const int mask = (pos ? 1 : 0) | (vel ? 2 : 0) | (acc ? 4 : 0);
-    if (!mask) return 0;
-    k_state_io<<<(N + 255) / 256, 256, 0, c->st>>>(c->d, c->d.stage, N, mask, 0);
-    CK(cudaGetLastError());
-    for (int k = 0; k < 3; k++)
-        if (outs[k])
-            CK(cudaMemcpyAsync(outs[k], c->d.stage + (size_t)k * 3 * N, 3 * (size_t)N * sizeof(double),
-                               cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return 0;
+    double *const outs[4] = {pos, vel, acc, nullptr};
+    return state_io(c, outs, 0);
 }
 
 int sesp_set_state(sesp_ctx *c, const double *pos, const double *vel, const double *acc, double eta) {
     if (int e = check_ctx(c, true)) return e;
     if (set_device(c)) return SESP_ECUDA;
-    const int N = c->nsite;
-    const double *ins[3] = {pos, vel, acc};
-    const int mask = (pos ? 1 : 0) | (vel ? 2 : 0) | (acc ? 4 : 0);
-    for (int k = 0; k < 3; k++)
-        if (ins[k])
-            CK(cudaMemcpyAsync(c->d.stage + (size_t)k * 3 * N, ins[k], 3 * (size_t)N * sizeof(double),
-                               cudaMemcpyHostToDevice, c->st));
-    if (mask) {
-        k_state_io<<<(N + 255) / 256, 256, 0, c->st>>>(c->d, c->d.stage, N, mask, 1);
-        CK(cudaGetLastError());
-    }
+    double *const ins[4] = {const_cast<double *>(pos), const_cast<double *>(vel), const_cast<double *>(acc), nullptr};
+    if (int e = state_io(c, ins, 1)) return e;
     const std::vector<double> etas(c->nrep, eta);   // every replica
     CK(cudaMemcpyAsync(c->d.eta, etas.data(), c->nrep * sizeof(double), cudaMemcpyHostToDevice, c->st));
     CK(cudaStreamSynchronize(c->st));
@@ -1429,12 +1461,8 @@ int sesp_download_forces(sesp_ctx *c, double *f) {
     if (int e = check_ctx(c, true)) return e;
     if (!f) return fail(SESP_EINVAL, "null output");
     if (set_device(c)) return SESP_ECUDA;
-    const int N = c->nsite;
-    k_state_io<<<(N + 255) / 256, 256, 0, c->st>>>(c->d, c->d.stage, N, 8, 0);
-    CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(f, c->d.stage + (size_t)9 * N, 3 * (size_t)N * sizeof(double), cudaMemcpyDeviceToHost, c->st));
-    CK(cudaStreamSynchronize(c->st));
-    return 0;
+    double *const outs[4] = {nullptr, nullptr, nullptr, f};
+    return state_io(c, outs, 0);
 }
 
 int sesp_init_accel(sesp_ctx *c) {
