@@ -23,6 +23,8 @@ void upload_tables_force(const Tables &t, cudaStream_t st) {
     cudaMemcpyToSymbolAsync(cT, &t, sizeof(Tables), 0, cudaMemcpyHostToDevice, st);
 }
 
+typedef unsigned long long u64;
+
 constexpr int NEAR_THREADS = 128;
 constexpr int SORT_CAP = 2048, SORT_SHIFT = 29;   // site indices stay below 2^29
 
@@ -286,8 +288,17 @@ __device__ inline double cell_centre(const Dev &d, const Rep &r, int a, int i) {
     return t[i];
 }
 
-// fixed point of the FP64 pair field (see near_block64)
-constexpr double FIX_ONE = 4503599627370496.0;   // 2^52
+// A coordinate in the fixed point of the FP64 pair field (see near_block64):
+// units of 2^-59 modulo 2^64, rounded to 2^-58, so every coordinate of at least
+// 2^-6 is exact and differences of up to 16 are the state's own.  Integer
+// operations alone (GB300 converts at its FP64 rate); |v| < 2^59.
+__device__ __forceinline__ long long fix_of(double v) {
+    const long long b = __double_as_longlong(v);
+    const int e = (int)(b >> 52) & 0x7ff, s = e - (1023 + 52 - 58);
+    const u64 m = ((u64)b & (((u64)1 << 52) - 1)) | (u64)(e != 0) << 52;
+    const u64 u = s >= 0 ? m << (s & 63) : s > -55 ? (m + ((u64)1 << ((-s - 1) & 63))) >> (-s & 63) : 0;
+    return (long long)((b < 0 ? 0 - u : u) << 1);
+}
 constexpr double FIX_REACH = 2.7;   // along an axis from a site to its cell's centre; beyond it the replica's items run in FP64
 
 // Slot positions of the step: the site's position (on the periodic preset
@@ -321,7 +332,7 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mode) {
         for (int a = 0; a < 3; a++) {
             const double ca = cell_centre(d, r, a, ic[a]);
             const bool in = fabs(p[a] - ca) < FIX_REACH && fabs(ca) < 1024.0;
-            d.srt_fix[s + a * (size_t)d.nsite] = in ? (__double2ll_rn(p[a] * FIX_ONE) - __double2ll_rn(ca * FIX_ONE)) << 7 : 0;
+            d.srt_fix[s + a * (size_t)d.nsite] = in ? fix_of(p[a]) - fix_of(ca) : 0;
             ok = ok && in;
         }
         if (!ok) d.near_far[d.crep[c]] = 1;   // cleared by the finish kernel
@@ -961,31 +972,30 @@ __device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, con
 // coordinates are fixed point, the squared distance, r^-3 and the force terms
 // are formed from 64-bit products, and the terms of up to 32 partners are added
 // as integers.  FP64 enters once a block, for LJ terms (a ninth of the pairs),
-// partners with charges of their own and close pairs.  About 157 instructions
-// a pair with LJ's share; the heavy half of the FMA pipe (64-bit products) is
-// busy for 63 % of the cycles, the integer pipe 57, FP64 23.  FP64 pair field of
-// 62,400 sites, ms: 10.5 with 22 FP64 instructions a pair (two Newton steps),
+// partners with charges of their own and pairs closer than 1 sigma (a 300th).
+// FP64 pair field of 62,400 sites, ms: 10.5 with 22 FP64 instructions a pair (two Newton steps),
 // 7.14 with 15 (r^-3 from one exact FP64 residual), 2.64 with the three force
-// sums alone, 1.98 now, and 1.80 with items ordered by a warp's cost; 3,000
-// sites 3.2, 0.317, 0.158, 0.136, 0.119.
+// sums alone, 1.82 now.
 //
-// Coordinates: 2^-59 sigma relative to the partner's cell centre, from
-// positions and centres rounded to 2^-52 (exact for |x| >= 1), so a
-// difference carries at most that rounding.  r^2: units of 2^-56, within 2.5 of
+// Coordinates: 2^-59 sigma relative to the partner's cell centre, the state's
+// own down to 2^-58 (fix_of).  r^2: units of 2^-56, within 2.5 of
 // them.  r^-3: y ~ r^-1 from the special-function unit on r^2
 // scaled by a power of 4 to [1, 4), a little low; e = 1 - r^2 y^2 >= 0 exactly
 // (the product modulo 2^64 below its known top), r^-3 = y^3 (1 + e (3/2 + 15/8
-// e)) up to 35/16 e^3 < 2^-57, then one rounding: to units of 2^-57 for the
-// Coulomb terms, to FP64 for the others (against 80-bit arithmetic over
+// e)) up to 35/16 e^3 < 2^-57, then one rounding: to units of 2^-61 for the
+// summed Coulomb terms, to FP64 for the others (against 80-bit arithmetic over
 // distances of 0.4 to 9 sigma 0.7e-16 RMS; a plain FP64 evaluation 1.2e-16).
-// Terms: units of 2^-53, within one of them; an FP64 sum of 30 terms of a
-// cell, which reaches 4 to 8, rounds each of the last ones to 2^-51.  Force of
-// 62,400 sites against a 64-bit reference, two draws: 5.2e-15 and 1.2e-14 RMS,
-// with FP64 arithmetic 7.3e-15 and 1.3e-14.
-typedef unsigned long long u64;
-constexpr u64 FIX_NEAR2 = (u64)1 << 53;   // r^2 of 1/8: closer pairs are evaluated in FP64
+// Terms: units of 2^-57, within one of them, of pairs at least 1 sigma apart:
+// a term is at most 1, so 32 of them fit, and closer pairs, whose FP64 sums
+// round coarser than that anyway, are left to FP64.  Both units are fine enough for a
+// site whose only partners are far: one water 8 sigma from another, whose
+// charges nearly cancel, has errors of 4e-18 (unscaled), as in FP64.  (Units
+// of 2^-57 and 2^-53, with every pair beyond 0.35 sigma summed so, had 6e-17
+// there, at 1.79 ms.)
+constexpr u64 FIX_CLOSE2 = (u64)1 << 53;   // r^2 of 1/8: r^-3 of closer pairs is evaluated in FP64
+constexpr u64 FIX_NEAR2 = (u64)1 << 56;    // r^2 of 1: the terms of closer pairs are summed in FP64
 
-// a difference (units of 2^-59) as FP64
+// a difference (units of 2^-59) as FP64, to nearest
 __device__ __forceinline__ double fix_to_double(long long v) {
     const long long s = v >> 63;
     const u64 u = (u64)((v ^ s) - s);
@@ -995,9 +1005,10 @@ __device__ __forceinline__ double fix_to_double(long long v) {
     const int lz = __clz(a);
     const unsigned mh = __funnelshift_l(b, a, lz), ml = b << (lz & 31);
     const unsigned e = (unsigned)(1023 + 63 - 59 - 1 - lz - (z ? 32 : 0)) << 20;
-    unsigned hi = e + (mh >> 11);   // the leading bit adds 1 to the exponent
-    if (a == 0) hi = 0;
-    return __hiloint2double((int)(hi | ((unsigned)s & 0x80000000u)), (int)__funnelshift_r(ml, mh, 11));
+    // the leading bit adds 1 to the exponent, the first bit cut off rounds
+    u64 m = ((u64)(e + (mh >> 11)) << 32 | __funnelshift_r(ml, mh, 11)) + (ml >> 10 & 1);
+    if (a == 0) m = 0;
+    return __longlong_as_double((long long)(m | ((u64)s & 0x8000000000000000ull)));
 }
 // w 2^ex as FP64, w >= 2^32
 __device__ __forceinline__ double scale_to_double(u64 w, int ex) {
@@ -1005,7 +1016,7 @@ __device__ __forceinline__ double scale_to_double(u64 w, int ex) {
     const u64 m = w << lz;
     return __longlong_as_double((long long)(((u64)(1023 + 63 - 1 - lz + ex) << 52) + (m >> 11) + ((m >> 10) & 1)));
 }
-// a difference's halves: h 2^32 + 2 l, with l signed (its low 7 bits are zero)
+// a difference's halves: h 2^32 + 2 l, with l signed (its lowest bit is zero)
 struct Fix {
     int h, l;
     __device__ __forceinline__ explicit Fix(long long v) : h((int)(v >> 32) + (int)((unsigned)v >> 31)), l((int)(unsigned)v >> 1) {}
@@ -1042,17 +1053,22 @@ __device__ __forceinline__ FixInv fix_inverse(u64 r2) {
     v.w = m3 + (u64)mh * kh + (((u64)mh * kl + (u64)ml * kh) >> 32);
     return v;
 }
-// r^-3 in units of 2^-57, to nearest: h 2^31 + l
+// r^-3 and r^-2 in FP64
+__device__ __forceinline__ double2 fix_powers(const FixInv &v) {
+    return make_double2(scale_to_double(v.w, -70 + 3 * (v.lz >> 1)),
+                        scale_to_double(v.mm + __umul64hi(v.mm, (v.e60 + (v.e2 >> 4)) << 4), -68 + v.lz));
+}
+// r^-3 of r2 >= 2^56 in units of 2^-61, to nearest: h 2^31 + l (any value for closer pairs)
 struct FixTerm {
     int h, l;
     __device__ __forceinline__ explicit FixTerm(const FixInv &v) {
-        const int k = v.lz + (v.lz >> 1);   // 3 lz / 2 <= 15
-        const u64 w = (v.w + (4096u >> k)) << 2;
-        const unsigned wh = (unsigned)(w >> 32), t0 = __funnelshift_r((unsigned)w, wh, 15 - k), t1 = wh >> (15 - k);
+        const int k = v.lz + (v.lz >> 1), n = (9 - k) & 31;   // 3 lz / 2 <= 9
+        const u64 w = v.w + (256u >> k);
+        const unsigned wh = (unsigned)(w >> 32), t0 = __funnelshift_r((unsigned)w, wh, n), t1 = wh >> n;
         h = (int)__funnelshift_l(t0, t1, 1); l = (int)(t0 & 0x7fffffffu);
     }
 };
-// a += the product of a difference and r^-3, in units of 2^-53, to nearest
+// a += the product of a difference and r^-3, in units of 2^-57, to nearest
 __device__ __forceinline__ void fix_add(long long &a, const Fix &x, const FixTerm &t) {
     const long long c = (long long)x.h * t.l + (long long)x.l * t.h + (1 << 30);
     a += (long long)x.h * t.h + (c >> 31);
@@ -1080,21 +1096,25 @@ struct Tgt64 {
 __device__ __forceinline__ void near_sum64(double (&f)[3], double dx, double dy, double dz, double ft) {
     f[0] = fma(dx, ft, f[0]); f[1] = fma(dy, ft, f[1]); f[2] = fma(dz, ft, f[2]);
 }
-// The LJ term of a pair within rc added to its Coulomb term (zero adds nothing)
-__device__ __forceinline__ double near_lj64(double ft, double2 p, bool in, double i3, double i2) {
+// The LJ term of a pair within rc added to its Coulomb term
+__device__ __forceinline__ double near_lj64(double ft, double2 p, double i3, double i2) {
     const double i6 = i3 * i3;
-    return fma(((in ? p.x : 0.0) * i6) * fma(p.y, i6, -0.5), i2, ft);
+    return fma((p.x * i6) * fma(p.y, i6, -0.5), i2, ft);
 }
 
 // The pairs of one staged block.  LJ: 0 Coulomb of a run with one charge, 1
 // water-O partners with LJ, 2 any partners.  Partners of the target's own
 // molecule, and the target itself, are left out.  S: the unscaled Coulomb sum
-// of runs with one charge; f: all else, scaled except with LJ 0.
+// of runs with one charge; f: all else, scaled except with LJ 0.  With LJ 0
+// the close pairs wait for the end of the block, where every lane takes its own next
+// one: three turns for the own cell's blocks, one or none for most (62,400 sites
+// 1.82 ms, 3,000 sites 122 us; with a vote on every partner 1.89 and 146).
 template <int LJ>
 __device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const Stage64 &s, int n, const double2 *ljt,
                                              double (&S)[3], double (&f)[3]) {
     const u64 rc2 = (u64)(RC * RC * 72057594037927936.0);   // 2^56
-    long long a[3] = {0, 0, 0};   // at most 32 terms of 8 (2^56)
+    long long a[3] = {0, 0, 0};   // at most 32 terms of 1 (2^57)
+    unsigned late = 0;            // LJ 0: the partners closer than 1 sigma
 #pragma unroll 1
     for (int k = 0; k < n; k++) {
         const long long x = t.x - s.x[k], y = t.y - s.y[k], z = t.z - s.z[k];
@@ -1103,36 +1123,44 @@ __device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const St
         const Fix X(x), Y(y), Z(z);
         const u64 r2 = fix_r2(X, Y, Z);
         const FixInv v = fix_inverse(r2);
-        const bool close = r2 < FIX_NEAR2;
+        const bool near = r2 < FIX_NEAR2;
         if constexpr (LJ != 2) {
             FixTerm w(v);
-            if (same || close) w.h = w.l = 0;
+            if (same || near) w.h = w.l = 0;
             fix_add(a[0], X, w); fix_add(a[1], Y, w); fix_add(a[2], Z, w);
         }
-        const bool cl = close && !same, in = LJ != 0 && !same && r2 <= rc2;
-        if (LJ == 2 || __any_sync(0xffffffffu, cl || in)) {
+        if constexpr (LJ == 0) {
+            if (near && !same) late |= 1u << k;
+        } else {
+            const bool in = !same && r2 <= rc2;
+            if (LJ == 1 && !__any_sync(0xffffffffu, in)) continue;
             const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
-            double i3 = 0.0, i2 = 0.0;
-            if (LJ != 0) {
-                i3 = scale_to_double(v.w, -70 + 3 * (v.lz >> 1));
-                i2 = scale_to_double(v.mm + __umul64hi(v.mm, (v.e60 + (v.e2 >> 4)) << 4), -68 + v.lz);
+            double2 u = fix_powers(v);
+            if (in && r2 < FIX_CLOSE2) u = near_inverse(dx, dy, dz);
+            double ft = 0.0;
+            if constexpr (LJ == 1) {
+                if (in && near) ft = qq * u.x;
+            } else {
+                if (!same) ft = qq * s.q[k] * u.x;
             }
-            if (cl) {
-                const double2 u = near_inverse(dx, dy, dz);
-                i3 = u.x; i2 = u.y;
-            }
-            double ft;
-            if constexpr (LJ == 0) ft = cl ? i3 : 0.0;
-            if constexpr (LJ == 1) ft = cl ? qq * i3 : 0.0;
-            if constexpr (LJ == 2) ft = same ? 0.0 : qq * s.q[k] * i3;
-            if constexpr (LJ != 0)
-                if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], in, i3, i2);
+            if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], u.x, u.y);
             near_sum64(f, dx, dy, dz, ft);
+        }
+    }
+    if constexpr (LJ == 0) {
+        for (; __any_sync(0xffffffffu, late); late &= late - 1) {
+            const int k = late ? __ffs(late) - 1 : 0;
+            const long long x = t.x - s.x[k], y = t.y - s.y[k], z = t.z - s.z[k];
+            const u64 r2 = fix_r2(Fix(x), Fix(y), Fix(z));
+            const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
+            double i3 = fix_powers(fix_inverse(r2)).x;
+            if (late && r2 < FIX_CLOSE2) i3 = near_inverse(dx, dy, dz).x;
+            near_sum64(f, dx, dy, dz, late ? i3 : 0.0);
         }
     }
     if constexpr (LJ != 2) {
 #pragma unroll
-        for (int b = 0; b < 3; b++) S[b] = fma((double)a[b], 0x1p-53, S[b]);
+        for (int b = 0; b < 3; b++) S[b] = fma((double)a[b], 0x1p-57, S[b]);
     }
 }
 
@@ -1151,7 +1179,7 @@ __device__ __noinline__ void near_run64_any(const Dev &d, double tx, double ty, 
         if constexpr (LJ != 0) {
             ft *= LJ == 2 ? qq * p.w : qq;
             const bool in = fma(dz, dz, fma(dy, dy, dx * dx)) <= RC * RC;
-            if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], in, v.x, v.y);
+            if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], v.x, v.y);
         }
         near_sum64(f, dx, dy, dz, ft);
     }
@@ -1173,9 +1201,8 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
     // a partner cell across a periodic face holds positions one box length
     // away, so the targets move by that length into its frame
     const double sy = (double)(jy - wy) * RS;
-    auto fixed = [](double v) { return __double2ll_rn(v * FIX_ONE); };
     auto shift = [&](int a, int own, int cell, double box) {   // own cell's frame to the partner cell's
-        return (fixed(cell_centre(d, r, a, own)) - fixed(cell_centre(d, r, a, cell)) - fixed(box)) << 7;
+        return fix_of(cell_centre(d, r, a, own)) - fix_of(cell_centre(d, r, a, cell)) - fix_of(box);
     };
     const long long shy = shift(1, iy, wy, sy), shz = shift(2, iz, jz, 0.0);
     Tgt64 t = {0, 5ll << 59, 0, 0.0, -2, NTYPE};   // no site: no molecule, water H (no LJ), clear of every partner
