@@ -299,7 +299,9 @@ __device__ __forceinline__ long long fix_of(double v) {
     const u64 u = s >= 0 ? m << (s & 63) : s > -55 ? (m + ((u64)1 << ((-s - 1) & 63))) >> (-s & 63) : 0;
     return (long long)((b < 0 ? 0 - u : u) << 1);
 }
-constexpr double FIX_REACH = 2.7;   // along an axis from a site to its cell's centre; beyond it the replica's items run in FP64
+// Along an axis from a site to its cell's centre; beyond it the site's bit in
+// far_bits is set, and its pairs run in FP64.
+constexpr double FIX_REACH = 2.7;
 
 // Slot positions of the step: the site's position (on the periodic preset
 // wrapped by the image it had at the last rebuild, so it stays beside its
@@ -309,7 +311,9 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mode) {
     griddep_wait();
     int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s == 0) d.near_ctl[0] = 0;   // the pair field's work counter
-    if (s >= nslot || s >= d.cstart[ncell]) return;
+    const bool in = s < nslot && s < d.cstart[ncell];
+    const unsigned live = __ballot_sync(0xffffffffu, in);   // a warp's first lanes
+    if (!in) return;
     int g = d.srt_site[s];
     const int c = d.srt_cell[s];
     double x = d.x[g], y = d.y[g], z = d.z[g];
@@ -331,11 +335,11 @@ __global__ void k_gather(Dev d, int nslot, int ncell, int mode) {
 #pragma unroll
         for (int a = 0; a < 3; a++) {
             const double ca = cell_centre(d, r, a, ic[a]);
-            const bool in = fabs(p[a] - ca) < FIX_REACH && fabs(ca) < 1024.0;
-            d.srt_fix[s + a * (size_t)d.nsite] = in ? fix_of(p[a]) - fix_of(ca) : 0;
-            ok = ok && in;
+            ok = ok && fabs(p[a] - ca) < FIX_REACH;
+            d.srt_fix[s + a * (size_t)d.nsite] = fix_of(p[a]) - fix_of(ca);
         }
-        if (!ok) d.near_far[d.crep[c]] = 1;   // cleared by the finish kernel
+        const unsigned far = __ballot_sync(live, !ok);
+        if ((s & 31) == 0) d.far_bits[s >> 5] = far;
     }
     if (mode == GATHER_MIXED) {
         const float4 p = make_float4((float)(x - cell_centre(d, r, 0, ix)), (float)(y - cell_centre(d, r, 1, iy)),
@@ -448,16 +452,6 @@ __device__ inline void local_grad(const LF &L, R x, R y, R z, R &gx, R &gy, R &g
 }
 
 // ------------------------------------------------------------------ near field
-
-// 1/sqrt(r2) in FP64 from the FP32 hardware estimate and two Newton steps
-// (relative error of the seed ~2^-22, after two steps at the FP64 rounding level)
-__device__ inline double rsqrt_fp64(double r2) {
-    double y = (double)rsqrtf((float)r2);
-    double h = 0.5 * r2;
-    y = y * (1.5 - h * y * y);
-    y = y * (1.5 - h * y * y);
-    return y;
-}
 
 // Work items, rebuilt with the cell lists: one per (target cell, partner row,
 // chunk of `tile` target sites).  A partner row is the (up to) 3 cells at
@@ -1074,10 +1068,21 @@ __device__ __forceinline__ void fix_add(long long &a, const Fix &x, const FixTer
     a += (long long)x.h * t.h + (c >> 31);
 }
 
-// r^-3 and r^-2 of a close pair, in FP64
-__device__ __noinline__ double2 near_inverse(double x, double y, double z) {
-    const double r2 = fma(z, z, fma(y, y, x * x)), i = 1.0 / sqrt(r2);
+// r^-3 and r^-2 in FP64: any r2 (infinities and NaN as 1 / r gives them)
+__device__ __noinline__ double2 near_inverse(double r2) {
+    const double i = 1.0 / sqrt(r2);
     return make_double2(i * i * i, i * i);
+}
+// the same in seven FP64 instructions for r2 within 2^-100 .. 2^100: y ~ r^-1
+// from the special-function unit on r2's leading bits, y^2 exact (48 bits), e =
+// 1 - r^2 y^2 with one rounding, and the series of fix_inverse
+__device__ __forceinline__ double2 powers64(double r2) {
+    if ((unsigned)(__double2hiint(r2) - ((1023 - 100) << 20)) >= 200u << 20) return near_inverse(r2);
+    const unsigned f = __funnelshift_l((unsigned)__double2loint(r2), (unsigned)__double2hiint(r2), 3) + 0x40000000u;
+    const unsigned b = __float_as_uint(rsqrt_ftz(__uint_as_float(f)));
+    const double y = __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    const double y2 = y * y, e = fma(-r2, y2, 1.0), y3 = y2 * y;
+    return make_double2(fma(y3, e * fma(e, 1.875, 1.5), y3), fma(y2, fma(e, e, e), y2));
 }
 
 constexpr int NEAR_STAGE64 = 32;
@@ -1136,7 +1141,7 @@ __device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const St
             if (LJ == 1 && !__any_sync(0xffffffffu, in)) continue;
             const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
             double2 u = fix_powers(v);
-            if (in && r2 < FIX_CLOSE2) u = near_inverse(dx, dy, dz);
+            if (in && r2 < FIX_CLOSE2) u = near_inverse(fma(dz, dz, fma(dy, dy, dx * dx)));
             double ft = 0.0;
             if constexpr (LJ == 1) {
                 if (in && near) ft = qq * u.x;
@@ -1154,7 +1159,7 @@ __device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const St
             const u64 r2 = fix_r2(Fix(x), Fix(y), Fix(z));
             const double dx = fix_to_double(x), dy = fix_to_double(y), dz = fix_to_double(z);
             double i3 = fix_powers(fix_inverse(r2)).x;
-            if (late && r2 < FIX_CLOSE2) i3 = near_inverse(dx, dy, dz).x;
+            if (late && r2 < FIX_CLOSE2) i3 = near_inverse(fma(dz, dz, fma(dy, dy, dx * dx))).x;
             near_sum64(f, dx, dy, dz, late ? i3 : 0.0);
         }
     }
@@ -1164,22 +1169,28 @@ __device__ __forceinline__ void near_block64(const Tgt64 &t, double qq, const St
     }
 }
 
-// the same in FP64 throughout, from the FP64 positions: systems with a site
-// far from its cell (a state that is blowing up)
-template <int LJ>
-__device__ __noinline__ void near_run64_any(const Dev &d, double tx, double ty, double tz, const Tgt64 &t, double qq, int t0,
-                                            int t1, const double2 *ljt, double (&f)[3]) {
+// The pairs of a run t0..t1 in FP64 throughout, from the FP64 positions, for the
+// target in slot s: pairs of cells with a site far from its cell (lists frozen
+// for long, a state that is blowing up).  bx, by: cells by which the partner
+// lies across a periodic face.  15 FP64 instructions a Coulomb pair: 62,400
+// sites that have all drifted so far 7.9 ms, 3,000 sites 0.28 (22 instructions
+// a pair 10.3 and 2.9); one such site, in reach 1.81 and 0.111, 1.87 and 0.16 (whole
+// replicas with a division and a root a pair: 11.0 and 0.37).
+__device__ __noinline__ void near_far64(const Dev &d, int s, int bx, int by, const Tgt64 &t, double qq, int LJ, int t0, int t1,
+                                        const double2 *ljt, double (&f)[3]) {
+    const double4 own = d.srt_pos[s];
+    const double x = own.x - (double)bx * RS, y = own.y - (double)by * RS, z = own.z;
     for (int k = t0; k < t1; k++) {
         const double4 p = d.srt_pos[k];
         const int key = d.srt_key[k];
-        const double dx = tx - p.x, dy = ty - p.y, dz = tz - p.z;
+        const double dx = x - p.x, dy = y - p.y, dz = z - p.z;
         if ((key >> 5) == t.m) continue;
-        const double2 v = near_inverse(dx, dy, dz);
+        const double r2 = fma(dz, dz, fma(dy, dy, dx * dx));
+        const double2 v = powers64(r2);
         double ft = v.x;
-        if constexpr (LJ != 0) {
+        if (LJ) {
             ft *= LJ == 2 ? qq * p.w : qq;
-            const bool in = fma(dz, dz, fma(dy, dy, dx * dx)) <= RC * RC;
-            if (in) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], v.x, v.y);
+            if (r2 <= RC * RC) ft = near_lj64(ft, ljt[t.trow + (LJ == 2 ? key & 31 : 0)], v.x, v.y);
         }
         near_sum64(f, dx, dy, dz, ft);
     }
@@ -1192,19 +1203,28 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
                                             int first, int ni, int lane, Stage64 &st) {
     const int dzc = pr / 3 - 1, dyc = pr % 3 - 1;
     const int s0 = d.cstart[c], nslot = d.nsite, i = first + lane;
-    const int rep = d.crep[c];
-    const Rep &r = d.rep[rep];
+    const Rep &r = d.rep[d.crep[c]];
     int ix, iy, iz;
     cell_xyz(r, c, ix, iy, iz);
     const int jy = iy + dyc, jz = iz + dzc, wy = PER ? wrap1(jy, r.nc[1]) : jy;
-    const bool far = d.near_far[rep] != 0;
     // a partner cell across a periodic face holds positions one box length
     // away, so the targets move by that length into its frame
-    const double sy = (double)(jy - wy) * RS;
     auto shift = [&](int a, int own, int cell, double box) {   // own cell's frame to the partner cell's
         return fix_of(cell_centre(d, r, a, own)) - fix_of(cell_centre(d, r, a, cell)) - fix_of(box);
     };
-    const long long shy = shift(1, iy, wy, sy), shz = shift(2, iz, jz, 0.0);
+    const long long shy = shift(1, iy, wy, (double)(jy - wy) * RS), shz = shift(2, iz, jz, 0.0);
+    // bit xo + 1: a target, or a site of the partner cell at xo, is far from its cell
+    unsigned far_cells = 0;
+    for (int xo = xo0; xo <= xo1; xo++) {
+        const int cn = cell_index(r, PER ? wrap1(ix + xo, r.nc[0]) : ix + xo, wy, jz);
+        const int p0 = d.cstart[cn], p1 = d.cstart[cn + 1];
+        for (int k = (p0 >> 5) + lane; 32 * k < p1; k += 32) {
+            unsigned m = d.far_bits[k];
+            if (32 * k < p0) m &= ~0u << (p0 - 32 * k);
+            if (p1 - 32 * k < 32) m &= ~(~0u << (p1 - 32 * k));
+            if (m) far_cells |= 1u << (xo + 1);
+        }
+    }
     Tgt64 t = {0, 5ll << 59, 0, 0.0, -2, NTYPE};   // no site: no molecule, water H (no LJ), clear of every partner
     long long ox = 0;
     if (i < ni) {
@@ -1213,32 +1233,28 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
         ox = fp[0]; t.y = fp[nslot] + shy; t.z = fp[2 * (size_t)nslot] + shz;
         t.q = d.srt_pos[s0 + i].w * XPI;
         t.m = kk >> 5; t.trow = (kk & 31) * NTYPE;
+        if (d.far_bits[(s0 + i) >> 5] >> ((s0 + i) & 31) & 1u) far_cells = 7u;
     }
+    far_cells = __reduce_or_sync(0xffffffffu, far_cells);
     const bool lj = first < d.cnh[c];
-    const double qo = d.tq[0], qh = d.tq[1];
     double row[3] = {0.0, 0.0, 0.0};
     for (int xo = xo0; xo <= xo1; xo++) {
         const int wx = PER ? wrap1(ix + xo, r.nc[0]) : ix + xo;
         const int cn = cell_index(r, wx, wy, jz);
         const int p0 = d.cstart[cn], po = p0 + d.cno[cn], ph = p0 + d.cnh[cn], p1 = d.cstart[cn + 1];
         if (p0 == p1) continue;
-        const double sx = (double)(ix + xo - wx) * RS;
-        t.x = ox + shift(0, ix, wx, sx);
+        t.x = ox + shift(0, ix, wx, (double)(ix + xo - wx) * RS);
         double cell[3] = {0.0, 0.0, 0.0};
+        const bool far = far_cells >> (xo + 1) & 1u;
 #pragma unroll 1
         for (int g = 0; g < 3; g++) {   // water O, other LJ sites, water H
             const int a = g == 0 ? p0 : g == 1 ? po : ph, b = g == 0 ? po : g == 1 ? ph : p1;
             if (a == b) continue;
             const bool one = g == 0 && lj;
-            const double qq = g == 1 ? t.q : t.q * (g ? qh : qo);
+            const double qq = g == 1 ? t.q : t.q * d.tq[g >> 1];
             double S[3] = {0.0, 0.0, 0.0}, f[3] = {0.0, 0.0, 0.0};
             if (far) {
-                if (i < ni) {
-                    const double4 p = d.srt_pos[s0 + i];
-                    if (g == 1) near_run64_any<2>(d, p.x - sx, p.y - sy, p.z, t, qq, a, b, ljt, f);
-                    else if (one) near_run64_any<1>(d, p.x - sx, p.y - sy, p.z, t, qq, a, b, ljt, f);
-                    else near_run64_any<0>(d, p.x - sx, p.y - sy, p.z, t, qq, a, b, ljt, f);
-                }
+                if (i < ni) near_far64(d, s0 + i, ix + xo - wx, jy - wy, t, qq, g == 1 ? 2 : one, a, b, ljt, f);
             } else {
                 for (int b0 = a; b0 < b; b0 += NEAR_STAGE64) {
                     const int n = min(NEAR_STAGE64, b - b0);
@@ -1357,7 +1373,6 @@ __global__ void k_near_finish(Dev d, int nslot, int ncell, int terms, int split)
     griddep_wait();
     typedef typename std::conditional<MIXED, float, double>::type R;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (!MIXED && s < d.nrep) d.near_far[s] = 0;   // for the next gather (fewer replicas than slots)
     if (s >= nslot || s >= d.cstart[ncell]) return;
     const int c = d.srt_cell[s];
     // FP32 partials summed in FP32 on the mixed path (one conversion to FP64

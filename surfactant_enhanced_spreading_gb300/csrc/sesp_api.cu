@@ -882,7 +882,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.sslot, N)) || (e = dalloc(c, &d.srt_site, N)) || (e = dalloc(c, &d.srt_pos, N)) ||
         (e = dalloc(c, &d.srt_pos32, N)) || (e = dalloc(c, &d.srt_meta, N)) || (e = dalloc(c, &d.srt_key, N)) ||
         (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) || (e = dalloc(c, &d.srt_fix, c->p.precision == SESP_PLAIN_FP64 ? 3 * (size_t)N : 1)) ||
-        (e = dalloc(c, &d.near_far, R)) ||
+        (e = dalloc(c, &d.far_bits, (size_t)N / 32 + 1)) ||
         (e = dalloc(c, &d.pair_xyz, 3 * pair_max)) || (e = dalloc(c, &d.pair_key, pair_max)) || (e = dalloc(c, &d.crun, 8 * (size_t)C)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
         (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
         (e = dalloc(c, &d.near_mask, C)) || (e = dalloc(c, &d.srt_cell, N)) || (e = dalloc(c, &d.near_ctl, 2 + 2 * NEAR_CLASSES)) ||

@@ -166,7 +166,7 @@ struct Dev {
     double4 *srt_pos;    // x, y, z, q in slot order (FP64)
     float4 *srt_pos32;   // x, y, z relative to the slot's own cell centre, q (mixed)
     long long *srt_fix;  // plain: x, y, z from the cell centre in units of 2^-59, three arrays of nsite
-    int *near_far;       // plain: per replica, set by the gather when a site is too far from its cell for that
+    unsigned *far_bits;  // plain: a bit per slot, set by the gather when the site is too far from its cell for that
     // pair layout (mixed): the slots of a cell in groups of four, negated
     // cell-relative coordinates x[4], y[4], z[4] and keys, every run padded;
     // crun: per cell its first group and the ends of its five runs in groups
