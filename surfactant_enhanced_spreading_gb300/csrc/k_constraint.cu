@@ -377,20 +377,44 @@ __device__ __forceinline__ bool gt_abs_num(double x, double t) {
     const long long a = __double_as_longlong(x) & 0x7fffffffffffffffLL;
     return a > __double_as_longlong(t) && a <= 0x7ff0000000000000LL;
 }
-// FP64 to FP32 (truncated; below FP32's normal range 0) and back as bit moves
-// on the integer pipe: GB300 converts at its FP64 rate, 64 cycles a warp
-// instruction against about 14 for these.  With them and fused predictors a
-// water's SHAKE half takes 185 FP64 instructions, not 258 (100,000 waters: 79
-// -> 67 us; RATTLE 50 -> 43)
-__device__ __forceinline__ float to32(double v) {
-    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v);
-    const unsigned a = hi & 0x7fffffffu;
-    const unsigned f = __funnelshift_l(lo, a, 3) + 0x40000000u;   // exponent bias 1023 -> 127
-    return __uint_as_float(a < 897u << 20 ? 0u : (f & 0x7fffffffu) | (hi & 0x80000000u));
+// FP64 to FP32 and back as integer operations: GB300 converts at its FP64 rate,
+// 64 cycles a warp instruction against about 18 for these.  With them and fused
+// predictors a water's SHAKE half takes 185 FP64 instructions, not 258 (100,000
+// waters: 79 -> 67 us; RATTLE 50 -> 43).  A group with a value outside FP32's
+// normal range (zero, infinities and NaN among them) takes the conversion, as
+// calls; tested once a group (value by value it cost a step of 3,000 sites 2 us).
+__device__ __noinline__ float convert32(double v) { return (float)v; }
+__device__ __noinline__ double convert64(float v) { return (double)v; }
+template <int N>
+__device__ __forceinline__ void to32(const double *v, float *o) {
+    bool rare = false;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(v[k]);
+        rare = rare || ((unsigned)(b >> 32) & 0x7fffffffu) - (897u << 20) >= (1150u - 897u) << 20;
+        const unsigned long long m = b + (0x0fffffffu + ((unsigned)b >> 29 & 1u));   // to nearest, ties to even
+        const unsigned hi = (unsigned)(m >> 32);
+        const unsigned f = __funnelshift_l((unsigned)m, hi & 0x7fffffffu, 3) + 0x40000000u;   // exponent bias 1023 -> 127
+        o[k] = __uint_as_float((f & 0x7fffffffu) | (hi & 0x80000000u));
+    }
+    if (rare) {
+#pragma unroll
+        for (int k = 0; k < N; k++) o[k] = convert32(v[k]);
+    }
 }
-__device__ __forceinline__ double to64(float v) {   // (0 becomes 2^-127)
-    const unsigned f = __float_as_uint(v);
-    return __hiloint2double((int)((((f & 0x7fffffffu) >> 3) + 0x38000000u) | (f & 0x80000000u)), (int)(f << 29));
+template <int N>
+__device__ __forceinline__ void to64(const float *v, double *o) {
+    bool rare = false;
+#pragma unroll
+    for (int k = 0; k < N; k++) {
+        const unsigned f = __float_as_uint(v[k]), a = f & 0x7fffffffu;
+        rare = rare || a - 0x00800000u >= 0x7f000000u;
+        o[k] = __hiloint2double((int)(((a >> 3) + 0x38000000u) | (f & 0x80000000u)), (int)(f << 29));
+    }
+    if (rare) {
+#pragma unroll
+        for (int k = 0; k < N; k++) o[k] = convert64(v[k]);
+    }
 }
 
 __device__ __forceinline__ void inv3f(const float (&A)[3][3], float (&B)[3][3]) {
@@ -466,10 +490,8 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, const double (&t
     }
     // the Jacobian and its inverse in FP32: they only steer the steps
     float R32[3][3], P32[3][3], J[3][3], Ji[3][3];
-#pragma unroll
-    for (int b = 0; b < 3; b++)
-#pragma unroll
-        for (int a = 0; a < 3; a++) { R32[b][a] = to32(R[b][a]); P32[b][a] = to32(P[b][a]); }
+    to32<9>(&R[0][0], &R32[0][0]);
+    to32<9>(&P[0][0], &P32[0][0]);
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -480,8 +502,9 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, const double (&t
     // tolerance (its rounding, ~1e-9 of d^2 ~ 0.1, is about the tolerance
     // band itself, so these only bring the corrections near the answer)
     float c32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
-    const float D0f[3] = {to32(D0[0]), to32(D0[1]), to32(D0[2])};
-    const float thrf[3] = {to32(thr[0]), to32(thr[1]), to32(thr[2])};
+    float D0f[3], thrf[3];
+    to32<3>(D0, D0f);
+    to32<3>(thr, thrf);
     int it = 0;
     for (int k32 = 0; k32 < WMAT_FP32_STEPS && it <= maxit; k32++) {
         float f[3];
@@ -503,10 +526,7 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, const double (&t
         it++;
     }
     double cc[3][3];
-#pragma unroll
-    for (int k = 0; k < 3; k++)
-#pragma unroll
-        for (int a = 0; a < 3; a++) cc[k][a] = to64(c32[k][a]);
+    to64<9>(&c32[0][0], &cc[0][0]);
     // the tolerance test in FP64, as the reference's; a failed test takes
     // one more step from the FP64 residual (solved in FP32: it is small)
     bool done = false;
@@ -526,12 +546,15 @@ __device__ __forceinline__ int water_a_mat(const Dev &d, int m, const double (&t
             done = done && !gt_abs_num(f[b], thr[b]);
         }
         if (done) break;
-        float f32[3] = {to32(f[0]), to32(f[1]), to32(f[2])}, d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        float f32[3], d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        to32<3>(f, f32);
         water_step32(Ji, R32, f32, d32);
+        double dd[3][3];
+        to64<9>(&d32[0][0], &dd[0][0]);
 #pragma unroll
         for (int k = 0; k < 3; k++)
 #pragma unroll
-            for (int a = 0; a < 3; a++) cc[k][a] += to64(d32[k][a]);
+            for (int a = 0; a < 3; a++) cc[k][a] += dd[k][a];
         it++;
     }
     double ke1 = 0.0;
@@ -574,10 +597,7 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
         for (int a = 0; a < 3; a++) R[b][a] = r[wbi(b)][a] - r[wbj(b)][a];
     // the matrix and its inverse in FP32 (they steer the solve; the test is FP64)
     float R32[3][3], A[3][3], Ai[3][3];
-#pragma unroll
-    for (int b = 0; b < 3; b++)
-#pragma unroll
-        for (int c = 0; c < 3; c++) R32[b][c] = to32(R[b][c]);
+    to32<9>(&R[0][0], &R32[0][0]);
 #pragma unroll
     for (int b = 0; b < 3; b++)
 #pragma unroll
@@ -598,15 +618,19 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
         }
         if (done) break;
         // A h = -R.V in FP32 (R.V is small: the rounding of h is far below the tolerance)
-        float rv32[3] = {to32(rv[0]), to32(rv[1]), to32(rv[2])}, d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        float rv32[3], d32[3][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+        to32<3>(rv, rv32);
         float h[3];
 #pragma unroll
         for (int b = 0; b < 3; b++) h[b] = -(Ai[b][0] * rv32[0] + Ai[b][1] * rv32[1] + Ai[b][2] * rv32[2]);
         water_move32(R32, h, d32);
 #pragma unroll
-        for (int k = 0; k < 3; k++)
+        for (int k = 0; k < 3; k++) {
+            double dd[3];
+            to64<3>(d32[k], dd);
 #pragma unroll
-            for (int a = 0; a < 3; a++) v[k][a] += to64(d32[k][a]);
+            for (int a = 0; a < 3; a++) v[k][a] += dd[a];
+        }
         it++;
     }
 #pragma unroll
@@ -1141,8 +1165,9 @@ __device__ __forceinline__ void chains_b(const Dev &d, const CPlan &p, int item,
 // chains.  Same queue, same per-water arithmetic, same counter reset.  The
 // flexible chains are the queue's last items (a launch of their own took 6 us
 // of the SHAKE half and 8 of the RATTLE half).
+// (three CTAs per SM for RATTLE: 100,000 waters 34.8 us, 37.1 at two)
 template <bool SHAKE>
-__global__ void __launch_bounds__(CW_THREADS) k_water_mat(Dev d, CPlan p, double tol, int maxit) {
+__global__ void __launch_bounds__(CW_THREADS, SHAKE ? 2 : 3) k_water_mat(Dev d, CPlan p, double tol, int maxit) {
     griddep_wait();
     const int lane = threadIdx.x & 31;
     // the CTAs of one SM start on different schedulers (a scheduler's FP64
