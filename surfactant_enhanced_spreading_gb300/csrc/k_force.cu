@@ -775,11 +775,13 @@ __device__ __forceinline__ void near_block32(const Tgt32<K> &t, const float (&qq
         // r^-3 (1 + 3/2 e), r^-2 (1 + e) with e = 1 - r^2 r^-2: the special
         // function's 2^-22.9 and the products' roundings are most of what the
         // compensated sums leave (pair forces of 41,600 sites against FP64:
-        // 7.3e-7 without, 6.1e-7 with; 154 and 169 us)
+        // 7.3e-7 without, 6.1e-7 with; 154 and 169 us).  r^2 is bounded in it: where
+        // it overflows r^-3 is 0, and must not meet an infinity (172 and 175 us)
         if constexpr (COMP) {
 #pragma unroll
             for (int c = 0; c < C; c++) {
-                const float2 e = __ffma2_rn(__fmul2_rn(r2[c], make_float2(-1.5f, -1.5f)), i2[c], make_float2(1.5f, 1.5f));
+                const float2 rb = make_float2(fminf(r2[c].x, 1e38f), fminf(r2[c].y, 1e38f));
+                const float2 e = __ffma2_rn(__fmul2_rn(rb, make_float2(-1.5f, -1.5f)), i2[c], make_float2(1.5f, 1.5f));
                 ft[c] = __ffma2_rn(ft[c], e, ft[c]);
                 if constexpr (LJ != 0) i2[c] = __ffma2_rn(__fmul2_rn(i2[c], make_float2(2.f / 3.f, 2.f / 3.f)), e, i2[c]);
             }
