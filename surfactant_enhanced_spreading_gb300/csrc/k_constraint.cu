@@ -767,90 +767,97 @@ __device__ __forceinline__ double tri_sum(double v, int base) {
     return (v0 + v1) + v2;
 }
 
-// The wavefront for FP64 corrections, one molecule at a time with each bond
-// split over 3 lanes, one per Cartesian component.  Every FP64 warp
+// The wavefront for FP64 corrections, with each bond split over 3 lanes, one
+// per Cartesian component.  Every FP64 warp
 // instruction costs the same whatever its active lanes (64 cycles of a
 // scheduler), so a step costs the same for one bond as for ten, and what
 // counts is the number of steps.  A bond has a fixed place in its sweep, so
-// that sweeps follow each other at a lag of 4 steps and not 8 (TAU: a sweep's
+// that sweeps can follow each other at a lag of 4 steps and not 8 (TAU: a sweep's
 // bonds 0..22 at steps 0..22, the second branch of site 17, bonds 23..26,
 // beside the first at 19..22, bond 27 at 23): of two bonds that share a site
 // the later in the reference's order comes 1 to 3 steps after the other, so
-// every site sees the sequential order's updates.  Six sweeps are in flight,
-// seven bonds a step: lane 3 u + k is component k of the main line of sweep u
-// (mod 6) for u < 6, and of the second branch for u = 6.  S sweeps take 4 S +
-// 20 steps (8 S + 20 at a lag of 8, which ran two molecules in a warp).
+// every site sees the sequential order's updates.  One molecule (N = 1): a lag
+// of 4, six sweeps in flight, seven bonds a step, S sweeps in 4 S + 20 steps.  Two at
+// once: a lag of 6, four sweeps each, ten bonds a step, 6 S + 20 steps for both:
+// 2,600 surfactants on four warps an SM, SHAKE / RATTLE 226 / 168 us one at a
+// time, 178 / 141 two at once (256 / 199 one after the other, and 208 / 164
+// both at a lag of 8).  Lane 3 u + k of a molecule's group is component k of the main line of
+// sweep u (mod LINES) for u < LINES, and of the second branch for u = LINES.
 // Splitting the components takes a SHAKE bond from 25 to 18 FP64 warp
 // instructions (9 to 6 for a bond within tolerance) and a RATTLE bond from 12
 // to 7; the two dot products go over shuffles.  Returns a ballot whose bit
 // 12 q is set if molecule q ran out of sweeps.
-constexpr int TAU_LAG = 4, TAU_END = 23, TAU_LINES = 6;
-template <bool SHAKE>
-__device__ __forceinline__ unsigned surf_wavefront3(const Dev &d, MolSmem<double, SHAKE ? 16 : 11> *sms, int n,
-                                                    double tol, int maxit) {
-    const int lane = threadIdx.x & 31;
-    const int u = lane / 3, k = lane - 3 * u, base = min(3 * u, 29);
-    const bool line = u < TAU_LINES, branch = u == TAU_LINES;
-    unsigned failed = 0;
+constexpr int TAU_END = 23;   // step of a sweep's last bond
+template <bool SHAKE, int N>
+__device__ __forceinline__ unsigned surf_wavefront3(const Dev &d, MolSmem<double, SHAKE ? 16 : 11> *sms, double tol,
+                                                    int maxit) {
+    constexpr int LAG = N == 1 ? 4 : 6, LINES = (TAU_END + 1) / LAG, GROUP = 3 * (LINES + 1);
+    static_assert(N * GROUP <= 32 && LINES * LAG == TAU_END + 1, "a line's next sweep follows its last at once");
+    const int lane = threadIdx.x & 31, q = min(lane / GROUP, N - 1), r = lane - q * GROUP;
+    const int u = r / 3, k = r - 3 * u, base = min(lane - k, 29);
+    const bool line = u < LINES, branch = u == LINES;
+    const unsigned group = ((1u << GROUP) - 1) << (q * GROUP);
     if (maxit < 0) return 0x1001u;   // no sweep allowed
-    for (int q = 0; q < n; q++) {
-        MolSmem<double, SHAKE ? 16 : 11> &sm = sms[q];
-        double *rec = &sm.rec[0][0];
-        int kmine = line ? u : 0;   // the lane's current sweep
-        bool changed = false, branch_changed = false;   // in it; on its second branch (kept one step for the main line)
-        for (int t = 0;; t++) {
-            const int tau = t - TAU_LAG * kmine;
-            const bool valid = kmine <= maxit && (line ? tau >= 0 : branch && tau >= 19 && tau <= 22);
-            const int b = valid ? (branch ? tau + 4 : tau == TAU_END ? NBOND - 1 : tau) : 0;
-            const int sb = skew8(b), i = sbi32(b), si = skew8(i), sj = skew8(b + 1);
-            double ci = 0.0, cj = 0.0, dx = 0.0, pr = 0.0;
-            if (valid) {
-                ci = sm.sc[k][si];
-                cj = sm.sc[k][sj];
-                dx = ci - cj;
-                pr = SHAKE ? dx * (dx + rec[k * SK + sb]) : rec[k * SK + sb] * dx;   // c_k (c_k + 2P_k)  /  -fb R_k c_k
-            }
-            const double sum = tri_sum(pr, base);
-            double gab = 0.0;
-            bool act = false;
-            if constexpr (SHAKE) {
-                const double diffsq = valid ? rec[12 * SK + sb] - sum : 0.0;   // D0 - c.(c + 2P)
-                act = valid && gt_abs(diffsq, rec[14 * SK + sb]);
-                if (__any_sync(FULL, act)) {   // the step only when some bond of the warp is corrected
-                    const double tk = valid ? rec[(3 + k) * SK + sb] * dx : 0.0;
-                    const double tt = tri_sum(tk, base);
-                    const double y0 = valid ? rec[13 * SK + sb] : 0.0;
-                    const double t2 = tt * tt;
-                    const double ya = fma(-y0, tt, y0), yb = fma(tt, tt, 1.0), yc = fma(t2, t2, 1.0);
-                    gab = (diffsq * ya) * (yb * yc);
-                }
-            } else {
-                gab = valid ? rec[9 * SK + sb] + sum : 0.0;   // -fb R.(V + c)
-                act = valid && gt_abs(gab, tol);
-            }
-            if (act) {
-                const int fa = SHAKE ? 6 : 3, fb = SHAKE ? 9 : 6;
-                sm.sc[k][si] = fma(rec[(fa + k) * SK + sb], gab, ci);
-                sm.sc[k][sj] = fma(-rec[(fb + k) * SK + sb], gab, cj);
-                changed = true;
-            }
-            // a sweep ends with its main line; the branch's flag dates from the step before
-            const bool ends = line && valid && tau == TAU_END;
-            const bool bc = __any_sync(FULL, branch && branch_changed);
-            const unsigned clean = __ballot_sync(FULL, ends && !changed && !bc);
-            const unsigned last = __ballot_sync(FULL, ends && kmine == maxit);
-            if (ends) { changed = false; kmine += TAU_LINES; }
-            if (branch && tau == 22) { branch_changed = changed; changed = false; kmine++; }
-            __syncwarp();
-            if (clean) break;
-            if (last) {
-                failed |= 1u << (12 * q);
-                break;
-            }
+    MolSmem<double, SHAKE ? 16 : 11> &sm = sms[q];
+    double *rec = &sm.rec[0][0];
+    int kmine = line ? u : 0;   // the lane's current sweep
+    bool changed = false, branch_changed = false;   // in it; on its second branch (kept until its next for the main line)
+    bool done = false, fail = false;                // of the molecule
+    for (int t = 0;; t++) {
+        const int tau = t - LAG * kmine;
+        const bool valid = !done && kmine <= maxit && (line ? tau >= 0 : branch && tau >= 19 && tau <= 22);
+        const int b = valid ? (branch ? tau + 4 : tau == TAU_END ? NBOND - 1 : tau) : 0;
+        const int sb = skew8(b), i = sbi32(b), si = skew8(i), sj = skew8(b + 1);
+        double ci = 0.0, cj = 0.0, dx = 0.0, pr = 0.0;
+        if (valid) {
+            ci = sm.sc[k][si];
+            cj = sm.sc[k][sj];
+            dx = ci - cj;
+            pr = SHAKE ? dx * (dx + rec[k * SK + sb]) : rec[k * SK + sb] * dx;   // c_k (c_k + 2P_k)  /  -fb R_k c_k
         }
+        const double sum = tri_sum(pr, base);
+        double gab = 0.0;
+        bool act = false;
+        if constexpr (SHAKE) {
+            const double diffsq = valid ? rec[12 * SK + sb] - sum : 0.0;   // D0 - c.(c + 2P)
+            act = valid && gt_abs(diffsq, rec[14 * SK + sb]);
+            if (__any_sync(FULL, act)) {   // the step only when some bond of the warp is corrected
+                const double tk = valid ? rec[(3 + k) * SK + sb] * dx : 0.0;
+                const double tt = tri_sum(tk, base);
+                const double y0 = valid ? rec[13 * SK + sb] : 0.0;
+                const double t2 = tt * tt;
+                const double ya = fma(-y0, tt, y0), yb = fma(tt, tt, 1.0), yc = fma(t2, t2, 1.0);
+                gab = (diffsq * ya) * (yb * yc);
+            }
+        } else {
+            gab = valid ? rec[9 * SK + sb] + sum : 0.0;   // -fb R.(V + c)
+            act = valid && gt_abs(gab, tol);
+        }
+        if (act) {
+            const int fa = SHAKE ? 6 : 3, fb = SHAKE ? 9 : 6;
+            sm.sc[k][si] = fma(rec[(fa + k) * SK + sb], gab, ci);
+            sm.sc[k][sj] = fma(-rec[(fb + k) * SK + sb], gab, cj);
+            changed = true;
+        }
+        // a sweep ends with its main line; the branch's flag dates from the step before
+        const bool ends = line && valid && tau == TAU_END;
+        const bool bc = (__ballot_sync(FULL, branch && branch_changed) & group) != 0;
+        const unsigned clean = __ballot_sync(FULL, ends && !changed && !bc) & group;
+        const unsigned last = __ballot_sync(FULL, ends && kmine == maxit) & group;
+        if (ends) { changed = false; kmine += LINES; }
+        if (branch && tau == 22) { branch_changed = changed; changed = false; kmine++; }
         __syncwarp();
+        if constexpr (N == 1) {
+            if (clean) return 0;
+            if (last) return 1u;
+        } else {
+            fail = fail || (!done && !clean && last);
+            done = done || clean || last;
+            if (__all_sync(FULL, done)) break;
+        }
     }
-    return failed;
+    const unsigned f = __ballot_sync(FULL, fail);
+    return (f & 1u) | (f >> GROUP & 1u) << 12;
 }
 
 // whether molecule g of the warp ran out of sweeps, from the wavefront's ballot
@@ -934,7 +941,7 @@ __device__ __forceinline__ void surf_a(const Dev &d, const int *mols, int n, dou
         for (int s = w; s < NSURF; s += WF_LANES) ke0 = __dadd_rn(ke0, sms[grp].kes[s]);
     ke0 = group_sum(ke0);
     unsigned failed;
-    if constexpr (sizeof(C) == 8) failed = surf_wavefront3<true>(d, sms, n, tol, maxit);
+    if constexpr (sizeof(C) == 8) failed = n == 1 ? surf_wavefront3<true, 1>(d, sms, tol, maxit) : surf_wavefront3<true, 2>(d, sms, tol, maxit);
     else failed = surf_wavefront<C, true>(d, sms, mine.g0, n, tol, maxit);
     // sites: positions, velocities, m v^2 after
     for (int it = lane; it < n * NSURF; it += 32) {
@@ -1006,7 +1013,7 @@ __device__ __forceinline__ void surf_b(const Dev &d, const int *mols, int n, dou
     }
     __syncwarp();
     unsigned failed;
-    if constexpr (sizeof(C) == 8) failed = surf_wavefront3<false>(d, sms, n, tol, maxit);
+    if constexpr (sizeof(C) == 8) failed = n == 1 ? surf_wavefront3<false, 1>(d, sms, tol, maxit) : surf_wavefront3<false, 2>(d, sms, tol, maxit);
     else failed = surf_wavefront<C, false>(d, sms, mine.g0, n, tol, maxit);
     for (int it = lane; it < n * NSURF; it += 32) {
         const int q = it / NSURF, s = it - q * NSURF;
