@@ -715,6 +715,7 @@ __device__ __forceinline__ unsigned surf_wavefront(const Dev &d, MolSmem<C, SHAK
     const int lane = threadIdx.x & 31, w = lane & (WF_LANES - 1), grp = lane >> 2;
     const unsigned gmask = 0xFu << (4 * grp);
     MolSmem<C, SHAKE ? 16 : 11> &sm = sms[grp < n ? grp : 0];
+    if (maxit < 0) return 0x11111111u;   // no sweep allowed
     const double tol2d = 2.0 * tol;
     const C tolc = (C)tol;
     int kmine = w;
