@@ -1097,8 +1097,10 @@ __global__ void __launch_bounds__(CW_THREADS) k_constrain(Dev d, CPlan p, double
     }
     // the other warps of a surfactant CTA stay idle, so its chains keep the SM's FP64 pipe
     if (!surf_cta || warp < p.s_warps) {
-        // (FP32 sweeps are no FP64 queue: 5,000 waters ran 51 us from the
-        // counter alone, 58 spread over all SMs)
+        // (FP32 sweeps are no FP64 queue, and a warp alone on its scheduler waits:
+        // SHAKE + RATTLE from the counter alone / spread over all SMs, us: 1,200
+        // waters 66 / 78, 3,600 with 36 surfactants 93 / 105, 5,800 with 58 98 /
+        // 106, 12,000 with 60 109 / 117, 24,000 89 / 95)
         const unsigned free_ctas = sizeof(C) == 8 ? gridDim.x - p.n_scta : 0;
         for (bool first = !surf_cta && free_ctas;; first = false) {
             const unsigned item = water_item(p, lane, first, warp * free_ctas + blockIdx.x - p.n_scta, CW * free_ctas);

@@ -474,17 +474,19 @@ int dalloc(sesp_ctx *c, T **p, size_t n) {
 
 // Systems up to this size run the pair field with one work item per partner
 // cell (27 partials per site) instead of per row of three (9): a small system
-// has too few rows to fill the GPU.  The field alone gains up to 45,000 sites
-// (us, rows against cells: 3,000 sites 30.9 / 26.6, FP64 614 / 317; 21,400
-// sites 64.9 / 57.1; 62,400 sites 142.6 / 150.7), a step with the graphite and
-// chain kernels beside it up to 15,000 (16,450 sites 162.8 / 164.1, 21,400
-// sites 96.5 / 99.7, 38,700 sites 131.8 / 139.4; FP64 36,600 sites 1,421 /
-// 1,445).
-constexpr int NEAR_SPLIT_MAX = 20000;
+// has too few rows to fill the GPU, and more partials cost more to add.  Mean
+// of a step, a tenth of them with a rebuild (us, rows / cells), FP32: 10,300
+// sites 84.8 / 84.7, 12,500 92.1 / 90.6, 14,400 95.3 / 95.9, 18,100 102.0 /
+// 103.7, 23,700 110.7 / 114.4; compensated 12,500 114.0 / 111.3, 14,400 119.6 /
+// 120.8; reference preset 11,800 170.0 / 168.0, 14,100 172.6 / 173.8.  FP64:
+// 10,300 603 / 554, 18,100 835 / 798, 20,300 988 / 953, 23,700 1,061 / 1,060.
+// (The server's memory estimate restates the two.)
+constexpr int NEAR_SPLIT_MAX = 13000, NEAR_SPLIT_MAX64 = 23000;
+bool near_split(int nsite, int precision) { return nsite <= (precision == SESP_PLAIN_FP64 ? NEAR_SPLIT_MAX64 : NEAR_SPLIT_MAX); }
 // work items of the pair field: 9 rows (or 27 cells) x the chunks of every
 // occupied cell (LJ-carrying sites and water H, each rounded up to 32s)
-size_t near_items_max(int nsite, int ncell) {
-    return (nsite <= NEAR_SPLIT_MAX ? 27 : 9) * ((size_t)nsite / 32 + 2 * (size_t)std::min(nsite, ncell)) + 16;
+size_t near_items_max(int nsite, int ncell, bool split) {
+    return (split ? 27 : 9) * ((size_t)nsite / 32 + 2 * (size_t)std::min(nsite, ncell)) + 16;
 }
 
 void free_state(sesp_ctx *c) {
@@ -867,7 +869,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
     int N = nsite, M = nmol, C = ncell;
     d.nsite = N;
     d.nrep = R;
-    d.near_split = N <= NEAR_SPLIT_MAX;
+    d.near_split = near_split(N, c->p.precision);
     int e = 0;
     double **a12[12] = {&d.x, &d.y, &d.z, &d.vx, &d.vy, &d.vz, &d.ax, &d.ay, &d.az, &d.fx, &d.fy, &d.fz};
     for (auto q : a12) if ((e = dalloc(c, q, N))) return e;
@@ -884,7 +886,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) || (e = dalloc(c, &d.srt_fix, c->p.precision == SESP_PLAIN_FP64 ? 3 * (size_t)N : 1)) ||
         (e = dalloc(c, &d.far_bits, (size_t)N / 32 + 1)) ||
         (e = dalloc(c, &d.pair_xyz, 3 * pair_max)) || (e = dalloc(c, &d.pair_key, pair_max)) || (e = dalloc(c, &d.crun, 8 * (size_t)C)) || (e = dalloc(c, &d.nf, 3 * (size_t)N)) ||
-        (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C))) ||
+        (e = dalloc(c, &d.near_part, (d.near_split ? 81 : 27) * (size_t)N)) || (e = dalloc(c, &d.near_items, near_items_max(N, C, d.near_split))) ||
         (e = dalloc(c, &d.near_mask, C)) || (e = dalloc(c, &d.srt_cell, N)) || (e = dalloc(c, &d.near_ctl, 2 + 2 * NEAR_CLASSES)) ||
         (e = dalloc(c, &d.isub, (size_t)c->ssite * nsm)) || (e = dalloc(c, &d.O4, (size_t)LP * C)) ||
         (e = dalloc(c, &d.L4, (size_t)LP * C)) || (e = dalloc(c, &d.L4f, (size_t)LP * C)) ||

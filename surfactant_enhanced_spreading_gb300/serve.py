@@ -96,8 +96,14 @@ def make_request(rid: int, n_water: int, n_surf: int, steps: int, seed: int, arr
     raise RuntimeError(f"no box found for {n_water} waters and {n_surf} surfactants")
 
 
-def estimate_bytes(system: S.System) -> int:
-    """Upper estimate of an engine's device memory for this system, from the
+# sites up to which an engine's pair field runs single cells as items, FP32 and
+# FP64 paths (the library's constants of the same names)
+NEAR_SPLIT_MAX, NEAR_SPLIT_MAX64 = 13000, 23000
+
+
+def estimate_bytes(system: S.System, precision: int = E.PLAIN_FP64) -> int:
+    """Upper estimate of an engine's device memory for this system (the plain
+    path's is an upper one for every precision), from the
     engine's allocation list: per-site, per-molecule and per-cell arrays, the
     multipole tables of the three levels, the translation operators and the
     per-column carbon lists (each carbon lies within reach of at most about
@@ -113,7 +119,7 @@ def estimate_bytes(system: S.System) -> int:
     w2 = 2 * d2 + 1
     # pair field: partials of 9 rows, or of 27 cells in small contexts; its
     # work items and the padded partner layout
-    parts = 27 if n <= 20000 else 9
+    parts = 27 if n <= (NEAR_SPLIT_MAX64 if precision == E.PLAIN_FP64 else NEAR_SPLIT_MAX) else 9
     per_site = 12 * 8 + 1 + 4 * 4 + 32 + 16 + 8 + 4 + 3 * 8 + parts * 3 * 8 + 6 + 3 * 8 + 12 * 8 + 4 + 16 + 24 + parts * 8 / 32 + 4
     per_mol = 5 * 4 + 2 * 8 + 4 + 4 + 2 * 4 + 2   # incl. the constraint halves' water lists and sweep counts
     cz = 25 * 16
@@ -152,7 +158,7 @@ class Server:
     def run(self, requests: list[Request], clock=time.perf_counter) -> list[Result]:
         pending = sorted(requests, key=lambda r: (r.arrival, r.rid))
         for r in pending:
-            if estimate_bytes(r.system) > self.budget:
+            if estimate_bytes(r.system, self.precision) > self.budget:
                 raise E.SespError(f"EBUDGET: request {r.rid} needs more than the whole budget")
         active = []
         results = []
@@ -164,7 +170,7 @@ class Server:
             # admission in arrival order while the budget allows (no overtaking)
             while pending and pending[0].arrival <= now and len(active) < self.max_active:
                 req = pending[0]
-                est = estimate_bytes(req.system)
+                est = estimate_bytes(req.system, self.precision)
                 if used + est > self.budget:
                     break
                 pending.pop(0)
@@ -292,7 +298,7 @@ class SlotServer:
         if len(presets) > 1:
             raise ValueError("the requests of one batched context share one force field (preset)")
         for r in pending:
-            if estimate_bytes(r.system) > self.budget:
+            if estimate_bytes(r.system, self.precision) > self.budget:
                 raise E.SespError(f"EBUDGET: request {r.rid} needs more than the whole budget")
             if r.steps % self.interval:
                 raise ValueError(f"request {r.rid}: steps must be a multiple of {self.interval}")
@@ -316,7 +322,7 @@ class SlotServer:
             for req in pending:
                 if req.arrival > now or len(runs) - len(leaving) + len(joining) >= self.max_active:
                     break
-                est = estimate_bytes(req.system)
+                est = estimate_bytes(req.system, self.precision)
                 if free + est > self.budget:
                     break
                 free += est
@@ -344,7 +350,7 @@ class SlotServer:
             self.peak_used = max(self.peak_used, used)
             for req in joining:
                 pending.remove(req)
-                runs.append({"req": req, "done": 0, "est": estimate_bytes(req.system), "admitted": clock() - t0,
+                runs.append({"req": req, "done": 0, "est": estimate_bytes(req.system, self.precision), "admitted": clock() - t0,
                              "pos": None, "vel": None, "acc": None, "eta": 0.0, "fails": 0, "fails0": 0})
             if not runs:
                 if pending:
