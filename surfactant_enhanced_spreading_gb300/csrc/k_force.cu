@@ -126,14 +126,28 @@ __device__ inline void occupied_boxes(const Dev &d, int c, int ncell) {
 
 // First slot of every cell, the first group of its pair layout, and the lists
 // of occupied boxes.  A CTA takes 1,024 cells and adds up the counts before
-// them itself (coalesced; nothing waits on another CTA).  One CTA scanning all
-// cells in strided runs took 49 us on 25,600 cells.
-constexpr int SCAN_CELLS = 1024;
+// them itself (coalesced; nothing waits on another CTA), or from SCAN_DIRECT
+// cells on the CTAs' sums, which a launch before it writes: adding up every cell
+// is work for the square of their number.  (Counts alone, us, cell by cell /
+// by sums / one CTA in strided runs: 25,600 cells 8.1 / 8.9 / 21, 102,400 12.0 /
+// 9.6 / 116, 1.6 M 332 / 28 / 3,021, 16.8 M 29,987 / 246 / 28,153.)
+constexpr int SCAN_CELLS = 1024, SCAN_DIRECT = 65536;
+__global__ void __launch_bounds__(SCAN_CELLS) k_scan_sums(Dev d, int ncell) {
+    griddep_wait();
+    const int c = blockIdx.x * SCAN_CELLS + threadIdx.x, n = c < ncell ? d.ccount[c] : 0;
+    int s, q;
+    block_exscan(n, &s);
+    block_exscan(pair_groups(n), &q);
+    if (threadIdx.x == 0) d.scan_sums[blockIdx.x] = make_int2(s, q);
+}
 __global__ void __launch_bounds__(SCAN_CELLS) k_scan(Dev d, int ncell) {
     griddep_wait();
     const int c0 = blockIdx.x * SCAN_CELLS, c = c0 + threadIdx.x;
     int s = 0, q = 0;
-    for (int k = threadIdx.x; k < c0; k += SCAN_CELLS) { const int n = d.ccount[k]; s += n; q += pair_groups(n); }
+    if (ncell > SCAN_DIRECT)
+        for (int k = threadIdx.x; k < blockIdx.x; k += SCAN_CELLS) { const int2 n = d.scan_sums[k]; s += n.x; q += n.y; }
+    else
+        for (int k = threadIdx.x; k < c0; k += SCAN_CELLS) { const int n = d.ccount[k]; s += n; q += pair_groups(n); }
     int sites0, groups0, t;
     block_exscan(s, &sites0);
     block_exscan(q, &groups0);
@@ -276,7 +290,9 @@ __global__ void __launch_bounds__(256) k_sort_cells(Dev d) {
 }
 
 void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st) {
-    launch_pdl(k_scan, dim3((ncell + SCAN_CELLS - 1) / SCAN_CELLS), dim3(SCAN_CELLS), 0, st, d, ncell);
+    const dim3 sg((ncell + SCAN_CELLS - 1) / SCAN_CELLS), sb(SCAN_CELLS);
+    if (ncell > SCAN_DIRECT) launch_pdl(k_scan_sums, sg, sb, 0, st, d, ncell);
+    launch_pdl(k_scan, sg, sb, 0, st, d, ncell);
     launch_pdl(k_scatter, dim3((nsite + 255) / 256 > 0 ? (nsite + 255) / 256 : 1), dim3(256), 0, st, d, nsite);
     launch_pdl(k_sort_cells, dim3(min(ncell, 152 * 8)), dim3(256), 0, st, d);
 }

@@ -880,7 +880,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         (e = dalloc(c, &d.mw1, M)) || (e = dalloc(c, &d.ke, 2 * M)) || (e = dalloc(c, &d.mfail, M)) ||
         (e = dalloc(c, &d.rep, R)) || (e = dalloc(c, &d.eta, R)) || (e = dalloc(c, &d.crep, C)) ||
         (e = dalloc(c, &d.b3rep, n3)) || (e = dalloc(c, &d.b2rep, n2)) || (e = dalloc(c, &d.cstart, C + 1)) ||
-        (e = dalloc(c, &d.ccount, C + 16 * (size_t)R + 3)) || (e = dalloc(c, &d.cfill, C)) || (e = dalloc(c, &d.sloc, N)) ||
+        (e = dalloc(c, &d.ccount, C + 16 * (size_t)R + 3)) || (e = dalloc(c, &d.cfill, C)) || (e = dalloc(c, &d.scan_sums, (size_t)C / 1024 + 1)) || (e = dalloc(c, &d.sloc, N)) ||
         (e = dalloc(c, &d.sslot, N)) || (e = dalloc(c, &d.srt_site, N)) || (e = dalloc(c, &d.srt_pos, N)) ||
         (e = dalloc(c, &d.srt_pos32, N)) || (e = dalloc(c, &d.srt_meta, N)) || (e = dalloc(c, &d.srt_key, N)) ||
         (e = dalloc(c, &d.srt_xmask, N)) || (e = dalloc(c, &d.srt_pair, N)) || (e = dalloc(c, &d.srt_fix, c->p.precision == SESP_PLAIN_FP64 ? 3 * (size_t)N : 1)) ||

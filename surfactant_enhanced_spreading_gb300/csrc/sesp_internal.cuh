@@ -159,6 +159,7 @@ struct Dev {
     // cells
     int *crep, *b3rep, *b2rep;
     int *cstart, *ccount, *cfill;
+    int2 *scan_sums;     // sites and pair groups of every 1,024 cells (large contexts)
     int *sloc, *sslot;
     int *cnh;            // per cell: slots with LJ (every kind but water H), which the sort puts first
     int *cno;            // per cell: water O among them, which come first of all
