@@ -477,12 +477,19 @@ __device__ inline void local_grad(const LF &L, R x, R y, R z, R &gx, R &gy, R &g
 // picks it.  near_split: one per partner cell instead of row.
 // Chunks do not mix LJ-carrying targets (the first nh of a cell) and water H:
 // the two take different loops, and a target's loop must not depend on the tile.
+// On the FP32 paths a cell of up to near_merge sites, which fit one pass of a
+// warp, is not parted: all its targets take the LJ loop.  (Two chunks
+// stage the row twice and leave lanes idle; with more targets the water H's LJ
+// code costs more.  Us: 800 replicas of 936 sites 932 -> 757, 800 of 300 sites
+// 165 -> 111, 100 of 3,120 sites 400 -> 375, 312,000 sites in one 632 -> 629.)
 // item.x = cell, item.y = part << 24 | chunk, part = plane * 3 + row, or
 // 3 (plane * 3 + row) + cell with near_split.
 
 __host__ __device__ inline int near_chunks(int nh, int ni, int tile) {
     return (nh + tile - 1) / tile + (ni - nh + tile - 1) / tile;
 }
+// targets of cell c (ni sites) that take the LJ loop, its first ones
+__device__ __forceinline__ int near_lj_targets(const Dev &d, int c, int ni) { return ni <= d.near_merge ? ni : d.cnh[c]; }
 // first and past-the-end target of a chunk
 __device__ inline void near_chunk(int nh, int ni, int tile, int ch, int &b, int &e) {
     const int k = (nh + tile - 1) / tile;
@@ -556,7 +563,7 @@ __device__ __forceinline__ void near_cell_items(const Dev &d, int c, int tile, b
         if (lane == 0) d.near_mask[c] = (int)m;
     }
     if (npart == 0) return;
-    const int ni = d.cstart[c + 1] - d.cstart[c], nh = d.cnh[c], nch = near_chunks(nh, ni, tile);
+    const int ni = d.cstart[c + 1] - d.cstart[c], nh = near_lj_targets(d, c, ni), nch = near_chunks(nh, ni, tile);
     for (int ch = 0; ch < nch; ch++) {
         int tb, te;
         near_chunk(nh, ni, tile, ch, tb, te);
@@ -832,10 +839,10 @@ __device__ __forceinline__ void near_block32(const Tgt32<K> &t, const float (&qq
 
 // One FP32 work item with K target sites per lane (lane + 32 j from `first`):
 // the force of the partner cells xo0..xo1 of row pr on them, written to
-// partial `part`.  qt: charges by kind.
+// partial `part`.  lj: some of them carry LJ.  qt: charges by kind.
 template <int K, bool PER, bool COMP>
 __device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, const float *qt, float *part, int c, int pr,
-                                            int xo0, int xo1, int first, int ni, int lane, Stage32<COMP> &st) {
+                                            int xo0, int xo1, int first, int ni, bool lj, int lane, Stage32<COMP> &st) {
     const int dzc = pr / 3 - 1, dyc = pr % 3 - 1;
     const int s0 = d.cstart[c];
     // lane l holds the pair layout of the row's cell at x offset l - 1: first
@@ -872,7 +879,6 @@ __device__ __forceinline__ void near_item32(const Dev &d, const float2 *ljt, con
         }
     }
     const unsigned excl = __reduce_or_sync(0xffffffffu, xm);
-    const bool lj = first < d.cnh[c];   // the other chunks are water H alone
     // a block: groups q0..q0 + NEAR_Q of the cell at offset xo
     int xo = xo0, q0 = -NEAR_Q;
     auto advance = [&]() -> bool {   // to the next block; false past the last
@@ -1369,12 +1375,14 @@ __global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, i
         R *part = (R *)d.near_part + (size_t)p * 3 * nslot;
         // 64 targets at a time, two per lane where there are more than 32
         int first, end;
-        near_chunk(d.cnh[c], ni, tile, chunk, first, end);
+        const int nh = near_lj_targets(d, c, ni);
+        near_chunk(nh, ni, tile, chunk, first, end);
         for (; first < end; first += 64) {
             const int e = min(first + 64, end);
             if constexpr (MODE != 0) {
-                if (e - first > 32) near_item32<2, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
-                else near_item32<1, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lane, s_stage[w]);
+                const bool lj = first < nh;
+                if (e - first > 32) near_item32<2, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lj, lane, s_stage[w]);
+                else near_item32<1, PER, MODE == 2>(d, s_lj, s_q, part, c, pr, xo0, xo1, first, e, lj, lane, s_stage[w]);
             } else {
                 for (int f = first; f < e; f += 32) near_item64<PER>(d, s_lj, part, c, pr, xo0, xo1, f, min(f + 32, e), lane, s_stage[w]);
             }
