@@ -472,6 +472,16 @@ int dalloc(sesp_ctx *c, T **p, size_t n) {
     return 0;
 }
 
+// n doubles of mapped host memory, or nulls where none is to be had (the values then go by copies)
+void mapped_alloc(double **host, double **dev, size_t n) {
+    if (cudaHostAlloc((void **)host, n * sizeof(double), cudaHostAllocMapped) == cudaSuccess &&
+        cudaHostGetDevicePointer((void **)dev, *host, 0) == cudaSuccess)
+        return;
+    cudaGetLastError();
+    cudaFreeHost(*host);
+    *host = *dev = nullptr;
+}
+
 // Systems up to this size run the pair field with one work item per partner
 // cell (27 partials per site) instead of per row of three (9): a small system
 // has too few rows to fill the GPU, and more partials cost more to add.  Mean
@@ -727,12 +737,11 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
         cudaEventCreateWithFlags(&c->ev_join, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_eta, cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&c->ev_list, cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&c->ev_items, cudaEventDisableTiming) != cudaSuccess ||
-        cudaHostAlloc(&c->host_values, HOST_VALUES * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
-        cudaHostGetDevicePointer((void **)&c->host_values_dev, c->host_values, 0) != cudaSuccess) {
+        cudaEventCreateWithFlags(&c->ev_items, cudaEventDisableTiming) != cudaSuccess) {
         delete c;
         return fail(SESP_ECUDA, "stream");
     }
+    mapped_alloc(&c->host_values, &c->host_values_dev, HOST_VALUES);
     for (int k = 0; k < 16; k++) cudaEventCreate(&c->ev[k]);
     init_force_kernels();
     init_constraint_kernels();
@@ -904,13 +913,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
         return e;
     const int w2x = 2 * d2.x + 1, w2y = 2 * d2.y + 1, w2z = 2 * d2.z + 1;
     const size_t nh2 = (size_t)w2x * w2y * w2z * NHARM;
-    if (N <= HOST_STATE_MAX &&
-        (cudaHostAlloc(&c->host_state, 12 * (size_t)N * sizeof(double), cudaHostAllocMapped) != cudaSuccess ||
-         cudaHostGetDevicePointer((void **)&c->host_state_dev, c->host_state, 0) != cudaSuccess)) {
-        cudaGetLastError();   // none to be had: the state goes by copies
-        cudaFreeHost(c->host_state);
-        c->host_state = c->host_state_dev = nullptr;
-    }
+    if (N <= HOST_STATE_MAX) mapped_alloc(&c->host_state, &c->host_state_dev, 12 * (size_t)N);
     lap("allocation");
     // real-form M2L at L4 and L3: work items (tiles of targets) of one parity
     // class, each split into M2C_GROUPS offset groups (a constant, so a
@@ -1794,7 +1797,7 @@ int sesp_temperature(sesp_ctx *c, double *t) {
     if (int e = check_ctx(c, true)) return e;
     if (!t) return fail(SESP_EINVAL, "null output");
     if (set_device(c)) return SESP_ECUDA;
-    const bool small = c->nrep <= HOST_VALUES;
+    const bool small = c->host_values && c->nrep <= HOST_VALUES;
     launch_temperature(c->d, c->nrep, small ? c->host_values_dev : nullptr, c->st);
     CK(cudaGetLastError());
     std::vector<double> sums(c->nrep);
