@@ -38,9 +38,9 @@ ROOT = os.path.dirname(os.path.abspath(__file__))
 sys.path.insert(0, ROOT)
 
 DT_FS = 2.0
-FLOPS_COUL = 18       # per ordered site pair, Coulomb only (sqrt and divide as 1 each)
-FLOPS_LJ_EXTRA = 11   # added when the pair is LJ-active within rc
-FLOPS_L2P = 25 * 40   # local-expansion force per site
+FLOPS_COUL = 16       # per ordered site pair, Coulomb only, as the pair field forms it (the reciprocal root apart)
+FLOPS_LJ_EXTRA = 8    # added when the pair is LJ-active within rc
+FLOPS_L2P = 270       # local-expansion force per site
 # kernels launched per step on the configuration preset's mixed path (gather;
 # graphite and chain terms on the side stream; pair field + finish; site
 # forces; SHAKE half and eta update; RATTLE half) and per rebuild step (cell

@@ -24,14 +24,15 @@
 //
 // Scheduling.  GB300 issues FP64 at one warp instruction per ~19 cycles per
 // SM whatever the active lanes, with ~64 cycles of dependent latency.  A water
-// (one thread, 3 bonds) is FP64-throughput work; a surfactant (4 lanes, 28
-// bonds swept as a wavefront, 8 molecules per warp) is one long FP64
-// dependency chain, latency work.  One launch of gridDim = SM count CTAs of
-// 8 warps runs both: the first n_scta CTAs start s_warps warps each on the
-// surfactant queue (groups of 8 molecules; few chains per SM, so they do not
-// wait behind water instructions), every other warp takes items of 32 waters
-// from the water queue, and surfactant warps join the water queue when no
-// surfactant is left.  The water list is ordered
+// (one thread, 3 bonds) is FP64-throughput work; a surfactant (28 bonds swept
+// as a wavefront) is one long dependency chain, latency work.  One launch of
+// gridDim = SM count CTAs of 8 warps runs both: the first n_scta CTAs start
+// s_warps warps each on the surfactant queue (groups of 1 or 2 molecules with
+// FP64 corrections, up to 8 with FP32; few chains per SM, so they do not wait
+// behind water instructions), every other warp takes items of 32 waters, and
+// surfactant warps join the water queue when no surfactant is left.  With FP64
+// corrections a warp's first item of waters is fixed, the next come from the
+// queue; with FP32 all do.  The water list is ordered
 // by each molecule's sweep count in the previous call (most first, reordered
 // at every list rebuild), so the 32 lanes of an item iterate alike and the
 // longest items start first.  Which warp takes which molecule changes no
@@ -644,7 +645,8 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
 
 // ---------------------------------------------------------------- surfactants
 
-// Gauss-Seidel sweeps as a wavefront: sweep k starts WF_LAG bonds after
+// Gauss-Seidel sweeps as a wavefront, with FP32 corrections (FP64 ones take
+// surf_wavefront3 below): sweep k starts WF_LAG bonds after
 // sweep k - 1 and runs on wavefront lane k mod WF_LANES, one bond per lane
 // and step.  Two bonds that share a site are never more than 7 apart in the
 // bond order (site 17: bonds 16 and 23), so with a lag of 8 every site sees
@@ -656,13 +658,11 @@ __device__ __forceinline__ int water_b_mat(const Dev &d, int m, double tol, int 
 // sequential loop.
 //
 // A warp carries up to MPW = 8 molecules, one per group of 4 lanes (the
-// launch picks how many: mpw).  An FP64 warp instruction costs a scheduler
-// partition ~64 cycles whatever its active lanes, so a wavefront step costs
-// the same for 1 molecule as for 8: more molecules per warp is more
-// throughput for many surfactants, while with one molecule per warp a step
-// whose 4 bonds all lie within tolerance more often skips the correction
-// arithmetic.  Each group stops when its molecule has converged or failed;
-// the warp stops when all have.
+// launch picks how many: mpw): more molecules per warp is more throughput for
+// many surfactants, while with one molecule per warp a step whose 4 bonds all
+// lie within tolerance more often skips the correction arithmetic.  Each group
+// stops when its molecule has converged or failed; the warp stops when all
+// have.
 constexpr int WF_LAG = 8;
 constexpr int WF_LANES = 4;   // ceil(NBOND / WF_LAG) sweeps in flight
 constexpr int MPW = 32 / WF_LANES;   // molecules per warp
@@ -703,11 +703,8 @@ __device__ __forceinline__ double group_sum(double v) {
     return v;
 }
 
-// The wavefront of SHAKE (SHAKE = true) or RATTLE over the 8 molecules of a
-// warp.  Lane (g, w): molecule g, wavefront lane w.  Returns through fail
-// whether its molecule ran out of sweeps.
-// The wavefront with one bond per lane (FP32 corrections): lane (g, w),
-// molecule g of the warp, wavefront lane w.  Returns a ballot whose bit 4g
+// The wavefront of SHAKE (SHAKE = true) or RATTLE with one bond per lane (FP32
+// corrections): lane (g, w), molecule g of the warp, wavefront lane w.  Returns a ballot whose bit 4g
 // is set if molecule g ran out of sweeps.
 template <typename C, bool SHAKE>
 __device__ __forceinline__ unsigned surf_wavefront(const Dev &d, MolSmem<C, SHAKE ? 16 : 11> *sms, int g0, int n,
@@ -887,8 +884,8 @@ __device__ __forceinline__ SurfMol surf_mol(const SurfMol &mine, int q) {
 
 // SHAKE half of up to 8 surfactants (the whole warp): molecules mols[0..n).
 // The per-site and per-bond work of the n molecules is spread over all 32
-// lanes (an FP64 warp instruction costs the same for 4 lanes as for 32), the
-// sweeps run in the molecules' groups of 4 lanes.
+// lanes (an FP64 warp instruction costs the same for 4 lanes as for 32); for the
+// sweeps each molecule has its lanes (the wavefronts above).
 template <typename C>
 __device__ __forceinline__ void surf_a(const Dev &d, const int *mols, int n, double tol, int maxit,
                                        MolSmem<C, 16> *sms) {
@@ -1042,7 +1039,7 @@ struct CPlan {
     int ns, nw;
     int n_scta;         // CTAs that start on the surfactant queue
     int s_warps;        // surfactant warps in each of them
-    int mpw;            // surfactants per warp (groups of 4 lanes), 1..MPW
+    int mpw;            // surfactants per warp, 1..wavefront_mols
     int nmol, nsite;    // bounds every listed molecule is checked against
     const int *chains;  // flexible chains advanced by the same launch (k_water_mat)
     int nch;

@@ -175,7 +175,7 @@ __global__ void k_isub(Dev d, int nsurf_sites, const int *surf_mol_of) {
 // division of infinities inlined); 20,000 waters (a lane each) 381 -> 254 and
 // 417 -> 244 us (346).
 constexpr int WATERS_SPLIT = 10;                       // waters of a warp with three lanes each
-constexpr int MOVE_SPLIT_MAX = WATERS_SPLIT * 4 * 152;
+constexpr int MOVE_SPLIT_MAX = WATERS_SPLIT * 4 * GB300_SMS;
 constexpr int MOVE_BLOCK = 32;
 
 // a rare division as a call: inlined, the compiler runs it beside the common

@@ -294,7 +294,7 @@ void launch_sort(const Dev &d, int nsite, int ncell, cudaStream_t st) {
     if (ncell > SCAN_DIRECT) launch_pdl(k_scan_sums, sg, sb, 0, st, d, ncell);
     launch_pdl(k_scan, sg, sb, 0, st, d, ncell);
     launch_pdl(k_scatter, dim3((nsite + 255) / 256 > 0 ? (nsite + 255) / 256 : 1), dim3(256), 0, st, d, nsite);
-    launch_pdl(k_sort_cells, dim3(min(ncell, 152 * 8)), dim3(256), 0, st, d);
+    launch_pdl(k_sort_cells, dim3(min(ncell, GB300_SMS * 8)), dim3(256), 0, st, d);
 }
 
 // ------------------------------------------------------------------ gather
@@ -388,8 +388,6 @@ template <typename R>
 __device__ inline Cx<R> cmul(Cx<R> a, Cx<R> b) { return {a.re * b.re - a.im * b.im, a.re * b.im + a.im * b.re}; }
 template <typename R>
 __device__ inline Cx<R> cscale(Cx<R> a, R s) { return {a.re * s, a.im * s}; }
-template <typename R>
-__device__ inline Cx<R> cadd(Cx<R> a, Cx<R> b) { return {a.re + b.re, a.im + b.im}; }
 template <typename R>
 __device__ inline Cx<R> csub(Cx<R> a, Cx<R> b) { return {a.re - b.re, a.im - b.im}; }
 
@@ -610,7 +608,7 @@ __global__ void __launch_bounds__(256) k_near_items_place(Dev d, int tile) {
 // (the lists of the last rebuild must be in place)
 void launch_near_items(const Dev &d, int ncell, int tile, cudaStream_t st) {
     cudaMemsetAsync(d.near_ctl + 2, 0, 2 * NEAR_CLASSES * sizeof(int), st);
-    const dim3 g(min((ncell + 7) / 8, 152 * 4)), b(256);
+    const dim3 g(min((ncell + 7) / 8, GB300_SMS * 4)), b(256);
     k_near_items_count<<<g, b, 0, st>>>(d, tile);
     launch_pdl(k_near_items_place, g, b, 0, st, d, tile);
 }
@@ -1310,7 +1308,7 @@ __device__ __forceinline__ void near_item64(const Dev &d, const double2 *ljt, do
 // Near field as a persistent kernel: each warp takes items from a global
 // counter until none are left, and for its item sums the force of one
 // partner row (or one of its cells, near_split) on up to `tile` target
-// sites, two per lane.  Each item writes its own partial per slot; the
+// sites, two per lane (FP64: one).  Each item writes its own partial per slot; the
 // finish kernel adds the cells of a row and the 9 rows in a fixed order.
 // Which warp takes which item does not change any arithmetic, so results are
 // bit-reproducible.
@@ -2013,10 +2011,6 @@ __global__ void __launch_bounds__(256) k_m2l_all(Dev d, const C2<R> *Htab, const
     }
 }
 
-// opt-in shared-memory sizes, called once per context creation; every
-// force kernel now fits the default 48 KB
-void init_force_kernels() {}
-
 template <typename R>
 size_t m2c_smem() { return sizeof(R) * M2C_CH * LP * M2C_LD; }
 
@@ -2025,7 +2019,7 @@ void fma_build(const Dev &d, int ncell, int n3, int n2, int3 d2, const OP *m43, 
                const OP *l34, const C2<R> *h2, const C2<R> *hper, const R *cf, cudaStream_t st) {
     // one chain of dependent launches (programmatic: each waits for its
     // predecessor first); grids that stride over the occupied boxes
-    constexpr int GRID = 152 * 16;
+    constexpr int GRID = GB300_SMS * 16;
     launch_pdl(k_p2m<R>, dim3(min(ncell, GRID)), dim3(64), 0, st, d);
     launch_pdl(k_m2m<R, OP>, dim3(min(n3, GRID)), dim3(128), 0, st, d, m43, 3);
     launch_pdl(k_m2m<R, OP>, dim3(n2), dim3(128), 0, st, d, m32, 2);
@@ -2318,8 +2312,8 @@ void launch_site_forces(const Dev &d, int nsite, int terms, int mixed, cudaStrea
 
 void launch_graphite(const Dev &d, int terms, int mixed, cudaStream_t st) {
     if (terms & SESP_T_GRAPHITE) {
-        if (mixed) k_graphite<float><<<152 * 4, 256, 0, st>>>(d);
-        else k_graphite<double><<<152 * 4, 256, 0, st>>>(d);
+        if (mixed) k_graphite<float><<<GB300_SMS * 4, 256, 0, st>>>(d);
+        else k_graphite<double><<<GB300_SMS * 4, 256, 0, st>>>(d);
     }
 }
 
@@ -2977,7 +2971,7 @@ __global__ void k_flush(float4 *buf, size_t n) {
 }
 
 void launch_flush(void *buf, size_t bytes, cudaStream_t st) {
-    k_flush<<<152 * 8, 256, 0, st>>>((float4 *)buf, bytes / sizeof(float4));
+    k_flush<<<GB300_SMS * 8, 256, 0, st>>>((float4 *)buf, bytes / sizeof(float4));
 }
 
 void launch_energies(const Dev &d, int ncell, int nsite, const int *smols, int ns, int chains, double *e_slot,

@@ -65,8 +65,8 @@ int near_resident_ctas(int mode, int per);
 int near_max_ctas_per_sm(int mode, int per);
 // reset_counter: clear the pair field's work counter first; without it the
 // caller must have launched launch_gather (which clears it) on the same
-// stream since the last pair-field launch, or the launch finds every work
-// item taken and computes nothing
+// stream since the last pair-field launch, or only each warp's first item is
+// computed and the other partials stay the last launch's
 void launch_near(const Dev &d, int ncell, int nslot, int mode, int terms, const NearShape &shape, cudaStream_t st,
                  bool reset_counter, int per);
 // d2: the largest L2 offset per axis (the H table's half-widths)
@@ -74,7 +74,6 @@ void launch_fma_build(const Dev &d, int ncell, int n3, int n2, int mixed, int3 d
 void launch_site_forces(const Dev &d, int nsite, int terms, int mixed, cudaStream_t st);
 void launch_graphite(const Dev &d, int terms, int mixed, cudaStream_t st);
 void launch_graphite_list(const Dev &d, int nsite, cudaStream_t st);
-void init_force_kernels();
 void upload_intra_map(const void *host_map, cudaStream_t st);
 size_t intra_map_size();
 // chains: the surfactants are the configuration preset's 12-bead chains

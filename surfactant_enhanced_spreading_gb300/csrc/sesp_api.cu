@@ -640,8 +640,8 @@ void seq_force(sesp_ctx *c, int rebuild, int terms) {
 }
 
 // fork_eta: the eta update goes to the side stream, beside the next force
-// call, which joins it before the site forces (a step's sequence on the
-// mixed paths); otherwise it follows the SHAKE half on the main stream
+// call, which joins it before the site forces (a step's
+// sequence); otherwise it follows the SHAKE half on the main stream
 void seq_move_a(sesp_ctx *c, bool fork_eta = false) {
     tstart(c, 2);
     launch_move_a(c->d, c->wmols, c->nwm, c->smols, c->nsm, c->nrep, c->nmol, c->nsite, c->p.shake_tol, c->p.shake_maxit,
@@ -743,7 +743,6 @@ int sesp_create(const sesp_params *p, sesp_ctx **out) {
     }
     mapped_alloc(&c->host_values, &c->host_values_dev, HOST_VALUES);
     for (int k = 0; k < 16; k++) cudaEventCreate(&c->ev[k]);
-    init_force_kernels();
     init_constraint_kernels();
     {
         int dev = 0;
