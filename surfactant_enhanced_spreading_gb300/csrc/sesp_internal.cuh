@@ -184,6 +184,7 @@ struct Dev {
     double *nf;          // near + far force by slot [3 * nslot]
     double *near_part;   // partial near forces [9 rows, or 27 cells with near_split][3 * nslot] (float on the mixed path)
     int near_split;      // pair-field items are single partner cells, not rows of three
+    int near_few;        // cells of up to this many turns of near_few32 are its items
     int near_merge;      // cells of up to this many sites have no chunks of water H alone
     int2 *near_items;    // near-field work items (cell, row << 24 | chunk), most expensive first
     int *near_mask;      // per occupied cell: its parts (rows or cells) that have partners
