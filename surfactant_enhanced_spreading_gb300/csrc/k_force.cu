@@ -480,19 +480,21 @@ __device__ inline void local_grad(const LF &L, R x, R y, R z, R &gx, R &gy, R &g
 // stage the row twice and leave lanes idle; with more targets the water H's LJ
 // code costs more.  Us: 800 replicas of 936 sites 932 -> 757, 800 of 300 sites
 // 165 -> 111, 100 of 3,120 sites 400 -> 375, 312,000 sites in one 632 -> 629.)
-// On the FP32 paths a cell whose targets, FEW at a time, take the partners of
-// its shell, 32 at a time, in up to near_few turns (48, compensated 36) is one
-// item per plane (near_few32), whose force goes to the plane's first part.  The
-// rule sees the cell and its shell alone, so a replica's sums do not depend on
-// what it is batched with.  Mean step, us, FP32 / compensated, by rows alone, with
-// 24, 36, 48 and 64 turns: one water a cell (20,736 sites) 199 / 251, then 107 /
-// 117 at any; three a cell (62,208) 245 / 314, 181 / 213, 170 / 202, 173 / 204;
-// four (195,000) 576 / 750, 528 / 679, 468 / 589, 436 / 547; 16 droplets of 936
-// sites 79.7 / 90.8, 78.8 / 91.0, 79.0 / 92.5, 79.5 / 98.6, and a batch of 200 of
-// 300 sites, FP32, 220, 221, 220, 221, 229.  Dense droplets keep their times.
+// On the FP32 paths a cell of up to FEW_MAX sites with a thin shell is worked off
+// by near_few32: an item takes FEW targets and the partners of a plane of the
+// shell, 32 a turn, and its force goes to the plane's first part.  Thin: at most
+// FEW_TURNS turns an item (longer ones were the tail of a small launch: 3,000
+// sites, a step of 50.5 us, up to 58 at 16) and near_few (48) for the cell (beyond
+// it rows have their lanes full).  The rule sees the cell and its shell alone, so a
+// replica's sums do not depend on what it is batched with.  Mean step by rows
+// alone / so, us, FP32 and compensated: one water a cell (20,736 sites) 199 / 107,
+// 252 / 117; three (62,208) 246 / 181, 314 / 219; four (195,000) 576 / 477, 753 /
+// 599; with 4 turns an item 552 / 717 for the last.  Droplets keep their times.
 // item.x = cell, item.y = part << 24 | chunk, part = plane * 3 + row,
-// 3 (plane * 3 + row) + cell with near_split, or NEAR_PLANE + plane.
-constexpr int FEW = 4, NEAR_PLANE = 28;
+// 3 (plane * 3 + row) + cell with near_split, or NEAR_PLANE + plane (chunk: of
+// FEW targets; FEW_MAX keeps such a cell's items within the 18 of its two chunks).
+constexpr int FEW = 4, FEW_MAX = 24, FEW_TURNS = 6, NEAR_PLANE = 28;
+static_assert(3 * (FEW_MAX / FEW) <= 18, "items of a cell");
 __host__ __device__ inline int near_plane_part(int plane, int split) { return plane * (split ? 9 : 3); }
 
 __host__ __device__ inline int near_chunks(int nh, int ni, int tile) {
@@ -569,25 +571,23 @@ __device__ __forceinline__ void near_cell_items(const Dev &d, int c, int tile, b
             nlj += d.cnh[cn];
         }
     const int ni = d.cstart[c + 1] - d.cstart[c];
-    int turns[3], all = 0;   // of near_few32, by plane
+    int turns[3];   // of a near_few32 item, by plane
     unsigned planes = 0;
 #pragma unroll
     for (int k = 0; k < 3; k++) {
-        const int n = __reduce_add_sync(0xffffffffu, pr / 3 == k ? npart : 0);
-        turns[k] = (ni + FEW - 1) / FEW * ((n + 31) / 32);
-        all += turns[k];
-        if (n > 0) planes |= 1u << near_plane_part(k, d.near_split);
+        turns[k] = (__reduce_add_sync(0xffffffffu, pr / 3 == k ? npart : 0) + 31) / 32;
+        if (turns[k] > 0) planes |= 1u << near_plane_part(k, d.near_split);
     }
-    const bool few = all <= d.near_few;
+    const int nb = (ni + FEW - 1) / FEW;
+    const bool few = ni <= FEW_MAX && max(max(turns[0], turns[1]), turns[2]) <= FEW_TURNS && nb * (turns[0] + turns[1] + turns[2]) <= d.near_few;
     if (mask) {
         const unsigned m = few ? planes : __ballot_sync(0xffffffffu, npart > 0);
         if (lane == 0) d.near_mask[c] = (int)m;
     }
     if (few) {
-#pragma unroll
-        for (int k = 0; k < 3; k++)
-            if (lane == k && turns[k] > 0)   // first: cheap, but long for one warp (last, they were the launch's tail)
-                emit(NEAR_CLASSES - 1, make_int2(c, (NEAR_PLANE + k) << 24));
+        // first: cheap, but long for one warp
+        if (lane < 3 && (lane == 0 ? turns[0] : lane == 1 ? turns[1] : turns[2]) > 0)
+            for (int b = 0; b < nb; b++) emit(NEAR_CLASSES - 1, make_int2(c, (NEAR_PLANE + lane) << 24 | b));
         return;
     }
     if (npart == 0) return;
@@ -1040,16 +1040,16 @@ __device__ __forceinline__ void tree_add(float (&v)[16], float (&vc)[16], const 
         for (int i = 0; i < o; i++) add(i, v[i], vc[i], v[i + o], vc[i + o], o);
 }
 
-// The force of a plane of the shell on the ni sites of a cell of few, written to
-// the plane's first part.  Items of one row leave most lanes of such a cell
-// idle and pay their staging and ends of runs for a handful of partners, nine
-// times.  Here a lane takes partners, from the plane's 9 cells as one list in
-// cell and slot order, and FEW targets at a time; the lanes' sums are added as a
-// tree.  Coulomb sums are in units of the target's and water H's charges, in which
-// a water's charges are exact: a neutral molecule's terms cancel unrounded.  Bound
-// by issue and by the loads of a list that is short.
+// The force of a plane of the shell on FEW sites, from t0 on, of a cell of ni,
+// written to the plane's first part.  Items of one row leave most lanes of a cell
+// of few idle and pay their staging and ends of runs for a handful of partners,
+// nine times.  Here a lane takes partners, from the plane's 9 cells as one list in
+// cell and slot order, and the lanes' sums are added as a tree.  Coulomb sums are
+// in units of the target's and water H's charges, in which a water's charges are
+// exact: a neutral molecule's terms cancel unrounded.  Bound by issue and by the
+// loads of a list that is short.
 template <bool PER, bool COMP>
-__device__ __forceinline__ void near_few32(const Dev &d, const float2 *ljt, const float *qt, float *part, int c, int plane, int ni, int lane) {
+__device__ __forceinline__ void near_few32(const Dev &d, const float2 *ljt, const float *qt, float *part, int c, int plane, int t0, int ni, int lane) {
     const float rc2 = (float)(RC * RC), rs = (float)RS;
     const int s0 = d.cstart[c];
     // lane l < 9: cell (l % 3, l / 3) of the plane
@@ -1091,107 +1091,105 @@ __device__ __forceinline__ void near_few32(const Dev &d, const float2 *ljt, cons
     };
     constexpr int H = FEW / 2;   // targets in pairs
     const float qo = __fdiv_rn(qt[0], qt[1]), qi = __fdiv_rn(1.f, qt[1]);
-    for (int t0 = 0; t0 < ni; t0 += FEW) {
-        float2 x[H], y[H], z[H], q[H], f[H][3], g[H][3], e[COMP ? H : 1][3], ge[COMP ? H : 1][3];   // f Coulomb, g LJ
-        int m[FEW], trow[FEW];
+    float2 x[H], y[H], z[H], q[H], f[H][3], g[H][3], e[COMP ? H : 1][3], ge[COMP ? H : 1][3];   // f Coulomb, g LJ
+    int m[FEW], trow[FEW];
+#pragma unroll
+    for (int h = 0; h < H; h++) {
+        float4 t[2];
+#pragma unroll
+        for (int u = 0; u < 2; u++) {
+            const int s = s0 + min(t0 + 2 * h + u, ni - 1), kk = d.srt_key[s];
+            t[u] = d.srt_pos32[s];
+            m[2 * h + u] = kk >> 5; trow[2 * h + u] = (kk & 31) * NTYPE;
+        }
+        x[h] = make_float2(t[0].x, t[1].x); y[h] = make_float2(t[0].y, t[1].y); z[h] = make_float2(t[0].z, t[1].z);
+        q[h] = make_float2(t[0].w * (float)XPI * qt[1], t[1].w * (float)XPI * qt[1]);
+#pragma unroll
+        for (int a = 0; a < 3; a++) {
+            f[h][a] = g[h][a] = make_float2(0.f, 0.f);
+            if constexpr (COMP) e[h][a] = ge[h][a] = make_float2(0.f, 0.f);
+        }
+    }
+    float4 p;
+    int key, cell = 0;
+    load(lane, p, key, cell);
+#pragma unroll 1
+    for (int k0 = 0; k0 < all; k0 += 32) {
+        const float2 ox = make_float2(-p.x, -p.x), oy = make_float2(-p.y, -p.y), oz = make_float2(-p.z, -p.z);
+        const int mo = key >> 5, to = key & 31;
+        const float w0 = to == 0 ? qo : to == 1 ? 1.f : p.w * qi;
+        const float2 oq = make_float2(w0, w0);
+        // the targets move into the partner's frame: the shift's rounding is the same for
+        // all sites of a cell, and a neutral molecule's cancel (moving the partners instead
+        // made the forces of a thin gas 5 to 12 % less accurate)
+        const float fx = (float)(1 - cell % 3) * rs, fy = (float)(1 - cell / 3) * rs, fz = (float)(1 - plane) * rs;
+        const float2 sx = make_float2(fx, fx), sy = make_float2(fy, fy), sz = make_float2(fz, fz);
+        const bool none = k0 + lane >= all;
+        if (k0 + 32 < all) load(k0 + 32 + lane, p, key, cell);
+        float2 dx[H], dy[H], dz[H], r2[H], i2[H], ft[H];
+        bool any = false;
 #pragma unroll
         for (int h = 0; h < H; h++) {
-            float4 t[2];
-#pragma unroll
-            for (int u = 0; u < 2; u++) {
-                const int s = s0 + min(t0 + 2 * h + u, ni - 1), kk = d.srt_key[s];
-                t[u] = d.srt_pos32[s];
-                m[2 * h + u] = kk >> 5; trow[2 * h + u] = (kk & 31) * NTYPE;
+            dx[h] = __fadd2_rn(__fadd2_rn(x[h], sx), ox); dy[h] = __fadd2_rn(__fadd2_rn(y[h], sy), oy); dz[h] = __fadd2_rn(__fadd2_rn(z[h], sz), oz);
+            r2[h] = __ffma2_rn(dz[h], dz[h], __ffma2_rn(dy[h], dy[h], __fmul2_rn(dx[h], dx[h])));
+            float2 ir = make_float2(rsqrt_ftz(r2[h].x), rsqrt_ftz(r2[h].y));
+            if (none || mo == m[2 * h]) ir.x = 0.f;
+            if (none || mo == m[2 * h + 1]) ir.y = 0.f;
+            i2[h] = __fmul2_rn(ir, ir);
+            ft[h] = __fmul2_rn(ir, i2[h]);
+            if constexpr (COMP) {   // as in near_block32
+                const float2 rb = make_float2(fminf(r2[h].x, 1e38f), fminf(r2[h].y, 1e38f));
+                const float2 w = __ffma2_rn(__fmul2_rn(rb, make_float2(-1.5f, -1.5f)), i2[h], make_float2(1.5f, 1.5f));
+                ft[h] = __ffma2_rn(ft[h], w, ft[h]);
+                i2[h] = __ffma2_rn(__fmul2_rn(i2[h], make_float2(2.f / 3.f, 2.f / 3.f)), w, i2[h]);
             }
-            x[h] = make_float2(t[0].x, t[1].x); y[h] = make_float2(t[0].y, t[1].y); z[h] = make_float2(t[0].z, t[1].z);
-            q[h] = make_float2(t[0].w * (float)XPI * qt[1], t[1].w * (float)XPI * qt[1]);
+            any = any || (r2[h].x <= rc2 && ir.x != 0.f) || (r2[h].y <= rc2 && ir.y != 0.f);
+        }
+        const bool lj = __any_sync(0xffffffffu, any);
+#pragma unroll
+        for (int h = 0; h < H; h++) {
+            const float2 i3 = ft[h], dd[3] = {dx[h], dy[h], dz[h]}, fc = __fmul2_rn(oq, i3);
 #pragma unroll
             for (int a = 0; a < 3; a++) {
-                f[h][a] = g[h][a] = make_float2(0.f, 0.f);
-                if constexpr (COMP) e[h][a] = ge[h][a] = make_float2(0.f, 0.f);
+                if constexpr (COMP) kahan2(f[h][a], e[h][a], dd[a], fc);
+                else f[h][a] = __ffma2_rn(dd[a], fc, f[h][a]);
             }
-        }
-        float4 p;
-        int key, cell = 0;
-        load(lane, p, key, cell);
-#pragma unroll 1
-        for (int k0 = 0; k0 < all; k0 += 32) {
-            const float2 ox = make_float2(-p.x, -p.x), oy = make_float2(-p.y, -p.y), oz = make_float2(-p.z, -p.z);
-            const int mo = key >> 5, to = key & 31;
-            const float w0 = to == 0 ? qo : to == 1 ? 1.f : p.w * qi;
-            const float2 oq = make_float2(w0, w0);
-            // the targets move into the partner's frame: the shift's rounding is the same for
-            // all sites of a cell, and a neutral molecule's cancel (moving the partners instead
-            // made the forces of a thin gas 5 to 12 % less accurate)
-            const float fx = (float)(1 - cell % 3) * rs, fy = (float)(1 - cell / 3) * rs, fz = (float)(1 - plane) * rs;
-            const float2 sx = make_float2(fx, fx), sy = make_float2(fy, fy), sz = make_float2(fz, fz);
-            const bool none = k0 + lane >= all;
-            if (k0 + 32 < all) load(k0 + 32 + lane, p, key, cell);
-            float2 dx[H], dy[H], dz[H], r2[H], i2[H], ft[H];
-            bool any = false;
-#pragma unroll
-            for (int h = 0; h < H; h++) {
-                dx[h] = __fadd2_rn(__fadd2_rn(x[h], sx), ox); dy[h] = __fadd2_rn(__fadd2_rn(y[h], sy), oy); dz[h] = __fadd2_rn(__fadd2_rn(z[h], sz), oz);
-                r2[h] = __ffma2_rn(dz[h], dz[h], __ffma2_rn(dy[h], dy[h], __fmul2_rn(dx[h], dx[h])));
-                float2 ir = make_float2(rsqrt_ftz(r2[h].x), rsqrt_ftz(r2[h].y));
-                if (none || mo == m[2 * h]) ir.x = 0.f;
-                if (none || mo == m[2 * h + 1]) ir.y = 0.f;
-                i2[h] = __fmul2_rn(ir, ir);
-                ft[h] = __fmul2_rn(ir, i2[h]);
-                if constexpr (COMP) {   // as in near_block32
-                    const float2 rb = make_float2(fminf(r2[h].x, 1e38f), fminf(r2[h].y, 1e38f));
-                    const float2 w = __ffma2_rn(__fmul2_rn(rb, make_float2(-1.5f, -1.5f)), i2[h], make_float2(1.5f, 1.5f));
-                    ft[h] = __ffma2_rn(ft[h], w, ft[h]);
-                    i2[h] = __ffma2_rn(__fmul2_rn(i2[h], make_float2(2.f / 3.f, 2.f / 3.f)), w, i2[h]);
-                }
-                any = any || (r2[h].x <= rc2 && ir.x != 0.f) || (r2[h].y <= rc2 && ir.y != 0.f);
-            }
-            const bool lj = __any_sync(0xffffffffu, any);
-#pragma unroll
-            for (int h = 0; h < H; h++) {
-                const float2 i3 = ft[h], dd[3] = {dx[h], dy[h], dz[h]}, fc = __fmul2_rn(oq, i3);
+            if (lj) {
+                const float2 v0 = ljt[trow[2 * h] + to], v1 = ljt[trow[2 * h + 1] + to];
+                const float2 on = make_float2(r2[h].x <= rc2 ? v0.x : 0.f, r2[h].y <= rc2 ? v1.x : 0.f), i6 = __fmul2_rn(i3, i3);
+                const float2 w = __ffma2_rn(make_float2(v0.y, v1.y), i6, make_float2(-0.5f, -0.5f));
+                const float2 fl = __fmul2_rn(__fmul2_rn(__fmul2_rn(on, i6), w), i2[h]);
 #pragma unroll
                 for (int a = 0; a < 3; a++) {
-                    if constexpr (COMP) kahan2(f[h][a], e[h][a], dd[a], fc);
-                    else f[h][a] = __ffma2_rn(dd[a], fc, f[h][a]);
-                }
-                if (lj) {
-                    const float2 v0 = ljt[trow[2 * h] + to], v1 = ljt[trow[2 * h + 1] + to];
-                    const float2 on = make_float2(r2[h].x <= rc2 ? v0.x : 0.f, r2[h].y <= rc2 ? v1.x : 0.f), i6 = __fmul2_rn(i3, i3);
-                    const float2 w = __ffma2_rn(make_float2(v0.y, v1.y), i6, make_float2(-0.5f, -0.5f));
-                    const float2 fl = __fmul2_rn(__fmul2_rn(__fmul2_rn(on, i6), w), i2[h]);
-#pragma unroll
-                    for (int a = 0; a < 3; a++) {
-                        if constexpr (COMP) kahan2(g[h][a], ge[h][a], dd[a], fl);
-                        else g[h][a] = __ffma2_rn(dd[a], fl, g[h][a]);
-                    }
+                    if constexpr (COMP) kahan2(g[h][a], ge[h][a], dd[a], fl);
+                    else g[h][a] = __ffma2_rn(dd[a], fl, g[h][a]);
                 }
             }
         }
-        float v[16] = {}, vc[16] = {}, w[16] = {}, wc[16] = {};
-#pragma unroll
-        for (int k = 0; k < 3 * FEW; k++) {
-            const int h = k / 6, a = k % 3;
-            const bool u = k / 3 & 1;
-            v[k] = u ? f[h][a].y : f[h][a].x; w[k] = u ? g[h][a].y : g[h][a].x;
-            if constexpr (COMP) { vc[k] = u ? e[h][a].y : e[h][a].x; wc[k] = u ? ge[h][a].y : ge[h][a].x; }
-        }
-        tree_add<COMP, 3 * FEW>(v, vc, w, wc, lane);
-        const int j = lane / 3;   // lane 3 j + a: component a of target j
-        const float qs = j == 0 ? q[0].x : j == 1 ? q[0].y : j == 2 ? q[1].x : q[1].y;
-        float o = __shfl_down_sync(0xffffffffu, v[0], 16);
-        if constexpr (COMP) {   // o += qs (v - vc)
-            float oc = __shfl_down_sync(0xffffffffu, vc[0], 16);
-            const float t = __fmul_rn(qs, v[0]);
-            kahan(o, oc, t);
-            kahan(o, oc, __fmaf_rn(qs, v[0], -t));
-            kahan(o, oc, -__fmul_rn(qs, vc[0]));
-            o = __fsub_rn(o, oc);
-        } else {
-            o = __fmaf_rn(qs, v[0], o);
-        }
-        if (lane < 3 * min(FEW, ni - t0)) part[3 * (size_t)(s0 + t0) + lane] = o;
     }
+    float v[16] = {}, vc[16] = {}, w[16] = {}, wc[16] = {};
+#pragma unroll
+    for (int k = 0; k < 3 * FEW; k++) {
+        const int h = k / 6, a = k % 3;
+        const bool u = k / 3 & 1;
+        v[k] = u ? f[h][a].y : f[h][a].x; w[k] = u ? g[h][a].y : g[h][a].x;
+        if constexpr (COMP) { vc[k] = u ? e[h][a].y : e[h][a].x; wc[k] = u ? ge[h][a].y : ge[h][a].x; }
+    }
+    tree_add<COMP, 3 * FEW>(v, vc, w, wc, lane);
+    const int j = lane / 3;   // lane 3 j + a: component a of target j
+    const float qs = j == 0 ? q[0].x : j == 1 ? q[0].y : j == 2 ? q[1].x : q[1].y;
+    float o = __shfl_down_sync(0xffffffffu, v[0], 16);
+    if constexpr (COMP) {   // o += qs (v - vc)
+        float oc = __shfl_down_sync(0xffffffffu, vc[0], 16);
+        const float t = __fmul_rn(qs, v[0]);
+        kahan(o, oc, t);
+        kahan(o, oc, __fmaf_rn(qs, v[0], -t));
+        kahan(o, oc, -__fmul_rn(qs, vc[0]));
+        o = __fsub_rn(o, oc);
+    } else {
+        o = __fmaf_rn(qs, v[0], o);
+    }
+    if (lane < 3 * min(FEW, ni - t0)) part[3 * (size_t)(s0 + t0) + lane] = o;
 }
 
 // ---- FP64
@@ -1575,7 +1573,7 @@ __global__ void __launch_bounds__(NEAR_THREADS, near_ctas(MODE)) k_near(Dev d, i
         if constexpr (MODE != 0)
             if (p >= NEAR_PLANE) {
                 R *part = (R *)d.near_part + (size_t)near_plane_part(p - NEAR_PLANE, split) * 3 * nslot;
-                near_few32<PER, MODE == 2>(d, s_lj, s_q, part, c, p - NEAR_PLANE, d.cstart[c + 1] - d.cstart[c], lane);
+                near_few32<PER, MODE == 2>(d, s_lj, s_q, part, c, p - NEAR_PLANE, FEW * chunk, d.cstart[c + 1] - d.cstart[c], lane);
                 k = __shfl_sync(0xffffffffu, next, 0);
                 continue;
             }

@@ -879,7 +879,7 @@ int upload_impl(sesp_ctx *c, const std::vector<RepIn> &in) {
     d.nrep = R;
     d.near_split = near_split(N, c->p.precision);
     d.near_merge = c->p.precision == SESP_PLAIN_FP64 ? 0 : 64;
-    d.near_few = c->p.precision == SESP_PLAIN_FP64 ? 0 : c->p.precision == SESP_MIXED_COMP ? 36 : 48;
+    d.near_few = c->p.precision == SESP_PLAIN_FP64 ? 0 : 48;
     int e = 0;
     double **a12[12] = {&d.x, &d.y, &d.z, &d.vx, &d.vy, &d.vz, &d.ax, &d.ay, &d.az, &d.fx, &d.fy, &d.fz};
     for (auto q : a12) if ((e = dalloc(c, q, N))) return e;

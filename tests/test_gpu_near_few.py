@@ -39,7 +39,8 @@ def gas(preset, water, surf, cells, seed, kept=1.0):
     return dataclasses.replace(s, n_water=len(wat), cells=tuple(cells), pos=pos, vel=np.zeros_like(pos))
 
 
-# about 1/3, 1, 2, 3, 4 and 6 waters a cell; surfactants of 12 or 29 sites in
+# about 1/3, 1, 2, 3, 4 and 6 waters a cell (6 turns a plane and 24 sites a cell
+# are the limits); surfactants of 12 or 29 sites in
 # place of some.  Bar: the mixed paths'
 @pytest.mark.parametrize("preset", [0, 1])
 @pytest.mark.parametrize("water,surf", [(170, 0), (512, 0), (1024, 0), (1500, 0), (2048, 0), (3000, 0), (150, 12), (600, 20)])
