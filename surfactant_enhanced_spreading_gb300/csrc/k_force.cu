@@ -2025,11 +2025,15 @@ __device__ __forceinline__ void m2c_row2(const float *op, float va, float vb, fl
     }
 }
 
-// A tile of a class's occupied targets (fm_list).  Up to M2C_FEW targets (a
-// tile of the FP64 path never has more): a warp takes one target at a time,
-// lane o its output o, so a target and offset costs 25 multiply-adds of the
-// warp and not 625 however few of its lanes have a target.  More: two targets
-// per lane.  Both forms add the same products in the same order.  What bounds
+// A tile of a class's occupied targets (fm_list).  Up to M2C_FEW targets: a warp
+// takes one target at a time, lane o its output o, so a target and offset costs
+// 25 multiply-adds of the warp and not 625 however few of its lanes have a
+// target.  More: two targets per lane.  FP64 tiles have up to M2C_FEW targets,
+// but in a class of M2C_MANY or more every eighth takes the next 128, one per
+// lane (19.5 FP64 instructions a target and offset, not 25; force call with a
+// rebuild, one water a cell, 76,800 sites 11.9 -> 10.1 ms and 10.5 from 512 on,
+// 20,736 sites 3.13 -> 2.94 and 2.97; 62,400 sites of a droplet have fewer).  All
+// forms add the same products in the same order.  What bounds
 // it is staging the operators and loading the sources: four warps share a
 // staged operator (far-field build of 312,000 sites with 1, 2 and 4 warps:
 // 236, 155 and 150 us; 3,000 sites: 91, 69, 57), and up to 16 targets the
@@ -2041,8 +2045,10 @@ __global__ void __launch_bounds__(32 * M2C_W) k_m2l_cls(Dev d, int ncell) {
     R *sop = (R *)smraw;   // [M2C_CH][LP][M2C_LD]
     const int4 it = d.m2c_items[blockIdx.x];
     const int level = it.x >> 28, cls = it.y, t0 = it.z, q = it.x & 0x0FFFFFFF;
-    const int cnt = min(it.w, d.fm_cnt[16 * q + (level == 4 ? 0 : 8) + cls] - t0);
-    if (cnt <= 0) return;
+    const int all = d.fm_cnt[16 * q + (level == 4 ? 0 : 8) + cls];
+    const bool many = sizeof(R) == 8 && all >= M2C_MANY;
+    const int cnt = min(many ? 32 * M2C_W : it.w, all - t0);
+    if (cnt <= 0 || (many && t0 % (32 * M2C_W) != 0)) return;
     const Rep r = d.rep[q];
     const int *list = d.fm_list + class_list(r, level, cls, ncell) + t0;
     constexpr int G = M2C_GROUPS;
@@ -2086,7 +2092,7 @@ __global__ void __launch_bounds__(32 * M2C_W) k_m2l_cls(Dev d, int ncell) {
         const int x = t % h0, y = (t / h0) % h1, z = t / (h0 * h1);
         return base + (2 * x + px) + n0 * ((2 * y + py) + n1 * (2 * z + pz));
     };
-    if (cnt <= M2C_FEW) {
+    if (!many && cnt <= M2C_FEW) {
         constexpr int NT = M2C_FEW / M2C_W;
         R acc[NT];
         int at[NT];
@@ -2151,6 +2157,30 @@ __global__ void __launch_bounds__(32 * M2C_W) k_m2l_cls(Dev d, int ncell) {
         };
         if (ka < cnt) put(ta, pa);
         if (kb < cnt) put(tb, pb);
+    } else {
+        const int k = w * 32 + lane, t = list[min(k, cnt - 1)], at = pidx(t);
+        R acc[LP];
+#pragma unroll
+        for (int o = 0; o < LP; o++) acc[o] = R(0);
+        for (int c0 = k0; c0 < k1; c0 += M2C_CH) {
+            const int nch = stage(c0);
+            if (w * 32 >= cnt) continue;   // no target of this warp
+            for (int kk = 0; kk < nch; kk++) {
+                const R *src = src_of(c0 + kk) + at;
+                const R *op = sop + kk * LP * M2C_LD;
+#pragma unroll 5
+                for (int i = 0; i < LP; i++) {
+                    const R v = src[(size_t)i * vol];
+#pragma unroll
+                    for (int o = 0; o < LP; o++) acc[o] = fma(op[i * M2C_LD + o], v, acc[o]);
+                }
+            }
+        }
+        if (k < cnt) {
+            R *o = part + ((size_t)cell(t) * G + g) * LP;
+#pragma unroll
+            for (int i = 0; i < LP; i++) o[i] = acc[i];
+        }
     }
 }
 

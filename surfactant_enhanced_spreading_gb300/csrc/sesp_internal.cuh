@@ -77,6 +77,7 @@ constexpr int M2C_LD = 28;    // padded output stride of a real M2L operator row
 constexpr int M2C_W = 4;      // warps of an M2L CTA, 64 targets each (2 per lane)
 constexpr int NEAR_CLASSES = 64;   // cost classes of the pair field's items
 constexpr int M2C_FEW = 16;   // targets of a tile that are taken one per warp
+constexpr int M2C_MANY = 256;   // targets of a class that FP64 tiles take one per lane
 constexpr int M2C_TILE = 64 * M2C_W, M2C_TILE64 = M2C_FEW;   // targets of a tile, FP32 and FP64
 constexpr int M2C_GROUPS = 21; // offset groups of an M2L work item, 9 offsets each (partial sums added in group order)
 constexpr int GGRP = 8;       // carbon groups per graphite column
