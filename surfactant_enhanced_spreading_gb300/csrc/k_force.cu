@@ -483,13 +483,14 @@ __device__ inline void local_grad(const LF &L, R x, R y, R z, R &gx, R &gy, R &g
 // On the FP32 paths a cell of up to FEW_MAX sites with a thin shell is worked off
 // by near_few32: an item takes FEW targets and the partners of a plane of the
 // shell, 32 a turn, and its force goes to the plane's first part.  Thin: at most
-// FEW_TURNS turns an item (longer ones were the tail of a small launch: 3,000
-// sites, a step of 50.5 us, up to 58 at 16) and near_few (48) for the cell (beyond
-// it rows have their lanes full).  The rule sees the cell and its shell alone, so a
-// replica's sums do not depend on what it is batched with.  Mean step by rows
-// alone / so, us, FP32 and compensated: one water a cell (20,736 sites) 199 / 107,
-// 252 / 117; three (62,208) 246 / 181, 314 / 219; four (195,000) 576 / 477, 753 /
-// 599; with 4 turns an item 552 / 717 for the last.  Droplets keep their times.
+// FEW_TURNS turns an item (longer ones were the tail of a small launch: a run of
+// 20 force calls of 3,000 sites 1,346 us, 1,429 to 1,534 without this limit) and
+// near_few (48) for the cell (beyond it rows have their lanes full).  The rule
+// sees the cell and its shell alone, so a replica's sums do not depend on what it
+// is batched with.  Mean step by rows alone / so, us, FP32 and compensated: one
+// water a cell (20,736 sites) 199 / 107, 252 / 117; three (62,208) 246 / 181, 314 /
+// 219; four (195,000) 576 / 477, 753 / 599 (with 4 turns an item 552 and 717).
+// Droplets keep their times.
 // item.x = cell, item.y = part << 24 | chunk, part = plane * 3 + row,
 // 3 (plane * 3 + row) + cell with near_split, or NEAR_PLANE + plane (chunk: of
 // FEW targets; FEW_MAX keeps such a cell's items within the 18 of its two chunks).
